@@ -513,8 +513,10 @@ def log_estimate(wait=False):
 
 def log_eligible(tree, opt):
     """Whether the logged forward / replay backward pair applies to this call."""
-    return (opt.format != FORMAT_RGBA and opt.basis_dim in (1, 4, 9, 16, 25)
-            and tree.data.shape[1] == 2 and tree.data.shape[4] == 3 * opt.basis_dim + 1
+    K = tree.data.shape[4]
+    layout = K == 4 if opt.format == FORMAT_RGBA else \
+        opt.basis_dim in (1, 4, 9, 16, 25) and K == 3 * opt.basis_dim + 1
+    return (layout and tree.data.shape[1] == 2
             and opt.sigma_thresh == 0.0 and opt.stop_thresh == 0.0
             and tree.data.dtype == torch.float32)
 

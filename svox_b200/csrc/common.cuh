@@ -55,7 +55,6 @@ struct LeafHit {
 struct TopTable {
     const int32_t* cells;  // shared or global memory
     int level;             // L (0 = no table)
-    const int32_t* bricks = nullptr;  // queue kernels only: see render_queue.cuh
 };
 
 // Descent of query_single_from_root (svox/csrc/include/common.cuh:52-90) for
@@ -148,13 +147,6 @@ struct TopScratch {
     int build(const svoxb_tree* t, int max_level, cudaStream_t s);
     ~TopScratch() { if (cells) cudaFreeAsync(cells, stream); }
 };
-
-// Queue kernels: lanes that must be idle before rays are loaded.  Measured on the training
-// step's logged forward: 1 to 3 are level, 4 costs 1 %, 8 3 %, 16 11 %.
-constexpr int kRefillBatch = 2;
-// Replay scatter: 1 = packets evict-first, 2 = gradient evict-last.  Measured (backward of the
-// training step): 3 -> 2.83 ms, 2 -> 2.78, 0 -> 2.79, 1 -> 2.89.
-constexpr int kReplayHints = 2;
 
 // The two switches the tests flip to show that an index or a bin size changes no result
 // (svoxb_test_knob).

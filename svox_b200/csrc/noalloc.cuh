@@ -1,8 +1,7 @@
 // svoxb_volume_render_noalloc: the forward ray render for callers that must
 // not allocate device memory.
 //
-// The regular entry points take their per-call scratch (the annotated copy of
-// the child array and the jump table over the top of the tree) from the CUDA
+// The regular entry points take their per-call scratch (the index of the tree) from the CUDA
 // memory pool.  Some hosts cannot do that: a renderer embedded in an
 // application that owns the whole device heap, a plug-in that runs inside
 // someone else's allocator-free real-time loop, or a process whose memory
@@ -16,12 +15,11 @@
 
 namespace svoxb {
 
-constexpr int64_t kNoAllocMaxNodes = 1 << 19;  // 524288 nodes -> 16 MiB of annotated entries
-constexpr int kNoAllocTopLevel = 6;            // leaf table: 64^3 entries (1 MiB)
-constexpr int64_t kNoAllocTopCells = 1 << (3 * kNoAllocTopLevel);
+constexpr int64_t kNoAllocMaxNodes = 1 << 19;  // 524288 nodes
+constexpr int64_t kNoAllocWords = kNoAllocMaxNodes * 8 + (1 << 18);  // 17 MiB
 
-// [0, 8 * kNoAllocMaxNodes): annotated child entries; then the leaf table.
-static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocMaxNodes * 8 + kNoAllocTopCells];
+// Holds the index of the call in progress (render_index.cuh), with as many bricks as fit.
+static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocWords];
 
 // Device address of the array, per device.  In host code the symbol's name is
 // only a stand-in: the address a kernel can use has to be asked for, once per
@@ -40,29 +38,23 @@ static int noalloc_scratch_address(int32_t** out) {
     return SVOXB_OK;
 }
 
-template <int BD>
 static int launch_noalloc(const RenderCall& c, const RayBatch& src, int32_t* scratch) {
     const svoxb_tree* t = c.tree;
-    int32_t* annotated = scratch;
-    int32_t* table = scratch + kNoAllocMaxNodes * 8;
-    const int64_t n = t->M * 8;
-    // Both scratch regions are fully overwritten before they are read, so nothing
-    // left over from an earlier call matters.
-    annotate_sigma_kernel<<<index_grid(n, 256, sm_count()), 256, 0, c.stream>>>(
-        t->child, t->data, t->K, n, c.opt.sigma_thresh, c.opt.density_softplus, annotated,
-        LogGate{});
-    SVOXB_CUDA(cudaGetLastError());
-    const int level = auto_top_level(t->M, kNoAllocTopLevel);
-    if (level > 0) {
-        const int cells = 1 << (3 * level);
-        build_leaf_table_kernel<<<index_grid(cells, 256, sm_count()), 256, 0, c.stream>>>(annotated, t->M, level,
-                                                                          table, LogGate{});
-        SVOXB_CUDA(cudaGetLastError());
-    }
-    const TopTable top{table, level};
-    TreeArgs tr = tree_args(t);
-    tr.child = annotated;
-    return launch_queue_fitted<BD>(c, src, tr, top);
+    IndexLayout layout = IndexLayout::of(t->M, 0);
+    const int64_t left = kNoAllocWords - (int64_t)layout.words - 64;
+    int64_t bricks = left / (kBrickWords + 1);
+    if (bricks > kMaxBricks) bricks = kMaxBricks;
+    layout = IndexLayout::of(t->M, (int)(bricks > 0 ? bricks : 0));
+    if ((int64_t)layout.words > kNoAllocWords) return SVOXB_ERR_TOO_LARGE;
+    // Every part of the scratch is overwritten before it is read, so nothing left over from an
+    // earlier call matters.
+    int st = build_index(t, layout, c.opt.sigma_thresh, c.opt.density_softplus, scratch,
+                         LogGate{}, c.stream);
+    if (st) return st;
+    const TreeIndex index = layout.view(scratch);
+    return with_basis(c.opt, [&](auto basis) {
+        return launch_mode<decltype(basis)::value>(c, src, index);
+    });
 }
 
 }  // namespace svoxb
@@ -90,12 +82,5 @@ extern "C" int svoxb_volume_render_noalloc(const svoxb_tree* tree, const svoxb_r
     c.out = out;
     c.stream = (cudaStream_t)stream;
     const RayBatch src{rays->origins, rays->dirs, rays->vdirs};
-    switch (opt->basis_dim) {
-        case 1: return launch_noalloc<1>(c, src, scratch);
-        case 4: return launch_noalloc<4>(c, src, scratch);
-        case 9: return launch_noalloc<9>(c, src, scratch);
-        case 16: return launch_noalloc<16>(c, src, scratch);
-        case 25: return launch_noalloc<25>(c, src, scratch);
-    }
-    return SVOXB_ERR_FORMAT;
+    return launch_noalloc(c, src, scratch);
 }

@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "query.cuh"
+#include "render_index.cuh"
 
 namespace svoxb {
 
@@ -147,9 +148,6 @@ __device__ __forceinline__ void colour_basis_any(const TreeArgs& tr,
     }
 }
 
-__device__ __forceinline__ float sigmoid_ref(float x) { return 1 / (1 + expf(-x)); }
-__device__ __forceinline__ float softplus_m1(float x) { return logf(1 + expf(x - 1)); }
-
 // _dda_unit (svox/csrc/rt_kernel.cu:203-220): slab test against the unit cube.
 template <int FUSED>
 __device__ __forceinline__ void dda_unit(float cx, float cy, float cz, float ix, float iy,
@@ -204,6 +202,10 @@ struct RayBatch {  // render_ray_kernel's inputs (svox/csrc/rt_kernel.cu:717-733
     const float* __restrict__ dirs;
     const float* __restrict__ vdirs;
 
+    // The order in which the queue kernels take the rays: ticket -> ray, for `tickets` tickets.
+    static int64_t tickets(const RayBatch&, int64_t n_rays) { return n_rays; }
+    __device__ __forceinline__ int64_t pick(int64_t ticket) const { return ticket; }
+
     __device__ __forceinline__ void load(int64_t i, const TreeArgs& tr,
                                          const svoxb_render_options&, Ray& r) const {
         r.ox = to_tree(__ldg(origins + 3 * i + 0), __ldg(tr.offset + 0), __ldg(tr.scaling + 0));
@@ -230,6 +232,19 @@ struct PixelRays {  // render_image_kernel's inputs (svox/csrc/rt_kernel.cu:758-
     const float* __restrict__ c2w;  // row-major, row stride 4
     float fx, fy;
     int width, height;
+
+    // Pixels are taken in tiles of 8 x 4, a warp's worth: neighbours share leaves and index
+    // words.  Tickets of a tile that hang over the image's edge yield no ray (-1).
+    static int64_t tickets(const PixelRays& p, int64_t) {
+        return 32 * (int64_t)((p.width + 7) / 8) * ((p.height + 3) / 4);
+    }
+    __device__ __forceinline__ int64_t pick(int64_t ticket) const {
+        const int64_t tile = ticket >> 5;
+        const int across = (width + 7) / 8, k = (int)ticket & 31;
+        const int ty = (int)(tile / across), tx = (int)(tile - (int64_t)ty * across);
+        const int x = tx * 8 + (k & 7), y = ty * 4 + (k >> 3);
+        return x < width && y < height ? (int64_t)y * width + x : -1;
+    }
 
     __device__ __forceinline__ void load(int64_t tid, const TreeArgs& tr,
                                          const svoxb_render_options& opt, Ray& r) const {

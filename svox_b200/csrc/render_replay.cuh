@@ -214,39 +214,30 @@ replay_bin_kernel(svoxb_render_options opt, const int32_t* __restrict__ log, int
     }
 }
 
-__device__ __forceinline__ int4 ld_stream16(const int4* a, uint64_t pol) {
-    int4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.s32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(a), "l"(pol));
-    return v;
-}
-
 template <int K>
 struct alignas(16) ScatterSmem {
     using Shape = RecordShape<K>;
-    uint32_t slot[32];
-    alignas(16) float rows[32 * Shape::STRIDE + 4];
+    alignas(16) float rows[32 * Shape::STRIDE];
 };
 
 template <int BD, int BLOCK, bool HESS, bool LOBES>
 __global__ void __launch_bounds__(BLOCK)
 replay_scatter_kernel(int64_t n_slots, svoxb_render_options opt, TreeArgs lobes,
                       float* __restrict__ grad_data, const int32_t* __restrict__ log,
-                      ReplayBins b, int flags, int part, int n_parts) {
-    constexpr int K = 3 * BD + 1;
+                      ReplayBins b, int part, int n_parts) {
+    constexpr int K = RecordLength<BD>::K;
     using Shape = RecordShape<K>;
     using SM = ScatterSmem<K>;
     extern __shared__ __align__(16) unsigned char s_raw[];
     const int lane = threadIdx.x & 31;
     SM& sm = *reinterpret_cast<SM*>(s_raw + (size_t)(threadIdx.x >> 5) * sizeof(SM));
-    const int sub = lane / Shape::GROUP, wj = lane % Shape::GROUP;
+    const bool vec_ok = (reinterpret_cast<uintptr_t>(grad_data) & 15) == 0;
     // packets of this part: those of its bin range
     int n_bins = log[3];
     if (n_bins > kMaxBins) n_bins = kMaxBins;
     const int64_t total = b.offset[replay_part_first_bin(part + 1, n_parts, n_bins)];
     const int shift = log[2];
-    const uint64_t pol_keep = l2_policy_keep(), pol_stream = l2_policy_stream();
+    const uint64_t pol_keep = l2_policy_keep();
     // Blocks take units of kScatterUnit packets in bin order from one counter, so the
     // whole grid works within a window much smaller than a bin.
     __shared__ int64_t s_unit;
@@ -267,13 +258,8 @@ replay_scatter_kernel(int64_t n_slots, svoxb_render_options opt, TreeArgs lobes,
         uint32_t slot = 0xffffffffu;
         int4 pa = make_int4(-1, 0, 0, 0), pb = make_int4(0, 0, 0, 0);
         if (lane < n) {
-            if (flags & 1) {
-                pa = ld_stream16(b.packet + 2 * (first + lane), pol_stream);
-                pb = ld_stream16(b.packet + 2 * (first + lane) + 1, pol_stream);
-            } else {
-                pa = __ldg(b.packet + 2 * (first + lane));
-                pb = __ldg(b.packet + 2 * (first + lane) + 1);
-            }
+            pa = __ldg(b.packet + 2 * (first + lane));
+            pb = __ldg(b.packet + 2 * (first + lane) + 1);
             slot = (uint32_t)pa.x;
         }
         // a position the bin pass left unwritten holds stale bytes: a packet counts only
@@ -287,61 +273,60 @@ replay_scatter_kernel(int64_t n_slots, svoxb_render_options opt, TreeArgs lobes,
             }
             if (!ok) slot = 0xffffffffu;
         }
-        sm.slot[lane] = slot;
+        // lane i expands packet i to its gradient record, placed in the row as in memory (offset
+        // within the first 16-byte word), zeros around it
+        const int off = record_offset<K>(grad_data, slot);
         if (slot != 0xffffffffu) {
             const float f[3] = {__int_as_float(pa.y), __int_as_float(pa.z), __int_as_float(pa.w)};
-            const float vdir[3] = {__int_as_float(pb.y), __int_as_float(pb.z), __int_as_float(pb.w)};
-            float basis[BD];
-            colour_basis<BD, LOBES>(lobes, opt, vdir, basis);
-#pragma unroll
-            for (int k = 0; k < BD; ++k)
-                if (k < opt.min_comp || k > opt.max_comp) basis[k] = 0.f;
             float v[K];
+            if constexpr (BD == 0) {
 #pragma unroll
-            for (int chn = 0; chn < 3; ++chn)
+                for (int chn = 0; chn < 3; ++chn) v[chn] = HESS ? f[chn] * f[chn] : f[chn];
+            } else {
+                const float vdir[3] = {__int_as_float(pb.y), __int_as_float(pb.z),
+                                       __int_as_float(pb.w)};
+                float basis[BD];
+                colour_basis<BD, LOBES>(lobes, opt, vdir, basis);
 #pragma unroll
-                for (int k = 0; k < BD; ++k) {
-                    const float gw = basis[k] * f[chn];
-                    v[chn * BD + k] = HESS ? gw * gw : gw;
-                }
+                for (int k = 0; k < BD; ++k)
+                    if (k < opt.min_comp || k > opt.max_comp) basis[k] = 0.f;
+#pragma unroll
+                for (int chn = 0; chn < 3; ++chn)
+#pragma unroll
+                    for (int k = 0; k < BD; ++k) {
+                        const float gw = basis[k] * f[chn];
+                        v[chn * BD + k] = HESS ? gw * gw : gw;
+                    }
+            }
             v[K - 1] = __int_as_float(pb.x);
             float* row = sm.rows + lane * Shape::STRIDE;
-            if (Shape::VEC) {
+            if (Shape::ALIGNED) {
 #pragma unroll
                 for (int w = 0; w < K / 4; ++w)
                     reinterpret_cast<float4*>(row)[w] =
                         make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
             } else {
 #pragma unroll
-                for (int w = 0; w < K; ++w) row[w] = v[w];
+                for (int i = 0; i < 3; ++i) {
+                    if (i < off) row[i] = 0.f;
+                    if (off + K + i < 4 * Shape::WORDS) row[off + K + i] = 0.f;
+                }
+#pragma unroll
+                for (int w = 0; w < K; ++w) row[off + w] = v[w];
             }
         }
         __syncwarp();
+        // groups of lanes add consecutive 16-byte words of a record
+        const int sub = lane / Shape::GROUP, w = lane % Shape::GROUP;
 #pragma unroll
-        for (int p = 0; p < 32 / Shape::IPP; ++p) {
-            const int k = p * Shape::IPP + sub;
-            if (k < n) {
-                const uint32_t sl = sm.slot[k];
-                if ((int64_t)sl < n_slots) {
-                    float* __restrict__ gp = grad_data + (size_t)sl * K;
-                    const float* row = sm.rows + k * Shape::STRIDE;
-#pragma unroll
-                    for (int w = 0; w < Shape::WPL; ++w) {
-                        const int word = wj + w * Shape::GROUP;
-                        if (word < Shape::WORDS) {
-                            if (Shape::VEC) {
-                                const float4 x = reinterpret_cast<const float4*>(row)[word];
-                                if (flags & 2)
-                                    red_add_v4_hint(gp + 4 * word, x.x, x.y, x.z, x.w, pol_keep);
-                                else
-                                    red_add_v4(gp + 4 * word, x.x, x.y, x.z, x.w);
-                            } else {
-                                atomicAdd(gp + word, row[word]);
-                            }
-                        }
-                    }
-                }
-            }
+        for (int p = 0; p < Shape::GROUP; ++p) {
+            const int k = p * Shape::RPP + sub;
+            const uint32_t sl = __shfl_sync(0xffffffffu, slot, k);
+            const int o = __shfl_sync(0xffffffffu, off, k);
+            if (k < n && w < Shape::WORDS && sl != 0xffffffffu)
+                flush_word<K>(grad_data + (size_t)sl * K, o, w,
+                              reinterpret_cast<const float4*>(sm.rows + k * Shape::STRIDE)[w],
+                              vec_ok, pol_keep);
         }
         __syncwarp();
     }

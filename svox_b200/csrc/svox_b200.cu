@@ -12,6 +12,12 @@
 
 namespace svoxb {
 
+// Queue kernels: idle lanes of a warp before it drains its queue and refills (4 and 12 measure
+// within 1 % of 8 on ray batches and images).
+constexpr int kRefillLanes = 8;
+// ... and warps per SM that a small batch is spread over before warps get 32 rays each.
+constexpr int kSpreadWarps = 16;
+
 struct RenderCall {
     const svoxb_tree* tree;
     svoxb_render_options opt;
@@ -28,7 +34,7 @@ struct RenderCall {
     int32_t* log = nullptr;
     int64_t log_capacity = 0;
     // forward with a scratch built earlier by svoxb_render_scratch_build (else per call)
-    int32_t* prepared = nullptr;
+    const int32_t* prepared = nullptr;
     // marching backward as the fallback of a replay: does its work only if this log overflowed
     LogGate gate{};
 };
@@ -38,12 +44,28 @@ static int out_dim_of(const svoxb_tree* t, const svoxb_render_options& o) {
     return o.format != SVOXB_FORMAT_RGBA ? (t->K - 1) / o.basis_dim : t->K - 1;
 }
 
-// The records hold three colour channels of basis_dim coefficients each and a density, and
-// basis_dim is one of the sizes the specialised kernels are compiled for.
-static bool basis3(const svoxb_tree* t, const svoxb_render_options& o) {
+// Whether the queue kernels are compiled for the records: three colour channels of basis_dim
+// coefficients each and a density, or plain RGBA.
+static bool queue_layout(const svoxb_tree* t, const svoxb_render_options& o) {
     const int b = o.basis_dim;
-    return o.format != SVOXB_FORMAT_RGBA && t->K == 3 * b + 1 &&
-           (b == 1 || b == 4 || b == 9 || b == 16 || b == 25);
+    if (o.format == SVOXB_FORMAT_RGBA) return t->K == 4;
+    return t->K == 3 * b + 1 && (b == 1 || b == 4 || b == 9 || b == 16 || b == 25);
+}
+
+// Calls f with the kernels' basis size (0: RGBA) as a compile-time constant.
+template <int N>
+struct Basis { static constexpr int value = N; };
+template <class F>
+static int with_basis(const svoxb_render_options& o, F f) {
+    if (o.format == SVOXB_FORMAT_RGBA) return f(Basis<0>{});
+    switch (o.basis_dim) {
+        case 1: return f(Basis<1>{});
+        case 4: return f(Basis<4>{});
+        case 9: return f(Basis<9>{});
+        case 16: return f(Basis<16>{});
+        case 25: return f(Basis<25>{});
+    }
+    return SVOXB_ERR_FORMAT;
 }
 
 static int validate_options(const svoxb_tree* t, const svoxb_render_options& o) {
@@ -116,10 +138,6 @@ static int launch_sh(const RenderCall& c, const Source& src, const TopTable& top
     return SVOXB_OK;
 }
 
-// Queue kernels (render_queue.cuh).  The block size is the largest whose
-// per-warp queues fit in shared memory next to the jump table.
-constexpr size_t kMaxSmem = 227 * 1024;
-
 // Replay bins: a bin is a range of 2^shift leaf slots whose gradient spans
 // about g_tuning.replay_bin_mb MB, at most kMaxBins of them.
 static int replay_bin_shift(int64_t M, int K) {
@@ -130,65 +148,48 @@ static int replay_bin_shift(int64_t M, int K) {
     return shift;
 }
 
-template <int BD, int BLOCK, class Source>
-static int launch_queue_block(const RenderCall& c, const Source& src, const TreeArgs& tr,
-                              const TopTable& top, size_t top_bytes) {
-    constexpr int K = 3 * BD + 1;
-    const int64_t n_gran = (c.Q + 31) / 32;
+// How the queue kernels deal out `tickets` rays.  With fewer rays than fill the device's warps
+// a warp takes fewer of them, so that every SM sub-partition has work: a march is a serial
+// chain, and what cannot be hidden by other warps should at least run side by side.
+static MarchShape march_shape(int64_t tickets, int sms) {
+    const int64_t warps = (int64_t)sms * kSpreadWarps;
+    MarchShape m{32, 5, kRefillLanes};
+    while (m.lanes > 4 && tickets <= warps * (m.lanes / 2)) m.lanes /= 2;
+    if (m.lanes == 4) m.granule_shift = 4;
+    if (m.lanes < 32) m.refill = m.lanes / 4;
+    return m;
+}
+
+template <int BD, int MODE, class Source>
+static int launch_march(const RenderCall& c, const Source& src, const TreeIndex& index) {
+    const size_t smem = (kMarchBlock / 32) * sizeof(WarpQueue<BD, MODE>);
+    const int64_t tickets = Source::tickets(src, c.Q);
+    const MarchShape shape = march_shape(tickets, sm_count());
+    auto k = render_queue_kernel<BD, MODE, Source>;
     unsigned grid = 1;
-    int st;
-    if (!c.backward && c.log != nullptr) {
-        const size_t smem = top_bytes + (size_t)(BLOCK / 32) * sizeof(WarpQueue<K, kModeForwardLogged>);
-        auto k = render_queue_kernel<BD, BLOCK, kModeForwardLogged, Source>;
-        if ((st = persistent_grid(k, BLOCK, smem, n_gran, &grid))) return st;
-        k<<<grid, BLOCK, smem, c.stream>>>(tr, src, c.opt, top, (int)top_bytes, c.Q, c.out,
-                                          nullptr, nullptr, nullptr, c.log, c.log_capacity,
-                                          replay_bin_shift(c.tree->M, K), kRefillBatch);
-    } else if (!c.backward) {
-        const size_t smem = top_bytes + (size_t)(BLOCK / 32) * sizeof(WarpQueue<K, kModeForward>);
-        auto k = render_queue_kernel<BD, BLOCK, kModeForward, Source>;
-        if ((st = persistent_grid(k, BLOCK, smem, n_gran, &grid))) return st;
-        k<<<grid, BLOCK, smem, c.stream>>>(tr, src, c.opt, top, (int)top_bytes, c.Q, c.out,
-                                          nullptr, nullptr, nullptr, nullptr, 0, 0, kRefillBatch);
-    } else {
-        const size_t smem = top_bytes + (size_t)(BLOCK / 32) * sizeof(WarpQueue<K, kModeBackward>);
-        const bool single = c.fwd_out != nullptr && c.opt.sigma_thresh == 0.f &&
-                            c.opt.stop_thresh == 0.f;
-        auto k = render_queue_kernel<BD, BLOCK, kModeBackward, Source>;
-        if ((st = persistent_grid(k, BLOCK, smem, n_gran, &grid))) return st;
-        k<<<grid, BLOCK, smem, c.stream>>>(tr, src, c.opt, top, (int)top_bytes, c.Q, nullptr,
-                                          c.grad_out, single ? c.fwd_out : nullptr, c.grad_data,
-                                          const_cast<int32_t*>(c.gate.log), c.gate.capacity, 0,
-                                          kRefillBatch);
-    }
+    const int64_t granules = (tickets + (1 << shape.granule_shift) - 1) >> shape.granule_shift;
+    // one granule per block at least (persistent_grid counts granules of 32 threads)
+    int st = persistent_grid(k, kMarchBlock, smem, granules * (kMarchBlock / 32), &grid);
+    if (st) return st;
+    const bool single = MODE == kModeBackward && c.fwd_out != nullptr && c.opt.sigma_thresh == 0.f &&
+                        c.opt.stop_thresh == 0.f;
+    int32_t* log = MODE == kModeForwardLogged ? c.log
+                   : MODE == kModeBackward    ? const_cast<int32_t*>(c.gate.log)
+                                              : nullptr;
+    const int64_t capacity = MODE == kModeForwardLogged ? c.log_capacity : c.gate.capacity;
+    k<<<grid, kMarchBlock, smem, c.stream>>>(
+        tree_args(c.tree), src, c.opt, index, tickets, c.out, c.grad_out,
+        single ? c.fwd_out : nullptr, c.grad_data, log, capacity,
+        replay_bin_shift(c.tree->M, c.tree->K), shape);
     SVOXB_CUDA(cudaGetLastError());
     return SVOXB_OK;
 }
 
-// Picks the block size: 640 threads where the record allows it (the kernel needs ~90
-// registers; at 768 threads it spilled inside the loop), fewer while the per-warp queues
-// do not fit in shared memory.
 template <int BD, class Source>
-static int launch_queue_fitted(const RenderCall& c, const Source& src, const TreeArgs& tr,
-                               const TopTable& top) {
-    constexpr int K = 3 * BD + 1;
-    const size_t top_bytes = 0;  // the leaf table stays in global memory
-    const size_t per_warp = c.backward ? sizeof(WarpQueue<K, kModeBackward>)
-                            : c.log    ? sizeof(WarpQueue<K, kModeForwardLogged>)
-                                       : sizeof(WarpQueue<K, kModeForward>);
-    // the lobe bases are compiled for the smallest block only
-    if constexpr (Source::kLobes) return launch_queue_block<BD, 256>(c, src, tr, top, top_bytes);
-    int want = 640;
-    // static shared memory: the ticket counter, and the bin histogram of the logged forward
-    const size_t fixed = 64 + (c.log ? (size_t)kMaxBins * sizeof(int) : 0);
-    while (want > 256 && top_bytes + (size_t)(want / 32) * per_warp + fixed > kMaxSmem) want -= 128;
-    if constexpr (BD <= 9) {
-        if (want >= 640) return launch_queue_block<BD, 640>(c, src, tr, top, top_bytes);
-    }
-    if constexpr (BD <= 16) {
-        if (want >= 512) return launch_queue_block<BD, 512>(c, src, tr, top, top_bytes);
-    }
-    return launch_queue_block<BD, 256>(c, src, tr, top, top_bytes);
+static int launch_mode(const RenderCall& c, const Source& src, const TreeIndex& index) {
+    if (c.backward) return launch_march<BD, kModeBackward>(c, src, index);
+    if (c.log != nullptr) return launch_march<BD, kModeForwardLogged>(c, src, index);
+    return launch_march<BD, kModeForward>(c, src, index);
 }
 
 // Replay backward (render_replay.cuh): prefix, pack, bin, then the scatter in one
@@ -200,7 +201,7 @@ struct ReplayJob {
     svoxb_render_options opt{};
     TreeArgs lobes{};            // for the lobe parameters of an SG / ASG basis
     int64_t n_slots = 0, n_rays = 0, chunks = 0;
-    int K = 0, basis_dim = 0, n_parts = 1, shift = 0, n_bins = 1;
+    int K = 0, n_parts = 1, shift = 0, n_bins = 1;
     bool hess = false;   // Gauss-Newton diagonal instead of the gradient
 };
 
@@ -244,7 +245,6 @@ static int replay_begin(const RenderCall& c, const Source& src, int64_t chunks, 
     job->n_rays = c.Q;
     job->chunks = chunks;
     job->K = c.tree->K;
-    job->basis_dim = c.opt.basis_dim;
     job->n_parts = n_parts;
     job->hess = hess;
     job->shift = replay_bin_shift(c.tree->M, c.tree->K);
@@ -280,7 +280,7 @@ static int replay_begin(const RenderCall& c, const Source& src, int64_t chunks, 
 template <int BD, int BLOCK, bool HESS, bool LOBES = false>
 static int replay_scatter_block(const ReplayJob& job, int part, float* grad, int reserve_sms,
                                 cudaStream_t stream) {
-    constexpr int K = 3 * BD + 1;
+    constexpr int K = RecordLength<BD>::K;
     const size_t smem = (size_t)(BLOCK / 32) * sizeof(ScatterSmem<K>);
     auto k = replay_scatter_kernel<BD, BLOCK, HESS, LOBES>;
     unsigned grid = 1;
@@ -293,7 +293,7 @@ static int replay_scatter_block(const ReplayJob& job, int part, float* grad, int
         if ((int64_t)grid > most) grid = (unsigned)(most > 1 ? most : 1);
     }
     k<<<grid, BLOCK, smem, stream>>>(job.n_slots, job.opt, job.lobes, grad, job.log, job.bins,
-                                    kReplayHints, part, job.n_parts);
+                                    part, job.n_parts);
     const cudaError_t e = cudaGetLastError();
     return e != cudaSuccess ? set_cuda_error(e) : SVOXB_OK;
 }
@@ -301,10 +301,13 @@ static int replay_scatter_block(const ReplayJob& job, int part, float* grad, int
 template <int BD>
 static int replay_scatter_bd(const ReplayJob& job, int part, float* grad, int reserve_sms,
                              cudaStream_t stream) {
-    if (job.opt.format != SVOXB_FORMAT_SH)
-        return job.hess ? replay_scatter_block<BD, 512, true, true>(job, part, grad, 0, stream)
-                        : replay_scatter_block<BD, 512, false, true>(job, part, grad, reserve_sms,
-                                                                     stream);
+    if constexpr (BD > 0) {
+        if (job.opt.format != SVOXB_FORMAT_SH)
+            return job.hess
+                       ? replay_scatter_block<BD, 512, true, true>(job, part, grad, 0, stream)
+                       : replay_scatter_block<BD, 512, false, true>(job, part, grad, reserve_sms,
+                                                                    stream);
+    }
     if (job.hess) return replay_scatter_block<BD, 512, true>(job, part, grad, 0, stream);
     if constexpr (BD <= 9) {
         if (reserve_sms > 0)
@@ -319,14 +322,9 @@ static int replay_scatter(const ReplayJob& job, int part, float* grad, int reser
                           cudaStream_t stream) {
     if (part < 0 || part >= job.n_parts) return SVOXB_ERR_OPTION;
     if (job.chunks < 1) return SVOXB_OK;
-    switch (job.basis_dim) {
-        case 1: return replay_scatter_bd<1>(job, part, grad, reserve_sms, stream);
-        case 4: return replay_scatter_bd<4>(job, part, grad, reserve_sms, stream);
-        case 9: return replay_scatter_bd<9>(job, part, grad, reserve_sms, stream);
-        case 16: return replay_scatter_bd<16>(job, part, grad, reserve_sms, stream);
-        case 25: return replay_scatter_bd<25>(job, part, grad, reserve_sms, stream);
-    }
-    return SVOXB_ERR_FORMAT;
+    return with_basis(job.opt, [&](auto basis) {
+        return replay_scatter_bd<decltype(basis)::value>(job, part, grad, reserve_sms, stream);
+    });
 }
 
 static void replay_end(ReplayJob* job, cudaStream_t stream) {
@@ -334,105 +332,45 @@ static void replay_end(ReplayJob* job, cudaStream_t stream) {
     job->base = nullptr;
 }
 
-// Per-call scratch of the queue kernels: the annotated child array followed by
-// the leaf table (render_queue.cuh); one pool allocation, freed on the stream.
+// The index of one call (render_index.cuh): a pool allocation, freed on the stream.
 struct QueueScratch {
-    int32_t* annotated = nullptr;
-    int32_t* table = nullptr;
-    int32_t* bricks = nullptr;
-    int level = 0;
-    bool owned = false;
+    int32_t* mem = nullptr;
     cudaStream_t stream = nullptr;
 
-    // annotated | table | brick counter (8 words) | brick roots | bricks
-    struct Layout {
-        int64_t n, cells, cap;
-        int level;
-        size_t head, words;
-    };
-    static Layout layout(const svoxb_tree* t, int max_level) {
-        Layout l{};
-        l.n = t->M * 8;
-        l.level = auto_top_level(t->M, max_level);
-        l.cells = l.level > 0 ? ((int64_t)1 << (3 * l.level)) : 0;
-        // bricks: one per table cell that holds a node, while the budget lasts
-        l.cap = 0;
-        if (l.level > 0 && g_tuning.render_bricks && t->M < kBrickMaxNodes &&
-            l.level + kBrickLevels < kCoordBits) {
-            l.cap = l.cells < t->M ? l.cells : t->M;
-            if (l.cap > kMaxBricks) l.cap = kMaxBricks;
-        }
-        l.head = (size_t)(l.n + l.cells) + 8 + (size_t)((l.cap + 7) & ~(int64_t)7);
-        l.words = l.head + (size_t)l.cap * kBrickWords;
-        return l;
+    static IndexLayout layout(const svoxb_tree* t) {
+        return IndexLayout::of(t->M, g_tuning.render_bricks ? kMaxBricks : 0);
     }
-    // Level of the leaf table: 6 (64^3 cells, 1 MB); 7 (128^3, 8 MB) for trees of several
-    // million nodes, whose leaves lie up to ten levels deep: the bricks below the table then
-    // still reach them in one step.
-    static int default_level(const svoxb_tree* t) {
-        return t->M >= (4LL << 20) ? 7 : 6;
-    }
-    void adopt(const Layout& l, int32_t* mem) {
-        annotated = mem;
-        table = mem + l.n;
-        bricks = l.cap > 0 ? mem + l.head : nullptr;
-        level = l.level;
-    }
-
-    // Fills `external` (layout(t, max_level).words int32) or a pool allocation of its own.
-    int build(const svoxb_tree* t, float thresh, int softplus, int max_level, cudaStream_t s,
-              int32_t* external = nullptr, LogGate gate = LogGate{}) {
+    int build(const svoxb_tree* t, const IndexLayout& l, float thresh, int softplus,
+              LogGate gate, cudaStream_t s) {
         stream = s;
-        const Layout l = layout(t, max_level);
-        int32_t* mem = external;
-        if (!mem) {
-            int st = keep_pool_cached();
-            if (st) return st;
-            SVOXB_CUDA(cudaMallocAsync((void**)&mem, l.words * sizeof(int32_t), s));
-            owned = true;
-        }
-        adopt(l, mem);
-        const int sms = sm_count();
-        annotate_sigma_kernel<<<index_grid(l.n, 256, sms), 256, 0, s>>>(
-            t->child, t->data, t->K, l.n, thresh, softplus, annotated, gate);
-        SVOXB_CUDA(cudaGetLastError());
-        if (level > 0) {
-            build_leaf_table_kernel<<<index_grid(l.cells, 256, sms), 256, 0, s>>>(
-                annotated, t->M, level, table, gate);
-            SVOXB_CUDA(cudaGetLastError());
-        }
-        if (l.cap > 0) {
-            int32_t* counter = table + l.cells;
-            int32_t* roots = counter + 8;
-            SVOXB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int32_t), s));
-            assign_bricks_kernel<<<index_grid(l.cells, 256, sms), 256, 0, s>>>(
-                table, (int)l.cells, (int)l.cap, counter, roots, gate);
-            fill_bricks_kernel<<<index_grid(l.cap * kBrickCells, kBrickCells, sms), kBrickCells, 0, s>>>(
-                annotated, t->M, level, (int)l.cap, counter, roots, bricks, gate);
-            SVOXB_CUDA(cudaGetLastError());
-        }
-        return SVOXB_OK;
+        int st = keep_pool_cached();
+        if (st) return st;
+        SVOXB_CUDA(cudaMallocAsync((void**)&mem, l.words * sizeof(int32_t), s));
+        return build_index(t, l, thresh, softplus, mem, gate, s);
     }
-    ~QueueScratch() { if (owned && annotated) cudaFreeAsync(annotated, stream); }
+    ~QueueScratch() { if (mem) cudaFreeAsync(mem, stream); }
 };
 
-template <int BD, class Source>
+template <class Source>
 static int launch_queue(const RenderCall& c, const Source& src) {
+    const IndexLayout layout = QueueScratch::layout(c.tree);
     QueueScratch scratch;
-    if (c.prepared != nullptr && !c.backward) {
-        scratch.adopt(QueueScratch::layout(c.tree, QueueScratch::default_level(c.tree)), c.prepared);
-    } else {
-        const int st = scratch.build(c.tree, c.backward ? 0.f : c.opt.sigma_thresh,
-                                     c.opt.density_softplus, QueueScratch::default_level(c.tree),
-                                     c.stream, nullptr, c.gate);
+    const int32_t* mem = c.prepared;
+    if (mem == nullptr || c.backward) {
+        const int st = scratch.build(c.tree, layout, c.backward ? 0.f : c.opt.sigma_thresh,
+                                     c.opt.density_softplus, c.gate, c.stream);
         if (st) return st;
+        mem = scratch.mem;
     }
-    TreeArgs tr = tree_args(c.tree);
-    tr.child = scratch.annotated;
-    const TopTable top{scratch.table, scratch.level, scratch.bricks};
-    if (c.opt.format != SVOXB_FORMAT_SH)
-        return launch_queue_fitted<BD>(c, WithLobes<Source>{src}, tr, top);
-    return launch_queue_fitted<BD>(c, src, tr, top);
+    const TreeIndex index = layout.view(mem);
+    return with_basis(c.opt, [&](auto basis) {
+        constexpr int BD = decltype(basis)::value;
+        if constexpr (BD > 0) {
+            if (c.opt.format != SVOXB_FORMAT_SH)
+                return launch_mode<BD>(c, WithLobes<Source>{src}, index);
+        }
+        return launch_mode<BD>(c, src, index);
+    });
 }
 
 template <int BLOCK, class Source>
@@ -462,7 +400,7 @@ template <int BLOCK, class Source>
 static int dispatch_layout(const RenderCall& c, const Source& src, const TopTable& top,
                            bool in_smem, size_t smem) {
     const svoxb_tree* t = c.tree;
-    const bool sh3 = basis3(t, c.opt) && c.opt.format == SVOXB_FORMAT_SH;
+    const bool sh3 = queue_layout(t, c.opt) && c.opt.format == SVOXB_FORMAT_SH;
     if (!sh3) return launch_generic<BLOCK>(c, src, top, in_smem, smem);
     const bool aligned = ((uintptr_t)t->data % 16 == 0) &&
                          (!c.backward || (uintptr_t)c.grad_data % 16 == 0);
@@ -495,23 +433,15 @@ static int render_dispatch(const RenderCall& c, const Source& src) {
     if (c.Q == 0) return SVOXB_OK;
     if (c.backward ? !c.grad_out : !c.out) return SVOXB_ERR_NULL;
 
-    // Default path: the queue kernels, for octrees with three colour channels of 1, 4, 9, 16
-    // or 25 basis functions whose buffers allow the record's word size.
+    // Default path: the queue kernels, for octrees with records they are compiled for, in
+    // buffers that allow the record's 16-byte words.
     {
         const svoxb_tree* t = c.tree;
-        const bool sh3 = basis3(t, c.opt);
         const bool aligned = ((uintptr_t)t->data % 16 == 0) &&
                              (!c.backward || (uintptr_t)c.grad_data % 16 == 0);
-        if (sh3 && t->N == 2 && (aligned || t->K % 4 != 0) &&
-            t->M < (1LL << 28)) {
-            switch (c.opt.basis_dim) {
-                case 1: return launch_queue<1>(c, src);
-                case 4: return launch_queue<4>(c, src);
-                case 9: return launch_queue<9>(c, src);
-                case 16: return launch_queue<16>(c, src);
-                case 25: return launch_queue<25>(c, src);
-            }
-        }
+        if (queue_layout(t, c.opt) && t->N == 2 && (aligned || t->K % 4 != 0) &&
+            t->M < (1LL << 28))
+            return launch_queue(c, src);
     }
 
     TopScratch scratch;
@@ -606,7 +536,7 @@ static int queue_eligible(const svoxb_tree* t, const svoxb_render_options* o) {
     int st = validate_tree(t);
     if (st) return st;
     if ((st = validate_options(t, *o))) return st;
-    if (!basis3(t, *o) || t->N != 2)
+    if (!queue_layout(t, *o) || t->N != 2)
         return SVOXB_ERR_FORMAT;
     if (t->K % 4 == 0 && (uintptr_t)t->data % 16 != 0) return SVOXB_ERR_FORMAT;
     if (t->M >= (1LL << 28)) return SVOXB_ERR_TOO_LARGE;
@@ -615,7 +545,7 @@ static int queue_eligible(const svoxb_tree* t, const svoxb_render_options* o) {
 
 int64_t svoxb_render_scratch_words(const svoxb_tree* tree) {
     if (!tree || tree->M < 1 || tree->N != 2) return 0;
-    return (int64_t)QueueScratch::layout(tree, QueueScratch::default_level(tree)).words;
+    return (int64_t)QueueScratch::layout(tree).words;
 }
 
 int svoxb_render_scratch_build(const svoxb_tree* tree, const svoxb_render_options* opt,
@@ -623,9 +553,8 @@ int svoxb_render_scratch_build(const svoxb_tree* tree, const svoxb_render_option
     if (!tree || !opt || !scratch) return SVOXB_ERR_NULL;
     int st = queue_eligible(tree, opt);
     if (st) return st;
-    QueueScratch q;
-    return q.build(tree, opt->sigma_thresh, opt->density_softplus, QueueScratch::default_level(tree),
-                   (cudaStream_t)stream, scratch);
+    return build_index(tree, QueueScratch::layout(tree), opt->sigma_thresh,
+                       opt->density_softplus, scratch, LogGate{}, (cudaStream_t)stream);
 }
 
 int svoxb_volume_render_prepared(const svoxb_tree* tree, const svoxb_rays* rays,
@@ -638,7 +567,7 @@ int svoxb_volume_render_prepared(const svoxb_tree* tree, const svoxb_rays* rays,
     RenderCall c{tree, *opt, rays->Q};
     c.out = out;
     c.stream = (cudaStream_t)stream;
-    c.prepared = const_cast<int32_t*>(scratch);
+    c.prepared = scratch;
     return render_dispatch(c, RayBatch{rays->origins, rays->dirs, rays->vdirs});
 }
 
@@ -652,7 +581,7 @@ int svoxb_volume_render_image_prepared(const svoxb_tree* tree, const svoxb_camer
     RenderCall c{tree, *opt, (int64_t)cam->width * cam->height};
     c.out = out;
     c.stream = (cudaStream_t)stream;
-    c.prepared = const_cast<int32_t*>(scratch);
+    c.prepared = scratch;
     return render_dispatch(c, PixelRays{cam->c2w, cam->fx, cam->fy, cam->width, cam->height});
 }
 
@@ -700,7 +629,7 @@ int svoxb_volume_render_image_backward(const svoxb_tree* tree, const svoxb_camer
 
 // Whether a call can take the logged forward / replay backward pair.
 static int log_eligible(const svoxb_tree* t, const svoxb_render_options* o, const float* grad) {
-    if (!basis3(t, *o) || t->N != 2)
+    if (!queue_layout(t, *o) || t->N != 2)
         return SVOXB_ERR_FORMAT;
     if (o->sigma_thresh != 0.f || o->stop_thresh != 0.f) return SVOXB_ERR_OPTION;
     if (t->M >= (1LL << 28)) return SVOXB_ERR_TOO_LARGE;
@@ -726,14 +655,7 @@ static int logged_forward(const svoxb_tree* tree, const Source& src, int64_t Q,
     c.stream = (cudaStream_t)stream;
     c.log = log;
     c.log_capacity = capacity_chunks;
-    switch (opt->basis_dim) {
-        case 1: return launch_queue<1>(c, src);
-        case 4: return launch_queue<4>(c, src);
-        case 9: return launch_queue<9>(c, src);
-        case 16: return launch_queue<16>(c, src);
-        case 25: return launch_queue<25>(c, src);
-    }
-    return SVOXB_ERR_FORMAT;
+    return launch_queue(c, src);
 }
 
 template <class Source>
