@@ -569,6 +569,15 @@ class N3Tree(nn.Module):
                 as_tuple=False).cpu()
         return self._last_all_leaves
 
+    def _leaf_slots(self):
+        """Packed ids of the leaves in the order of ``_all_leaves``, on the tree's device (kept,
+        like those, until the structure changes)."""
+        slots = self._last_leaf_slots
+        if slots is None or slots.device != self.child.device:
+            slots = self._last_leaf_slots = torch.nonzero(
+                self.child[:self.n_internal].reshape(-1) == 0).flatten()
+        return slots
+
     def _calc_corners(self, nodes, cuda=True):
         """Lower corner of each ``(node, u, v, w)`` cell in tree-local coordinates
         (svox/svox.py:990-1012): the native kernel on a CUDA tree, tensor ops otherwise."""
@@ -597,6 +606,7 @@ class N3Tree(nn.Module):
         self._ver += 1
         self._data_epoch += 1
         self._last_all_leaves = None
+        self._last_leaf_slots = None
         self._last_frontier = None
 
     def _spec(self, world=True):

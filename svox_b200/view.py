@@ -19,6 +19,7 @@ class N3TreeView:
         self.tree = tree
         self.single_key = False
         self._packed_ids = None
+        self._leaf_key = None       # which of the tree's leaves, for a view that is no query
         self._value = None
         local = False
 
@@ -45,6 +46,7 @@ class N3TreeView:
                 leaf_key = torch.tensor([leaf_key], device=tree.data.device)
                 self.single_key = True
             leaf_node = tuple(tree._all_leaves()[leaf_key].T)
+            self._leaf_key = leaf_key
         self.key = (*leaf_node, *extra)
         self._tree_ver = tree._ver
 
@@ -63,6 +65,15 @@ class N3TreeView:
         return tuple(k.to(dev) if torch.is_tensor(k) else k for k in self.key[:n])
 
     def _gather(self, arr):
+        if len(self.key) == 4 and arr.is_contiguous():
+            # whole records: one packed id each instead of four coordinates, which for a view
+            # of leaves lie in host memory (295 MB to copy for the 9.2 M leaves of a 512^3
+            # scene: 26 of the 29.5 ms of a weight accumulation over two 800x800 views)
+            slots = self._packed_ids
+            if slots is None and isinstance(self._leaf_key, slice):
+                slots = self.tree._leaf_slots()[self._leaf_key]
+            if slots is not None and slots.device == arr.device:
+                return arr.view(-1, *arr.shape[4:])[slots]
         if self._require_subindex():
             return arr[self._dev_key(4)][..., self.key[-1]]
         return arr[self._dev_key(len(self.key))]
