@@ -186,13 +186,13 @@ int svoxb_volume_render_image_prepared(const svoxb_tree* tree, const svoxb_camer
 /* Logged forward + replay backward (no counterpart in the reference; the
  * pair computes what volume_render followed by volume_render_backward
  * computes, svox/csrc/rt_kernel.cu:1019-1083).  The logged forward also
- * writes every contributing sample (leaf slot, ray, weight, transmittance,
- * step, colour sigmoids, the ray's colour sums so far) into `log`, a
+ * writes every contributing sample (leaf slot, ray, colour and density factors,
+ * view direction: 48 bytes) into `log`, a
  * caller-allocated int32 device buffer of svoxb_item_log_words(capacity_chunks)
- * words (one chunk = 32 samples).  The replay backward streams that log instead
- * of marching the rays and reading the leaf records again: it sorts the
- * samples by leaf range (scratch from the stream's memory pool, 32 bytes per
- * sample) and reduces the gradient range by range so that it stays in L2.
+ * words (one chunk = up to 32 samples).  The replay backward streams that log
+ * instead of marching the rays and reading the leaf records again.  A forward
+ * of many rays sorts its samples by leaf range, so that the gradient of a range
+ * stays in L2 while it is reduced.
  * Only for octrees with three colour channels of 1, 4, 9, 16 or 25 basis
  * functions (SH, SG or ASG) and sigma_thresh =
  * stop_thresh = 0 (else SVOXB_ERR_FORMAT / SVOXB_ERR_OPTION).  `data` must not change between the two calls.
@@ -203,15 +203,19 @@ int svoxb_volume_render_image_prepared(const svoxb_tree* tree, const svoxb_camer
  *        device and do nothing if the forward asked for more chunks than
  *        `capacity_chunks`; a marching backward (as
  *        svoxb_volume_render_backward) is enqueued behind them that does its
- *        work only in that case.  No host synchronisation; the scratch is
- *        sized for the whole log; the result is the gradient either way.
+ *        work only in that case.  No host synchronisation; the result is the
+ *        gradient either way.
  *   > 0  the caller read the count with svoxb_item_log_used (which
- *        synchronises) and found it <= capacity_chunks: the scratch is sized
- *        for that many chunks and no fallback is enqueued.  With a larger
+ *        synchronises) and found it <= capacity_chunks: no fallback is
+ *        enqueued.  With a larger
  *        count the caller must call svoxb_volume_render_backward instead.
- * If the scratch cannot be had, the call marches like
- * svoxb_volume_render_backward. */
+ */
 int64_t svoxb_item_log_words(int64_t capacity_chunks);
+/* 1 if a logged forward of n_rays rays (image != 0: pixels) sorts its samples.
+ * The replay then clears the gradient on the way (zero_first != 0), at no cost;
+ * else a caller does better to clear it beside the forward, on another stream. */
+int svoxb_log_is_sorted(const svoxb_tree* tree, int64_t n_rays, int image,
+                        int64_t capacity_chunks);
 int svoxb_volume_render_logged(const svoxb_tree* tree, const svoxb_rays* rays,
                                const svoxb_render_options* opt, float* out, int32_t* log,
                                int64_t capacity_chunks, void* stream);
@@ -251,6 +255,20 @@ int svoxb_volume_render_image_hessdiag_replay(const svoxb_tree* tree, const svox
                                               int64_t capacity_chunks, int64_t chunks_used,
                                               float* hessdiag_out, int zero_first,
                                               void* stream);
+
+/* Gradient and diagonal at once, from one pass over the log: `residual` = render
+ * - colour takes grad_output's place.  chunks_used as for the replay backward
+ * (0: a march enqueued behind the replay covers a log that was too small). */
+int svoxb_se_grad_replay(const svoxb_tree* tree, const svoxb_rays* rays,
+                         const svoxb_render_options* opt, const float* residual,
+                         const float* fwd_out, int32_t* log, int64_t capacity_chunks,
+                         int64_t chunks_used, float* grad_data_out, float* hessdiag_out,
+                         int zero_first, void* stream);
+int svoxb_se_grad_image_replay(const svoxb_tree* tree, const svoxb_camera* cam,
+                               const svoxb_render_options* opt, const float* residual,
+                               const float* fwd_out, int32_t* log, int64_t capacity_chunks,
+                               int64_t chunks_used, float* grad_data_out, float* hessdiag_out,
+                               int zero_first, void* stream);
 
 /* se_grad / se_grad_persp (svox/csrc/rt_kernel.cu:479-715,846-897,1111-1173)
  * for any record layout with at most 4 output channels (the reference's bound,

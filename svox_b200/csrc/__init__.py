@@ -439,12 +439,8 @@ def volume_render_image(tree, cam, opt, prepared=None):
 # ---------------------------------------------------------------------------
 # Logged forward / replay backward (training step without a second march)
 
-# Layout of the log's head (render_queue.cuh): word 0 = chunks the forward asked for,
-# word 2 = bin shift, word 3 = number of bins, words LOG_HIST .. LOG_HIST + LOG_MAX_BINS =
-# samples per bin of the last logged forward.
-LOG_HIST, LOG_MAX_BINS = 32, 1024
-_LOG_SLACK_CHUNKS = 2 * 16384   # every warp of the forward takes log chunks 8 at a time
-_items_per_ray = 48.0           # running estimate used to size the item log
+_LOG_SLACK_CHUNKS = 2 * 16384   # chunks the forward's warps take and leave partly empty
+_items_per_ray = 80.0           # running estimate used to size the item log
 _WATCH_SLOTS = 8
 
 
@@ -462,7 +458,7 @@ class _LogWatch:
     def _state(cls, device):
         st = cls.slots.get(device)
         if st is None:
-            st = [torch.zeros(_WATCH_SLOTS, dtype=torch.int32).pin_memory(), 0, []]
+            st = [torch.zeros((_WATCH_SLOTS, 2), dtype=torch.int32).pin_memory(), 0, []]
             cls.slots[device] = st
         return st
 
@@ -474,7 +470,7 @@ class _LogWatch:
             cls.poll(log.device, wait=True)
         slot = st[1]
         st[1] = (slot + 1) % _WATCH_SLOTS
-        st[0][slot:slot + 1].copy_(log[:1], non_blocking=True)
+        st[0][slot].copy_(log[:2], non_blocking=True)
         ev = torch.cuda.Event()
         ev.record()
         pending.append((slot, ev, n_rays, cap))
@@ -493,11 +489,12 @@ class _LogWatch:
                 elif not ev.query():
                     keep.append((slot, ev, n_rays, cap))
                     continue
-                used = int(st[0][slot])
+                used, items = st[0][slot].tolist()
                 cls.last_used, cls.last_cap = used, cap
                 if n_rays:
-                    # chunks are 32 items, partly filled ones included: keep 25 % head room
-                    need = max(8.0, 1.25 * 32.0 * used / n_rays)
+                    # items, or the chunks they took beyond the slack: keep 25 % head room
+                    items = max(items, 32 * (used - _LOG_SLACK_CHUNKS))
+                    need = max(8.0, 1.25 * items / n_rays)
                     _items_per_ray = need if used > cap else max(need, 0.9 * _items_per_ray)
             st[2] = keep
         return _items_per_ray
@@ -521,11 +518,24 @@ def log_eligible(tree, opt):
             and tree.data.dtype == torch.float32)
 
 
+def _log_capacity(n_rays, device):
+    """Chunks of the next log for ``n_rays`` rays."""
+    return int(n_rays * _LogWatch.poll(device) / 32) + _LOG_SLACK_CHUNKS
+
+
+def log_is_sorted(tree, n_rays, image):
+    """Whether a logged forward of this size sorts its samples, so that the replay clears the
+    gradient on the way."""
+    ct = _pack_tree(tree)
+    return bool(library().svoxb_log_is_sorted(
+        C.byref(ct), C.c_int64(n_rays), C.c_int(int(image)),
+        C.c_int64(_log_capacity(n_rays, tree.data.device))))
+
+
 def _log_alloc(n_rays, device):
     lib = library()
     lib.svoxb_item_log_words.restype = C.c_int64
-    _LogWatch.poll(device)
-    cap = int(n_rays * _items_per_ray / 32) + _LOG_SLACK_CHUNKS
+    cap = _log_capacity(n_rays, device)
     words = lib.svoxb_item_log_words(C.c_int64(cap))
     return torch.empty(words, dtype=torch.int32, device=device), cap
 
@@ -588,7 +598,7 @@ def volume_render_backward_replay(tree, rays_or_cam, opt, grad_output, fwd_out, 
         if used > cap:
             raise RuntimeError("the item log overflowed: it cannot be replayed")
         grad = zeroed if zeroed is not None else \
-            torch.zeros_like(tree.data, memory_format=torch.contiguous_format)
+            torch.empty_like(tree.data, memory_format=torch.contiguous_format)
         if image:
             cs = _pack_camera(rays_or_cam, dev)
             fn = lib.svoxb_volume_render_image_backward_replay
@@ -598,39 +608,39 @@ def volume_render_backward_replay(tree, rays_or_cam, opt, grad_output, fwd_out, 
         with _timed("volume_render_backward"):
             st = fn(C.byref(ct), C.byref(cs), C.byref(co), C.c_void_p(grad_output.data_ptr()),
                     C.c_void_p(fwd_out.data_ptr()), C.c_void_p(log.data_ptr()), C.c_int64(cap),
-                    C.c_int64(used), C.c_void_p(grad.data_ptr()), C.c_int(0), _stream())
+                    C.c_int64(used), C.c_void_p(grad.data_ptr()), C.c_int(int(zeroed is None)),
+                    _stream())
     if st:
         _raise(st, "volume_render_backward_replay")
     return grad
 
 
-def volume_render_hessdiag_replay(tree, rays_or_cam, opt, fwd_out, logpair, used, image=False):
-    """Gauss-Newton diagonal of the squared error from the item log (third result of the
-    reference's ``se_grad``).  ``used``: the count from ``log_chunks_used`` (there is no
-    marching fallback for this result, so the caller has to know that the log was large
-    enough)."""
+def se_grad_replay(tree, rays_or_cam, opt, residual, fwd_out, logpair, grad, hess, zeroed,
+                   image=False):
+    """Gradient and Gauss-Newton diagonal of the squared error (second and third result of the
+    reference's ``se_grad``) from the item log, into ``grad`` and ``hess`` (``zeroed``: which
+    already are zero).  The host does not wait: a log that was too small is noticed on the
+    device, where a march enqueued behind the replay then takes over."""
     lib = library()
     log, cap = logpair
     dev = tree.data.device
-    if not 0 < used <= cap:
-        raise RuntimeError("the item log overflowed or its chunk count is not known")
     with torch.cuda.device(dev):
         ct = _pack_tree(tree)
         co = opt._pack()
+        _check_input(residual, "residual")
         _check_input(fwd_out, "fwd_out")
-        hess = torch.zeros_like(tree.data, memory_format=torch.contiguous_format)
         if image:
             cs = _pack_camera(rays_or_cam, dev)
-            fn = lib.svoxb_volume_render_image_hessdiag_replay
+            fn = lib.svoxb_se_grad_image_replay
         else:
             cs = _pack_rays(rays_or_cam, dev)
-            fn = lib.svoxb_volume_render_hessdiag_replay
-        st = fn(C.byref(ct), C.byref(cs), C.byref(co), C.c_void_p(fwd_out.data_ptr()),
-                C.c_void_p(log.data_ptr()), C.c_int64(cap), C.c_int64(used),
-                C.c_void_p(hess.data_ptr()), C.c_int(0), _stream())
+            fn = lib.svoxb_se_grad_replay
+        st = fn(C.byref(ct), C.byref(cs), C.byref(co), C.c_void_p(residual.data_ptr()),
+                C.c_void_p(fwd_out.data_ptr()), C.c_void_p(log.data_ptr()), C.c_int64(cap),
+                C.c_int64(0), C.c_void_p(grad.data_ptr()), C.c_void_p(hess.data_ptr()),
+                C.c_int(int(not zeroed)), _stream())
     if st:
-        _raise(st, "volume_render_hessdiag_replay")
-    return hess
+        _raise(st, "se_grad_replay")
 
 
 def se_grad_march(tree, rays_or_cam, opt, fwd_out, colors, image=False):

@@ -148,11 +148,14 @@ struct TopScratch {
     ~TopScratch() { if (cells) cudaFreeAsync(cells, stream); }
 };
 
+// Gradient MB one log bin spans.  Measured on the scatter of the training step: 32 -> 1.49 ms,
+// 64 -> 1.62, 128 -> 2.39, 256 -> 3.40, unsorted 4.50.
+constexpr int kReplayBinMB = 32;
+
 // The two switches the tests flip to show that an index or a bin size changes no result
 // (svoxb_test_knob).
 struct Tuning {
-    int replay_bin_mb = 32;  // gradient MB one replay bin spans (measured: 16 -> 3.05 ms of
-                             // backward per training step, 32 and 64 -> 2.94, 128 -> 3.86)
+    int replay_bin_mb = kReplayBinMB;
     int render_bricks = 1;   // queue kernels: bricks below the leaf table
 };
 extern Tuning g_tuning;

@@ -198,6 +198,7 @@ __device__ __forceinline__ void ray_setup(Ray& r, const float* __restrict__ scal
 // Ray sources ---------------------------------------------------------------
 struct RayBatch {  // render_ray_kernel's inputs (svox/csrc/rt_kernel.cu:717-733)
     static constexpr bool kLobes = false;
+    static constexpr bool kImage = false;
     const float* __restrict__ origins;
     const float* __restrict__ dirs;
     const float* __restrict__ vdirs;
@@ -218,17 +219,11 @@ struct RayBatch {  // render_ray_kernel's inputs (svox/csrc/rt_kernel.cu:717-733
         r.vdir[1] = __ldg(vdirs + 3 * i + 1);
         r.vdir[2] = __ldg(vdirs + 3 * i + 2);
     }
-    // The view direction alone (colour basis of the backward's gradient records).
-    __device__ __forceinline__ void load_vdir(int64_t i, const TreeArgs&,
-                                              const svoxb_render_options&, float v[3]) const {
-        v[0] = __ldg(vdirs + 3 * i + 0);
-        v[1] = __ldg(vdirs + 3 * i + 1);
-        v[2] = __ldg(vdirs + 3 * i + 2);
-    }
 };
 
 struct PixelRays {  // render_image_kernel's inputs (svox/csrc/rt_kernel.cu:758-819)
     static constexpr bool kLobes = false;
+    static constexpr bool kImage = true;
     const float* __restrict__ c2w;  // row-major, row stride 4
     float fx, fy;
     int width, height;
@@ -291,12 +286,6 @@ struct PixelRays {  // render_image_kernel's inputs (svox/csrc/rt_kernel.cu:758-
         r.oy = to_tree(o[1], __ldg(tr.offset + 1), __ldg(tr.scaling + 1));
         r.oz = to_tree(o[2], __ldg(tr.offset + 2), __ldg(tr.scaling + 2));
         r.dx = d[0]; r.dy = d[1]; r.dz = d[2];
-    }
-    __device__ __forceinline__ void load_vdir(int64_t i, const TreeArgs& tr,
-                                              const svoxb_render_options& opt, float v[3]) const {
-        Ray r;
-        load(i, tr, opt, r);
-        v[0] = r.vdir[0]; v[1] = r.vdir[1]; v[2] = r.vdir[2];
     }
 };
 
@@ -859,15 +848,18 @@ render_bwd_generic(TreeArgs tr, Source src, svoxb_render_options opt, TopTable t
 // record layout: what the reference's se_grad kernel adds up in its second and third march
 // (svox/csrc/rt_kernel.cu:566-709), with its per-channel running sums.  One march is enough
 // here because the colour the reference re-accumulates in its second march is the forward's
-// output (`fwd_out`, rendered without thresholds), which the caller already has.
+// output (`fwd_out`, rendered without thresholds), which the caller already has.  The residual
+// is given, or formed as fwd_out - color_ref.
 template <int BLOCK, class Source>
 __global__ void __launch_bounds__(BLOCK)
 render_se_grad_generic(TreeArgs tr, Source src, svoxb_render_options opt, TopTable topg,
                        bool top_in_smem, const float* __restrict__ fwd_out,
-                       const float* __restrict__ color_ref, float* __restrict__ grad,
-                       float* __restrict__ hess, int64_t Q, int out_dim) {
+                       const float* __restrict__ color_ref, const float* __restrict__ residual,
+                       float* __restrict__ grad, float* __restrict__ hess, int64_t Q, int out_dim,
+                       LogGate gate) {
     extern __shared__ int32_t s_top[];
     __shared__ unsigned s_next;
+    if (gate.closed()) return;
     if (threadIdx.x == 0) s_next = 0;
     const TopTable top = stage_top(topg, s_top, top_in_smem);
     __syncthreads();
@@ -892,7 +884,9 @@ render_se_grad_generic(TreeArgs tr, Source src, svoxb_render_options opt, TopTab
         float accum[kMaxSeGradOut], curr[kMaxSeGradOut], resid[kMaxSeGradOut];
         for (int j = 0; j < out_dim; ++j) {
             accum[j] = r.hit ? __ldg(fwd_out + ray * out_dim + j) : 0.f;
-            resid[j] = r.hit ? accum[j] - __ldg(color_ref + ray * out_dim + j) : 0.f;
+            resid[j] = !r.hit               ? 0.f
+                       : residual != nullptr ? __ldg(residual + ray * out_dim + j)
+                                             : accum[j] - __ldg(color_ref + ray * out_dim + j);
         }
         float light = 1.f, t = r.tmin;
         int it = 0;

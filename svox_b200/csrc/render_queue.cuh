@@ -64,23 +64,58 @@ struct RecordShape {
 // Item log: what a logged forward leaves behind so that the backward pass can
 // replay the contributing samples without marching again and without reading
 // the leaf records a second time.  int32 words:
-//   [0] chunks allocated   [2] bin shift   [3] number of bins
-//   [kLogHeads + b]        items whose leaf slot falls into bin b (= slot >> shift)
-//   chunk c at kLogChunks + c * kLogChunkWords: 12 rows of 32 words,
-//     row 0: word 0 = items in the chunk
-//     rows 1-11, one word per item: slot, ray, weight, T after, delta_t*delta_scale
-//     (times the derivative of the density's softplus, if that is on), sigmoid of the
-//     three channels, colour sums of the ray up to and including the item (three channels)
-// With the partial colour sums every item is self-contained: the reference's
-// running `accum` after item k (svox/csrc/rt_kernel.cu:462-471) equals
-// <grad_out, out> - <grad_out, partial sums>, so the backward can take the
-// items in any order.
-constexpr int kLogHeads = 32;
-constexpr int kMaxBins = 256;
-constexpr int kLogChunks = kLogHeads + kMaxBins;
-constexpr int kLogRows = 12;
-constexpr int kLogChunkWords = kLogRows * 32;
-constexpr int kLogGrab = 8;  // chunks a warp takes per bump of the allocation counter
+//   [0] chunks asked for   [1] items   [2] bin shift   [3] number of bins
+//   [kLogNext + p]         units taken of scatter part p, [kLogNext + kMaxParts + p] blocks done
+//   [kLogBins + b]         groups of bin b      [kLogCleared + b]  cleared units of bin b
+//   [kLogCounts + g]       items of group g (bits 0-7) and its bin (bits 8-)
+//   then, 128-byte aligned, 32 packets of 12 words per chunk, and the order of the groups by
+//   bin (one word per group; only with several bins).
+// A PACKET is one contributing sample: {slot, ray, q0, q1} {q2, h0, h1, h2} {dd, view
+// direction}, with q = weight * sg * (1 - sg) per colour channel (sg the channel's sigmoid), h =
+// colour * T + S (T the transmittance after the sample, S the ray's colour sum up to and
+// including it) and dd = delta_t * delta_scale, times the derivative of the density's softplus
+// if that is on.  With g = grad_out[ray] the reference's gradient of the sample is
+//   d/d coef  = basis[i] * q * g * (1 + 2 pad)                  (svox/csrc/rt_kernel.cu:386-392)
+//   d/d sigma = dd * sum_ch g (h - out[ray])                    (:462-471)
+// because its running `accum` after the sample equals <g, out> - <g, S>: every packet is
+// self-contained and the backward can take them in any order.
+//
+// One bin: a GROUP is one chunk, a batch of the forward, in the order of the march.  Several
+// bins (ranges of leaf slots): a group is kSortedChunks chunks, and every block keeps an open
+// group per bin, so that the backward can take the packets range by range and the gradient
+// stays in L2 meanwhile.
+constexpr int kMaxParts = 16;   // the scatter can run in up to 16 parts (bin ranges)
+constexpr int kLogNext = 32;
+constexpr int kLogBins = kLogNext + 2 * kMaxParts;
+constexpr int kMaxBins = 128;
+constexpr int kLogCleared = kLogBins + kMaxBins;
+constexpr int kLogCounts = kLogCleared + kMaxBins;
+constexpr int kPacketWords = 12;
+constexpr int kLogGrab = 8;        // groups a warp takes at least per bump of the counter ...
+constexpr int kSortedGrab = 2;     // ... of a sorted log
+constexpr int kSortedChunks = 4;   // chunks per group of a sorted log
+constexpr int kSortedItems = 32 * kSortedChunks;
+// A block remembers this many of a bin's last groups.  A warp reads the id of its item's group
+// a few instructions after it has taken the item's place; a block has at most 24 * 32 items under
+// way, so their groups are among the last 7 (see the wait in `evaluate` for the rest).
+constexpr int kOpenGroups = 16;
+
+__host__ __device__ inline int64_t log_packets_at(int64_t capacity) {
+    return (kLogCounts + capacity + 31) & ~(int64_t)31;
+}
+__host__ __device__ inline int64_t log_order_at(int64_t capacity) {
+    return log_packets_at(capacity) + capacity * (32 * kPacketWords);
+}
+__host__ __device__ inline int64_t log_words(int64_t capacity) {
+    return log_order_at(capacity) + capacity + kMaxBins;   // ... and cursors of the ordering
+}
+
+// The log as a kernel gets it: written by a logged forward, the gate of a fallback march.
+struct LogArgs {
+    int32_t* log = nullptr;
+    int64_t capacity = 0;
+    int shift = 0, n_bins = 1;
+};
 
 // L2 residency hints.  The index (tens of MB, re-read hundreds of times per launch) must stay
 // in L2 while the leaf records and gradients (GBs, touched a few times each) stream through it.
@@ -99,8 +134,10 @@ __device__ __forceinline__ int32_t ld_keep(const int32_t* a, uint64_t pol) {
     asm volatile("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(pol));
     return v;
 }
-__device__ __forceinline__ void st_stream(int32_t* a, int32_t v, uint64_t pol) {
-    asm volatile("st.global.L2::cache_hint.s32 [%0], %1, %2;" ::"l"(a), "r"(v), "l"(pol) : "memory");
+__device__ __forceinline__ void st_hint16(void* a, int4 v, uint64_t pol) {
+    asm volatile("st.global.L2::cache_hint.v4.s32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(a), "r"(v.x),
+                 "r"(v.y), "r"(v.z), "r"(v.w), "l"(pol)
+                 : "memory");
 }
 // The 64-byte L2 fetch granularity is a measured choice: records are 112-196 bytes at arbitrary
 // 16-byte offsets, and the logged forward of the training step runs 1 % faster with it than with the
@@ -152,7 +189,8 @@ struct alignas(16) WarpQueue {
     using Shape = RecordShape<K>;
     // three batches: items being collected, what spills over, and the batch in flight
     static constexpr int CAP = 96;
-    static constexpr int RAYW = (BD + (BWD ? 3 : 0)) | 1;  // odd stride: no bank conflicts
+    // colour basis, upstream gradient or view direction; odd stride: no bank conflicts
+    static constexpr int RAYW = (BD + (BWD || LOG ? 3 : 0)) | 1;
     // Staging rows (cp.async targets).  After lane i has read row i it reuses the
     // row's first words for the item's results.
     alignas(16) float rows[32 * Shape::STRIDE];
@@ -161,24 +199,33 @@ struct alignas(16) WarpQueue {
     float T[(BWD || LOG) ? CAP : 4];   // transmittance after the sample
     float dd[(BWD || LOG) ? CAP : 4];  // delta_t * delta_scale
     unsigned char owner[CAP];          // bits 0-4 owner lane, bit 7 accumulation march
-    float rayv[32][RAYW];              // per lane: colour basis [0,BD), upstream gradient
+    float rayv[32][RAYW];
 };
 
 enum { kNeedRay = 0, kMarching = 1, kEnded = 2, kExhausted = 3 };
 
 constexpr int kMarchBlock = 128;
 
-// Blocks per SM the kernel is compiled for: as many as shared memory holds, at most 6 (24
-// warps, 80 registers per thread).  Measured on the logged forward of 2^20 rays, SH9: 8 blocks
-// (64 registers, no L1 left beside 213 KB of queues) 5.0 ms, 7 blocks 3.6, 6 blocks 3.5, 5
-// blocks 3.7.
+// Blocks of kMarchBlock threads per SM the kernel is compiled for: as many as shared memory
+// holds, at most 6 (24 warps, 80 registers per thread).  Measured on the logged forward of 2^20
+// rays, SH9: 8 blocks (64 registers, no L1 left beside 213 KB of queues) 5.0 ms, 7 blocks 3.6,
+// 6 blocks 3.5, 5 blocks 3.7.
 constexpr int kMarchBlocks = 6;
 template <int BD, int MODE>
 constexpr int march_blocks_per_sm() {
-    const size_t smem = (kMarchBlock / 32) * sizeof(WarpQueue<BD, MODE>) + 1024 +
-                        (MODE == kModeForwardLogged ? kMaxBins * sizeof(int) : 0);
+    const size_t smem = (kMarchBlock / 32) * sizeof(WarpQueue<BD, MODE>) + 1024;
     const int fit = (int)(227 * 1024 / smem);
     return fit > kMarchBlocks ? kMarchBlocks : fit < 1 ? 1 : fit;
+}
+
+// A forward that sorts its log into bins runs as one block per SM, so that a bin has one open
+// group per SM and the lines being filled stay in L2 until they are full.
+constexpr size_t kBinSmem = (size_t)kMaxBins * (1 + kOpenGroups) * sizeof(uint32_t);
+template <int BD>
+constexpr int sorted_march_block() {
+    const int fit = (int)((227 * 1024 - 1024 - kBinSmem) / sizeof(WarpQueue<BD, kModeForwardLogged>));
+    const int warps = 4 * march_blocks_per_sm<BD, kModeForwardLogged>();
+    return 32 * (fit < warps ? fit : warps);
 }
 
 // clamp01's upper bound
@@ -206,13 +253,13 @@ struct MarchShape {
     int lanes, granule_shift, refill;
 };
 
-template <int BD, int MODE, class Source>
-__global__ void __launch_bounds__(kMarchBlock, march_blocks_per_sm<BD, MODE>())
+template <int BD, int MODE, int BLOCK, class Source>
+__global__ void
+__launch_bounds__(BLOCK, BLOCK == kMarchBlock ? march_blocks_per_sm<BD, MODE>() : 1)
 render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex index,
                     int64_t tickets, float* __restrict__ out,
                     const float* __restrict__ grad_out, const float* __restrict__ fwd_out,
-                    float* __restrict__ grad_data, int32_t* __restrict__ log,
-                    int64_t log_capacity, int log_shift, MarchShape shape) {
+                    float* __restrict__ grad_data, LogArgs lg, MarchShape shape) {
     constexpr int K = RecordLength<BD>::K;
     constexpr bool BWD = MODE == kModeBackward;
     constexpr bool LOG = MODE == kModeForwardLogged;
@@ -220,16 +267,19 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     using Shape = RecordShape<K>;
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ unsigned s_next;
-    __shared__ int s_hist[LOG ? kMaxBins : 1];  // logged forward: items per bin
     // backward with a log: the marching fallback of a replay, needed only if the log overflowed
-    if (BWD && LogGate{log, log_capacity}.closed()) return;
+    if (BWD && LogGate{lg.log, lg.capacity}.closed()) return;
     if (threadIdx.x == 0) s_next = 0;
-    if (LOG) {
-        for (int i = threadIdx.x; i < kMaxBins; i += kMarchBlock) s_hist[i] = 0;
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            log[2] = log_shift;
-            log[3] = (int)(((tr.M * 8 - 1) >> log_shift) + 1);
-        }
+    // sorted log: items this block has put into each bin, and its last groups of the bin, each
+    // as (1 + the group's number among them) mod 256 in the top byte and the group's id
+    constexpr bool SORTED = LOG && BLOCK != kMarchBlock;
+    uint32_t* s_count = reinterpret_cast<uint32_t*>(s_raw + (BLOCK / 32) * sizeof(WQ));
+    uint32_t* s_open = s_count + lg.n_bins;
+    if (SORTED)
+        for (int i = threadIdx.x; i < lg.n_bins * (1 + kOpenGroups); i += BLOCK) s_count[i] = 0;
+    if (LOG && blockIdx.x == 0 && threadIdx.x == 0) {
+        lg.log[2] = lg.shift;
+        lg.log[3] = lg.n_bins;
     }
     const int lane = threadIdx.x & 31;
     WQ& q = *reinterpret_cast<WQ*>(s_raw + (size_t)(threadIdx.x >> 5) * sizeof(WQ));
@@ -262,9 +312,11 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     int head = 0, qn = 0;
     unsigned mine = 0u, mine_next = 0u, mine_fly = 0u;  // my items: first 32, spilled, in flight
     int fly = 0;                       // items in flight, in the batch before `head`
-    // logged forward: the warp takes kLogGrab chunks at a time from the log
-    int64_t log_chunk = 0;
-    int log_left = 0;
+    // logged forward: groups the warp has taken from the log but not used, items written
+    int log_group = 0, log_left = 0, log_items = 0;
+    const int log_limit = SORTED ? (int)(lg.capacity / kSortedChunks) : (int)lg.capacity;
+    int32_t* const log_counts = lg.log + kLogCounts;
+    int4* const packets = reinterpret_cast<int4*>(lg.log + log_packets_at(lg.capacity));
 
     // Places the cursor at parameter t and requests the index words there, to be consumed one
     // iteration later: the brick's, if the ray is still in the table cell whose brick it used
@@ -288,6 +340,11 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         const uint32_t x = ux >> s3, y = uy >> s3, z = uz >> s3;
         const uint32_t c = ((x & 6) << 6) | ((y & 6) << 4) | ((z & 6) << 2) |
                            ((x & 1) << 2) | ((y & 1) << 1) | (z & 1);
+        if (BWD && index.table == nullptr) {       // fallback march: no index was built
+            word = kWordWalk;
+            in_brick = false;
+            return;
+        }
         word = ld_keep(index.table + (in_brick ? cur_brick + c : (uint32_t)cell), pol_keep);
         if (in_brick)
             group = ld_keep(index.table + (cur_brick + kBrickCells + (c >> 3)), pol_keep);
@@ -336,7 +393,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         const int off = record_offset<K>(tr.data, b_slot);
         const int own = b_own & 31;
         const bool acc_item = BWD && (b_own & 0x80) != 0;
-        float sg[3] = {0.f, 0.f, 0.f};
+        float sg[3] = {0.f, 0.f, 0.f}, col[3] = {0.f, 0.f, 0.f};
         float raw_sigma = 0.f;
         if (active) {
             float tmp[3] = {0.f, 0.f, 0.f};
@@ -371,7 +428,6 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                     raw_sigma = rec[K - 1];
                 }
             }
-            float col[3];
 #pragma unroll
             for (int ch = 0; ch < 3; ++ch) {
                 sg[ch] = sigmoid_ref(tmp[ch]);
@@ -409,40 +465,84 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         fly = 0;
         __syncwarp();
         if (LOG) {
-            // lane i writes item i, now with its ray's colour sums, into the log
-            if (log_left == 0) {
-                int c = 0;
-                if (lane == 0) c = atomicAdd(log, kLogGrab);
-                log_chunk = __shfl_sync(0xffffffffu, c, 0);
-                log_left = kLogGrab;
-            }
+            // lane i writes the packet of item i, now that its ray's colour sums are known: to
+            // place i of the batch's chunk, or to the next place of its bin
             const int ray_id = __shfl_sync(0xffffffffu, (int)ray, own);
-            if (log_chunk < log_capacity) {
-                int32_t* ch = log + kLogChunks + log_chunk * kLogChunkWords;
-                if (lane == 0) ch[0] = nb;
-                if (active) {
-                    const float4 sums = *reinterpret_cast<const float4*>(row);
-                    // the logged step length carries d softplus / d raw density, the one factor
-                    // the replayed density gradient needs from the raw value
-                    // (svox/csrc/rt_kernel.cu:469-470)
-                    if (opt.density_softplus) b_dd *= sigmoid_ref(raw_sigma - 1);
-                    st_stream(ch + 32 * 1 + lane, (int32_t)b_slot, pol_stream);
-                    st_stream(ch + 32 * 2 + lane, ray_id, pol_stream);
-                    st_stream(ch + 32 * 3 + lane, __float_as_int(b_w), pol_stream);
-                    st_stream(ch + 32 * 4 + lane, __float_as_int(b_T), pol_stream);
-                    st_stream(ch + 32 * 5 + lane, __float_as_int(b_dd), pol_stream);
-                    st_stream(ch + 32 * 6 + lane, __float_as_int(sg[0]), pol_stream);
-                    st_stream(ch + 32 * 7 + lane, __float_as_int(sg[1]), pol_stream);
-                    st_stream(ch + 32 * 8 + lane, __float_as_int(sg[2]), pol_stream);
-                    st_stream(ch + 32 * 9 + lane, __float_as_int(sums.x), pol_stream);
-                    st_stream(ch + 32 * 10 + lane, __float_as_int(sums.y), pol_stream);
-                    st_stream(ch + 32 * 11 + lane, __float_as_int(sums.z), pol_stream);
-                    const uint32_t bin = b_slot >> log_shift;
-                    atomicAdd(&s_hist[bin < (uint32_t)kMaxBins ? bin : kMaxBins - 1], 1);
-                }
+            int bin = 0, place = lane;
+            uint32_t number = 0;
+            if (SORTED && active) {
+                bin = (int)(b_slot >> lg.shift);
+                const uint32_t n = atomicAdd(&s_count[bin], 1u);
+                place = (int)(n % kSortedItems);
+                number = n / kSortedItems;
             }
-            ++log_chunk;
-            --log_left;
+            // lanes that open a group: the first of its items
+            const bool opens = SORTED ? active && place == 0 : lane == 0;
+            const unsigned opening = __ballot_sync(0xffffffffu, opens);
+            const int n_open = __popc(opening);
+            const int mine_open = __popc(opening & ((1u << lane) - 1u));
+            int group_id = log_group + mine_open;
+            if (n_open > log_left) {
+                constexpr int GRAB = SORTED ? kSortedGrab : kLogGrab;
+                constexpr int UNIT = SORTED ? kSortedChunks : 1;
+                const int more = n_open - log_left > GRAB ? n_open - log_left : GRAB;
+                int c = 0;
+                if (lane == 0) c = atomicAdd(lg.log, more * UNIT) / UNIT;
+                c = __shfl_sync(0xffffffffu, c, 0);
+                if (mine_open >= log_left) group_id = c + mine_open - log_left;
+                log_group = c + n_open - log_left;
+                log_left += more - n_open;
+            } else {
+                log_group += n_open;
+                log_left -= n_open;
+            }
+            if (opens && group_id < log_limit)
+                log_counts[group_id] = SORTED ? kSortedItems | (bin << 8) : nb;
+            if (SORTED) {
+                volatile uint32_t* open = s_open + bin * kOpenGroups + (number & (kOpenGroups - 1));
+                const uint32_t tag = (number + 1u) & 0xffu;
+                if (opens)
+                    *open = (tag << 24) | (uint32_t)(group_id < 0xffffff ? group_id : 0xffffff);
+                __syncwarp();
+                if (active && !opens) {
+                    // another warp may be about to publish the group's id
+                    uint32_t v = *open;
+                    int tries = 0;
+                    while ((v >> 24) != tag && ++tries < (1 << 14)) {
+                        __nanosleep(32);
+                        v = *open;
+                    }
+                    group_id = (int)(v & 0xffffffu);
+                    if ((v >> 24) != tag) {     // never seen: give the log up, march instead
+                        atomicMax(lg.log, 1 << 30);
+                        group_id = 0x7fffffff;
+                    }
+                }
+                __syncwarp();
+            } else {
+                group_id = __shfl_sync(0xffffffffu, group_id, 0);
+            }
+            if (active && group_id < log_limit) {
+                const float4 sums = *reinterpret_cast<const float4*>(row);
+                // the step length carries d softplus / d raw density, the one factor the
+                // density gradient needs from the raw value (svox/csrc/rt_kernel.cu:469-470)
+                if (opt.density_softplus) b_dd *= sigmoid_ref(raw_sigma - 1);
+                int qf[3];
+#pragma unroll
+                for (int ch = 0; ch < 3; ++ch)
+                    qf[ch] = __float_as_int((float)(b_w * sg[ch] * (1.0 - sg[ch])));
+                const float* vd = &q.rayv[own][BD];
+                int4* to = packets + ((int64_t)group_id * (SORTED ? kSortedItems : 32) + place) *
+                                         (kPacketWords / 4);
+                const uint64_t pol = SORTED ? pol_keep : pol_stream;
+                st_hint16(to, make_int4((int)b_slot, ray_id, qf[0], qf[1]), pol);
+                st_hint16(to + 1, make_int4(qf[2], __float_as_int(__fmaf_rn(col[0], b_T, sums.x)),
+                                            __float_as_int(__fmaf_rn(col[1], b_T, sums.y)),
+                                            __float_as_int(__fmaf_rn(col[2], b_T, sums.z))), pol);
+                st_hint16(to + 2, make_int4(__float_as_int(b_dd), __float_as_int(vd[0]),
+                                            __float_as_int(vd[1]), __float_as_int(vd[2])), pol);
+            }
+            log_items += nb;
             __syncwarp();
         }
         if (BWD) {
@@ -556,6 +656,10 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                             for (int i = 0; i < BD; ++i)
                                 q.rayv[lane][i] =
                                     (i < opt.min_comp || i > opt.max_comp) ? 0.f : basis[i];
+                        }
+                        if (LOG) {
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) q.rayv[lane][BD + i] = r.vdir[i];
                         }
                         a0 = a1 = a2 = 0.f;
                         if (BWD) {
@@ -715,12 +819,21 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         }
     }
     if (LOG) {
-        // chunks taken but not used hold no items
-        if (lane < log_left && log_chunk + lane < log_capacity)
-            log[kLogChunks + (log_chunk + lane) * kLogChunkWords] = 0;
-        __syncthreads();
-        for (int i = threadIdx.x; i < kMaxBins; i += kMarchBlock)
-            if (s_hist[i] != 0) atomicAdd(log + kLogHeads + i, s_hist[i]);
+        // groups taken but not used hold no items; the last group of a bin holds what it got
+        for (int i = lane; i < log_left; i += 32)
+            if (log_group + i < log_limit) log_counts[log_group + i] = 0;
+        if (lane == 0 && log_items > 0) atomicAdd(lg.log + 1, log_items);
+        if (SORTED) {
+            __syncthreads();
+            for (int b = threadIdx.x; b < lg.n_bins; b += BLOCK) {
+                const uint32_t n = s_count[b];
+                if (n == 0) continue;
+                const uint32_t last = (n - 1) / kSortedItems;
+                const int g = (int)(s_open[b * kOpenGroups + (last & (kOpenGroups - 1))] & 0xffffffu);
+                if (g < log_limit) log_counts[g] = (int)(n - kSortedItems * last) | (b << 8);
+                atomicAdd(lg.log + kLogBins + b, (int)last + 1);
+            }
+        }
     }
 }
 

@@ -8,6 +8,7 @@
 #include "render_queue.cuh"
 #include "render_replay.cuh"
 #include "collective.cuh"
+#include <initializer_list>
 #include <new>
 
 namespace svoxb {
@@ -15,6 +16,8 @@ namespace svoxb {
 // Queue kernels: idle lanes of a warp before it drains its queue and refills (4 and 12 measure
 // within 1 % of 8 on ray batches and images).
 constexpr int kRefillLanes = 8;
+// Quarters of the leaf slots a batch has to touch for its log to be sorted.
+constexpr int kSortTouches = 1;
 // ... and warps per SM that a small batch is spread over before warps get 32 rays each.
 constexpr int kSpreadWarps = 16;
 
@@ -138,21 +141,33 @@ static int launch_sh(const RenderCall& c, const Source& src, const TopTable& top
     return SVOXB_OK;
 }
 
-// Replay bins: a bin is a range of 2^shift leaf slots whose gradient spans
+// Log bins: a bin is a range of 2^shift leaf slots whose gradient spans
 // about g_tuning.replay_bin_mb MB, at most kMaxBins of them.
 static int replay_bin_shift(int64_t M, int K) {
     const int64_t per_bin = ((int64_t)g_tuning.replay_bin_mb << 20) / (K * 4);
-    int shift = 0;
+    int shift = 2;               // a bin of the gradient is a whole number of 16-byte words
     while ((2LL << shift) <= per_bin) ++shift;
     while (((M * 8 - 1) >> shift) + 1 > kMaxBins) ++shift;
     return shift;
+}
+static int replay_bins(int64_t M, int K) {
+    return (int)(((M * 8 - 1) >> replay_bin_shift(M, K)) + 1);
+}
+
+// Whether a logged forward sorts its items into bins: when the gradient outgrows a bin and a
+// good part of it is touched (64 contributing samples per ray of a random batch, 24 per pixel,
+// against the leaf slots).  Then the scatter finds the gradient in L2 and clears it on the way.
+// A group's id has 24 bits there.
+static bool sorts_log(const svoxb_tree* t, int64_t rays, bool image, int64_t capacity) {
+    if (capacity / kSortedChunks >= 0xffffff || replay_bins(t->M, t->K) < 2) return false;
+    return g_tuning.replay_bin_mb != kReplayBinMB ||
+           rays * (image ? 24 : 64) >= kSortTouches * 8 * t->M / 4;
 }
 
 // How the queue kernels deal out `tickets` rays.  With fewer rays than fill the device's warps
 // a warp takes fewer of them, so that every SM sub-partition has work: a march is a serial
 // chain, and what cannot be hidden by other warps should at least run side by side.
-static MarchShape march_shape(int64_t tickets, int sms) {
-    const int64_t warps = (int64_t)sms * kSpreadWarps;
+static MarchShape march_shape(int64_t tickets, int64_t warps) {
     MarchShape m{32, 5, kRefillLanes};
     while (m.lanes > 4 && tickets <= warps * (m.lanes / 2)) m.lanes /= 2;
     if (m.lanes == 4) m.granule_shift = 4;
@@ -160,128 +175,89 @@ static MarchShape march_shape(int64_t tickets, int sms) {
     return m;
 }
 
-template <int BD, int MODE, class Source>
-static int launch_march(const RenderCall& c, const Source& src, const TreeIndex& index) {
-    const size_t smem = (kMarchBlock / 32) * sizeof(WarpQueue<BD, MODE>);
+template <int BD, int MODE, int BLOCK, class Source>
+static int launch_march(const RenderCall& c, const Source& src, const TreeIndex& index,
+                        LogArgs log) {
+    const size_t smem = (BLOCK / 32) * sizeof(WarpQueue<BD, MODE>) +
+                        (BLOCK == kMarchBlock ? 0 : kBinSmem);
     const int64_t tickets = Source::tickets(src, c.Q);
-    const MarchShape shape = march_shape(tickets, sm_count());
-    auto k = render_queue_kernel<BD, MODE, Source>;
+    const MarchShape shape = march_shape(
+        tickets, (int64_t)sm_count() * (BLOCK == kMarchBlock ? kSpreadWarps : BLOCK / 32));
+    auto k = render_queue_kernel<BD, MODE, BLOCK, Source>;
     unsigned grid = 1;
     const int64_t granules = (tickets + (1 << shape.granule_shift) - 1) >> shape.granule_shift;
     // one granule per block at least (persistent_grid counts granules of 32 threads)
-    int st = persistent_grid(k, kMarchBlock, smem, granules * (kMarchBlock / 32), &grid);
+    int st = persistent_grid(k, BLOCK, smem, granules * (BLOCK / 32), &grid);
     if (st) return st;
     const bool single = MODE == kModeBackward && c.fwd_out != nullptr && c.opt.sigma_thresh == 0.f &&
                         c.opt.stop_thresh == 0.f;
-    int32_t* log = MODE == kModeForwardLogged ? c.log
-                   : MODE == kModeBackward    ? const_cast<int32_t*>(c.gate.log)
-                                              : nullptr;
-    const int64_t capacity = MODE == kModeForwardLogged ? c.log_capacity : c.gate.capacity;
-    k<<<grid, kMarchBlock, smem, c.stream>>>(
-        tree_args(c.tree), src, c.opt, index, tickets, c.out, c.grad_out,
-        single ? c.fwd_out : nullptr, c.grad_data, log, capacity,
-        replay_bin_shift(c.tree->M, c.tree->K), shape);
+    k<<<grid, BLOCK, smem, c.stream>>>(tree_args(c.tree), src, c.opt, index, tickets, c.out,
+                                       c.grad_out, single ? c.fwd_out : nullptr, c.grad_data, log,
+                                       shape);
     SVOXB_CUDA(cudaGetLastError());
     return SVOXB_OK;
 }
 
 template <int BD, class Source>
 static int launch_mode(const RenderCall& c, const Source& src, const TreeIndex& index) {
-    if (c.backward) return launch_march<BD, kModeBackward>(c, src, index);
-    if (c.log != nullptr) return launch_march<BD, kModeForwardLogged>(c, src, index);
-    return launch_march<BD, kModeForward>(c, src, index);
+    LogArgs log;
+    if (c.backward) {
+        log.log = const_cast<int32_t*>(c.gate.log);
+        log.capacity = c.gate.capacity;
+        return launch_march<BD, kModeBackward, kMarchBlock>(c, src, index, log);
+    }
+    if (c.log == nullptr) return launch_march<BD, kModeForward, kMarchBlock>(c, src, index, log);
+    log.log = c.log;
+    log.capacity = c.log_capacity;
+    log.shift = replay_bin_shift(c.tree->M, c.tree->K);
+    if (!sorts_log(c.tree, c.Q, Source::kImage, c.log_capacity))
+        return launch_march<BD, kModeForwardLogged, kMarchBlock>(c, src, index, log);
+    log.n_bins = replay_bins(c.tree->M, c.tree->K);
+    const int st = launch_march<BD, kModeForwardLogged, sorted_march_block<BD>()>(c, src, index, log);
+    if (st) return st;
+    int32_t* cursor = c.log + log_words(c.log_capacity) - kMaxBins;
+    SVOXB_CUDA(cudaMemsetAsync(cursor, 0, kMaxBins * sizeof(int32_t), c.stream));
+    order_groups_kernel<<<index_grid(c.log_capacity / kSortedChunks, kOrderTile, sm_count()), 256,
+                          0, c.stream>>>(c.log, c.log_capacity, cursor);
+    SVOXB_CUDA(cudaGetLastError());
+    return SVOXB_OK;
 }
 
-// Replay backward (render_replay.cuh): prefix, pack, bin, then the scatter in one
-// or several parts (bin ranges).  A ReplayJob holds the scratch between the calls.
+// Replay backward (render_replay.cuh) in one or several parts (bin ranges).
 struct ReplayJob {
-    ReplayBins bins{};
-    int32_t* base = nullptr;     // pool allocation
-    const int32_t* log = nullptr;
+    int32_t* log = nullptr;
+    int64_t capacity = 0;
+    int64_t chunks = 0;          // at most this many are in the log
     svoxb_render_options opt{};
-    TreeArgs lobes{};            // for the lobe parameters of an SG / ASG basis
-    int64_t n_slots = 0, n_rays = 0, chunks = 0;
-    int K = 0, n_parts = 1, shift = 0, n_bins = 1;
-    bool hess = false;   // Gauss-Newton diagonal instead of the gradient
+    TreeArgs tree{};
+    ScatterOut to{};
+    int64_t n_slots = 0;
+    int n_parts = 1, shift = 0, n_bins = 1;
 };
 
-// Prefix + pack + bin.  SVOXB_ERR_TOO_LARGE when the packet buffer cannot be had
-// (the caller then marches instead).
-template <class Source>
-static int replay_begin(const RenderCall& c, const Source& src, int64_t chunks, int n_parts,
-                        ReplayJob* job, bool hess = false) {
-    if (chunks > c.log_capacity) chunks = c.log_capacity;
+static int replay_job(const RenderCall& c, int64_t chunks, int n_parts, ReplayJob* job) {
     if (n_parts < 1 || n_parts > kMaxParts) return SVOXB_ERR_OPTION;
-    const int64_t packets = (chunks > 0 ? chunks : 1) * 32;
-    if (packets >= (1LL << 30)) return SVOXB_ERR_TOO_LARGE;
-
-    int st = keep_pool_cached();
-    if (st) return st;
-    // cursors | offsets | work counters | packed rays | packets
-    const size_t head_words =
-        (size_t)kMaxBins * kCursorStride + kMaxBins + 8 + 2 * kMaxParts;  // 32-byte multiple
-    const size_t ray_words = (size_t)c.Q * 12;
-    const size_t pad = (8 - (head_words + ray_words) % 8) % 8;
-    int32_t* base = nullptr;
-    if (cudaMallocAsync((void**)&base,
-                        (head_words + ray_words + pad + 8 * (size_t)packets) * sizeof(int32_t),
-                        c.stream) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return SVOXB_ERR_TOO_LARGE;
-    }
-    ReplayBins& b = job->bins;
-    b.cursor = base;
-    b.offset = base + (size_t)kMaxBins * kCursorStride;
-    b.work = reinterpret_cast<int64_t*>(b.offset + kMaxBins + 2);  // 8-byte aligned
-    float4* rays = reinterpret_cast<float4*>(base + head_words);
-    b.rays = rays;
-    b.capacity = packets;
-    b.packet = reinterpret_cast<int4*>(base + head_words + ray_words + pad);
-    job->base = base;
     job->log = c.log;
+    job->capacity = c.log_capacity;
+    job->chunks = chunks > c.log_capacity ? c.log_capacity : chunks;
     job->opt = c.opt;
-    job->lobes = tree_args(c.tree);
+    job->tree = tree_args(c.tree);
+    job->to = ScatterOut{c.grad_data, nullptr, c.grad_out, c.fwd_out, 0};
     job->n_slots = c.tree->M * 8;
-    job->n_rays = c.Q;
-    job->chunks = chunks;
-    job->K = c.tree->K;
     job->n_parts = n_parts;
-    job->hess = hess;
     job->shift = replay_bin_shift(c.tree->M, c.tree->K);
-    job->n_bins = (int)(((job->n_slots - 1) >> job->shift) + 1);
-
-    replay_prefix_kernel<<<1, 256, 0, c.stream>>>(c.log, b, n_parts, c.log_capacity);
-    if (chunks > 0) {
-        replay_pack_rays_kernel<<<(unsigned)((c.Q + 255) / 256), 256, 0, c.stream>>>(
-            tree_args(c.tree), src, c.opt, c.grad_out, c.fwd_out, c.Q, rays);
-        unsigned grid = 1;
-        auto run_bin = [&](auto k, int block) {
-            int s2 = persistent_grid(k, block, 0, chunks, &grid);
-            if (s2 == SVOXB_OK)
-                k<<<grid, block, 0, c.stream>>>(c.opt, c.log, chunks, c.log_capacity, c.Q, b,
-                                                c.tree->data, c.tree->K);
-            return s2;
-        };
-        st = hess ? run_bin(replay_bin_kernel<128, 2, 12, true>, 128)
-                  : run_bin(replay_bin_kernel<128, 2, 12, false>, 128);
-    }
-    const cudaError_t e = cudaGetLastError();
-    if (st == SVOXB_OK && e != cudaSuccess) st = set_cuda_error(e);
-    if (st != SVOXB_OK) {
-        cudaFreeAsync(base, c.stream);
-        job->base = nullptr;
-    }
-    return st;
+    job->n_bins = replay_bins(c.tree->M, c.tree->K);
+    return SVOXB_OK;
 }
 
-// Scatter of one part.  With `reserve_sms` > 0 that many SMs are left without a block
-// (for a collective that runs beside the scatter); small records then use one 1024-thread
-// block per SM, so that the SMs left out are really empty.
-template <int BD, int BLOCK, bool HESS, bool LOBES = false>
-static int replay_scatter_block(const ReplayJob& job, int part, float* grad, int reserve_sms,
+// Scatter of one part.  With `reserve_sms` > 0 that many SMs are left without a block (for a
+// collective that runs beside the scatter); one 1024-thread block per SM then, so that the SMs
+// left out are really empty.
+template <int BD, int BLOCK, bool HESS, bool LOBES>
+static int replay_scatter_block(const ReplayJob& job, int part, int reserve_sms,
                                 cudaStream_t stream) {
     constexpr int K = RecordLength<BD>::K;
-    const size_t smem = (size_t)(BLOCK / 32) * sizeof(ScatterSmem<K>);
+    const size_t smem = (size_t)(BLOCK / 32) * sizeof(ScatterSmem<K, HESS ? 2 : 1>);
     auto k = replay_scatter_kernel<BD, BLOCK, HESS, LOBES>;
     unsigned grid = 1;
     int st = persistent_grid(k, BLOCK, smem, job.chunks, &grid);
@@ -292,44 +268,35 @@ static int replay_scatter_block(const ReplayJob& job, int part, float* grad, int
         const int64_t most = ((int64_t)sms - reserve_sms) * per_sm;
         if ((int64_t)grid > most) grid = (unsigned)(most > 1 ? most : 1);
     }
-    k<<<grid, BLOCK, smem, stream>>>(job.n_slots, job.opt, job.lobes, grad, job.log, job.bins,
-                                    part, job.n_parts);
+    k<<<grid, BLOCK, smem, stream>>>(job.tree, job.opt, job.log, job.capacity, job.to, part,
+                                    job.n_parts);
     const cudaError_t e = cudaGetLastError();
     return e != cudaSuccess ? set_cuda_error(e) : SVOXB_OK;
 }
 
-template <int BD>
-static int replay_scatter_bd(const ReplayJob& job, int part, float* grad, int reserve_sms,
+template <int BD, bool LOBES>
+static int replay_scatter_bd(const ReplayJob& job, int part, int reserve_sms,
                              cudaStream_t stream) {
-    if constexpr (BD > 0) {
-        if (job.opt.format != SVOXB_FORMAT_SH)
-            return job.hess
-                       ? replay_scatter_block<BD, 512, true, true>(job, part, grad, 0, stream)
-                       : replay_scatter_block<BD, 512, false, true>(job, part, grad, reserve_sms,
-                                                                    stream);
-    }
-    if (job.hess) return replay_scatter_block<BD, 512, true>(job, part, grad, 0, stream);
-    if constexpr (BD <= 9) {
+    if (job.to.hess != nullptr)
+        return replay_scatter_block<BD, kScatterBlock, true, LOBES>(job, part, 0, stream);
+    if constexpr (BD <= 9 && !LOBES) {
         if (reserve_sms > 0)
-            return replay_scatter_block<BD, 1024, false>(job, part, grad, reserve_sms, stream);
+            return replay_scatter_block<BD, 1024, false, LOBES>(job, part, reserve_sms, stream);
     }
-    // 256-thread blocks: measured 2.83 ms of backward per training step against 2.94 with 512
-    // (more, smaller blocks keep the window of packets in flight narrower)
-    return replay_scatter_block<BD, 256, false>(job, part, grad, reserve_sms, stream);
+    return replay_scatter_block<BD, kScatterBlock, false, LOBES>(job, part, reserve_sms, stream);
 }
 
-static int replay_scatter(const ReplayJob& job, int part, float* grad, int reserve_sms,
-                          cudaStream_t stream) {
+static int replay_scatter(const ReplayJob& job, int part, int reserve_sms, cudaStream_t stream) {
     if (part < 0 || part >= job.n_parts) return SVOXB_ERR_OPTION;
     if (job.chunks < 1) return SVOXB_OK;
     return with_basis(job.opt, [&](auto basis) {
-        return replay_scatter_bd<decltype(basis)::value>(job, part, grad, reserve_sms, stream);
+        constexpr int BD = decltype(basis)::value;
+        if constexpr (BD > 0) {
+            if (job.opt.format != SVOXB_FORMAT_SH)
+                return replay_scatter_bd<BD, true>(job, part, reserve_sms, stream);
+        }
+        return replay_scatter_bd<BD, false>(job, part, reserve_sms, stream);
     });
-}
-
-static void replay_end(ReplayJob* job, cudaStream_t stream) {
-    if (job->base) cudaFreeAsync(job->base, stream);
-    job->base = nullptr;
 }
 
 // The index of one call (render_index.cuh): a pool allocation, freed on the stream.
@@ -356,13 +323,17 @@ static int launch_queue(const RenderCall& c, const Source& src) {
     const IndexLayout layout = QueueScratch::layout(c.tree);
     QueueScratch scratch;
     const int32_t* mem = c.prepared;
-    if (mem == nullptr || c.backward) {
+    if (c.gate.log != nullptr) {
+        // the fallback of a replay hardly ever runs: one launch that walks the tree itself
+        mem = nullptr;
+    } else if (mem == nullptr || c.backward) {
         const int st = scratch.build(c.tree, layout, c.backward ? 0.f : c.opt.sigma_thresh,
                                      c.opt.density_softplus, c.gate, c.stream);
         if (st) return st;
         mem = scratch.mem;
     }
-    const TreeIndex index = layout.view(mem);
+    TreeIndex index = layout.view(mem);
+    if (mem == nullptr) index = TreeIndex{nullptr, 0, 0, 1};
     return with_basis(c.opt, [&](auto basis) {
         constexpr int BD = decltype(basis)::value;
         if constexpr (BD > 0) {
@@ -648,7 +619,7 @@ static int logged_forward(const svoxb_tree* tree, const Source& src, int64_t Q,
     if ((st = log_eligible(tree, opt, nullptr))) return st;
     if (!log || capacity_chunks < 1 || Q < 0) return SVOXB_ERR_SHAPE;
     if (Q > 0 && !out) return SVOXB_ERR_NULL;
-    SVOXB_CUDA(cudaMemsetAsync(log, 0, kLogChunks * sizeof(int32_t), (cudaStream_t)stream));
+    SVOXB_CUDA(cudaMemsetAsync(log, 0, kLogCounts * sizeof(int32_t), (cudaStream_t)stream));
     if (Q == 0) return SVOXB_OK;
     RenderCall c{tree, *opt, Q};
     c.out = out;
@@ -658,21 +629,29 @@ static int logged_forward(const svoxb_tree* tree, const Source& src, int64_t Q,
     return launch_queue(c, src);
 }
 
+// Gradient (`grad_data_out`) and / or Gauss-Newton diagonal (`hess_out`) from the log.
 template <class Source>
 static int replay_backward(const svoxb_tree* tree, const Source& src, int64_t Q,
                            const svoxb_render_options* opt, const float* grad_output,
                            const float* fwd_out, int32_t* log, int64_t capacity_chunks,
-                           int64_t chunks_used, float* grad_data_out, int zero_first,
-                           void* stream, bool hess = false) {
+                           int64_t chunks_used, float* grad_data_out, float* hess_out,
+                           int zero_first, void* stream) {
     int st = validate_tree(tree);
     if (st) return st;
     if ((st = validate_options(tree, *opt))) return st;
-    if (!grad_data_out || !log) return SVOXB_ERR_NULL;
-    if ((st = log_eligible(tree, opt, grad_data_out))) return st;
-    if (zero_first && (st = zero_grad(tree, grad_data_out, tree->K, (cudaStream_t)stream)))
-        return st;
+    if ((!grad_data_out && !hess_out) || !log) return SVOXB_ERR_NULL;
+    // a sorted log's scatter clears its outputs itself
+    bool clears = zero_first && Q > 0 && sorts_log(tree, Q, Source::kImage, capacity_chunks);
+    for (float* out : {grad_data_out, hess_out}) clears = clears && (uintptr_t)out % 16 == 0;
+    for (float* out : {grad_data_out, hess_out}) {
+        if (!out) continue;
+        if ((st = log_eligible(tree, opt, out))) return st;
+        if (zero_first && !clears &&
+            (st = zero_grad(tree, out, tree->K, (cudaStream_t)stream)))
+            return st;
+    }
     if (Q == 0) return SVOXB_OK;
-    if ((!hess && !grad_output) || !fwd_out) return SVOXB_ERR_NULL;
+    if ((grad_data_out && !grad_output) || !fwd_out) return SVOXB_ERR_NULL;
     RenderCall c{tree, *opt, Q};
     c.backward = true;
     c.grad_out = grad_output;
@@ -682,33 +661,37 @@ static int replay_backward(const svoxb_tree* tree, const Source& src, int64_t Q,
     c.log = log;
     c.log_capacity = capacity_chunks;
     // chunks_used > 0: the caller has read the count (svoxb_item_log_used) and vouches that
-    // the log did not overflow.  Otherwise the count stays on the device: the scratch is sized
-    // for the whole log, the kernels read the count themselves, and a marching backward is
-    // enqueued behind them that does its work only if the log overflowed.
+    // the log did not overflow.  Otherwise the count stays on the device: the kernel reads it
+    // itself, and a march enqueued behind it does its work only if the log overflowed.
     const bool known = chunks_used > 0 && chunks_used <= capacity_chunks;
-    if (hess && !known) return SVOXB_ERR_OPTION;
+    if (hess_out && !grad_data_out && !known) return SVOXB_ERR_OPTION;
     ReplayJob job;
-    st = replay_begin(c, src, known ? chunks_used : capacity_chunks, 1, &job, hess);
-    if (st == SVOXB_OK) {
-        st = replay_scatter(job, 0, grad_data_out, 0, c.stream);
-        replay_end(&job, c.stream);
-    }
-    if (hess) return st;
-    RenderCall march = c;
-    march.log = nullptr;
-    march.log_capacity = 0;
-    if (st == SVOXB_ERR_TOO_LARGE) return render_dispatch(march, src);  // no room for packets
-    if (st == SVOXB_OK && !known) {
-        march.gate = LogGate{log, capacity_chunks};
-        st = render_dispatch(march, src);
-    }
-    return st;
+    if ((st = replay_job(c, known ? chunks_used : capacity_chunks, 1, &job))) return st;
+    job.to.hess = hess_out;
+    if (clears) job.to.zero_slots = job.n_slots;
+    if ((st = replay_scatter(job, 0, 0, c.stream)) || known) return st;
+    c.log = nullptr;
+    c.gate = LogGate{log, capacity_chunks};
+    if (!hess_out) return render_dispatch(c, src);
+    auto k = render_se_grad_generic<256, Source>;
+    unsigned grid = 1;
+    if ((st = persistent_grid(k, 256, 0, (Q + 31) / 32, &grid))) return st;
+    k<<<grid, 256, 0, c.stream>>>(tree_args(tree), src, *opt, TopTable{nullptr, 0}, false, fwd_out,
+                                  nullptr, grad_output, grad_data_out, hess_out, Q, 3, c.gate);
+    SVOXB_CUDA(cudaGetLastError());
+    return SVOXB_OK;
 }
 
 extern "C" {
 
+int svoxb_log_is_sorted(const svoxb_tree* tree, int64_t n_rays, int image,
+                        int64_t capacity_chunks) {
+    if (!tree || tree->M < 1 || tree->K < 1) return 0;
+    return sorts_log(tree, n_rays, image != 0, capacity_chunks) ? 1 : 0;
+}
+
 int64_t svoxb_item_log_words(int64_t capacity_chunks) {
-    return (int64_t)kLogChunks + capacity_chunks * kLogChunkWords;
+    return log_words(capacity_chunks);
 }
 
 int svoxb_volume_render_logged(const svoxb_tree* tree, const svoxb_rays* rays,
@@ -740,7 +723,7 @@ int svoxb_volume_render_backward_replay(const svoxb_tree* tree, const svoxb_rays
     if (rays->Q > 0 && (!rays->origins || !rays->dirs || !rays->vdirs)) return SVOXB_ERR_NULL;
     return replay_backward(tree, RayBatch{rays->origins, rays->dirs, rays->vdirs}, rays->Q, opt,
                            grad_output, fwd_out, log, capacity_chunks, chunks_used, grad_data_out,
-                           zero_first, stream);
+                           nullptr, zero_first, stream);
 }
 
 int svoxb_volume_render_image_backward_replay(const svoxb_tree* tree, const svoxb_camera* cam,
@@ -753,7 +736,8 @@ int svoxb_volume_render_image_backward_replay(const svoxb_tree* tree, const svox
     if (cam->width < 0 || cam->height < 0) return SVOXB_ERR_SHAPE;
     return replay_backward(tree, PixelRays{cam->c2w, cam->fx, cam->fy, cam->width, cam->height},
                            (int64_t)cam->width * cam->height, opt, grad_output, fwd_out, log,
-                           capacity_chunks, chunks_used, grad_data_out, zero_first, stream);
+                           capacity_chunks, chunks_used, grad_data_out, nullptr, zero_first,
+                           stream);
 }
 
 /* Gauss-Newton diagonal of the squared error from the item log (the third result of the
@@ -766,8 +750,8 @@ int svoxb_volume_render_hessdiag_replay(const svoxb_tree* tree, const svoxb_rays
     if (!tree || !rays || !opt) return SVOXB_ERR_NULL;
     if (rays->Q > 0 && (!rays->origins || !rays->dirs || !rays->vdirs)) return SVOXB_ERR_NULL;
     return replay_backward(tree, RayBatch{rays->origins, rays->dirs, rays->vdirs}, rays->Q, opt,
-                           nullptr, fwd_out, log, capacity_chunks, chunks_used, hessdiag_out,
-                           zero_first, stream, true);
+                           nullptr, fwd_out, log, capacity_chunks, chunks_used, nullptr,
+                           hessdiag_out, zero_first, stream);
 }
 
 int svoxb_volume_render_image_hessdiag_replay(const svoxb_tree* tree, const svoxb_camera* cam,
@@ -780,7 +764,35 @@ int svoxb_volume_render_image_hessdiag_replay(const svoxb_tree* tree, const svox
     if (cam->width < 0 || cam->height < 0) return SVOXB_ERR_SHAPE;
     return replay_backward(tree, PixelRays{cam->c2w, cam->fx, cam->fy, cam->width, cam->height},
                            (int64_t)cam->width * cam->height, opt, nullptr, fwd_out, log,
-                           capacity_chunks, chunks_used, hessdiag_out, zero_first, stream, true);
+                           capacity_chunks, chunks_used, nullptr, hessdiag_out, zero_first,
+                           stream);
+}
+
+/* Both at once: the packets are read once. */
+int svoxb_se_grad_replay(const svoxb_tree* tree, const svoxb_rays* rays,
+                         const svoxb_render_options* opt, const float* residual,
+                         const float* fwd_out, int32_t* log, int64_t capacity_chunks,
+                         int64_t chunks_used, float* grad_data_out, float* hessdiag_out,
+                         int zero_first, void* stream) {
+    if (!tree || !rays || !opt || !grad_data_out || !hessdiag_out) return SVOXB_ERR_NULL;
+    if (rays->Q > 0 && (!rays->origins || !rays->dirs || !rays->vdirs)) return SVOXB_ERR_NULL;
+    return replay_backward(tree, RayBatch{rays->origins, rays->dirs, rays->vdirs}, rays->Q, opt,
+                           residual, fwd_out, log, capacity_chunks, chunks_used, grad_data_out,
+                           hessdiag_out, zero_first, stream);
+}
+
+int svoxb_se_grad_image_replay(const svoxb_tree* tree, const svoxb_camera* cam,
+                               const svoxb_render_options* opt, const float* residual,
+                               const float* fwd_out, int32_t* log, int64_t capacity_chunks,
+                               int64_t chunks_used, float* grad_data_out, float* hessdiag_out,
+                               int zero_first, void* stream) {
+    if (!tree || !cam || !opt || !cam->c2w || !grad_data_out || !hessdiag_out)
+        return SVOXB_ERR_NULL;
+    if (cam->width < 0 || cam->height < 0) return SVOXB_ERR_SHAPE;
+    return replay_backward(tree, PixelRays{cam->c2w, cam->fx, cam->fy, cam->width, cam->height},
+                           (int64_t)cam->width * cam->height, opt, residual, fwd_out, log,
+                           capacity_chunks, chunks_used, grad_data_out, hessdiag_out, zero_first,
+                           stream);
 }
 
 }  // extern "C"
@@ -815,8 +827,8 @@ static int se_grad_march(const svoxb_tree* tree, const Source& src, int64_t Q,
     auto run = [&](auto k, int block) {
         int s2 = persistent_grid(k, block, smem, n_gran, &grid);
         if (s2) return s2;
-        k<<<grid, block, smem, stream>>>(tr, src, *opt, top, in_smem, fwd_out, color_ref, grad,
-                                        hess, Q, od);
+        k<<<grid, block, smem, stream>>>(tr, src, *opt, top, in_smem, fwd_out, color_ref, nullptr,
+                                        grad, hess, Q, od, LogGate{});
         const cudaError_t e = cudaGetLastError();
         return e != cudaSuccess ? set_cuda_error(e) : (int)SVOXB_OK;
     };
@@ -867,6 +879,7 @@ static int replay_begin_checked(const svoxb_tree* tree, const Source& src, int64
     c.backward = true;
     c.grad_out = grad_output;
     c.fwd_out = fwd_out;
+    c.grad_data = grad_data_out;
     c.stream = (cudaStream_t)stream;
     c.log = log;
     c.log_capacity = capacity_chunks;
@@ -875,18 +888,14 @@ static int replay_begin_checked(const svoxb_tree* tree, const Source& src, int64
     if (Q == 0) chunks_used = 0;
     ReplayJob* job = new (std::nothrow) ReplayJob;
     if (!job) return SVOXB_ERR_TOO_LARGE;
-    st = replay_begin(c, src, chunks_used, n_parts, job);
+    st = replay_job(c, chunks_used, n_parts, job);
     if (st == SVOXB_OK && !known && Q > 0) {
         // the fallback for an overflowed log goes BEFORE the parts: if it runs, it produces the
         // whole gradient and the parts add nothing, so every part's rows are final when the
         // caller hands them on, whichever of the two happened
-        RenderCall march = c;
-        march.grad_data = grad_data_out;
-        march.log = nullptr;
-        march.log_capacity = 0;
-        march.gate = LogGate{log, capacity_chunks};
-        st = render_dispatch(march, src);
-        if (st != SVOXB_OK) replay_end(job, c.stream);
+        c.log = nullptr;
+        c.gate = LogGate{log, capacity_chunks};
+        st = render_dispatch(c, src);
     }
     if (st != SVOXB_OK) {
         delete job;
@@ -943,16 +952,15 @@ int svoxb_replay_part_range(const void* job, int part, int64_t* slot_begin, int6
 int svoxb_replay_scatter(const void* job, int part, float* grad_data_out, int reserve_sms,
                          void* stream) {
     if (!job || !grad_data_out) return SVOXB_ERR_NULL;
-    const ReplayJob* j = static_cast<const ReplayJob*>(job);
-    if (j->K % 4 == 0 && (uintptr_t)grad_data_out % 16 != 0) return SVOXB_ERR_FORMAT;
-    return replay_scatter(*j, part, grad_data_out, reserve_sms, (cudaStream_t)stream);
+    ReplayJob j = *static_cast<const ReplayJob*>(job);
+    if (j.tree.K % 4 == 0 && (uintptr_t)grad_data_out % 16 != 0) return SVOXB_ERR_FORMAT;
+    j.to.grad = grad_data_out;
+    return replay_scatter(j, part, reserve_sms, (cudaStream_t)stream);
 }
 
-int svoxb_replay_end(void* job, void* stream) {
+int svoxb_replay_end(void* job, void*) {
     if (!job) return SVOXB_ERR_NULL;
-    ReplayJob* j = static_cast<ReplayJob*>(job);
-    replay_end(j, (cudaStream_t)stream);
-    delete j;
+    delete static_cast<ReplayJob*>(job);
     return SVOXB_OK;
 }
 

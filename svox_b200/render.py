@@ -114,10 +114,13 @@ def _forward(ctx, data, tree, src, opt, prepared, train, image):
     log = None
     ctx.grad_buffer = None
     if train and USE_ITEM_LOG and _C.log_eligible(tree, opt):
-        # training step: record the contributing samples for the backward pass, and clear the
-        # gradient buffer the backward will add into on a second stream meanwhile (the march
-        # leaves a third of the memory bandwidth unused)
-        ctx.grad_buffer = _zeroed_beside(tree.data)
+        # training step: record the contributing samples for the backward pass, and unless the
+        # backward does it on the way clear the gradient buffer it will add into on a second
+        # stream meanwhile (the march leaves memory bandwidth unused)
+        n = src.width * src.height if image else src.origins.shape[0]
+        if GRAD_PARTS is not None or GRAD_BUFFER is not None or \
+                not _C.log_is_sorted(tree, n, image):
+            ctx.grad_buffer = _zeroed_beside(tree.data)
         out, (log, ctx.log_capacity) = _C.volume_render_logged(tree, src, opt, image=image)
     elif image:
         out = _C.volume_render_image(tree, src, opt, prepared=prepared)
@@ -302,19 +305,20 @@ class VolumeRenderer(nn.Module):
                                               colors.reshape(out.shape).contiguous(),
                                               image=image)
                 return out, grad, hess
-            for _ in range(4):      # a log that was too small is enlarged and the render redone
-                out, log = _C.volume_render_logged(tree, src, opt, image=image)
-                used = _C.log_chunks_used(log[0])
-                _C.log_estimate(wait=True)
-                if used > log[1]:
-                    continue
-                resid = (out - colors.reshape(out.shape)).contiguous()
-                grad = _C.volume_render_backward_replay(tree, src, opt, resid, out, log,
-                                                        image=image, used=max(used, 1))
-                hess = _C.volume_render_hessdiag_replay(tree, src, opt, out, log, max(used, 1),
-                                                        image=image)
-                return out, grad, hess
-        raise RuntimeError("se_grad: the item log kept overflowing")
+            data = self.tree.data
+            grad, hess = (torch.empty_like(data, memory_format=torch.contiguous_format)
+                          for _ in range(2))
+            n = src.width * src.height if image else src.origins.shape[0]
+            # unless the replay does it on the way, both results are cleared beside the forward
+            zeroed = [] if _C.log_is_sorted(tree, n, image) else \
+                [_C.zero_beside(x) for x in (grad, hess)]
+            out, log = _C.volume_render_logged(tree, src, opt, image=image)
+            resid = (out - colors.reshape(out.shape)).contiguous()
+            for done in zeroed:
+                torch.cuda.current_stream(data.device).wait_event(done)
+            _C.se_grad_replay(tree, src, opt, resid, out, log, grad, hess, bool(zeroed),
+                              image=image)
+            return out, grad, hess
 
     @staticmethod
     def persp_rays(c2w, width=800, height=800, fx=1111.111, fy=None):
