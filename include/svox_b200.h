@@ -324,6 +324,11 @@ int svoxb_replay_end(void* job, void* stream);
  * capacity means that it overflowed. */
 int svoxb_item_log_used(const int32_t* log, int64_t* chunks_used, void* stream);
 
+/* Enqueues the copy of {chunks asked for, samples} of a log into two int32 of
+ * pinned host memory, for a caller that sizes its next log by them and looks
+ * later whether they have arrived. */
+int svoxb_item_log_watch(const int32_t* log, int32_t* counts, void* stream);
+
 /* Forward ray render that allocates nothing (no counterpart in the
  * reference).  Same inputs, outputs and results as svoxb_volume_render, for
  * hosts that may not touch a device allocator while rendering: an application

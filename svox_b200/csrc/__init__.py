@@ -4,7 +4,7 @@ Same spec classes (``TreeSpec``, ``RaysSpec``, ``CameraSpec``,
 ``RenderOptions``) and the same functions with the same arguments and
 results as the reference's pybind11 module (svox/csrc/svox.cpp:63-122), but
 implemented by the C-ABI library ``libsvox_b200.so`` (hand-written sm_100a
-kernels) loaded with ctypes.  Tensors are allocated by PyTorch and handed to
+kernels) loaded with ctypes; the hot calls go through the extension ``_host``.  Tensors are allocated by PyTorch and handed to
 the library as raw device pointers together with the current CUDA stream.
 
 There is no CPU implementation: if the library is missing or a tensor is
@@ -66,7 +66,7 @@ class TreeSpec:
         counter does not see (``tree[...] = v`` writes through ``data.data``); -1 without
         an owner."""
         tree = self._owner() if self._owner is not None else None
-        return tree._data_epoch if tree is not None else -1
+        return int(tree._data_epoch) if tree is not None else -1
 
 
 class RaysSpec:
@@ -124,8 +124,27 @@ def library():
     return _lib
 
 
+_extension = None
+
+
+def host():
+    """The Python extension that makes the hot calls (host.cpp), bound to ``library()``."""
+    global _extension
+    if _extension is None:
+        library()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError(
+                "svox_b200: the host extension is missing or does not load; build it with "
+                f"`python -m svox_b200.csrc.build` ({e})") from e
+        module.load(LIB_PATH)
+        _extension = module
+    return _extension
+
+
 def is_built():
-    return os.path.exists(LIB_PATH)
+    return os.path.exists(LIB_PATH) and os.path.exists(os.path.join(_HERE, "_host.so"))
 
 
 def _raise(status, what):
@@ -250,19 +269,7 @@ def _check_indices(indices):
 
 def query_vertical(tree, indices):
     """-> (values (Q, K) float32, node_ids (Q,) int64); svox_kernel.cu:120-143."""
-    lib = library()
-    ct = _pack_tree(tree)
-    _check_indices(indices)
-    with torch.cuda.device(indices.device):
-        Q = indices.shape[0]
-        values = torch.empty((Q, ct.K), dtype=indices.dtype, device=indices.device)
-        node_ids = torch.empty((Q,), dtype=torch.int64, device=tree.child.device)
-        st = lib.svoxb_query_vertical(C.byref(ct), C.c_void_p(indices.data_ptr()), C.c_int64(Q),
-                                      C.c_void_p(values.data_ptr()),
-                                      C.c_void_p(node_ids.data_ptr()), _stream())
-    if st:
-        _raise(st, "query_vertical")
-    return values, node_ids
+    return host().query_vertical(tree, indices)
 
 
 _side_streams = {}
@@ -301,29 +308,7 @@ def _is_symmetric(buf):
 def query_vertical_backward(tree, indices, grad_output, zeroed=None):
     """-> gradient w.r.t. data, (M, N, N, N, Kg); svox_kernel.cu:160-182.  ``zeroed``: a zero
     tensor of that shape to add the rows into (else one is made and cleared here)."""
-    lib = library()
-    ct = _pack_tree(tree)
-    _check_indices(indices)
-    _check_input(grad_output, "grad_output")
-    Q = indices.shape[0]
-    if grad_output.dim() != 2 or grad_output.shape[0] != Q:
-        raise RuntimeError("grad_output must be (Q, K)")
-    Kg = grad_output.shape[1]
-    with torch.cuda.device(indices.device):
-        shape = (ct.M, ct.N, ct.N, ct.N, Kg)
-        if zeroed is not None:
-            _check_input(zeroed, "zeroed")
-            if tuple(zeroed.shape) != shape:
-                raise RuntimeError("zeroed must be (M, N, N, N, Kg)")
-        grad = zeroed if zeroed is not None else \
-            torch.empty(shape, dtype=grad_output.dtype, device=grad_output.device)
-        st = lib.svoxb_query_vertical_backward(
-            C.byref(ct), C.c_void_p(indices.data_ptr()), C.c_int64(Q),
-            C.c_void_p(grad_output.data_ptr()), C.c_int32(Kg), C.c_void_p(grad.data_ptr()),
-            C.c_int(0 if zeroed is not None else 1), _stream())
-    if st:
-        _raise(st, "query_vertical_backward")
-    return grad
+    return host().query_vertical_backward(tree, indices, grad_output, zeroed)
 
 
 def assign_vertical(tree, indices, values):
@@ -394,46 +379,14 @@ def render_scratch(tree, opt):
 def volume_render(tree, rays, opt, prepared=None):
     """-> (Q, out_dim); svox/csrc/rt_kernel.cu:1019-1036.  ``prepared``: a tensor from
     ``render_scratch`` for the same tree and options (skips the per-call index build)."""
-    lib = library()
-    ct = _pack_tree(tree)
-    cr = _pack_rays(rays, tree.data.device)
-    co = opt._pack()
-    with torch.cuda.device(tree.data.device):
-        out = torch.empty((cr.Q, _out_dim(opt, ct.K)), dtype=torch.float32,
-                          device=tree.data.device)
-        with _timed("volume_render"):
-            if prepared is not None:
-                st = lib.svoxb_volume_render_prepared(
-                    C.byref(ct), C.byref(cr), C.byref(co), C.c_void_p(prepared.data_ptr()),
-                    C.c_void_p(out.data_ptr()), _stream())
-            else:
-                st = lib.svoxb_volume_render(C.byref(ct), C.byref(cr), C.byref(co),
-                                             C.c_void_p(out.data_ptr()), _stream())
-    if st:
-        _raise(st, "volume_render")
-    return out
+    with _timed("volume_render"):
+        return host().volume_render(tree, rays, opt, False, prepared)
 
 
 def volume_render_image(tree, cam, opt, prepared=None):
     """-> (height, width, out_dim); svox/csrc/rt_kernel.cu:1038-1057.  ``prepared`` as for
     ``volume_render``."""
-    lib = library()
-    ct = _pack_tree(tree)
-    cc = _pack_camera(cam, tree.data.device)
-    co = opt._pack()
-    with torch.cuda.device(tree.data.device):
-        out = torch.empty((cc.height, cc.width, _out_dim(opt, ct.K)), dtype=torch.float32,
-                          device=tree.data.device)
-        if prepared is not None:
-            st = lib.svoxb_volume_render_image_prepared(
-                C.byref(ct), C.byref(cc), C.byref(co), C.c_void_p(prepared.data_ptr()),
-                C.c_void_p(out.data_ptr()), _stream())
-        else:
-            st = lib.svoxb_volume_render_image(C.byref(ct), C.byref(cc), C.byref(co),
-                                               C.c_void_p(out.data_ptr()), _stream())
-    if st:
-        _raise(st, "volume_render_image")
-    return out
+    return host().volume_render(tree, cam, opt, True, prepared)
 
 
 # ---------------------------------------------------------------------------
@@ -441,65 +394,33 @@ def volume_render_image(tree, cam, opt, prepared=None):
 
 _LOG_SLACK_CHUNKS = 2 * 16384   # chunks the forward's warps take and leave partly empty
 _items_per_ray = 80.0           # running estimate used to size the item log
-_WATCH_SLOTS = 8
 
 
 class _LogWatch:
     """Learns how large the item log has to be WITHOUT making the host wait for the device.
 
-    After a logged forward the number of chunks it asked for is copied to pinned host
-    memory, asynchronously; whenever the next log is sized, the counts that have arrived by
-    then adapt the per-ray estimate.  A log that was too small costs that one step a marching
-    backward (decided on the device, see ``volume_render_backward_replay``), never a wrong
-    gradient."""
-    slots = {}     # device -> [pinned int32 ring, next slot, pending [(slot, event, rays, cap)]]
+    After a logged forward the number of chunks it asked for and of samples it wrote are copied
+    to pinned host memory, asynchronously (host.cpp); whenever the next log is sized, the counts
+    that have arrived by then adapt the per-ray estimate.  A log that was too small costs that
+    one step a marching backward (decided on the device, see ``volume_render_backward_replay``),
+    never a wrong gradient."""
+    last_used = last_cap = 0
 
     @classmethod
-    def _state(cls, device):
-        st = cls.slots.get(device)
-        if st is None:
-            st = [torch.zeros((_WATCH_SLOTS, 2), dtype=torch.int32).pin_memory(), 0, []]
-            cls.slots[device] = st
-        return st
-
-    @classmethod
-    def watch(cls, log, cap, n_rays):
-        st = cls._state(log.device)
-        pending = st[2]
-        if len(pending) >= _WATCH_SLOTS:           # nobody has polled for a while
-            cls.poll(log.device, wait=True)
-        slot = st[1]
-        st[1] = (slot + 1) % _WATCH_SLOTS
-        st[0][slot].copy_(log[:2], non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record()
-        pending.append((slot, ev, n_rays, cap))
-
-    @classmethod
-    def poll(cls, device=None, wait=False):
+    def poll(cls, wait=False):
         """Fold the counts that have arrived into the estimate; ``wait`` blocks for all."""
         global _items_per_ray
-        for dev, st in cls.slots.items():
-            if device is not None and dev != device:
-                continue
-            keep = []
-            for slot, ev, n_rays, cap in st[2]:
-                if wait:
-                    ev.synchronize()
-                elif not ev.query():
-                    keep.append((slot, ev, n_rays, cap))
-                    continue
-                used, items = st[0][slot].tolist()
-                cls.last_used, cls.last_cap = used, cap
-                if n_rays:
-                    # items, or the chunks they took beyond the slack: keep 25 % head room
-                    items = max(items, 32 * (used - _LOG_SLACK_CHUNKS))
-                    need = max(8.0, 1.25 * items / n_rays)
-                    _items_per_ray = need if used > cap else max(need, 0.9 * _items_per_ray)
-            st[2] = keep
+        if wait and host().logs_pending():
+            for dev in range(torch.cuda.device_count()):
+                torch.cuda.synchronize(dev)
+        for used, items, n_rays, cap in host().poll_logs():
+            cls.last_used, cls.last_cap = used, cap
+            if n_rays:
+                # items, or the chunks they took beyond the slack: keep 25 % head room
+                items = max(items, 32 * (used - _LOG_SLACK_CHUNKS))
+                need = max(8.0, 1.25 * items / n_rays)
+                _items_per_ray = need if used > cap else max(need, 0.9 * _items_per_ray)
         return _items_per_ray
-
-    last_used = last_cap = 0
 
 
 def log_estimate(wait=False):
@@ -518,26 +439,19 @@ def log_eligible(tree, opt):
             and tree.data.dtype == torch.float32)
 
 
-def _log_capacity(n_rays, device):
+def log_capacity(n_rays):
     """Chunks of the next log for ``n_rays`` rays."""
-    return int(n_rays * _LogWatch.poll(device) / 32) + _LOG_SLACK_CHUNKS
+    return int(n_rays * _LogWatch.poll() / 32) + _LOG_SLACK_CHUNKS
 
 
 def log_is_sorted(tree, n_rays, image):
     """Whether a logged forward of this size sorts its samples, so that the replay clears the
     gradient on the way."""
-    ct = _pack_tree(tree)
-    return bool(library().svoxb_log_is_sorted(
-        C.byref(ct), C.c_int64(n_rays), C.c_int(int(image)),
-        C.c_int64(_log_capacity(n_rays, tree.data.device))))
+    return host().log_is_sorted(tree, n_rays, image, log_capacity(n_rays))
 
 
-def _log_alloc(n_rays, device):
-    lib = library()
-    lib.svoxb_item_log_words.restype = C.c_int64
-    cap = _log_capacity(n_rays, device)
-    words = lib.svoxb_item_log_words(C.c_int64(cap))
-    return torch.empty(words, dtype=torch.int32, device=device), cap
+def n_rays_of(rays_or_cam, image):
+    return rays_or_cam.height * rays_or_cam.width if image else rays_or_cam.origins.shape[0]
 
 
 def volume_render_logged(tree, rays_or_cam, opt, image=False):
@@ -545,27 +459,9 @@ def volume_render_logged(tree, rays_or_cam, opt, image=False):
 
     -> (out, (log, capacity_chunks)); pass the pair to ``volume_render_backward_replay``.
     """
-    lib = library()
-    ct = _pack_tree(tree)
-    co = opt._pack()
-    dev = tree.data.device
-    with torch.cuda.device(dev):
-        if image:
-            cs = _pack_camera(rays_or_cam, dev)
-            shape, n = (cs.height, cs.width, 3), cs.height * cs.width
-            fn = lib.svoxb_volume_render_image_logged
-        else:
-            cs = _pack_rays(rays_or_cam, dev)
-            shape, n = (cs.Q, 3), cs.Q
-            fn = lib.svoxb_volume_render_logged
-        out = torch.empty(shape, dtype=torch.float32, device=dev)
-        log, cap = _log_alloc(n, dev)
-        with _timed("volume_render"):
-            st = fn(C.byref(ct), C.byref(cs), C.byref(co), C.c_void_p(out.data_ptr()),
-                    C.c_void_p(log.data_ptr()), C.c_int64(cap), _stream())
-        if st:
-            _raise(st, "volume_render_logged")
-        _LogWatch.watch(log, cap, n)
+    cap = log_capacity(n_rays_of(rays_or_cam, image))
+    with _timed("volume_render"):
+        out, log = host().volume_render_logged(tree, rays_or_cam, opt, image, cap)
     return out, (log, cap)
 
 
@@ -587,60 +483,19 @@ def volume_render_backward_replay(tree, rays_or_cam, opt, grad_output, fwd_out, 
     takes over in that case.  ``used`` > 0: a count read with ``log_chunks_used`` that fits
     the capacity (smaller scratch, no fallback enqueued).  ``zeroed``: a zero tensor like
     ``data`` to add the gradient into (else one is made here)."""
-    lib = library()
     log, cap = logpair
-    dev = tree.data.device
-    with torch.cuda.device(dev):
-        ct = _pack_tree(tree)
-        co = opt._pack()
-        _check_input(grad_output, "grad_output")
-        _check_input(fwd_out, "fwd_out")
-        if used > cap:
-            raise RuntimeError("the item log overflowed: it cannot be replayed")
-        grad = zeroed if zeroed is not None else \
-            torch.empty_like(tree.data, memory_format=torch.contiguous_format)
-        if image:
-            cs = _pack_camera(rays_or_cam, dev)
-            fn = lib.svoxb_volume_render_image_backward_replay
-        else:
-            cs = _pack_rays(rays_or_cam, dev)
-            fn = lib.svoxb_volume_render_backward_replay
-        with _timed("volume_render_backward"):
-            st = fn(C.byref(ct), C.byref(cs), C.byref(co), C.c_void_p(grad_output.data_ptr()),
-                    C.c_void_p(fwd_out.data_ptr()), C.c_void_p(log.data_ptr()), C.c_int64(cap),
-                    C.c_int64(used), C.c_void_p(grad.data_ptr()), C.c_int(int(zeroed is None)),
-                    _stream())
-    if st:
-        _raise(st, "volume_render_backward_replay")
-    return grad
+    with _timed("volume_render_backward"):
+        return host().volume_render_backward_replay(tree, rays_or_cam, opt, image, grad_output,
+                                                    fwd_out, log, cap, used, zeroed)
 
 
-def se_grad_replay(tree, rays_or_cam, opt, residual, fwd_out, logpair, grad, hess, zeroed,
-                   image=False):
-    """Gradient and Gauss-Newton diagonal of the squared error (second and third result of the
-    reference's ``se_grad``) from the item log, into ``grad`` and ``hess`` (``zeroed``: which
-    already are zero).  The host does not wait: a log that was too small is noticed on the
-    device, where a march enqueued behind the replay then takes over."""
-    lib = library()
-    log, cap = logpair
-    dev = tree.data.device
-    with torch.cuda.device(dev):
-        ct = _pack_tree(tree)
-        co = opt._pack()
-        _check_input(residual, "residual")
-        _check_input(fwd_out, "fwd_out")
-        if image:
-            cs = _pack_camera(rays_or_cam, dev)
-            fn = lib.svoxb_se_grad_image_replay
-        else:
-            cs = _pack_rays(rays_or_cam, dev)
-            fn = lib.svoxb_se_grad_replay
-        st = fn(C.byref(ct), C.byref(cs), C.byref(co), C.c_void_p(residual.data_ptr()),
-                C.c_void_p(fwd_out.data_ptr()), C.c_void_p(log.data_ptr()), C.c_int64(cap),
-                C.c_int64(0), C.c_void_p(grad.data_ptr()), C.c_void_p(hess.data_ptr()),
-                C.c_int(int(not zeroed)), _stream())
-    if st:
-        _raise(st, "se_grad_replay")
+def se_grad(tree, rays_or_cam, opt, colors, image=False):
+    """-> (render, gradient, Gauss-Newton diagonal) of the squared error against ``colors``
+    (the reference's ``se_grad``) through the item log.  The host does not wait: a log that was
+    too small is noticed on the device, where a march enqueued behind the replay then takes
+    over."""
+    cap = log_capacity(n_rays_of(rays_or_cam, image))
+    return host().se_grad(tree, rays_or_cam, opt, image, colors, cap)
 
 
 def se_grad_march(tree, rays_or_cam, opt, fwd_out, colors, image=False):
@@ -754,58 +609,19 @@ def volume_render_backward_replay_parts(tree, rays_or_cam, opt, grad_output, fwd
     return grad
 
 
-def _fwd_ptr(fwd_out, shape):
-    if fwd_out is None:
-        return C.c_void_p(0)
-    _check_input(fwd_out, "fwd_out")
-    if tuple(fwd_out.shape) != tuple(shape):
-        raise RuntimeError("fwd_out must have the shape of the forward output")
-    return C.c_void_p(fwd_out.data_ptr())
-
-
 def volume_render_backward(tree, rays, opt, grad_output, fwd_out=None):
     """-> gradient w.r.t. data (like data); svox/csrc/rt_kernel.cu:1059-1083.
 
     ``fwd_out`` (optional, not in the reference signature) is the forward
     result for the same inputs; it lets the kernel march each ray once.
     """
-    lib = library()
-    ct = _pack_tree(tree)
-    cr = _pack_rays(rays, tree.data.device)
-    co = opt._pack()
-    _check_input(grad_output, "grad_output")
-    shape = (cr.Q, _out_dim(opt, ct.K))
-    if tuple(grad_output.shape) != shape:
-        raise RuntimeError(f"grad_output must be {shape}")
-    with torch.cuda.device(tree.data.device):
-        grad = torch.zeros_like(tree.data, memory_format=torch.contiguous_format)
-        with _timed("volume_render_backward"):
-            st = lib.svoxb_volume_render_backward(
-                C.byref(ct), C.byref(cr), C.byref(co), C.c_void_p(grad_output.data_ptr()),
-                _fwd_ptr(fwd_out, shape), C.c_void_p(grad.data_ptr()), C.c_int(0), _stream())
-    if st:
-        _raise(st, "volume_render_backward")
-    return grad
+    with _timed("volume_render_backward"):
+        return host().volume_render_backward(tree, rays, opt, False, grad_output, fwd_out)
 
 
 def volume_render_image_backward(tree, cam, opt, grad_output, fwd_out=None):
     """-> gradient w.r.t. data; svox/csrc/rt_kernel.cu:1085-1109."""
-    lib = library()
-    ct = _pack_tree(tree)
-    cc = _pack_camera(cam, tree.data.device)
-    co = opt._pack()
-    _check_input(grad_output, "grad_output")
-    shape = (cc.height, cc.width, _out_dim(opt, ct.K))
-    if tuple(grad_output.shape) != shape:
-        raise RuntimeError(f"grad_output must be {shape}")
-    with torch.cuda.device(tree.data.device):
-        grad = torch.empty_like(tree.data, memory_format=torch.contiguous_format)
-        st = lib.svoxb_volume_render_image_backward(
-            C.byref(ct), C.byref(cc), C.byref(co), C.c_void_p(grad_output.data_ptr()),
-            _fwd_ptr(fwd_out, shape), C.c_void_p(grad.data_ptr()), C.c_int(1), _stream())
-    if st:
-        _raise(st, "volume_render_image_backward")
-    return grad
+    return host().volume_render_backward(tree, cam, opt, True, grad_output, fwd_out)
 
 
 def march_stats(tree, rays, opt):

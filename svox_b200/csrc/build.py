@@ -1,4 +1,4 @@
-"""Compile the native library in-tree for sm_100a with nvcc.
+"""Compile the native library in-tree for sm_100a with nvcc, and its host extension.
 
     python -m svox_b200.csrc.build [--force] [--verbose]
 
@@ -18,15 +18,43 @@ DEPS = ["svox_b200.cu", "common.cuh", "arith.cuh", "host.cuh", "query.cuh", "ren
         os.path.join("..", "..", "include", "svox_b200.h")]
 
 
-def _stale():
-    if not os.path.exists(LIB):
+# the host side of the hot calls, a Python extension (host.cpp)
+HOST_SRC = os.path.join(HERE, "host.cpp")
+HOST_LIB = os.path.join(HERE, "_host.so")
+HOST_DEPS = ["host.cpp", os.path.join("..", "..", "include", "svox_b200.h")]
+
+
+def _stale(lib, deps):
+    if not os.path.exists(lib):
         return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(os.path.join(HERE, d)) > t for d in DEPS)
+    t = os.path.getmtime(lib)
+    return any(os.path.getmtime(os.path.join(HERE, d)) > t for d in deps)
+
+
+def _build_host():
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           "-DTORCH_EXTENSION_NAME=_host", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for d in [*cpp_extension.include_paths(), os.path.join(cuda, "include"),
+              sysconfig.get_paths()["include"]]:
+        cmd += ["-isystem", d]
+    cmd += ["-o", HOST_LIB, HOST_SRC]
+    for d in [*cpp_extension.library_paths(), os.path.join(cuda, "lib64")]:
+        cmd += ["-L" + d]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python",
+            "-lcudart"]
+    subprocess.run(cmd, check=True)
 
 
 def build(force=False, verbose=False):
-    if not force and not _stale():
+    if force or _stale(HOST_LIB, HOST_DEPS):
+        _build_host()
+    if not force and not _stale(LIB, DEPS):
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     cmd = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",

@@ -974,6 +974,13 @@ int svoxb_item_log_used(const int32_t* log, int64_t* chunks_used, void* stream) 
     return SVOXB_OK;
 }
 
+int svoxb_item_log_watch(const int32_t* log, int32_t* counts, void* stream) {
+    if (!log || !counts) return SVOXB_ERR_NULL;
+    SVOXB_CUDA(cudaMemcpyAsync(counts, log, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                               (cudaStream_t)stream));
+    return SVOXB_OK;
+}
+
 int svoxb_march_stats(const svoxb_tree* tree, const svoxb_rays* rays,
                       const svoxb_render_options* opt, int32_t* visits, int32_t* contrib_fwd,
                       int32_t* contrib_bwd, void* stream) {

@@ -117,9 +117,8 @@ def _forward(ctx, data, tree, src, opt, prepared, train, image):
         # training step: record the contributing samples for the backward pass, and unless the
         # backward does it on the way clear the gradient buffer it will add into on a second
         # stream meanwhile (the march leaves memory bandwidth unused)
-        n = src.width * src.height if image else src.origins.shape[0]
         if GRAD_PARTS is not None or GRAD_BUFFER is not None or \
-                not _C.log_is_sorted(tree, n, image):
+                not _C.log_is_sorted(tree, _C.n_rays_of(src, image), image):
             ctx.grad_buffer = _zeroed_beside(tree.data)
         out, (log, ctx.log_capacity) = _C.volume_render_logged(tree, src, opt, image=image)
     elif image:
@@ -156,6 +155,13 @@ def _backward(ctx, grad_out):
     if ctx.image:
         return (_C.volume_render_image_backward(ctx.tree, ctx.src, ctx.opt, grad_out, fwd),) + none
     return (_C.volume_render_backward(ctx.tree, ctx.src, ctx.opt, grad_out, fwd),) + none
+
+
+def _hooked():
+    """Whether something here asks for more than the native autograd node does: a gradient in
+    parts or in a buffer of the caller's, timing records, the switches of the tests."""
+    return GRAD_PARTS is not None or GRAD_BUFFER is not None or FORCE_TWO_MARCHES or \
+        not USE_ITEM_LOG or _C._timing is not None
 
 
 class _VolumeRenderFunction(autograd.Function):
@@ -225,15 +231,12 @@ class VolumeRenderer(nn.Module):
         be changed through ``.data`` without any version counter noticing."""
         return _FrozenTree(self)
 
-    def _training(self):
-        return self.tree.data.requires_grad and torch.is_grad_enabled()
-
-    def _prepared(self, opt):
-        if self._frozen is None or self._training():
+    def _prepared(self, tree, opt):
+        if self._frozen is None:
             return None
         key = (float(opt.sigma_thresh), bool(opt.density_softplus))
         if key not in self._frozen:
-            self._frozen[key] = _C.render_scratch(self.tree._spec(), opt)
+            self._frozen[key] = _C.render_scratch(tree, opt)
         return self._frozen[key]
 
     @property
@@ -249,10 +252,22 @@ class VolumeRenderer(nn.Module):
     def forward(self, rays: Rays, cuda=True, fast=False):
         """Render ``(B, 3)`` rays -> ``(B, rgb_dim)``.  Differentiable w.r.t. tree.data."""
         self._require_cuda(cuda)
+        return self._render(_rays_spec_from_rays(rays), fast, False)
+
+    def _render(self, src, fast, image):
         opt = self._get_options(fast)
-        return _VolumeRenderFunction.apply(self.tree.data, self.tree._spec(),
-                                           _rays_spec_from_rays(rays), opt, self._prepared(opt),
-                                           self._training())
+        tree = self.tree._spec()
+        data = tree.data
+        train = data.requires_grad and torch.is_grad_enabled()
+        if not train and _C._timing is None:
+            render = _C.volume_render_image if image else _C.volume_render
+            return render(tree, src, opt, self._prepared(tree, opt))
+        if train and not _hooked():
+            cap = _C.log_capacity(_C.n_rays_of(src, image)) if _C.log_eligible(tree, opt) else 0
+            return _C.host().render_node(data, tree, src, opt, image, cap, self.tree._data_epoch)
+        function = _VolumeRenderImageFunction if image else _VolumeRenderFunction
+        return function.apply(data, tree, src, opt, None if train else self._prepared(tree, opt),
+                              train)
 
     def render_persp(self, c2w, width=800, height=800, fx=1111.111, fy=None, cuda=True,
                      fast=False):
@@ -261,11 +276,7 @@ class VolumeRenderer(nn.Module):
         if fy is None:
             fy = fx
         c2w = c2w.to(dtype=self.tree.data.dtype, device=self.tree.data.device).contiguous()
-        opt = self._get_options(fast)
-        return _VolumeRenderImageFunction.apply(
-            self.tree.data, self.tree._spec(),
-            _make_camera_spec(c2w, width, height, fx, fy), opt, self._prepared(opt),
-            self._training())
+        return self._render(_make_camera_spec(c2w, width, height, fx, fy), fast, True)
 
     def se_grad(self, rays: Rays, colors):
         """Rendered colour, gradient and Gauss-Newton diagonal of the total squared error
@@ -305,20 +316,7 @@ class VolumeRenderer(nn.Module):
                                               colors.reshape(out.shape).contiguous(),
                                               image=image)
                 return out, grad, hess
-            data = self.tree.data
-            grad, hess = (torch.empty_like(data, memory_format=torch.contiguous_format)
-                          for _ in range(2))
-            n = src.width * src.height if image else src.origins.shape[0]
-            # unless the replay does it on the way, both results are cleared beside the forward
-            zeroed = [] if _C.log_is_sorted(tree, n, image) else \
-                [_C.zero_beside(x) for x in (grad, hess)]
-            out, log = _C.volume_render_logged(tree, src, opt, image=image)
-            resid = (out - colors.reshape(out.shape)).contiguous()
-            for done in zeroed:
-                torch.cuda.current_stream(data.device).wait_event(done)
-            _C.se_grad_replay(tree, src, opt, resid, out, log, grad, hess, bool(zeroed),
-                              image=image)
-            return out, grad, hess
+            return _C.se_grad(tree, src, opt, colors, image=image)
 
     @staticmethod
     def persp_rays(c2w, width=800, height=800, fx=1111.111, fy=None):
@@ -357,8 +355,6 @@ class VolumeRenderer(nn.Module):
         else:
             opts.ndc_width = -1
         opts.sigma_thresh = opts.stop_thresh = 1e-2 if fast else 0.0
-        if hasattr(self, "sigma_thresh"):
-            opts.sigma_thresh = self.sigma_thresh
-        if hasattr(self, "stop_thresh"):
-            opts.stop_thresh = self.stop_thresh
+        opts.sigma_thresh = getattr(self, "sigma_thresh", opts.sigma_thresh)
+        opts.stop_thresh = getattr(self, "stop_thresh", opts.stop_thresh)
         return opts

@@ -22,7 +22,7 @@ from warnings import warn
 
 import numpy as np
 import torch
-from torch import autograd, nn
+from torch import nn
 
 from . import csrc as _C
 from .formats import DataFormat, LocalIndex
@@ -31,25 +31,17 @@ from .view import N3TreeView
 __all__ = ["N3Tree", "WeightAccumulator", "_QueryVerticalFunction"]
 
 
-class _QueryVerticalFunction(autograd.Function):
-    """Autograd boundary of the point query (svox/svox.py:38-54)."""
+class _QueryVerticalFunction:
+    """Autograd boundary of the point query (svox/svox.py:38-54): a native node where a gradient
+    can follow, the plain call otherwise."""
 
     @staticmethod
-    def forward(ctx, data, tree_spec, indices):
-        out, node_ids = _C.query_vertical(tree_spec, indices)
-        ctx.mark_non_differentiable(node_ids)
-        ctx.tree_spec = tree_spec
-        ctx.save_for_backward(indices)
-        return out, node_ids
-
-    @staticmethod
-    def backward(ctx, grad_out, dummy):
+    def apply(data, tree_spec, indices):
         # (clearing the gradient buffer on a second stream beside the forward query, as the
         # renderer does, was measured: no gain, both are bound by DRAM)
-        if ctx.needs_input_grad[0]:
-            return _C.query_vertical_backward(ctx.tree_spec, ctx.saved_tensors[0],
-                                              grad_out.contiguous()), None, None
-        return None, None, None
+        if data.requires_grad and torch.is_grad_enabled():
+            return _C.host().query_node(data, tree_spec, indices)
+        return _C.query_vertical(tree_spec, indices)
 
 
 class N3Tree(nn.Module):
@@ -96,7 +88,9 @@ class N3Tree(nn.Module):
             self.extra_data = None
 
         self._ver = 0
-        self._data_epoch = 0     # bumped by every write that goes through ``data.data``
+        # counts the writes that go through ``data.data``; in a tensor so that the native
+        # autograd node can look at it
+        self._data_epoch = torch.zeros((), dtype=torch.int64)
         self._invalidate()
         self._lock_tree_structure = False
         self._weight_accum = None
@@ -613,19 +607,18 @@ class N3Tree(nn.Module):
         """Pack the tensors for the native library (svox/svox.py:1084-1103)."""
         spec = _C.TreeSpec()
         spec._owner = weakref.ref(self)
-        spec.data = self.data
-        spec.child = self.child
-        spec.parent_depth = self.parent_depth
-        dev, dt = self.data.device, self.data.dtype
-        spec.extra_data = self.extra_data if self.extra_data is not None else \
-            torch.empty((0, 0), dtype=dt, device=dev)
+        buffers = self._buffers        # (attribute look-up on a Module goes through __getattr__)
+        data = spec.data = self._parameters["data"]
+        spec.child = buffers["child"]
+        spec.parent_depth = buffers["parent_depth"]
+        spec.extra_data = self.extra_data if "extra_data" in buffers else \
+            self.__dict__["extra_data"]
         if world:
-            spec.offset, spec.scaling = self.offset, self.invradius
+            spec.offset, spec.scaling = buffers["offset"], buffers["invradius"]
         else:
-            spec.offset = torch.zeros(3, dtype=dt, device=dev)
-            spec.scaling = torch.ones(3, dtype=dt, device=dev)
-        spec._weight_accum = self._weight_accum if self._weight_accum is not None else \
-            torch.empty(0, dtype=dt, device=dev)
+            spec.offset = torch.zeros(3, dtype=data.dtype, device=data.device)
+            spec.scaling = torch.ones(3, dtype=data.dtype, device=data.device)
+        spec._weight_accum = self._weight_accum
         spec._weight_accum_max = (self._weight_accum_op == "max")
         return spec
 
