@@ -222,6 +222,19 @@ int svoxb_volume_render_logged(const svoxb_tree* tree, const svoxb_rays* rays,
 int svoxb_volume_render_image_logged(const svoxb_tree* tree, const svoxb_camera* cam,
                                      const svoxb_render_options* opt, float* out, int32_t* log,
                                      int64_t capacity_chunks, void* stream);
+/* The logged forward, which also clears one or two buffers shaped like data
+ * (clear1 may be null) on `clear_stream`, beside its march: for gradients that
+ * the replay does not clear on its way.  At least one ray.  The caller orders
+ * the buffers' earlier users before this call, and their next ones behind the
+ * work enqueued on `clear_stream`. */
+int svoxb_volume_render_logged_clear(const svoxb_tree* tree, const svoxb_rays* rays,
+                                     const svoxb_render_options* opt, float* out, int32_t* log,
+                                     int64_t capacity_chunks, void* stream, float* clear0,
+                                     float* clear1, void* clear_stream);
+int svoxb_volume_render_image_logged_clear(const svoxb_tree* tree, const svoxb_camera* cam,
+                                           const svoxb_render_options* opt, float* out,
+                                           int32_t* log, int64_t capacity_chunks, void* stream,
+                                           float* clear0, float* clear1, void* clear_stream);
 int svoxb_volume_render_backward_replay(const svoxb_tree* tree, const svoxb_rays* rays,
                                         const svoxb_render_options* opt,
                                         const float* grad_output, const float* fwd_out,

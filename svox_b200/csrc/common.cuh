@@ -128,6 +128,7 @@ __device__ __forceinline__ bool descendN(const int32_t* __restrict__ child, int6
 // Host helpers
 int set_cuda_error(cudaError_t e);  // records the text, returns SVOXB_ERR_CUDA
 int sm_count();                     // multiprocessors of the current device
+int blocks_per_sm(const void* kernel, int block, size_t smem, int* per_sm);
 
 #define SVOXB_CUDA(call)                                              \
     do {                                                              \

@@ -34,7 +34,8 @@ struct Library {
     X(volume_render_image_backward) X(volume_render_logged) X(volume_render_image_logged)       \
     X(volume_render_backward_replay) X(volume_render_image_backward_replay)                     \
     X(se_grad_replay) X(se_grad_image_replay) X(item_log_words) X(item_log_watch)               \
-    X(log_is_sorted) X(strerror) X(last_cuda_error)
+    X(volume_render_logged_clear) X(volume_render_image_logged_clear) X(log_is_sorted)          \
+    X(strerror) X(last_cuda_error)
 #define SVOXB_MEMBER(name) decltype(&svoxb_##name) name = nullptr;
     SVOXB_FUNCTIONS(SVOXB_MEMBER)
 } lib;
@@ -343,17 +344,63 @@ Tensor run_render(const Tree& t, const Source& s, const svoxb_render_options& o,
     return out;
 }
 
+// Gradients that the backward does not clear on its way are cleared on a side stream beside the
+// forward's march, which leaves memory bandwidth unused -- unless they are so small that the two
+// events cost more than the fill.
+constexpr int64_t kFillBeside = 16 << 20;   // bytes; 16 MB are cleared in about 4 us
+
+struct Zeroed {
+    std::vector<Tensor> buffers;
+    at::cuda::CUDAEvent done;
+    c10::cuda::CUDAStream side;
+
+    Zeroed(const Tensor& like, int count) : side(side_stream(like.device().index())) {
+        for (int i = 0; i < count; ++i) buffers.push_back(at::empty(like.sizes(), like.options()));
+    }
+    float* pointer(size_t i) { return i < buffers.size() ? buffers[i].data_ptr<float>() : nullptr; }
+    // After the call that enqueued the fills.  Should a tensor be dropped before anyone waited for
+    // its fill, its memory must not be handed out again while the side stream still writes to it.
+    void enqueued() {
+        done.record(side);
+        for (const Tensor& b : buffers)
+            c10::cuda::CUDACachingAllocator::recordStream(b.storage().data_ptr(), side);
+    }
+    Tensor claim(size_t i) {
+        done.block(at::cuda::getCurrentCUDAStream(buffers[i].device().index()));
+        return std::move(buffers[i]);
+    }
+    static c10::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
+        static std::mutex mutex;
+        static std::vector<optional<c10::cuda::CUDAStream>> streams(64);
+        std::lock_guard<std::mutex> lock(mutex);
+        auto& s = streams.at((size_t)dev);
+        if (!s) s = c10::cuda::getStreamFromPool(false, dev);
+        return *s;
+    }
+};
+
 std::pair<Tensor, Tensor> run_logged(const Tree& t, const Source& s, const svoxb_render_options& o,
-                                     int64_t capacity) {
+                                     int64_t capacity, Zeroed* zeroed = nullptr) {
     const c10::cuda::CUDAGuard guard(t.data.device());
     Tensor out = at::empty(s.shape(3), t.data.options());
     Tensor log = at::empty({lib.item_log_words(capacity)}, t.child.options());
     float* to = out.data_ptr<float>();
     int32_t* words = log.data_ptr<int32_t>();
     void* stream = stream_of(t.data);
-    check(s.image ? lib.volume_render_image_logged(&t.c, &s.cam, &o, to, words, capacity, stream)
-                  : lib.volume_render_logged(&t.c, &s.rays, &o, to, words, capacity, stream),
-          "volume_render_logged");
+    int st;
+    if (zeroed) {
+        float *c0 = zeroed->pointer(0), *c1 = zeroed->pointer(1);
+        void* side = zeroed->side.stream();
+        st = s.image ? lib.volume_render_image_logged_clear(&t.c, &s.cam, &o, to, words, capacity,
+                                                            stream, c0, c1, side)
+                     : lib.volume_render_logged_clear(&t.c, &s.rays, &o, to, words, capacity,
+                                                      stream, c0, c1, side);
+        zeroed->enqueued();
+    } else {
+        st = s.image ? lib.volume_render_image_logged(&t.c, &s.cam, &o, to, words, capacity, stream)
+                     : lib.volume_render_logged(&t.c, &s.rays, &o, to, words, capacity, stream);
+    }
+    check(st, "volume_render_logged");
     log_watch().watch(log, capacity, s.count());
     return {out, log};
 }
@@ -402,47 +449,9 @@ Tensor run_backward(const Tree& t, const Source& s, const svoxb_render_options& 
     return grad;
 }
 
-// A gradient that is not cleared by the backward on its way: cleared on a side stream beside the
-// forward, which leaves memory bandwidth unused -- unless it is so small that the two events cost
-// more than the fill.
-constexpr int64_t kFillBeside = 16 << 20;   // bytes; 16 MB are cleared in about 4 us
-
-struct Zeroed {
-    Tensor buffer;
-    at::cuda::CUDAEvent done;
-
-    explicit Zeroed(const Tensor& like) : buffer(at::empty(like.sizes(), like.options())) {
-        const auto dev = like.device().index();
-        const auto current = at::cuda::getCurrentCUDAStream(dev);
-        const auto side = side_stream(dev);
-        at::cuda::CUDAEvent before;       // the memory's earlier users
-        before.record(current);
-        before.block(side);
-        {
-            const c10::cuda::CUDAStreamGuard guard(side);
-            buffer.zero_();
-        }
-        done.record(side);
-        // should the tensor be dropped before anyone waited for the fill, its memory must not be
-        // handed out again while the side stream still writes to it
-        c10::cuda::CUDACachingAllocator::recordStream(buffer.storage().data_ptr(), side);
-    }
-    Tensor claim() {
-        done.block(at::cuda::getCurrentCUDAStream(buffer.device().index()));
-        return std::move(buffer);
-    }
-    static c10::cuda::CUDAStream side_stream(c10::DeviceIndex dev) {
-        static std::mutex mutex;
-        static std::vector<optional<c10::cuda::CUDAStream>> streams(64);
-        std::lock_guard<std::mutex> lock(mutex);
-        auto& s = streams.at((size_t)dev);
-        if (!s) s = c10::cuda::getStreamFromPool(false, dev);
-        return *s;
-    }
-};
-
-bool sorted_log(const Tree& t, const Source& s, int64_t capacity) {
-    return lib.log_is_sorted(&t.c, s.count(), s.image, capacity) != 0;
+bool fills_beside(const Tree& t, const Source& s, int64_t capacity) {
+    return s.count() > 0 && t.data.numel() * 4 >= kFillBeside &&
+           !lib.log_is_sorted(&t.c, s.count(), s.image, capacity);
 }
 
 // ---------------------------------------------------------------------------
@@ -490,9 +499,10 @@ class RenderNode : public torch::autograd::Function<RenderNode> {
         c.keeps_out = c.options.sigma_thresh == 0.f && c.options.stop_thresh == 0.f;
         Tensor out, log;
         if (c.capacity > 0) {
-            if (c.tree.data.numel() * 4 >= kFillBeside && !sorted_log(c.tree, c.source, c.capacity))
-                c.zeroed = std::make_shared<Zeroed>(c.tree.data);
-            std::tie(out, log) = run_logged(c.tree, c.source, c.options, c.capacity);
+            if (fills_beside(c.tree, c.source, c.capacity))
+                c.zeroed = std::make_shared<Zeroed>(c.tree.data, 1);
+            std::tie(out, log) =
+                run_logged(c.tree, c.source, c.options, c.capacity, c.zeroed.get());
         } else {
             out = run_render(c.tree, c.source, c.options, {});
         }
@@ -513,7 +523,7 @@ class RenderNode : public torch::autograd::Function<RenderNode> {
             if (c.tree.data._version() == c.version_then && c.epoch_now() == c.epoch_then) {
                 if (saved[1].defined()) {
                     optional<Tensor> zeroed;
-                    if (auto z = std::move(c.zeroed)) zeroed = z->claim();
+                    if (auto z = std::move(c.zeroed)) zeroed = z->claim(0);
                     return {run_replay(c.tree, c.source, c.options, grad_out, saved[0], saved[1],
                                        c.capacity, 0, zeroed),
                             Tensor()};
@@ -636,21 +646,20 @@ PYBIND11_MODULE(_host, m) {
         return unlocked([&] {
             const c10::cuda::CUDAGuard guard(t.data.device());
             Tensor grad, hess;
-            const bool beside = t.data.numel() * 4 >= kFillBeside && !sorted_log(t, s, capacity);
-            optional<Zeroed> zg, zh;
+            const bool beside = fills_beside(t, s, capacity);
+            optional<Zeroed> zeroed;
             if (beside) {
-                zg.emplace(t.data);
-                zh.emplace(t.data);
+                zeroed.emplace(t.data, 2);
             } else {
                 grad = at::empty(t.data.sizes(), t.data.options());
                 hess = at::empty(t.data.sizes(), t.data.options());
             }
-            auto [out, log] = run_logged(t, s, o, capacity);
+            auto [out, log] = run_logged(t, s, o, capacity, beside ? &*zeroed : nullptr);
             const Tensor resid = at::sub(out, colors.reshape(out.sizes())).contiguous();
             check_input(resid, "colors");
             if (beside) {
-                grad = zg->claim();
-                hess = zh->claim();
+                grad = zeroed->claim(0);
+                hess = zeroed->claim(1);
             }
             const float *r = resid.data_ptr<float>(), *f = out.template data_ptr<float>();
             int32_t* words = log.template data_ptr<int32_t>();

@@ -2,8 +2,11 @@
 // per-call top-of-tree jump table.
 #pragma once
 
+#include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 #include "common.cuh"
 
@@ -21,10 +24,41 @@ int set_cuda_error(cudaError_t e) {
 }
 
 int sm_count() {
+    static std::atomic<int> known[64];
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
     return n > 0 ? n : 148;
+}
+
+// Resident blocks per SM of a kernel on the current device, after raising its shared memory
+// limit where that is needed; asked of the runtime once per kernel and device (a microsecond or
+// two of the host's time per launch otherwise).
+int blocks_per_sm(const void* kernel, int block, size_t smem, int* per_sm) {
+    struct Known { const void* kernel; size_t smem; int block, dev, per_sm; };
+    static std::mutex mutex;
+    static std::vector<Known> all;
+    int dev = 0;
+    SVOXB_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        for (const Known& k : all)
+            if (k.kernel == kernel && k.dev == dev && k.block == block && k.smem == smem) {
+                *per_sm = k.per_sm;
+                return SVOXB_OK;
+            }
+    }
+    // the 48 KB a kernel gets without asking cover its static shared memory too (up to 4 KB here)
+    if (smem > 40 * 1024)
+        SVOXB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem));
+    SVOXB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, block, smem));
+    if (*per_sm < 1) *per_sm = 1;
+    std::lock_guard<std::mutex> lock(mutex);
+    all.push_back(Known{kernel, smem, block, dev, *per_sm});
+    return SVOXB_OK;
 }
 
 int validate_tree(const svoxb_tree* t) {

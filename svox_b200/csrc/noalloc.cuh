@@ -42,7 +42,7 @@ static int launch_noalloc(const RenderCall& c, const RayBatch& src, int32_t* scr
     const svoxb_tree* t = c.tree;
     IndexLayout layout = IndexLayout::of(t->M, 0);
     const int64_t left = kNoAllocWords - (int64_t)layout.words - 64;
-    int64_t bricks = left / (kBrickWords + 1);
+    int64_t bricks = left / (2 * kBrickCells + 1);
     if (bricks > kMaxBricks) bricks = kMaxBricks;
     layout = IndexLayout::of(t->M, (int)(bricks > 0 ? bricks : 0));
     if ((int64_t)layout.words > kNoAllocWords) return SVOXB_ERR_TOO_LARGE;

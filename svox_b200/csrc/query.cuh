@@ -215,8 +215,12 @@ static int launch_query(int mode, const svoxb_tree* tree, const float* indices, 
     if (Q == 0) return SVOXB_OK;
     if (!indices) return SVOXB_ERR_NULL;
     if ((Q + kQueryBlock - 1) / kQueryBlock > 0x7fffffffLL) return SVOXB_ERR_TOO_LARGE;
+    // The jump table saves a point its upper levels, at a cost of one walk per cell: it has at
+    // most a quarter as many cells as there are points, and few points go without.
     TopScratch top;
-    int st = top.build(tree, 7, stream);
+    int level = 0;
+    while (level < 7 && Q >= (int64_t)4 << (3 * (level + 1))) ++level;
+    int st = level >= 5 ? top.build(tree, level, stream) : (int)SVOXB_OK;
     if (st) return st;
     const TopTable tt{top.cells, top.level};
     const unsigned grid = (unsigned)((Q + kQueryBlock - 1) / kQueryBlock);

@@ -2,25 +2,23 @@
 // the root and fetching every leaf's density from its 100- to 300-byte record.
 //
 // Level L of the tree is a dense TABLE of 2^L cells per side; a table cell that holds a node
-// gets a BRICK, the 8x8x8 grid of the three levels below it.  Both consist of one word per
-// CELL and one word per 2x2x2 GROUP of cells:
-//   cell word   0x00000001 .. 0x7f800000   the cell lies in a leaf that passes the density
-//                                          test; the word is its density (softplus applied)
-//               kWordEmpty + d             in a leaf of depth d that fails it: a sample there
-//                                          needs nothing else
-//               kWordFetch + d             passes it, but the density is no positive float
-//                                          (possible below a negative threshold only)
-//               kWordWalk                  the tree goes deeper here: walk `child`
-//               negative (table only)      kWordBrick | brick id
-//   group word  bits 28-31 = k, bits 0-27 = payload: with k = the last level of the grid, the
-//               payload is the node whose children are the group's cells; below that, the whole
-//               group lies in a leaf k levels under the grid's root, whose slot it is
-// Brick cells are stored group by group (8 cells = one 32-byte sector), because consecutive
-// samples of a ray stay inside a group for two or three steps.
+// gets a BRICK, the 8x8x8 grid of the three levels below it.  Both consist of one ENTRY of two
+// words per cell, z fastest:
+//   word 0   0x00000001 .. 0x7f800000   the cell lies in a leaf that passes the density test;
+//                                       the word is its density (softplus applied)
+//            kWordEmpty                 in a leaf that fails it
+//            kWordFetch                 passes it, but the density is no positive float
+//                                       (possible below a negative threshold only)
+//            kWordWalk                  the tree goes deeper here: walk `child`
+//            negative (table only)      kWordBrick | brick id
+//   word 1   bits 28-31: the leaf's depth, in a brick less L; bits 0-27: its slot.  kWordWalk:
+//            the node whose cell this is, in bits 28-31 its depth likewise, or 0: walk from the
+//            root
+// so that one 8-byte load per sample brings all that the march needs of a leaf.
 //
 // Built per call (`data` can change between any two): one thread per table cell, then one per
-// brick group, each with eight independent density loads in flight.  The bound is the 32-byte
-// sector of every leaf's density (266 MB for the 8.3 M leaves of a 512^3 shell).
+// brick cell.  The bound is the 64 bytes that DRAM delivers for every leaf's density (530 MB for
+// the 8.3 M leaves of a 512^3 shell).
 #pragma once
 
 #include "query.cuh"
@@ -41,27 +39,24 @@ struct LogGate {
 
 constexpr int kBrickLevels = 3;
 constexpr int kBrickCells = 512;
-constexpr int kBrickGroups = kBrickCells / 8;
-constexpr int kBrickWords = kBrickCells + kBrickGroups;
-constexpr int64_t kIndexMaxNodes = 1 << 25;  // slots must fit the 28 bits of a group word
+constexpr int64_t kIndexMaxNodes = 1 << 25;  // slots must fit 28 bits
 constexpr int kMaxBricks = 1 << 17;
 constexpr int kMaxTableLevel = 7;
 constexpr int kPosBits = 23;                 // position bits below the binary point, see march
 
 constexpr int32_t kWordInf = 0x7f800000;
-constexpr int32_t kWordEmpty = kWordInf;        // + depth (1 .. 31)
-constexpr int32_t kWordWalk = kWordInf + 63;
-constexpr int32_t kWordFetch = kWordInf + 64;   // + depth
+constexpr int32_t kWordEmpty = kWordInf + 1;
+constexpr int32_t kWordFetch = kWordInf + 2;   // these two leave the march's ordinary route
+constexpr int32_t kWordWalk = kWordInf + 3;
 constexpr int32_t kWordBrick = INT32_MIN;
 
 __device__ __forceinline__ float sigmoid_ref(float x) { return 1 / (1 + expf(-x)); }
 __device__ __forceinline__ float softplus_m1(float x) { return logf(1 + expf(x - 1)); }
 
-// The index as the march sees it: one buffer of int32 words.
+// The index as the march sees it: one buffer of entries.
 struct TreeIndex {
-    const int32_t* table = nullptr;   // (2^level)^3 cell words, z fastest, at the start
-    uint32_t groups = 0;              // from this word on: (2^(level-1))^3 group words
-    uint32_t bricks = 0;              // ... and kBrickWords per brick
+    const int2* table = nullptr;      // (2^level)^3 entries, z fastest, at the start
+    uint32_t bricks = 0;              // from this entry on: kBrickCells per brick
     int level = 0;
 };
 
@@ -73,18 +68,21 @@ __device__ __forceinline__ float ld_density(const float* a) {
     return v;
 }
 
-__device__ __forceinline__ int32_t leaf_word(float raw, float thresh, int softplus, int depth) {
+__device__ __forceinline__ int32_t leaf_word(float raw, float thresh, int softplus) {
     const float sigma = softplus ? softplus_m1(raw) : raw;
-    if (!(sigma > thresh)) return kWordEmpty + depth;
+    if (!(sigma > thresh)) return kWordEmpty;
     const int32_t bits = __float_as_int(sigma);
-    return bits > 0 ? bits : kWordFetch + depth;
+    return bits > 0 ? bits : kWordFetch;
+}
+__device__ __forceinline__ int32_t leaf_place(int depth, int64_t slot) {
+    return (int32_t)(((uint32_t)depth << 28) | (uint32_t)slot);
 }
 
 __global__ void __launch_bounds__(256)
 build_table_kernel(const int32_t* __restrict__ child, const float* __restrict__ data, int K,
                    int64_t M, int L, float thresh, int softplus, int brick_cap,
-                   int32_t* __restrict__ table, int32_t* __restrict__ groups,
-                   int32_t* __restrict__ counter, int32_t* __restrict__ roots, LogGate gate) {
+                   int2* __restrict__ table, int32_t* __restrict__ counter,
+                   int32_t* __restrict__ roots, LogGate gate) {
     if (gate.closed()) return;
     const bool fits = M < kIndexMaxNodes;
     const int S = (1 << L) - 1;
@@ -92,18 +90,15 @@ build_table_kernel(const int32_t* __restrict__ child, const float* __restrict__ 
          idx += gridDim.x * blockDim.x) {
         const int iz = idx & S, iy = (idx >> L) & S, ix = idx >> (2 * L);
         int64_t node = 0;
-        int32_t word = kWordWalk;
-        uint32_t group = 0xf0000000u;
+        int2 entry = make_int2(kWordWalk, 0);
         for (int l = 0; l < L; ++l) {
             const int b = L - 1 - l;
             const int64_t slot = node * 8 + ((((ix >> b) & 1) << 2) | (((iy >> b) & 1) << 1) |
                                              ((iz >> b) & 1));
-            if (b == 0 && fits) group = ((uint32_t)l << 28) | (uint32_t)node;
             const int32_t e = __ldg(child + slot);
             if (e == 0) {
-                if (b != 0 && fits) group = ((uint32_t)l << 28) | (uint32_t)slot;
-                word = leaf_word(ld_density(data + slot * K + (K - 1)), thresh, softplus, l + 1);
-                if (!fits && (word <= kWordInf || word >= kWordFetch)) word = kWordWalk;
+                const int32_t word = leaf_word(ld_density(data + slot * K + (K - 1)), thresh, softplus);
+                if (fits) entry = make_int2(word, leaf_place(l + 1, slot));
                 break;
             }
             node += e;
@@ -112,71 +107,47 @@ build_table_kernel(const int32_t* __restrict__ child, const float* __restrict__ 
                 const int id = atomicAdd(counter, 1);
                 if (id < brick_cap) {
                     roots[id] = (int32_t)node;
-                    word = kWordBrick | id;
+                    entry.x = kWordBrick | id;
                 }
             }
         }
-        table[idx] = word;
-        if (((ix | iy | iz) & 1) == 0)
-            groups[((((ix >> 1) << (L - 1)) + (iy >> 1)) << (L - 1)) + (iz >> 1)] = (int32_t)group;
+        table[idx] = entry;
     }
 }
 
-// One thread per 2x2x2 group of a brick.
+// One thread per brick cell: the loads on the way down are shared by a warp's neighbouring cells,
+// the stores run through a brick.  (With one thread per 2x2x2 group and eight loads in flight each
+// the kernel took 183 us instead of 114 on the 512^3 shell, 980 instead of 619 on 1024^3 shells.)
 __global__ void __launch_bounds__(256)
 fill_bricks_kernel(const int32_t* __restrict__ child, const float* __restrict__ data, int K,
                    int64_t M, int L, float thresh, int softplus, int cap,
                    const int32_t* __restrict__ counter, const int32_t* __restrict__ roots,
-                   int32_t* __restrict__ bricks, LogGate gate) {
+                   int2* __restrict__ bricks, LogGate gate) {
     if (gate.closed()) return;
     int n = *counter;
     if (n > cap) n = cap;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n * kBrickGroups;
-         i += gridDim.x * blockDim.x) {
-        const int g = i & (kBrickGroups - 1);
-        const int gx = g >> 4, gy = (g >> 2) & 3, gz = g & 3;
-        int64_t node = __ldg(roots + (i >> 6));
-        int32_t w[8];
-        uint32_t group = 0xf0000000u;
-        int state = 0;                         // 0: on the way down, 1: words done
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)n * kBrickCells;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const int c = (int)(i & (kBrickCells - 1));
+        const int x = c >> 6, y = (c >> 3) & 7, z = c & 7;
+        int64_t node = __ldg(roots + (i >> 9));
+        int2 entry = make_int2(kWordWalk, 0);
 #pragma unroll
-        for (int l = 0; l < kBrickLevels - 1; ++l) {
-            if (state == 0) {
-                const int b = kBrickLevels - 2 - l;
-                const int64_t slot = node * 8 + ((((gx >> b) & 1) << 2) |
-                                                 (((gy >> b) & 1) << 1) | ((gz >> b) & 1));
-                const int32_t e = __ldg(child + slot);
-                int32_t word = kWordWalk;
-                if (e == 0) {
-                    word = leaf_word(ld_density(data + slot * K + (K - 1)), thresh, softplus, L + 1 + l);
-                    group = ((uint32_t)l << 28) | (uint32_t)slot;
-                    state = 1;
-                } else {
-                    node += e;
-                    if (node < 0 || node >= M) state = 1;      // corrupt: reported by the march
-                }
-#pragma unroll
-                for (int c = 0; c < 8; ++c) w[c] = word;
+        for (int l = 1; l <= kBrickLevels; ++l) {
+            const int b = kBrickLevels - l;
+            const int64_t slot = node * 8 + ((((x >> b) & 1) << 2) | (((y >> b) & 1) << 1) |
+                                             ((z >> b) & 1));
+            const int32_t e = __ldg(child + slot);
+            if (e == 0) {
+                entry = make_int2(leaf_word(ld_density(data + slot * K + (K - 1)), thresh, softplus),
+                                  leaf_place(l, slot));
+                break;
             }
+            if (l == kBrickLevels) entry.y = leaf_place(l, node);   // the tree goes deeper
+            node += e;
+            if (node < 0 || node >= M) break;              // corrupt: reported by the march
         }
-        if (state == 0) {
-            group = ((uint32_t)(kBrickLevels - 1) << 28) | (uint32_t)node;
-            int32_t e[8];
-            float raw[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) e[c] = __ldg(child + node * 8 + c);
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                raw[c] = e[c] == 0 ? ld_density(data + (node * 8 + c) * K + (K - 1)) : 0.f;
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                w[c] = e[c] == 0 ? leaf_word(raw[c], thresh, softplus, L + kBrickLevels) : kWordWalk;
-        }
-        int32_t* __restrict__ brick = bricks + (size_t)(i >> 6) * kBrickWords;
-        int4* __restrict__ out = reinterpret_cast<int4*>(brick + 8 * g);
-        out[0] = make_int4(w[0], w[1], w[2], w[3]);
-        out[1] = make_int4(w[4], w[5], w[6], w[7]);
-        brick[kBrickCells + g] = (int32_t)group;
+        bricks[i] = entry;
     }
 }
 
@@ -188,11 +159,11 @@ inline unsigned index_grid(int64_t n, int block, int sms) {
 }
 
 // Where the parts of the index lie in its buffer (int32 words, 128-byte aligned parts):
-// table | groups | brick counter | brick roots | bricks.
+// table | brick counter | brick roots | bricks.
 struct IndexLayout {
     int level = 0, cap = 0;
     int64_t cells = 0;
-    size_t groups = 0, counter = 0, roots = 0, bricks = 0, words = 0;
+    size_t counter = 0, roots = 0, bricks = 0, words = 0;
 
     // A complete tree (all leaves at one depth) that fits the largest table gets the table at
     // its leaves' level: no bricks, which would hold every leaf 8 or 64 times.  Any other
@@ -218,15 +189,14 @@ struct IndexLayout {
             if (l.cap > max_bricks) l.cap = max_bricks;
         }
         auto up = [](size_t w) { return (w + 31) & ~(size_t)31; };
-        l.groups = (size_t)l.cells;
-        l.counter = up(l.groups + (size_t)l.cells / 8);
+        l.counter = up(2 * (size_t)l.cells);
         l.roots = l.counter + 32;
         l.bricks = up(l.roots + (size_t)l.cap);
-        l.words = l.bricks + (size_t)l.cap * kBrickWords;
+        l.words = l.bricks + (size_t)l.cap * (2 * kBrickCells);
         return l;
     }
     TreeIndex view(const int32_t* mem) const {
-        return TreeIndex{mem, (uint32_t)groups, (uint32_t)bricks, level};
+        return TreeIndex{reinterpret_cast<const int2*>(mem), (uint32_t)(bricks / 2), level};
     }
 };
 
@@ -238,12 +208,12 @@ static int build_index(const svoxb_tree* t, const IndexLayout& l, float thresh, 
     int32_t* roots = mem + l.roots;
     if (l.cap > 0) SVOXB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int32_t), s));
     build_table_kernel<<<index_grid(l.cells, 256, sms), 256, 0, s>>>(
-        t->child, t->data, t->K, t->M, l.level, thresh, softplus, l.cap, mem, mem + l.groups,
-        counter, roots, gate);
+        t->child, t->data, t->K, t->M, l.level, thresh, softplus, l.cap,
+        reinterpret_cast<int2*>(mem), counter, roots, gate);
     if (l.cap > 0)
-        fill_bricks_kernel<<<index_grid((int64_t)l.cap * kBrickGroups, 256, sms), 256, 0, s>>>(
+        fill_bricks_kernel<<<index_grid((int64_t)l.cap * kBrickCells, 256, sms), 256, 0, s>>>(
             t->child, t->data, t->K, t->M, l.level, thresh, softplus, l.cap, counter, roots,
-            mem + l.bricks, gate);
+            reinterpret_cast<int2*>(mem + l.bricks), gate);
     SVOXB_CUDA(cudaGetLastError());
     return SVOXB_OK;
 }

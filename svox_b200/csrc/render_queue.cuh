@@ -129,9 +129,11 @@ __device__ __forceinline__ uint64_t l2_policy_stream() {
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-__device__ __forceinline__ int32_t ld_keep(const int32_t* a, uint64_t pol) {
-    int32_t v;
-    asm volatile("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(pol));
+__device__ __forceinline__ int2 ld_keep(const int2* a, uint64_t pol) {
+    int2 v;
+    asm volatile("ld.global.nc.L2::cache_hint.v2.s32 {%0, %1}, [%2], %3;"
+                 : "=r"(v.x), "=r"(v.y)
+                 : "l"(a), "l"(pol));
     return v;
 }
 __device__ __forceinline__ void st_hint16(void* a, int4 v, uint64_t pol) {
@@ -189,15 +191,16 @@ struct alignas(16) WarpQueue {
     using Shape = RecordShape<K>;
     // three batches: items being collected, what spills over, and the batch in flight
     static constexpr int CAP = 96;
-    // colour basis, upstream gradient or view direction; odd stride: no bank conflicts
-    static constexpr int RAYW = (BD + (BWD || LOG ? 3 : 0)) | 1;
+    // per ray: colour basis, upstream gradient or view direction, delta_scale; odd stride: no
+    // bank conflicts
+    static constexpr int SCALE = BD + (BWD || LOG ? 3 : 0);
+    static constexpr int RAYW = (SCALE + 1) | 1;
     // Staging rows (cp.async targets).  After lane i has read row i it reuses the
     // row's first words for the item's results.
     alignas(16) float rows[32 * Shape::STRIDE];
     uint32_t slot[CAP];
-    float w[CAP];                      // weight T * (1 - att)
-    float T[(BWD || LOG) ? CAP : 4];   // transmittance after the sample
-    float dd[(BWD || LOG) ? CAP : 4];  // delta_t * delta_scale
+    float dt[CAP];                     // step length
+    float sigma[CAP];
     unsigned char owner[CAP];          // bits 0-4 owner lane, bit 7 accumulation march
     float rayv[32][RAYW];
 };
@@ -291,22 +294,27 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     const uint32_t side = (1u << L) - 1u;
     const uint64_t pol_keep = l2_policy_keep(), pol_stream = l2_policy_stream();
     const bool vec_ok = (reinterpret_cast<uintptr_t>(grad_data) & 15) == 0;
+    // Only an early stop needs the transmittance while marching (with a threshold of 0 a ray
+    // stops where it is exactly 0, after which nothing contributes); otherwise items are
+    // evaluated 32 at a time, where all lanes have one, and folded into the ray in order.
+    const bool early = !BWD && opt.stop_thresh > 0.f;
 
     // ---- per-lane state -------------------------------------------------------
     Ray r;
     r.hit = false;
     int64_t ray = 0;
     int state = lane < shape.lanes ? kNeedRay : kExhausted;
-    float t = 0.f, light = 1.f;
+    float t = 0.f, light = 1.f, ahead = 1.f;   // transmittance after the items folded / pushed
     float a0 = 0.f, a1 = 0.f, a2 = 0.f;  // forward: colour sums; backward: a0 = accum
     bool stopped = false;
     int phase = 1;  // backward: 0 = accumulation march (reference PASS 1), 1 = scatter march
     int it = 0;
-    int cur_cell = -1;                 // table cell of the brick used last ...
+    uint32_t cur_cell = 0xffffffffu;   // table cell of the brick used last ...
     uint32_t cur_brick = 0;            // ... and where the brick lies in the index
     // cursor: the position of the lane's next sample, and the index words requested for it
     float px = 0.f, py = 0.f, pz = 0.f;
-    int32_t word = 0, group = 0;
+    int2 entry = make_int2(0, 0);
+    uint32_t cell = 0;                 // ... and its table cell
     bool in_brick = false;             // ... from the brick `cur_brick`, else from the table
     // queue: ring of three batches; `qn` items collected from ring position `head` on
     int head = 0, qn = 0;
@@ -328,26 +336,20 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     };
     // 1 + floor(p * 2^23) / 2^23, exactly: the low 23 bits are the position's bits
     auto bits = [](float p) { return __float_as_uint(__fadd_rz(p, 1.0f)); };
-    auto table_cell = [&](uint32_t ux, uint32_t uy, uint32_t uz) {
-        return (int)(((ux >> (kPosBits - 3 * L)) & (side << (2 * L))) |
-                     ((uy >> (kPosBits - 2 * L)) & (side << L)) | ((uz >> (kPosBits - L)) & side));
-    };
     auto request_words = [&]() {
         const uint32_t ux = bits(px), uy = bits(py), uz = bits(pz);
-        const int cell = table_cell(ux, uy, uz);
-        in_brick = cell == cur_cell;
-        const int s3 = kPosBits - kBrickLevels - L;
-        const uint32_t x = ux >> s3, y = uy >> s3, z = uz >> s3;
-        const uint32_t c = ((x & 6) << 6) | ((y & 6) << 4) | ((z & 6) << 2) |
-                           ((x & 1) << 2) | ((y & 1) << 1) | (z & 1);
         if (BWD && index.table == nullptr) {       // fallback march: no index was built
-            word = kWordWalk;
+            entry = make_int2(kWordWalk, 0);
             in_brick = false;
             return;
         }
-        word = ld_keep(index.table + (in_brick ? cur_brick + c : (uint32_t)cell), pol_keep);
-        if (in_brick)
-            group = ld_keep(index.table + (cur_brick + kBrickCells + (c >> 3)), pol_keep);
+        cell = ((ux >> (kPosBits - 3 * L)) & (side << (2 * L))) |
+               ((uy >> (kPosBits - 2 * L)) & (side << L)) | ((uz >> (kPosBits - L)) & side);
+        in_brick = cell == cur_cell;
+        const int s3 = kPosBits - kBrickLevels - L;
+        const uint32_t c = ((ux >> (s3 - 6)) & 0x1c0u) | ((uy >> (s3 - 3)) & 0x38u) |
+                           ((uz >> s3) & 7u);
+        entry = ld_keep(index.table + (in_brick ? cur_brick + c : cell), pol_keep);
     };
 
     // Takes the first n (<= 32) collected items as the batch in flight and requests their
@@ -385,17 +387,19 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         const bool active = lane < nb;
         const int at = (head == 0 ? 64 : head - 32) + lane;     // item of this lane
         const uint32_t b_slot = q.slot[at];
-        const float b_w = q.w[at];
         const int b_own = q.owner[at];
-        const float b_T = (BWD || LOG) ? q.T[(BWD || LOG) ? at : 0] : 0.f;
-        float b_dd = (BWD || LOG) ? q.dd[(BWD || LOG) ? at : 0] : 0.f;
         float* row = q.rows + lane * Shape::STRIDE;
         const int off = record_offset<K>(tr.data, b_slot);
         const int own = b_own & 31;
         const bool acc_item = BWD && (b_own & 0x80) != 0;
         float sg[3] = {0.f, 0.f, 0.f}, col[3] = {0.f, 0.f, 0.f};
-        float raw_sigma = 0.f;
+        float raw_sigma = 0.f, att = 0.f, b_dd = 0.f;
         if (active) {
+            const float delta_t = q.dt[at], sigma = q.sigma[at],
+                        delta_scale = q.rayv[own][WQ::SCALE];
+            b_dd = delta_t * delta_scale;
+            att = BWD ? expf(-delta_t * sigma * delta_scale)
+                      : expf(-delta_t * delta_scale * sigma);
             float tmp[3] = {0.f, 0.f, 0.f};
             if (BD == 0) {
                 const float4 x = *reinterpret_cast<const float4*>(row);
@@ -434,14 +438,13 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 col[ch] = sg[ch] * d_rgb_pad - opt.rgb_padding;
             }
             if (!BWD) {
-                *reinterpret_cast<float4*>(row) = make_float4(col[0], col[1], col[2], b_w);
-                if (tr.weight_accum != nullptr) accumulate_weight(tr, b_slot, b_w);
+                *reinterpret_cast<float4*>(row) = make_float4(col[0], col[1], col[2], att);
             } else {
                 float total_color = 0.f;
 #pragma unroll
                 for (int ch = 0; ch < 3; ++ch) total_color += col[ch] * q.rayv[own][BD + ch];
                 *reinterpret_cast<float4*>(row) =
-                    make_float4(total_color, b_w, acc_item ? -1.f : b_T, b_dd);
+                    make_float4(total_color, att, acc_item ? 1.f : 0.f, b_dd);
             }
         }
         __syncwarp();
@@ -450,20 +453,35 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             float4* res = reinterpret_cast<float4*>(q.rows + (__ffs(m) - 1) * Shape::STRIDE);
             const float4 x = *res;
             if (!BWD) {
-                a0 = __fmaf_rn(x.w, x.x, a0);
-                a1 = __fmaf_rn(x.w, x.y, a1);
-                a2 = __fmaf_rn(x.w, x.z, a2);
-                if (LOG) *res = make_float4(a0, a1, a2, 0.f);
-            } else if (x.z < 0.f) {
-                a0 += x.y * x.x;
+                // res->w: the transmittance before the item, 0 where the ray has stopped
+                const float before = stopped ? 0.f : light;
+                const float weight = before * (1.f - x.w);
+                if (!stopped) {
+                    a0 = __fmaf_rn(weight, x.x, a0);
+                    a1 = __fmaf_rn(weight, x.y, a1);
+                    a2 = __fmaf_rn(weight, x.z, a2);
+                    light = light * x.w;
+                    stopped = light <= opt.stop_thresh;
+                }
+                if (LOG) *res = make_float4(a0, a1, a2, before);
+                else if (tr.weight_accum != nullptr) res->w = before;
             } else {
-                a0 -= x.y * x.x;
-                res->x = x.w * (x.x * x.z - a0);    // density gradient
+                const float weight = light * (1.f - x.y);
+                light = light * x.y;
+                if (x.z != 0.f) {
+                    a0 += weight * x.x;
+                } else {
+                    a0 -= weight * x.x;
+                    res->x = x.w * (x.x * light - a0);    // density gradient
+                    res->y = weight;
+                }
             }
         }
         mine_fly = 0u;
         fly = 0;
         __syncwarp();
+        if (!BWD && tr.weight_accum != nullptr && active)
+            accumulate_weight(tr, b_slot, row[3] * (1.f - att));
         if (LOG) {
             // lane i writes the packet of item i, now that its ray's colour sums are known: to
             // place i of the batch's chunk, or to the next place of its bin
@@ -524,6 +542,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             }
             if (active && group_id < log_limit) {
                 const float4 sums = *reinterpret_cast<const float4*>(row);
+                const float b_w = sums.w * (1.f - att), b_T = sums.w * att;
                 // the step length carries d softplus / d raw density, the one factor the
                 // density gradient needs from the raw value (svox/csrc/rt_kernel.cu:469-470)
                 if (opt.density_softplus) b_dd *= sigmoid_ref(raw_sigma - 1);
@@ -549,7 +568,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             // lane i forms the gradient of record i in its staging row
             const int goff = record_offset<K>(grad_data, b_slot);
             if (active && !acc_item) {
-                const float gs = row[0];
+                const float gs = row[0], b_w = row[1];
                 float v[K];
 #pragma unroll
                 for (int ch = 0; ch < 3; ++ch) {
@@ -592,10 +611,11 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         }
     };
 
+    unsigned alive = __ballot_sync(0xffffffffu, state != kExhausted);
     for (;;) {
         // ---- lanes that are not marching: finish, refill, termination ---------------------
         unsigned marching = __ballot_sync(0xffffffffu, state == kMarching);
-        const unsigned waiting = __ballot_sync(0xffffffffu, state == kNeedRay || state == kEnded);
+        const unsigned waiting = alive & ~marching;
         if (marching == 0u || __popc(waiting) >= shape.refill) {
             if (__any_sync(0xffffffffu, state == kEnded && (mine | mine_next | mine_fly) != 0u)) {
                 __syncwarp();
@@ -646,7 +666,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                     } else {
                         march_ready(r);
                         state = kMarching;
-                        t = r.tmin; light = 1.f; it = 0; stopped = false;
+                        t = r.tmin; light = ahead = 1.f; it = 0; stopped = false;
+                        q.rayv[lane][WQ::SCALE] = r.delta_scale;
                         place_cursor();
                         request_words();
                         if (BD > 0) {
@@ -679,124 +700,81 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             }
             __syncwarp();
             marching = __ballot_sync(0xffffffffu, state == kMarching);
+            alive = __ballot_sync(0xffffffffu, state != kExhausted);
             if (marching == 0u) {
-                if (__all_sync(0xffffffffu, state == kExhausted)) break;
+                if (alive == 0u) break;
                 continue;
             }
         }
 
         // ---- G step: every lane consumes the words requested one iteration ago --------------
-        bool item = false;
-        uint32_t slot = 0;
-        float weight = 0.f, dd = 0.f;
-        if (state == kMarching) {
-            bool go = true;
-            if (!in_brick && word < 0) {
-                // the table cell has a brick: the sample is looked up there
-                cur_cell = table_cell(bits(px), bits(py), bits(pz));
-                cur_brick = index.bricks + (uint32_t)(word & 0x7fffffff) * kBrickWords;
-            } else {
-                const uint32_t ux = bits(px), uy = bits(py), uz = bits(pz);
-                int depth = in_brick ? L + 1 + (int)((uint32_t)group >> 28) : word - kWordEmpty;
-                float sigma = __int_as_float(word);
-                bool full = word <= kWordInf;       // passes the density test
-                bool fail = false, have_slot = false;
-                if ((full && !in_brick) || word >= kWordWalk) {
-                    // seldom in refined scenes: an occupied leaf in the table itself, a tree
-                    // deeper than the index, a density that is not in the word
-                    if (word == kWordWalk) {
-                        const bool from_group =
-                            in_brick && ((uint32_t)group >> 28) == kBrickLevels - 1;
-                        const float big = (float)(1 << 24);
-                        const Walked f = walk_to_leaf(
-                            tr.child, tr.data, K, tr.M, from_group ? (group & 0x0fffffff) : 0,
-                            from_group ? L + kBrickLevels - 1 : 0, (int)(px * big),
-                            (int)(py * big), (int)(pz * big));
-                        fail = !f.ok;
-                        slot = f.slot;
-                        have_slot = true;
-                        depth = f.depth;
-                        sigma = opt.density_softplus ? softplus_m1(f.raw) : f.raw;
-                        full = sigma > (BWD ? 0.f : opt.sigma_thresh);
-                    } else {
-                        if (!in_brick) {
-                            const int hs = kPosBits - L + 1, hL = L - 1;
-                            const uint32_t hside = side >> 1;
-                            group = ld_keep(
-                                index.table + (index.groups +
-                                               (((((ux >> hs) & hside) << hL |
-                                                  ((uy >> hs) & hside)) << hL) |
-                                                ((uz >> hs) & hside))), pol_keep);
-                            depth = 1 + (int)((uint32_t)group >> 28);
-                        }
-                        if (word >= kWordFetch) {
-                            full = true;
-                            slot = group & 0x0fffffff;
-                            const int b = kPosBits - depth;
-                            if (depth == (in_brick ? L + kBrickLevels : L))
-                                slot = slot * 8 + ((((ux >> b) & 1) << 2) |
-                                                   (((uy >> b) & 1) << 1) | ((uz >> b) & 1));
-                            have_slot = true;
-                            sigma = __ldg(tr.data + (size_t)slot * K + (K - 1));
-                            if (opt.density_softplus) sigma = softplus_m1(sigma);
-                        }
-                    }
-                }
-                float gx, gy, gz;                   // offset from the leaf's lower corner
-                if (depth <= kPosBits) {
-                    const uint32_t keep = 0xffffffffu << (kPosBits - depth);
-                    gx = __fsub_rn(px, __fsub_rn(__uint_as_float(ux & keep), 1.0f));
-                    gy = __fsub_rn(py, __fsub_rn(__uint_as_float(uy & keep), 1.0f));
-                    gz = __fsub_rn(pz, __fsub_rn(__uint_as_float(uz & keep), 1.0f));
-                } else {                        // 2^-24 leaves: a float resolves them below 1/2
-                    const float big = (float)(1 << 24);
-                    gx = __fsub_rn(px, truncf(px * big) * (1.f / big));
-                    gy = __fsub_rn(py, truncf(py * big) * (1.f / big));
-                    gz = __fsub_rn(pz, truncf(pz * big) * (1.f / big));
-                }
-                // Exit distance of the leaf (_dda_unit, svox/csrc/rt_kernel.cu:203-220, in the
-                // leaf's own scale).  The point lies inside, so the entry distance is 0 and per
-                // axis the larger of t1 = -f*inv and t1 + inv is t1 + max(inv, 0); powers of
-                // two commute with rounding, so everything can be done at the tree's scale.
-                const float inv_cube = __int_as_float((127 - depth) << 23);  // 2^-depth
-                const float ex = __fmaf_rn(fmaxf(r.ix, 0.f), inv_cube, __fmul_rn(-gx, r.ix));
-                const float ey = __fmaf_rn(fmaxf(r.iy, 0.f), inv_cube, __fmul_rn(-gy, r.iy));
-                const float ez = __fmaf_rn(fmaxf(r.iz, 0.f), inv_cube, __fmul_rn(-gz, r.iz));
-                const float delta_t = __fadd_rn(fminf(ex, fminf(ey, ez)), opt.step_size);
-                t = __fadd_rn(t, delta_t);
-                bool done = fail || !(t < r.tmax);
-                if (full && !fail) {
-                    if (!have_slot) {
-                        slot = group & 0x0fffffff;
-                        const int b = kPosBits - depth;
-                        if (depth == (in_brick ? L + kBrickLevels : L))
-                            slot = slot * 8 + ((((ux >> b) & 1) << 2) | (((uy >> b) & 1) << 1) |
-                                               ((uz >> b) & 1));
-                    }
-                    dd = delta_t * r.delta_scale;
-                    const float att = BWD ? expf(-delta_t * sigma * r.delta_scale)
-                                          : expf(-delta_t * r.delta_scale * sigma);
-                    weight = light * (1.f - att);
-                    light *= att;
-                    item = true;
-                    if (!BWD && light <= opt.stop_thresh) {
-                        stopped = true;
-                        done = true;
-                    }
-                }
-                if (++it > kMaxSteps) {
-                    report(SVOXB_ERR_MARCH);
-                    done = true;
-                }
-                if (done) {
-                    state = kEnded;
-                    go = false;
-                } else {
-                    place_cursor();
-                }
-            }
-            if (go) request_words();
+        // (without branches but for the rare cases: lanes that have nothing to do compute along)
+        bool on = state == kMarching;
+        if (on && !in_brick && entry.x < 0) {
+            // the table cell has a brick: the sample is looked up there
+            cur_cell = cell;
+            cur_brick = index.bricks + (uint32_t)(entry.x & 0x7fffffff) * kBrickCells;
+            on = false;
         }
+        int depth = (int)((uint32_t)entry.y >> 28) + (in_brick ? L : 0);
+        uint32_t slot = (uint32_t)entry.y & 0x0fffffffu;
+        float sigma = __int_as_float(entry.x);
+        bool item = on && entry.x <= kWordInf;      // the leaf passes the density test
+        bool done = false;
+        uint32_t ux = bits(px), uy = bits(py), uz = bits(pz);
+        if (on && entry.x >= kWordFetch) {
+            // seldom: a tree deeper than the index, a density that is not in the word
+            float raw = 0.f;
+            if (entry.x == kWordWalk) {
+                const float big = (float)(1 << 24);
+                const Walked f = walk_to_leaf(
+                    tr.child, tr.data, K, tr.M, depth > L ? (int64_t)slot : 0,
+                    depth > L ? depth - 1 : 0, (int)(px * big), (int)(py * big), (int)(pz * big));
+                done = !f.ok;
+                slot = f.slot;
+                depth = f.ok ? f.depth : 1;
+                raw = f.raw;
+            } else {
+                raw = __ldg(tr.data + (size_t)slot * K + (K - 1));
+            }
+            sigma = opt.density_softplus ? softplus_m1(raw) : raw;
+            item = !done && sigma > (BWD ? 0.f : opt.sigma_thresh);
+        }
+        // lower corner of the leaf, offset of the sample from it
+        const uint32_t keep = 0xffffffffu << (kPosBits - (depth < kPosBits ? depth : kPosBits));
+        float cx = __fsub_rn(__uint_as_float(ux & keep), 1.0f);
+        float cy = __fsub_rn(__uint_as_float(uy & keep), 1.0f);
+        float cz = __fsub_rn(__uint_as_float(uz & keep), 1.0f);
+        if (depth > kPosBits) {                     // 2^-24 leaves: a float resolves them below 1/2
+            const float big = (float)(1 << 24);
+            cx = truncf(px * big) * (1.f / big);
+            cy = truncf(py * big) * (1.f / big);
+            cz = truncf(pz * big) * (1.f / big);
+        }
+        // Exit distance of the leaf (_dda_unit, svox/csrc/rt_kernel.cu:203-220, in the leaf's own
+        // scale).  The point lies inside, so the entry distance is 0 and per axis the larger of
+        // t1 = -f*inv and t1 + inv is t1 + max(inv, 0); powers of two commute with rounding, so
+        // everything can be done at the tree's scale.
+        const float inv_cube = __int_as_float((127 - depth) << 23);  // 2^-depth
+        const float ex = __fmaf_rn(fmaxf(r.ix, 0.f), inv_cube, __fmul_rn(__fsub_rn(cx, px), r.ix));
+        const float ey = __fmaf_rn(fmaxf(r.iy, 0.f), inv_cube, __fmul_rn(__fsub_rn(cy, py), r.iy));
+        const float ez = __fmaf_rn(fmaxf(r.iz, 0.f), inv_cube, __fmul_rn(__fsub_rn(cz, pz), r.iz));
+        const float delta_t = __fadd_rn(fminf(ex, fminf(ey, ez)), opt.step_size);
+        if (on) {
+            t = __fadd_rn(t, delta_t);
+            if (!(t < r.tmax)) done = true;
+            if (early && item) {
+                ahead *= expf(-delta_t * r.delta_scale * sigma);
+                if (ahead <= opt.stop_thresh) done = true;
+            }
+            if (++it > kMaxSteps) {
+                report(SVOXB_ERR_MARCH);
+                done = true;
+            }
+            if (done) state = kEnded;
+        }
+        place_cursor();
+        if (state == kMarching) request_words();
 
         // ---- push items --------------------------------------------------------------
         const unsigned pushed = __ballot_sync(0xffffffffu, item);
@@ -804,8 +782,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             const int n = qn + __popc(pushed & ((1u << lane) - 1u));
             const int pos = head + n < WQ::CAP ? head + n : head + n - WQ::CAP;
             q.slot[pos] = slot;
-            q.w[pos] = weight;
-            if (BWD || LOG) { q.T[pos] = light; q.dd[pos] = dd; }
+            q.dt[pos] = delta_t;
+            q.sigma[pos] = sigma;
             q.owner[pos] = (unsigned char)(lane | ((BWD && phase == 0) ? 0x80 : 0));
             const unsigned bit = 1u << (n & 31);
             if (n < 32) mine |= bit;

@@ -38,6 +38,9 @@ struct RenderCall {
     int64_t log_capacity = 0;
     // forward with a scratch built earlier by svoxb_render_scratch_build (else per call)
     const int32_t* prepared = nullptr;
+    // logged forward: buffers like `data` to clear on `clear_stream` beside the march
+    float* clear[2] = {nullptr, nullptr};
+    cudaStream_t clear_stream = nullptr;
     // marching backward as the fallback of a replay: does its work only if this log overflowed
     LogGate gate{};
 };
@@ -98,13 +101,9 @@ static int validate_options(const svoxb_tree* t, const svoxb_render_options& o) 
 
 template <class Kernel>
 static int persistent_grid(Kernel kernel, int block, size_t smem, int64_t n_gran, unsigned* grid) {
-    // the 48 KB a kernel gets without asking cover its static shared memory too (up to 4 KB here)
-    if (smem > 40 * 1024)
-        SVOXB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
     int per_sm = 0;
-    SVOXB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem));
-    if (per_sm < 1) per_sm = 1;
+    const int st = blocks_per_sm(reinterpret_cast<const void*>(kernel), block, smem, &per_sm);
+    if (st) return st;
     int sms = sm_count() - g_reserved_sms;     // see svoxb_reserve_sms
     if (sms < 1) sms = 1;
     int64_t g = (int64_t)sms * per_sm;
@@ -318,6 +317,30 @@ struct QueueScratch {
     ~QueueScratch() { if (mem) cudaFreeAsync(mem, stream); }
 };
 
+// Clears the buffers of a logged forward once the index is built, behind the launch of the march,
+// which leaves most of the memory bandwidth and many places on the SMs unused.  (Started before
+// the index the fill put its blocks in front of it and delayed the march by all of its time.)
+struct ClearBeside {
+    const RenderCall& c;
+    cudaEvent_t ready = nullptr;
+
+    int index_built() {
+        if (!c.clear[0]) return SVOXB_OK;
+        SVOXB_CUDA(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        SVOXB_CUDA(cudaEventRecord(ready, c.stream));
+        return SVOXB_OK;
+    }
+    int march_launched() {
+        if (!c.clear[0]) return SVOXB_OK;
+        SVOXB_CUDA(cudaStreamWaitEvent(c.clear_stream, ready, 0));
+        const size_t n = (size_t)c.tree->M * 8 * (size_t)c.tree->K;
+        for (float* to : c.clear)
+            if (to) SVOXB_CUDA(cudaMemsetAsync(to, 0, n * sizeof(float), c.clear_stream));
+        return SVOXB_OK;
+    }
+    ~ClearBeside() { if (ready) cudaEventDestroy(ready); }
+};
+
 template <class Source>
 static int launch_queue(const RenderCall& c, const Source& src) {
     const IndexLayout layout = QueueScratch::layout(c.tree);
@@ -333,8 +356,11 @@ static int launch_queue(const RenderCall& c, const Source& src) {
         mem = scratch.mem;
     }
     TreeIndex index = layout.view(mem);
-    if (mem == nullptr) index = TreeIndex{nullptr, 0, 0, 1};
-    return with_basis(c.opt, [&](auto basis) {
+    if (mem == nullptr) index = TreeIndex{nullptr, 0, 1};
+    ClearBeside clear{c};
+    int st = clear.index_built();
+    if (st) return st;
+    st = with_basis(c.opt, [&](auto basis) {
         constexpr int BD = decltype(basis)::value;
         if constexpr (BD > 0) {
             if (c.opt.format != SVOXB_FORMAT_SH)
@@ -342,6 +368,7 @@ static int launch_queue(const RenderCall& c, const Source& src) {
         }
         return launch_mode<BD>(c, src, index);
     });
+    return st ? st : clear.march_launched();
 }
 
 template <int BLOCK, class Source>
@@ -612,7 +639,8 @@ static int log_eligible(const svoxb_tree* t, const svoxb_render_options* o, cons
 template <class Source>
 static int logged_forward(const svoxb_tree* tree, const Source& src, int64_t Q,
                           const svoxb_render_options* opt, float* out, int32_t* log,
-                          int64_t capacity_chunks, void* stream) {
+                          int64_t capacity_chunks, void* stream, float* clear0 = nullptr,
+                          float* clear1 = nullptr, void* clear_stream = nullptr) {
     int st = validate_tree(tree);
     if (st) return st;
     if ((st = validate_options(tree, *opt))) return st;
@@ -626,6 +654,9 @@ static int logged_forward(const svoxb_tree* tree, const Source& src, int64_t Q,
     c.stream = (cudaStream_t)stream;
     c.log = log;
     c.log_capacity = capacity_chunks;
+    c.clear[0] = clear0;
+    c.clear[1] = clear1;
+    c.clear_stream = (cudaStream_t)clear_stream;
     return launch_queue(c, src);
 }
 
@@ -711,6 +742,28 @@ int svoxb_volume_render_image_logged(const svoxb_tree* tree, const svoxb_camera*
     return logged_forward(tree, PixelRays{cam->c2w, cam->fx, cam->fy, cam->width, cam->height},
                           (int64_t)cam->width * cam->height, opt, out, log, capacity_chunks,
                           stream);
+}
+
+int svoxb_volume_render_logged_clear(const svoxb_tree* tree, const svoxb_rays* rays,
+                                     const svoxb_render_options* opt, float* out, int32_t* log,
+                                     int64_t capacity_chunks, void* stream, float* clear0,
+                                     float* clear1, void* clear_stream) {
+    if (!tree || !rays || !opt || !clear0) return SVOXB_ERR_NULL;
+    if (rays->Q > 0 && (!rays->origins || !rays->dirs || !rays->vdirs)) return SVOXB_ERR_NULL;
+    if (rays->Q <= 0) return SVOXB_ERR_SHAPE;
+    return logged_forward(tree, RayBatch{rays->origins, rays->dirs, rays->vdirs}, rays->Q, opt,
+                          out, log, capacity_chunks, stream, clear0, clear1, clear_stream);
+}
+
+int svoxb_volume_render_image_logged_clear(const svoxb_tree* tree, const svoxb_camera* cam,
+                                           const svoxb_render_options* opt, float* out,
+                                           int32_t* log, int64_t capacity_chunks, void* stream,
+                                           float* clear0, float* clear1, void* clear_stream) {
+    if (!tree || !cam || !opt || !cam->c2w || !clear0) return SVOXB_ERR_NULL;
+    if (cam->width <= 0 || cam->height <= 0) return SVOXB_ERR_SHAPE;
+    return logged_forward(tree, PixelRays{cam->c2w, cam->fx, cam->fy, cam->width, cam->height},
+                          (int64_t)cam->width * cam->height, opt, out, log, capacity_chunks,
+                          stream, clear0, clear1, clear_stream);
 }
 
 int svoxb_volume_render_backward_replay(const svoxb_tree* tree, const svoxb_rays* rays,
