@@ -119,6 +119,13 @@ int svoxb_query_vertical_backward(const svoxb_tree* tree, const float* indices, 
                                   const float* grad_output, int32_t Kg, float* grad_data_out,
                                   int zero_first, void* stream);
 
+/* The same for leaves that are known: node_ids (Q) are the packed ids that
+ * svoxb_query_vertical returned for the points (no counterpart in the
+ * reference, which descends again). */
+int svoxb_query_scatter(const svoxb_tree* tree, const int64_t* node_ids, int64_t Q,
+                        const float* grad_output, int32_t Kg, float* grad_data_out, int zero_first,
+                        void* stream);
+
 /* assign_vertical (svox/csrc/svox_kernel.cu:80-89,145-158): overwrite the first
  * Kv floats (1 <= Kv <= K) of the record of each point's leaf with row q of
  * values (Q, Kv).  data_out is the tree's own data array (writable).  Points

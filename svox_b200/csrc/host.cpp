@@ -29,7 +29,7 @@ using std::optional;
 // The library's functions, from the file that the Python side has loaded.
 struct Library {
 #define SVOXB_FUNCTIONS(X)                                                                      \
-    X(query_vertical) X(query_vertical_backward) X(volume_render) X(volume_render_image)        \
+    X(query_vertical) X(query_vertical_backward) X(query_scatter) X(volume_render) X(volume_render_image)        \
     X(volume_render_prepared) X(volume_render_image_prepared) X(volume_render_backward)         \
     X(volume_render_image_backward) X(volume_render_logged) X(volume_render_image_logged)       \
     X(volume_render_backward_replay) X(volume_render_image_backward_replay)                     \
@@ -540,6 +540,8 @@ class RenderNode : public torch::autograd::Function<RenderNode> {
 
 struct QueryCall {
     Tree tree;
+    Tensor ids;                // the leaves found, for as long as nobody writes to them or to
+    uint32_t ids_version = 0, child_version = 0;   // the tree's structure
 };
 
 class QueryNode : public torch::autograd::Function<QueryNode> {
@@ -550,6 +552,9 @@ class QueryNode : public torch::autograd::Function<QueryNode> {
         auto [values, ids] = run_query(call->tree, indices);
         ctx->mark_non_differentiable({ids});
         ctx->save_for_backward({indices});
+        call->ids = ids;
+        call->ids_version = ids._version();
+        call->child_version = call->tree.child._version();
         keep(ctx, std::move(call));
         return {values, ids};
     }
@@ -557,8 +562,16 @@ class QueryNode : public torch::autograd::Function<QueryNode> {
                                                    torch::autograd::variable_list grads) {
         if (!ctx->needs_input_grad(0)) return {Tensor(), Tensor(), Tensor()};
         QueryCall& c = *kept<std::shared_ptr<QueryCall>>(ctx);
-        return {run_query_backward(c.tree, ctx->get_saved_variables()[0], grads[0].contiguous(), {}),
-                Tensor(), Tensor()};
+        const Tensor indices = ctx->get_saved_variables()[0], grad_out = grads[0].contiguous();
+        if (c.ids._version() != c.ids_version || c.tree.child._version() != c.child_version)
+            return {run_query_backward(c.tree, indices, grad_out, {}), Tensor(), Tensor()};
+        const c10::cuda::CUDAGuard guard(indices.device());
+        Tensor grad = at::empty(c.tree.data.sizes(), grad_out.options());
+        check(lib.query_scatter(&c.tree.c, c.ids.data_ptr<int64_t>(), c.ids.numel(),
+                                grad_out.data_ptr<float>(), c.tree.c.K, grad.data_ptr<float>(), 1,
+                                stream_of(indices)),
+              "query_scatter");
+        return {grad, Tensor(), Tensor()};
     }
 };
 

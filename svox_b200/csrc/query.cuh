@@ -5,15 +5,17 @@
 // point's K-float record with a per-thread scalar loop, so every warp
 // instruction touches 32 different cache lines on both sides.  Here a thread
 // still descends for its own point, but the records of a warp's 32 points
-// are then moved by the whole warp: lane l handles elements l, l+32, ... of
-// the warp's contiguous (32, K) output block, so stores are fully coalesced
-// and loads walk each record contiguously.
+// are then moved by the whole warp, so that loads and stores run along rows.
+// The backward works on the leaf ids that the forward found.
 //
 // HBM roofline per point: 12 B in + K*4 B gathered + K*4 B written + 8 B id
-// (+ one 4-B child entry per level below the jump table, L2 resident).
+// (+ one 4-B child entry per level below the jump table, L2 resident).  2^24 points over 256^3
+// leaves of 49 floats, 268 of the 196 bytes per record read (64-byte pieces): 1.75 -> 1.63 ms.
+// Backward: 3.43 ms (clear, then reductions at random) -> 2.77 ms (binned, see below).
 #pragma once
 
 #include "common.cuh"
+#include "binned.cuh"
 
 namespace svoxb {
 
@@ -71,108 +73,90 @@ __device__ __forceinline__ int64_t locate_point(const TreeArgs& tr, const TopTab
     return ok ? hit.slot : -1;
 }
 
-// MODE 0: copy records out (forward).  MODE 1: scatter-add rows in (backward).
-// MODE 2: overwrite the first Kg floats of each point's record with its row of `grad_out`
-// (assign_single_kernel, svox/csrc/svox_kernel.cu:80-89; points that share a leaf race, as in
-// the reference).
-template <int MODE>
+// Records are fetched in 64-byte pieces of L2 lines (without the hint the L2 reads 128 bytes for
+// each of these scattered pieces).
+__device__ __forceinline__ float ld_row(const float* a) {
+    float v;
+    asm volatile("ld.global.nc.L2::64B.f32 %0, [%1];" : "=f"(v) : "l"(a));
+    return v;
+}
+
+// Forward: the records of the points' leaves, row by row.  G lanes copy a row, STEPS elements
+// each (0: as many as it takes); PASSES of them are under way at a time, loads first.  A flat walk
+// over the warp's output block, with a division's worth of index arithmetic per element, spent
+// 74 instructions per point of 49 floats and 73 % of the issue slots.
+template <int G, int STEPS>
 __global__ void __launch_bounds__(kQueryBlock)
 query_kernel(TreeArgs tr, TopTable top, const float* __restrict__ pts, int64_t Q,
-             float* __restrict__ values_out, int64_t* __restrict__ ids_out,
-             const float* __restrict__ grad_out, float* __restrict__ grad_data, int Kg) {
+             float* __restrict__ values_out, int64_t* __restrict__ ids_out) {
     const int64_t i = (int64_t)blockIdx.x * kQueryBlock + threadIdx.x;
     const int lane = threadIdx.x & 31;
     int64_t slot = -1;
     if (i < Q) {
         slot = locate_point(tr, top, pts, i);
-        if (MODE == 0 && ids_out != nullptr && slot >= 0) ids_out[i] = slot;
+        if (ids_out != nullptr) ids_out[i] = slot;      // -1: not a tree
     }
-    if (MODE == 0 && values_out == nullptr) return;
+    const int64_t wb = i - lane;            // first point of this warp
+    if (values_out == nullptr || wb >= Q) return;
+    const int K = tr.K;
+    const int sub = lane / G, e = lane % G;
+    constexpr int ROWS = 32 / G;            // rows per pass
+    constexpr int N = STEPS > 0 ? STEPS : 1;
+    constexpr int PASSES = G < 8 / N ? G : 8 / N;
+    const int n = (int)(Q - wb < 32 ? Q - wb : 32);
+    float* __restrict__ out = values_out + wb * K;
+    for (int base = 0; STEPS > 0 ? base == 0 : base < K; base += G) {
+#pragma unroll 1
+        for (int p0 = 0; p0 < G; p0 += PASSES) {
+            float v[PASSES][N];
+#pragma unroll
+            for (int p = 0; p < PASSES; ++p) {
+                const int k = (p0 + p) * ROWS + sub;
+                const int64_t s = __shfl_sync(0xffffffffu, slot, k);
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    v[p][j] = 0.f;
+                    if (s >= 0 && base + e + j * G < K)
+                        v[p][j] = ld_row(tr.data + s * K + (base + e + j * G));
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < PASSES; ++p) {
+                const int k = (p0 + p) * ROWS + sub;
+                // (a point without a leaf -- not a tree -- leaves its row as it is)
+                const bool there = __shfl_sync(0xffffffffu, slot, k) >= 0;
+#pragma unroll
+                for (int j = 0; j < N; ++j)
+                    if (k < n && there && base + e + j * G < K)
+                        out[k * K + (base + e + j * G)] = v[p][j];
+            }
+        }
+    }
+}
 
-    // Warp-cooperative record move.  `wb` is the first point of this warp.
+// Overwrites the first Kv floats of each point's record with its row of `values`
+// (assign_single_kernel, svox/csrc/svox_kernel.cu:80-89; points that share a leaf race, as in the
+// reference).
+__global__ void __launch_bounds__(kQueryBlock)
+assign_kernel(TreeArgs tr, TopTable top, const float* __restrict__ pts, int64_t Q,
+              const float* __restrict__ values, float* __restrict__ data_out, int Kv) {
+    const int64_t i = (int64_t)blockIdx.x * kQueryBlock + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int64_t slot = i < Q ? locate_point(tr, top, pts, i) : -1;
     const int64_t wb = i - lane;
     if (wb >= Q) return;
-    const int K = (MODE == 0) ? tr.K : Kg;
+    // lanes walk the warp's block of rows in order: coalesced reads, and writes that are
+    // contiguous within each record
     const int nvalid = (int)((Q - wb) < 32 ? (Q - wb) : 32);
-    if (MODE == 2) {
-        // lanes walk the warp's (nvalid, Kg) block of rows in order: coalesced reads, and
-        // writes that are contiguous within each record
-        const int total = nvalid * K;
-        int p = 0, e = lane;
-        while (e >= K) { e -= K; ++p; }
-        for (int base = 0; base < total; base += 32) {        // warp-uniform trip count
-            const int j = base + lane;
-            const int64_t s = __shfl_sync(0xffffffffu, slot, p < nvalid ? p : nvalid - 1);
-            if (j < total && s >= 0) grad_data[s * tr.K + e] = __ldg(grad_out + wb * K + j);
-            e += 32;
-            while (e >= K) { e -= K; ++p; }
-        }
-        return;
-    }
-    if (MODE == 1) {
-        // Backward: add row p of the upstream gradient into the record of point p's leaf.  A
-        // record is K floats at 4-byte alignment, so each is cut into at most 3 single floats
-        // up to the next 16-byte boundary, whole 16-byte words (one vector reduction each,
-        // a quarter of the requests of scalar atomics) and at most 3 single floats behind
-        // them.  Lanes take these pieces of the warp's 32 records round robin.
-        const int per_point = 6 + (K >> 2);        // 3 head + K/4 word + 3 tail places
-        const bool vec_ok = (reinterpret_cast<uintptr_t>(grad_data) & 15) == 0;
-        const int n_units = nvalid * per_point;
-        for (int base = 0; base < n_units; base += 32) {       // warp-uniform trip count
-            const int u = base + lane;
-            const int p = u < n_units ? u / per_point : 0, j = u - p * per_point;
-            const int64_t s = __shfl_sync(0xffffffffu, slot, p);
-            if (u >= n_units || s < 0) continue;
-            const int64_t first = s * K;                       // destination, in floats
-            int head = vec_ok ? (int)((4 - (first & 3)) & 3) : 0;
-            if (head > K) head = K;
-            const int words = vec_ok ? (K - head) >> 2 : 0;
-            const float* __restrict__ src = grad_out + (wb + p) * K;
-            if (j < 3) {
-                if (j < head && j < K) atomicAdd(grad_data + first + j, __ldg(src + j));
-            } else if (j < 3 + (K >> 2)) {
-                const int w = j - 3;
-                if (w < words) {
-                    const int e = head + 4 * w;
-                    red_add_v4(grad_data + first + e, __ldg(src + e), __ldg(src + e + 1),
-                               __ldg(src + e + 2), __ldg(src + e + 3));
-                } else if (!vec_ok) {                           // unaligned buffer: scalars
-                    for (int e = 4 * w; e < 4 * w + 4 && e < K; ++e)
-                        atomicAdd(grad_data + first + e, __ldg(src + e));
-                }
-            } else {
-                const int e = (vec_ok ? head + 4 * words : 4 * (K >> 2)) + (j - 3 - (K >> 2));
-                if (e < K) atomicAdd(grad_data + first + e, __ldg(src + e));
-            }
-        }
-        return;
-    }
-    const int total = nvalid * K;
-    int p = 0, e = lane;  // element j = p*K + e of the warp's (nvalid, K) block
-    while (e >= K) { e -= K; ++p; }
-    // Batches of kBatch steps: all loads of a batch are issued before the first store, so that
-    // a warp keeps kBatch 128-byte requests in flight (the path is bound by memory latency).
-    constexpr int kBatch = 8;
-    for (int base = 0; base < total; base += 32 * kBatch) {
-        float v[kBatch];
-        int64_t dst[kBatch];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            const int j = base + 32 * u + lane;
-            const int src_lane = p < nvalid ? p : nvalid - 1;
-            const int64_t s = __shfl_sync(0xffffffffu, slot, src_lane);
-            dst[u] = -1;
-            v[u] = 0.f;
-            if (j < total && s >= 0) {
-                v[u] = __ldg(tr.data + s * K + e);
-                dst[u] = wb * K + j;
-            }
-            e += 32;
-            while (e >= K) { e -= K; ++p; }
-        }
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-            if (dst[u] >= 0) values_out[dst[u]] = v[u];
+    const int total = nvalid * Kv;
+    int p = 0, e = lane;
+    while (e >= Kv) { e -= Kv; ++p; }
+    for (int base = 0; base < total; base += 32) {        // warp-uniform trip count
+        const int j = base + lane;
+        const int64_t s = __shfl_sync(0xffffffffu, slot, p < nvalid ? p : nvalid - 1);
+        if (j < total && s >= 0) data_out[s * tr.K + e] = __ldg(values + wb * Kv + j);
+        e += 32;
+        while (e >= Kv) { e -= Kv; ++p; }
     }
 }
 
@@ -209,9 +193,10 @@ __global__ void calc_corners_kernel(const int32_t* __restrict__ parent_depth, in
     out[3 * i + 2] = r[2];
 }
 
-static int launch_query(int mode, const svoxb_tree* tree, const float* indices, int64_t Q,
-                        float* values_out, int64_t* ids_out, const float* grad_out,
-                        float* grad_data, int Kg, cudaStream_t stream) {
+// Query, or with `rows` assignment.
+static int launch_query(const svoxb_tree* tree, const float* indices, int64_t Q,
+                        float* values_out, int64_t* ids_out, const float* rows, float* data_out,
+                        int Kv, cudaStream_t stream) {
     if (Q == 0) return SVOXB_OK;
     if (!indices) return SVOXB_ERR_NULL;
     if ((Q + kQueryBlock - 1) / kQueryBlock > 0x7fffffffLL) return SVOXB_ERR_TOO_LARGE;
@@ -224,20 +209,262 @@ static int launch_query(int mode, const svoxb_tree* tree, const float* indices, 
     if (st) return st;
     const TopTable tt{top.cells, top.level};
     const unsigned grid = (unsigned)((Q + kQueryBlock - 1) / kQueryBlock);
-    if (mode == 0)
-        query_kernel<0><<<grid, kQueryBlock, 0, stream>>>(tree_args(tree), tt, indices, Q,
-                                                          values_out, ids_out, nullptr,
-                                                          nullptr, 0);
-    else if (mode == 2)
-        query_kernel<2><<<grid, kQueryBlock, 0, stream>>>(tree_args(tree), tt, indices, Q,
-                                                          nullptr, nullptr, grad_out,
-                                                          grad_data, Kg);
-    else
-        query_kernel<1><<<grid, kQueryBlock, 0, stream>>>(tree_args(tree), tt, indices, Q,
-                                                          nullptr, nullptr, grad_out,
-                                                          grad_data, Kg);
+    auto forward = [&](auto kernel) {
+        kernel<<<grid, kQueryBlock, 0, stream>>>(tree_args(tree), tt, indices, Q, values_out,
+                                                 ids_out);
+    };
+    const int K = tree->K;
+    if (rows != nullptr)
+        assign_kernel<<<grid, kQueryBlock, 0, stream>>>(tree_args(tree), tt, indices, Q, rows,
+                                                        data_out, Kv);
+    else if (K <= 2) forward(query_kernel<2, 1>);
+    else if (K <= 4) forward(query_kernel<4, 1>);
+    else if (K <= 8) forward(query_kernel<8, 1>);
+    else if (K <= 16) forward(query_kernel<16, 1>);
+    else if (K <= 32) forward(query_kernel<32, 1>);
+    else if (K <= 64) forward(query_kernel<32, 2>);
+    else if (K <= 96) forward(query_kernel<32, 3>);
+    else forward(query_kernel<32, 0>);
     SVOXB_CUDA(cudaGetLastError());
     return SVOXB_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Backward of the query: row q of the upstream gradient is added into record ids[q].
+
+// 32 rows of a warp.  Groups of G lanes take a row each; lane w adds the 16-byte word w of the
+// record's place in memory (with zeros where the word reaches beyond the record), a quarter of
+// the requests of scalar atomics.  `slot` < 0: no row.
+template <int G>
+__device__ __forceinline__ void add_rows(int64_t slot, int64_t row, int n,
+                                         const float* __restrict__ rows, int K,
+                                         float* __restrict__ grad, int64_t n_floats, bool vec_ok,
+                                         uint64_t pol) {
+    const int lane = threadIdx.x & 31;
+    const int sub = lane / G, w = lane % G;
+#pragma unroll 4
+    for (int p = 0; p < G; ++p) {
+        const int k = p * (32 / G) + sub;
+        const int64_t s = __shfl_sync(0xffffffffu, slot, k);
+        const int64_t r = __shfl_sync(0xffffffffu, row, k);
+        if (k >= n || s < 0) continue;
+        const float* __restrict__ src = rows + r * K;
+        const int64_t first = s * K;
+        const int off = vec_ok ? (int)(first & 3) : 0;
+        for (int word = w; 4 * word < off + K; word += G) {
+            const int e = 4 * word - off;
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = e + i >= 0 && e + i < K ? ld_row(src + e + i) : 0.f;
+            float* to = grad + first + e;
+            if (vec_ok && first + e + 4 <= n_floats) {
+                red_add_v4_hint(to, v[0], v[1], v[2], v[3], pol);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (e + i >= 0 && e + i < K) atomicAdd(to + i, v[i]);
+            }
+        }
+    }
+}
+
+template <int G>
+__global__ void __launch_bounds__(kQueryBlock)
+scatter_rows_kernel(const int64_t* __restrict__ ids, int64_t Q, const float* __restrict__ rows,
+                    int K, float* __restrict__ grad, int64_t n_slots) {
+    const int64_t i = (int64_t)blockIdx.x * kQueryBlock + threadIdx.x;
+    const int64_t wb = i - (threadIdx.x & 31);
+    if (wb >= Q) return;
+    int64_t slot = i < Q ? ids[i] : -1;
+    if (slot >= n_slots) slot = -1;
+    add_rows<G>(slot, i, 32, rows, K, grad, n_slots * K,
+                (reinterpret_cast<uintptr_t>(grad) & 15) == 0, l2_policy_stream());
+}
+
+// Many rows into a gradient that outgrows the L2: the points are sorted into bins first (count,
+// place), then their rows are added bin by bin, each bin cleared on the way (binned.cuh).
+struct RowBins {
+    int32_t* count;      // [kMaxBins]
+    int32_t* cursor;     // [kMaxBins]
+    UnitCounters units;
+    int2* pair;          // [Q] {slot, row}
+    int shift, n_bins;
+};
+constexpr int kBinRows = 2048;       // points a block sorts at a time
+
+__global__ void __launch_bounds__(256)
+count_rows_kernel(const int64_t* __restrict__ ids, int64_t Q, int64_t n_slots, RowBins b) {
+    __shared__ int s_count[kMaxBins];
+    for (int i = threadIdx.x; i < kMaxBins; i += 256) s_count[i] = 0;
+    __syncthreads();
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < Q; i += (int64_t)gridDim.x * 256) {
+        const int64_t slot = ids[i];
+        if (slot >= 0 && slot < n_slots) atomicAdd(&s_count[(int)(slot >> b.shift)], 1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < b.n_bins; i += 256)
+        if (s_count[i]) atomicAdd(b.count + i, s_count[i]);
+}
+
+__global__ void __launch_bounds__(256)
+place_rows_kernel(const int64_t* __restrict__ ids, int64_t Q, int64_t n_slots, RowBins b) {
+    __shared__ int s_first[kMaxBins], s_count[kMaxBins];
+    for (int i = threadIdx.x; i < kMaxBins; i += 256) s_first[i] = b.count[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int run = 0;
+        for (int i = 0; i < kMaxBins; ++i) {
+            const int n = s_first[i];
+            s_first[i] = run;
+            run += n;
+        }
+    }
+    for (int64_t tile = blockIdx.x; tile * kBinRows < Q; tile += gridDim.x) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < kMaxBins; i += 256) s_count[i] = 0;
+        __syncthreads();
+        int slot[kBinRows / 256], rank[kBinRows / 256];
+#pragma unroll
+        for (int j = 0; j < kBinRows / 256; ++j) {
+            const int64_t i = tile * kBinRows + 256 * j + threadIdx.x;
+            const int64_t s = i < Q ? ids[i] : -1;
+            slot[j] = s >= 0 && s < n_slots ? (int)s : -1;
+            rank[j] = slot[j] >= 0 ? atomicAdd(&s_count[slot[j] >> b.shift], 1) : 0;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < b.n_bins; i += 256)
+            if (s_count[i] > 0) s_count[i] = s_first[i] + atomicAdd(b.cursor + i, s_count[i]);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kBinRows / 256; ++j)
+            if (slot[j] >= 0)
+                b.pair[s_count[slot[j] >> b.shift] + rank[j]] =
+                    make_int2(slot[j], (int)(tile * kBinRows + 256 * j + threadIdx.x));
+    }
+}
+
+template <int G>
+__global__ void __launch_bounds__(kQueryBlock)
+scatter_binned_rows_kernel(int64_t Q, const float* __restrict__ rows, int K,
+                           float* __restrict__ grad, int64_t n_slots, RowBins b, int per_warp) {
+    __shared__ UnitShared s_units;
+    const int lane = threadIdx.x & 31;
+    const uint64_t pol_keep = l2_policy_keep();
+    auto clear = [&](int64_t from, int64_t until) {
+        const int4 none = make_int4(0, 0, 0, 0);
+        int64_t i = from + 4 * threadIdx.x;
+        for (; i + 4 <= until; i += 4 * kQueryBlock) st_hint16(grad + i, none, pol_keep);
+        for (; i < until; ++i) grad[i] = 0.f;      // the end of a buffer of odd length
+    };
+    auto work = [&](int first, int end) {
+        first += (threadIdx.x >> 5) * per_warp * 32;
+        for (int j = 0; j < per_warp; ++j, first += 32) {
+            const int n = end - first < 32 ? end - first : 32;
+            if (n <= 0) break;
+            int2 p = make_int2(0, 0);
+            if (lane < n) p = __ldg(b.pair + first + lane);
+            add_rows<G>(p.x, p.y, n, rows, K, grad, n_slots * K, true, pol_keep);
+        }
+    };
+    ordered_units<kQueryBlock>(s_units, b.units, 0, b.n_bins, 0, kQueryBlock * per_warp,
+                               ((int64_t)1 << b.shift) * K, n_slots * K,
+                               [&](int i) { return b.count[i]; }, clear, work);
+}
+
+// Calls f with the lanes per row that suit K floats.
+template <int N>
+struct Lanes { static constexpr int value = N; };
+template <class F>
+static int with_row_lanes(int K, F f) {
+    const int words = (K + 3 + 3) / 4;
+    if (words <= 2) return f(Lanes<2>{});
+    if (words <= 4) return f(Lanes<4>{});
+    if (words <= 8) return f(Lanes<8>{});
+    if (words <= 16) return f(Lanes<16>{});
+    return f(Lanes<32>{});
+}
+
+static int zero_rows(float* grad, int64_t n_floats, cudaStream_t stream) {
+    SVOXB_CUDA(cudaMemsetAsync(grad, 0, (size_t)n_floats * sizeof(float), stream));
+    return SVOXB_OK;
+}
+
+static int launch_scatter(const svoxb_tree* tree, const int64_t* ids, int64_t Q, const float* rows,
+                          int K, float* grad, bool zero_first, cudaStream_t stream) {
+    const int64_t n_slots = tree->M * tree->N * tree->N * tree->N, n_floats = n_slots * K;
+    // Binned where the gradient outgrows the L2 and a good part of its records is touched (at
+    // least every eighth or so, with 8 * 16 bytes of sorting against 260 of every row).
+    const bool binned = zero_first && n_floats * 4 >= (96LL << 20) && Q >= n_slots / 4 &&
+                        Q < (1LL << 31) - kBinRows && n_slots < (1LL << 31) &&
+                        reinterpret_cast<uintptr_t>(grad) % 16 == 0;
+    int st;
+    if (!binned) {
+        if (zero_first && (st = zero_rows(grad, n_floats, stream))) return st;
+        if (Q == 0) return SVOXB_OK;
+        const int64_t grid = (Q + kQueryBlock - 1) / kQueryBlock;
+        if (grid > 0x7fffffffLL) return SVOXB_ERR_TOO_LARGE;
+        return with_row_lanes(K, [&](auto lanes) {
+            scatter_rows_kernel<decltype(lanes)::value><<<(unsigned)grid, kQueryBlock, 0, stream>>>(
+                ids, Q, rows, K, grad, n_slots);
+            SVOXB_CUDA(cudaGetLastError());
+            return (int)SVOXB_OK;
+        });
+    }
+    if ((st = keep_pool_cached())) return st;
+    RowBins b{};
+    b.shift = 2;                          // a bin is a whole number of 16-byte words
+    while ((2LL << b.shift) * K * 4 <= ((int64_t)kReplayBinMB << 20)) ++b.shift;
+    while (((n_slots - 1) >> b.shift) + 1 > kMaxBins) ++b.shift;
+    b.n_bins = (int)(((n_slots - 1) >> b.shift) + 1);
+    constexpr int kHead = 3 * kMaxBins + 32;
+    int32_t* mem = nullptr;
+    SVOXB_CUDA(cudaMallocAsync((void**)&mem, (kHead + 2 * (size_t)Q) * sizeof(int32_t), stream));
+    b.count = mem;
+    b.cursor = mem + kMaxBins;
+    b.units = UnitCounters{mem + 3 * kMaxBins, mem + 3 * kMaxBins + 1, mem + 2 * kMaxBins};
+    b.pair = reinterpret_cast<int2*>(mem + kHead);
+    st = [&] {
+        SVOXB_CUDA(cudaMemsetAsync(mem, 0, kHead * sizeof(int32_t), stream));
+        const int sms = sm_count();
+        int64_t grid = (Q + 256 * 16 - 1) / (256 * 16);
+        if (grid > 8LL * sms) grid = 8LL * sms;
+        count_rows_kernel<<<(unsigned)grid, 256, 0, stream>>>(ids, Q, n_slots, b);
+        grid = (Q + kBinRows - 1) / kBinRows;
+        if (grid > 8LL * sms) grid = 8LL * sms;
+        place_rows_kernel<<<(unsigned)grid, 256, 0, stream>>>(ids, Q, n_slots, b);
+        SVOXB_CUDA(cudaGetLastError());
+        return with_row_lanes(K, [&](auto lanes) {
+            auto k = scatter_binned_rows_kernel<decltype(lanes)::value>;
+            int per_sm = 0;
+            const int s2 = blocks_per_sm(reinterpret_cast<const void*>(k), kQueryBlock, 0, &per_sm);
+            if (s2) return s2;
+            const int blocks = sms * per_sm;
+            // rows a warp takes per unit: the grid's window stays below a bin
+            int64_t per_warp = Q / b.n_bins / ((int64_t)blocks * kQueryBlock);
+            per_warp = per_warp < 1 ? 1 : per_warp > 4 ? 4 : per_warp;
+            k<<<(unsigned)blocks, kQueryBlock, 0, stream>>>(Q, rows, K, grad, n_slots, b,
+                                                            (int)per_warp);
+            SVOXB_CUDA(cudaGetLastError());
+            return (int)SVOXB_OK;
+        });
+    }();
+    cudaFreeAsync(mem, stream);
+    return st;
+}
+
+// The same from the points themselves.
+static int launch_query_backward(const svoxb_tree* tree, const float* indices, int64_t Q,
+                                 const float* rows, int K, float* grad, bool zero_first,
+                                 cudaStream_t stream) {
+    if (Q == 0) return launch_scatter(tree, nullptr, 0, rows, K, grad, zero_first, stream);
+    int st = keep_pool_cached();
+    if (st) return st;
+    int64_t* ids = nullptr;
+    SVOXB_CUDA(cudaMallocAsync((void**)&ids, (size_t)Q * sizeof(int64_t), stream));
+    st = launch_query(tree, indices, Q, nullptr, ids, nullptr, nullptr, 0, stream);
+    if (st == SVOXB_OK) st = launch_scatter(tree, ids, Q, rows, K, grad, zero_first, stream);
+    cudaFreeAsync(ids, stream);
+    return st;
 }
 
 }  // namespace svoxb

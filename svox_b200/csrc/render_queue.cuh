@@ -35,6 +35,7 @@
 
 #include "render.cuh"
 #include "render_index.cuh"
+#include "binned.cuh"
 
 namespace svoxb {
 
@@ -87,7 +88,6 @@ struct RecordShape {
 constexpr int kMaxParts = 16;   // the scatter can run in up to 16 parts (bin ranges)
 constexpr int kLogNext = 32;
 constexpr int kLogBins = kLogNext + 2 * kMaxParts;
-constexpr int kMaxBins = 128;
 constexpr int kLogCleared = kLogBins + kMaxBins;
 constexpr int kLogCounts = kLogCleared + kMaxBins;
 constexpr int kPacketWords = 12;
@@ -117,29 +117,14 @@ struct LogArgs {
     int shift = 0, n_bins = 1;
 };
 
-// L2 residency hints.  The index (tens of MB, re-read hundreds of times per launch) must stay
-// in L2 while the leaf records and gradients (GBs, touched a few times each) stream through it.
-__device__ __forceinline__ uint64_t l2_policy_keep() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-__device__ __forceinline__ uint64_t l2_policy_stream() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
+// The index (tens of MB, re-read hundreds of times per launch) must stay in L2 while the leaf
+// records and gradients (GBs, touched a few times each) stream through it.
 __device__ __forceinline__ int2 ld_keep(const int2* a, uint64_t pol) {
     int2 v;
     asm volatile("ld.global.nc.L2::cache_hint.v2.s32 {%0, %1}, [%2], %3;"
                  : "=r"(v.x), "=r"(v.y)
                  : "l"(a), "l"(pol));
     return v;
-}
-__device__ __forceinline__ void st_hint16(void* a, int4 v, uint64_t pol) {
-    asm volatile("st.global.L2::cache_hint.v4.s32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(a), "r"(v.x),
-                 "r"(v.y), "r"(v.z), "r"(v.w), "l"(pol)
-                 : "memory");
 }
 // The 64-byte L2 fetch granularity is a measured choice: records are 112-196 bytes at arbitrary
 // 16-byte offsets, and the logged forward of the training step runs 1 % faster with it than with the
@@ -150,13 +135,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, uint64_
                  "l"(gmem), "l"(pol)
                  : "memory");
 }
-__device__ __forceinline__ void red_add_v4_hint(float* addr, float a, float b, float c, float d,
-                                                uint64_t pol) {
-    asm volatile("red.global.add.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(addr),
-                 "f"(a), "f"(b), "f"(c), "f"(d), "l"(pol)
-                 : "memory");
-}
-
 // Adds the 16-byte word `word` of a gradient row to its place.  The row holds the record's K
 // floats from offset `off` on, zeros around them; `rec` is the record's first float.  With a
 // gradient buffer that is not 16-byte aligned the record's floats go one by one.

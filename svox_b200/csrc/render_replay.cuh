@@ -25,7 +25,6 @@ namespace svoxb {
 
 constexpr int kScatterBlock = 256;
 constexpr int kScatterBatches = 8;   // batches of 32 packets a warp takes at a time at most
-constexpr int kZeroFloats = 16384;   // floats a block clears at a time
 constexpr int kOrderTile = 1024;     // groups a block of the order kernel takes at a time
 
 // First bin of part p when n_bins bins are cut into n_parts ranges.
@@ -103,20 +102,10 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
     const uint64_t pol_keep = l2_policy_keep();
     const float d_rgb_pad = 1 + 2 * opt.rgb_padding;
     constexpr int WARPS = BLOCK / 32;
-    // Units of work, taken by blocks in order from one counter, so that the whole grid works
-    // within a window much smaller than a bin (with a fixed assignment the blocks drift apart and
-    // the gradient of several bins competes for L2: 2.9 ms for the 2^20-ray step instead of 1.7;
-    // with a unit per warp the counter itself is the bound, some 6 ns per unit).
-    // s_start[b]: first unit of bin b; with `zero` its units are the clearing of bin b + 1
-    // followed by the packets of bin b, and the clearing of the first bin comes before all.
-    __shared__ int s_start[kMaxBins + 1];
-    __shared__ int s_group[kMaxBins + 1];   // first group of bin b in the order
-    __shared__ int s_zero[kMaxBins + 1];    // units of clearing of bin b
+    __shared__ UnitShared s_units;
     const bool overflow = (int64_t)log[0] > capacity;     // then no packet counts
     const int n_bins = log[3] > kMaxBins ? kMaxBins : log[3];
     const bool sorted = n_bins > 1;
-    const bool zero = to.zero_slots > 0 && sorted;
-    const int64_t bin_floats = ((int64_t)1 << log[2]) * K, all_floats = to.zero_slots * K;
     const int lo_bin = sorted ? replay_part_first_bin(part, n_parts, n_bins) : 0,
               hi_bin = sorted ? replay_part_first_bin(part + 1, n_parts, n_bins) : 1;
     // batches of 32 packets a warp takes per unit, and per group
@@ -124,95 +113,30 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
     const int share = chunks / ((int)gridDim.x * WARPS * (sorted ? n_bins : 4));
     const int per_group = sorted ? kSortedChunks : 1;
     const int per_warp = share < 1 ? 1 : share > kScatterBatches ? kScatterBatches : share;
-    const int groups_per_unit = WARPS * per_warp / per_group;
-    for (int b = threadIdx.x; b <= kMaxBins; b += BLOCK) {
-        const int64_t left = all_floats - b * bin_floats;
-        s_zero[b] = zero && b < hi_bin
-                        ? (int)(((left < bin_floats ? left : bin_floats) + kZeroFloats - 1) / kZeroFloats)
-                        : 0;
-        s_group[b] = overflow || b >= hi_bin ? 0 : sorted ? log[kLogBins + b] : chunks;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int group = 0;
-        for (int b = 0; b < lo_bin; ++b) group += s_group[b];
-        int unit = s_zero[lo_bin];
-        for (int b = lo_bin; b < hi_bin; ++b) {
-            const int n = s_group[b];
-            s_start[b] = unit;
-            s_group[b] = group;
-            unit += s_zero[b + 1];
-            unit += (n + groups_per_unit - 1) / groups_per_unit;
-            group += n;
-        }
-        s_start[hi_bin] = unit;
-        s_group[hi_bin] = group;
-    }
     const int32_t* __restrict__ counts = log + kLogCounts;
     const int32_t* __restrict__ order = log + log_order_at(capacity);
     const int4* __restrict__ packets =
         reinterpret_cast<const int4*>(log + log_packets_at(capacity));
-    int32_t* next = log + kLogNext + part;
-    int32_t* cleared = log + kLogCleared;
-    __shared__ int s_unit, s_bin, s_place;   // the unit, its bin, its place among the bin's units
-    int taken = 0, at_bin = lo_bin, ready = -1;   // thread 0; `ready`: bin known to be cleared
-    if (threadIdx.x == 0) taken = atomicAdd(next, 1);
-
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const int unit = taken;
-            int bin = lo_bin, u = unit, z = s_start[lo_bin];       // clearing of the first bin
-            if (unit >= z && unit < s_start[hi_bin]) {
-                while (unit >= s_start[at_bin + 1]) ++at_bin;    // a block's units ascend
-                bin = at_bin;
-                u = unit - s_start[bin];
-                z = s_zero[bin + 1];
-                if (u < z) {
-                    ++bin;
-                } else if (zero && bin != ready) {
-                    // the bin's units of clearing were all taken before this one, and a block
-                    // works on its units in order; they are usually long done
-                    const int want = s_zero[bin];
-                    int tries = 0;
-                    while (*(volatile int32_t*)(cleared + bin) < want && ++tries < (1 << 22))
-                        __nanosleep(64);
-                    if (tries == (1 << 22)) report(SVOXB_ERR_CUDA);
-                    __threadfence();
-                    ready = bin;
-                }
-            }
-            s_unit = unit;
-            s_bin = bin;
-            s_place = u - z;
+    int groups_before = 0;
+    for (int b = 0; b < lo_bin && !overflow; ++b) groups_before += log[kLogBins + b];
+    const UnitCounters counters{log + kLogNext + part, log + kLogNext + kMaxParts + part,
+                                log + kLogCleared};
+    auto count = [&](int b) { return overflow ? 0 : sorted ? log[kLogBins + b] : chunks; };
+    auto clear = [&](int64_t from, int64_t until) {
+        const int4 none = make_int4(0, 0, 0, 0);
+        for (int64_t i = from + 4 * threadIdx.x; i < until; i += 4 * BLOCK) {
+            if (!HESS || to.grad != nullptr) st_hint16(to.grad + i, none, pol_keep);
+            if (HESS) st_hint16(to.hess + i, none, pol_keep);
         }
-        __syncthreads();
-        const int unit = s_unit, bin = s_bin, u = s_place;
-        if (unit >= s_start[hi_bin]) break;
-        if (threadIdx.x == 0) taken = atomicAdd(next, 1);      // arrives during this unit's work
-        if (u < 0) {
-            const int64_t from = bin * bin_floats + (int64_t)(u + s_zero[bin]) * kZeroFloats;
-            int64_t until = from + kZeroFloats;
-            if (until > (bin + 1) * bin_floats) until = (bin + 1) * bin_floats;
-            if (until > all_floats) until = all_floats;
-            const int4 none = make_int4(0, 0, 0, 0);
-            for (int64_t i = from + 4 * threadIdx.x; i < until; i += 4 * BLOCK) {
-                if (!HESS || to.grad != nullptr) st_hint16(to.grad + i, none, pol_keep);
-                if (HESS) st_hint16(to.hess + i, none, pol_keep);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                __threadfence();
-                atomicAdd(cleared + bin, 1);
-            }
-            continue;
-        }
+    };
+    auto work = [&](int first, int end) {
         // lane j: first packet and length of the warp's batch j
         int64_t at = 0;
         int len = 0;
         {
             const int batch = (threadIdx.x >> 5) * per_warp + lane;
-            const int i = s_group[bin] + u * groups_per_unit + batch / per_group;
-            if (lane < per_warp && i < s_group[bin + 1]) {
+            const int i = first + batch / per_group;
+            if (lane < per_warp && i < end) {
                 const int g = sorted ? __ldg(order + i) : i;
                 const int sub = batch % per_group;
                 at = ((int64_t)g * per_group + sub) * 32;
@@ -222,10 +146,10 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
         }
         int4 na = make_int4(0, 0, 0, 0), nb = na, nc = na;
         auto fetch = [&](int j) {
-            const int64_t first = __shfl_sync(0xffffffffu, at, j);
+            const int64_t packet = __shfl_sync(0xffffffffu, at, j);
             const int m = __shfl_sync(0xffffffffu, len, j);
             if (lane < m) {
-                const int4* __restrict__ p = packets + (first + lane) * (kPacketWords / 4);
+                const int4* __restrict__ p = packets + (packet + lane) * (kPacketWords / 4);
                 na = __ldg(p); nb = __ldg(p + 1); nc = __ldg(p + 2);
             }
         };
@@ -336,19 +260,10 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
             if constexpr (HESS) flush(to.hess, sm.rows + 32 * Shape::STRIDE, hoff);
             __syncwarp();
         }
-        __syncthreads();
-    }
-    // the last block puts the counters back
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        int32_t* done = log + kLogNext + kMaxParts + part;
-        if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
-            *next = 0;
-            *done = 0;
-            for (int b = lo_bin; b < hi_bin; ++b) cleared[b] = 0;
-        }
-    }
+    };
+    ordered_units<BLOCK>(s_units, counters, lo_bin, hi_bin, groups_before,
+                         WARPS * per_warp / per_group, ((int64_t)1 << log[2]) * K,
+                         sorted ? to.zero_slots * K : 0, count, clear, work);
 }
 
 }  // namespace svoxb

@@ -469,7 +469,7 @@ int svoxb_query_vertical(const svoxb_tree* tree, const float* indices, int64_t Q
     int st = validate_tree(tree);
     if (st) return st;
     if (Q < 0) return SVOXB_ERR_SHAPE;
-    return launch_query(0, tree, indices, Q, values_out, node_ids_out, nullptr, nullptr, 0,
+    return launch_query(tree, indices, Q, values_out, node_ids_out, nullptr, nullptr, 0,
                         (cudaStream_t)stream);
 }
 
@@ -480,9 +480,20 @@ int svoxb_query_vertical_backward(const svoxb_tree* tree, const float* indices, 
     if (st) return st;
     if (Q < 0 || Kg < 1) return SVOXB_ERR_SHAPE;
     if (!grad_data_out || (Q > 0 && !grad_output)) return SVOXB_ERR_NULL;
-    if (zero_first && (st = zero_grad(tree, grad_data_out, Kg, (cudaStream_t)stream))) return st;
-    return launch_query(1, tree, indices, Q, nullptr, nullptr, grad_output, grad_data_out, Kg,
-                        (cudaStream_t)stream);
+    if (Q > 0 && !indices) return SVOXB_ERR_NULL;
+    return launch_query_backward(tree, indices, Q, grad_output, Kg, grad_data_out, zero_first != 0,
+                                 (cudaStream_t)stream);
+}
+
+int svoxb_query_scatter(const svoxb_tree* tree, const int64_t* node_ids, int64_t Q,
+                        const float* grad_output, int32_t Kg, float* grad_data_out, int zero_first,
+                        void* stream) {
+    int st = validate_tree(tree);
+    if (st) return st;
+    if (Q < 0 || Kg < 1) return SVOXB_ERR_SHAPE;
+    if (!grad_data_out || (Q > 0 && (!grad_output || !node_ids))) return SVOXB_ERR_NULL;
+    return launch_scatter(tree, node_ids, Q, grad_output, Kg, grad_data_out, zero_first != 0,
+                          (cudaStream_t)stream);
 }
 
 int svoxb_assign_vertical(const svoxb_tree* tree, const float* indices, int64_t Q,
@@ -491,7 +502,7 @@ int svoxb_assign_vertical(const svoxb_tree* tree, const float* indices, int64_t 
     if (st) return st;
     if (Q < 0 || Kv < 1 || Kv > tree->K) return SVOXB_ERR_SHAPE;
     if (!data_out || (Q > 0 && !values)) return SVOXB_ERR_NULL;
-    return launch_query(2, tree, indices, Q, nullptr, nullptr, values, data_out, Kv,
+    return launch_query(tree, indices, Q, nullptr, nullptr, values, data_out, Kv,
                         (cudaStream_t)stream);
 }
 
