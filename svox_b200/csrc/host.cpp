@@ -358,13 +358,15 @@ struct Zeroed {
         for (int i = 0; i < count; ++i) buffers.push_back(at::empty(like.sizes(), like.options()));
     }
     float* pointer(size_t i) { return i < buffers.size() ? buffers[i].data_ptr<float>() : nullptr; }
-    // After the call that enqueued the fills.  Should a tensor be dropped before anyone waited for
-    // its fill, its memory must not be handed out again while the side stream still writes to it.
-    void enqueued() {
-        done.record(side);
+    Zeroed(const Zeroed&) = delete;
+    // A buffer dropped before anyone waited for its fill: its memory must not be handed out again
+    // while the side stream still writes to it.
+    ~Zeroed() {
         for (const Tensor& b : buffers)
-            c10::cuda::CUDACachingAllocator::recordStream(b.storage().data_ptr(), side);
+            if (b.defined())
+                c10::cuda::CUDACachingAllocator::recordStream(b.storage().data_ptr(), side);
     }
+    void enqueued() { done.record(side); }      // after the call that enqueued the fills
     Tensor claim(size_t i) {
         done.block(at::cuda::getCurrentCUDAStream(buffers[i].device().index()));
         return std::move(buffers[i]);

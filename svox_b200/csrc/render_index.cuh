@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256)
 build_table_kernel(const int32_t* __restrict__ child, const float* __restrict__ data, int K,
                    int64_t M, int L, float thresh, int softplus, int brick_cap,
                    int2* __restrict__ table, int32_t* __restrict__ counter,
-                   int32_t* __restrict__ roots, LogGate gate) {
+                   int32_t* __restrict__ roots, const uint8_t* __restrict__ marks, LogGate gate) {
     if (gate.closed()) return;
     const bool fits = M < kIndexMaxNodes;
     const int S = (1 << L) - 1;
@@ -103,7 +103,7 @@ build_table_kernel(const int32_t* __restrict__ child, const float* __restrict__ 
             }
             node += e;
             if (node < 0 || node >= M) break;             // corrupt: reported by the march
-            if (b == 0 && brick_cap > 0) {
+            if (b == 0 && brick_cap > 0 && (marks == nullptr || marks[idx] != 0)) {
                 const int id = atomicAdd(counter, 1);
                 if (id < brick_cap) {
                     roots[id] = (int32_t)node;
@@ -200,16 +200,18 @@ struct IndexLayout {
     }
 };
 
-// Launches the kernels that fill an index buffer.
+// Launches the kernels that fill an index buffer.  `marks`: only the marked table cells get
+// bricks.
 static int build_index(const svoxb_tree* t, const IndexLayout& l, float thresh, int softplus,
-                       int32_t* mem, LogGate gate, cudaStream_t s) {
+                       int32_t* mem, LogGate gate, cudaStream_t s,
+                       const uint8_t* marks = nullptr) {
     const int sms = sm_count();
     int32_t* counter = mem + l.counter;
     int32_t* roots = mem + l.roots;
     if (l.cap > 0) SVOXB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int32_t), s));
     build_table_kernel<<<index_grid(l.cells, 256, sms), 256, 0, s>>>(
         t->child, t->data, t->K, t->M, l.level, thresh, softplus, l.cap,
-        reinterpret_cast<int2*>(mem), counter, roots, gate);
+        reinterpret_cast<int2*>(mem), counter, roots, marks, gate);
     if (l.cap > 0)
         fill_bricks_kernel<<<index_grid((int64_t)l.cap * kBrickCells, 256, sms), 256, 0, s>>>(
             t->child, t->data, t->K, t->M, l.level, thresh, softplus, l.cap, counter, roots,

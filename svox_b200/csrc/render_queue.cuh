@@ -183,6 +183,32 @@ struct alignas(16) WarpQueue {
     float rayv[32][RAYW];
 };
 
+// Marks the table cells that the rays pass, at points a quarter of a cell apart: for a few rays
+// only these get bricks, instead of the whole scene.  A cell that is clipped between two points
+// goes unmarked; the march then walks the tree for its samples there.  One warp per ray.
+template <class Source>
+__global__ void __launch_bounds__(128)
+mark_cells_kernel(TreeArgs tr, Source src, svoxb_render_options opt, int64_t tickets, int L,
+                  uint8_t* __restrict__ marks) {
+    const int64_t ticket = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int64_t ray = ticket < tickets ? src.pick(ticket) : -1;
+    if (ray < 0) return;
+    Ray r;
+    src.load(ray, tr, opt, r);
+    ray_setup(r, tr.scaling);
+    if (!r.hit) return;
+    const int side = 1 << L;
+    const float step = 0.25f / (float)side;
+    for (int k = threadIdx.x & 31; k < 8 * side; k += 32) {      // a diagonal is sqrt(3) long
+        const float t = r.tmin + (float)k * step;
+        if (!(t < r.tmax)) break;
+        const int x = (int)(clamp01(r.ox + t * r.dx) * (float)side),
+                  y = (int)(clamp01(r.oy + t * r.dy) * (float)side),
+                  z = (int)(clamp01(r.oz + t * r.dz) * (float)side);
+        marks[(((x << L) + y) << L) + z] = 1;
+    }
+}
+
 enum { kNeedRay = 0, kMarching = 1, kEnded = 2, kExhausted = 3 };
 
 constexpr int kMarchBlock = 128;
