@@ -1,0 +1,210 @@
+"""The branches that a call's size, record length or history selects, at the sizes where they
+begin and end: each against the branch beside it, the definition in torch, or the marching
+backward.  Needs a GPU."""
+import numpy as np
+import pytest
+import torch
+
+import svox_b200 as svox
+from svox_b200 import csrc, render as _render
+from svox_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _shell(fmt, refine, extra, dev, seed=5):
+    gen = torch.Generator().manual_seed(seed)
+    return W.shell_tree(refine, extra, fmt, gen, (5.0, 50.0), W._SHELL).to(dev)
+
+
+def _rays(n, dev, seed=6):
+    gen = torch.Generator().manual_seed(seed)
+    return svox.Rays(*[t.to(dev) for t in W.sphere_rays(n, gen, 4.0, 0.2, 0.8)])
+
+
+def _close(a, b):
+    # sums of the same 32-bit terms in another order: 1e-5 of the largest element, the bound that
+    # the reference's own two runs of a backward keep (parity_util.assert_grad_matches_reference)
+    return (a - b).abs().max().item() <= 1e-5 * b.abs().max().item()
+
+
+def _grad(renderer, call, upstream):
+    renderer.tree.data.grad = None
+    call().backward(upstream)
+    return renderer.tree.data.grad
+
+
+@pytest.fixture(scope="module")
+def big_tree(cuda_device):
+    """512^3 shell of 1.3 M nodes with the shortest records (large enough for bricks only where
+    the rays pass)."""
+    return _shell("SH1", 5, 3, cuda_device)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1024])
+def test_bricks_where_a_few_rays_pass(n, big_tree, cuda_device):
+    r = svox.VolumeRenderer(big_tree)
+    rays = _rays(2048, cuda_device)                      # more rays: every brick
+    with torch.no_grad():
+        every = r(rays)
+        some = r(svox.Rays(*[t[:n].contiguous() for t in rays]))
+    assert torch.equal(some, every[:n])
+    csrc.check_device_status()
+
+
+@pytest.mark.parametrize("fmt,refine,n_rays", [("RGBA", 5, 50000), ("SH9", 4, 12000),
+                                               ("SH16", 4, 12000)])
+@pytest.mark.parametrize("image", [False, True])
+def test_sorted_log_unsorted_log_and_march_agree(fmt, refine, n_rays, image, cuda_device):
+    # 169 k (RGBA: 1.3 M) nodes: the gradient (169, 152, 266 MB) outgrows a bin, and the rays (or
+    # 400 x 300 pixels) touch enough of it for the log to be sorted and the gradient cleared on
+    # the way
+    tree = _shell(fmt, refine, 3, cuda_device)
+    r = svox.VolumeRenderer(tree)
+    if image:
+        c2w = W.look_at_cameras(1, torch.Generator().manual_seed(1), 1.6)[0].to(cuda_device)
+
+        def call():
+            return r.render_persp(c2w, width=400, height=300, fx=560.0)
+    else:
+        rays = _rays(n_rays, cuda_device)
+
+        def call():
+            return r(rays)
+    up = torch.randn(call().shape, generator=torch.Generator(cuda_device).manual_seed(2),
+                     device=cuda_device)
+    n = up.numel() // 3
+    lib = csrc.library()
+    assert csrc.log_is_sorted(tree._spec(), n, image)
+    a = _grad(r, call, up)
+    try:
+        assert lib.svoxb_test_knob(5, 1024) == 0         # one bin: nothing to sort
+        assert not csrc.log_is_sorted(tree._spec(), n, image)
+        b = _grad(r, call, up)
+    finally:
+        lib.svoxb_test_knob(5, 32)
+    _render.USE_ITEM_LOG = False
+    try:
+        c = _grad(r, call, up)
+    finally:
+        _render.USE_ITEM_LOG = True
+    assert _close(a, c) and _close(b, c)
+    csrc.check_device_status()
+
+
+@pytest.mark.parametrize("fmt", ["RGBA", "SH4"])
+@pytest.mark.parametrize("n", [50, 30000])
+def test_se_grad_through_either_log_and_without(fmt, n, cuda_device):
+    # few rays: unsorted log, results cleared beside the march; many: sorted; a log that is too
+    # small: the march enqueued behind the replay
+    tree = _shell(fmt, 4, 3, cuda_device)
+    r = svox.VolumeRenderer(tree)
+    rays = _rays(n, cuda_device)
+    colors = torch.rand(n, 3, generator=torch.Generator(cuda_device).manual_seed(3),
+                        device=cuda_device)
+    out, grad, hess = r.se_grad(rays, colors)
+    old = csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS
+    csrc.log_estimate(wait=True)
+    try:
+        csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS = 0.0, 2
+        out2, grad2, hess2 = r.se_grad(rays, colors)
+        csrc.log_estimate(wait=True)
+        assert csrc._LogWatch.last_used > csrc._LogWatch.last_cap
+    finally:
+        csrc.log_estimate(wait=True)
+        csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS = old
+    assert torch.equal(out, out2)
+    # the reference adds the density's gradient once per channel, the replay the channels' sum:
+    # 3e-4 of the summed magnitude in the parity tests, of the largest element here
+    assert (grad - grad2).abs().max() <= 3e-4 * grad2.abs().max()
+    assert (hess - hess2).abs().max() <= 3e-4 * hess2.abs().max()
+    csrc.check_device_status()
+
+
+@pytest.mark.parametrize("n", [40, 12000])
+def test_backward_twice_over_one_forward(n, cuda_device):
+    # a gradient cleared beside the forward is handed out once; a sorted log is replayed twice
+    tree = _shell("SH9", 4, 3, cuda_device)
+    r = svox.VolumeRenderer(tree)
+    out = r(_rays(n, cuda_device))
+    up = torch.ones_like(out)
+    tree.data.grad = None
+    out.backward(up, retain_graph=True)
+    first = tree.data.grad
+    tree.data.grad = None
+    out.backward(up)
+    assert _close(tree.data.grad, first)
+    csrc.check_device_status()
+
+
+def _query_reference(tree, pts, rows):
+    with torch.no_grad():
+        _, ids = tree(pts, want_node_ids=True)
+    want = torch.zeros(tree.child.numel(), rows.shape[1], dtype=torch.float64, device=pts.device)
+    want.index_add_(0, ids, rows.double())
+    return ids, want
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 4, 5, 8, 9, 16, 17, 28, 33, 49, 65, 76, 97, 130])
+@pytest.mark.parametrize("N", [2, 3])
+def test_query_rows_of_any_length(K, N, cuda_device):
+    tree = svox.N3Tree(N=N, data_dim=K, data_format=None, init_refine=2, device=cuda_device)
+    gen = torch.Generator(cuda_device).manual_seed(K)
+    tree.data.data.normal_(generator=gen)
+    flat = tree.data.data.view(-1, K)
+    for Q in (1, 31, 32, 33, 1000):
+        pts = torch.rand(Q, 3, generator=gen, device=cuda_device)
+        rows = torch.randn(Q, K, generator=gen, device=cuda_device)
+        ids, want = _query_reference(tree, pts, rows)
+        tree.data.grad = None
+        vals, ids2 = tree(pts, want_node_ids=True)
+        assert torch.equal(ids, ids2) and torch.equal(vals, flat[ids])
+        vals.backward(rows)
+        got = tree.data.grad.view(-1, K)
+        # a few 32-bit additions per element against double sums
+        assert (got - want).abs().max().item() <= 1e-6 * max(1.0, want.abs().max().item())
+        direct = csrc.query_vertical_backward(tree._spec(), pts, rows).view(-1, K)
+        assert (direct - want).abs().max().item() <= 1e-6 * max(1.0, want.abs().max().item())
+    csrc.check_device_status()
+
+
+@pytest.mark.parametrize("K", [97, 100])
+@pytest.mark.parametrize("Q", [74000, 75000, 300001])
+def test_query_backward_binned(K, Q, cuda_device):
+    # 299592 slots of about 400 bytes: 116 MB and more; binned from a quarter as many points on
+    tree = svox.N3Tree(data_dim=K, data_format=None, init_refine=5, device=cuda_device)
+    gen = torch.Generator(cuda_device).manual_seed(Q)
+    pts = torch.rand(Q, 3, generator=gen, device=cuda_device)
+    rows = torch.randn(Q, K, generator=gen, device=cuda_device)
+    _, want = _query_reference(tree, pts, rows)
+    tree(pts).backward(rows)
+    got = tree.data.grad.view(-1, K)
+    assert (got - want).abs().max().item() <= 2e-6 * max(1.0, want.abs().max().item())
+    csrc.check_device_status()
+
+
+def test_query_backward_after_the_ids_were_written_to(cuda_device):
+    tree, _ = W.config1()
+    tree = tree.to(cuda_device)
+    pts = torch.rand(500, 3, device=cuda_device)
+    vals, ids = tree(pts, want_node_ids=True)
+    rows = torch.randn_like(vals)
+    _, want = _query_reference(tree, pts, rows)
+    ids.zero_()                                          # the points are looked up again
+    tree.data.grad = None
+    vals.backward(rows)
+    assert (tree.data.grad.view(-1, tree.data_dim) - want).abs().max().item() <= 1e-5
+    csrc.check_device_status()
+
+
+def test_leaf_views_equal_indexing_by_coordinates(cuda_device):
+    tree, _ = W.config1()
+    tree = tree.to(cuda_device)
+    aux = torch.rand(tree.child.shape, device=cuda_device)
+    for key in (slice(None), slice(5, 400, 3), torch.tensor([3, 1, 2])):
+        view = tree[key]
+        at = tuple(k.to(cuda_device) for k in view.key)
+        assert torch.equal(view.values, tree.data[at]) and torch.equal(view.aux(aux), aux[at])
+    tree.data.grad = None
+    (tree[:].values * 2).sum().backward()
+    assert np.array_equal(tree.data.grad[tree.child == 0].unique().cpu().numpy(), [2.0])
