@@ -10,7 +10,10 @@
 namespace svoxb {
 
 constexpr int kMaxBins = 128;
-constexpr int kZeroFloats = 16384;   // floats a block clears at a time
+// Floats a block clears at a time.  Measured (scatter of 2^24 query rows, of an 800x800 SH16 view,
+// of se_grad for 100000 rays, of 2^20 rays; ms): 8192: 2.86, 1.44, 1.13, 1.86; 16384: 2.60, 1.35,
+// 1.13, 1.86; 65536: 2.40, 1.30, 1.10, 1.88.
+constexpr int kZeroFloats = 65536;
 
 // L2 residency hints.
 __device__ __forceinline__ uint64_t l2_policy_keep() {
