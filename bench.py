@@ -55,18 +55,15 @@ METRICS = {
     "image3": "Mrays/s render_persp forward (SH deg 3, 512^3 shell, 800x800 views)",
     "image5": "Mrays/s render_persp forward (SH deg 3, three shells at 1024^3, 1920x1080 views)",
 }
-# DRAM bytes (read + write) of one launch of the dominant kernel of the training step (the
-# logged forward march), from an ncu capture of a 2^17-ray launch (1.450 GB read + 0.353 GB
-# written) scaled by 8 to the 2^20-ray launch: its traffic grows with the rays.  The backward's
-# does not (the gradient is read and written once whatever the number of rays), so its figure
-# comes from a one-pass capture (DRAM bytes and duration only) of the two replay kernels at
-# full size: bin pass 3.583 GB read + 2.227 GB written, scatter 3.167 GB + 0.900 GB.
-# Printed only together with `traffic_source`, which names the capture.
-NCU_TRAFFIC = {"forward": 8 * (1.449616e9 + 0.352721e9),
-               "backward": 3.583350e9 + 2.226789e9 + 3.167486e9 + 0.900214e9}
-NCU_TRAFFIC_SOURCE = ("ncu --set full of render_queue_kernel<9,640,ForwardLogged> at 2^17 rays "
-                      "x 8 (profiles/training_step_rays131072_ncu_full.md); valid for the "
-                      "kernel as of library version " + "0.3.0")
+# DRAM bytes (read + write) of one launch of the training step's kernels: the logged march from an
+# ncu capture of a 2^17-ray launch (1.657 GB read + 0.381 GB written), scaled by 8 because its
+# traffic grows with the rays; the scatter's does not (the gradient is written once whatever the
+# number of rays), so no scaled figure is given for it.  Printed only together with
+# `traffic_source`, which names the capture.
+NCU_TRAFFIC = {"forward": 8 * (1.657470e9 + 0.381325e9), "backward": None}
+NCU_TRAFFIC_SOURCE = ("ncu --set full of render_queue_kernel<9,2,768> at 2^17 rays x 8 "
+                      "(profiles/training_step_rays131072_ncu_full.md); valid for the kernel as "
+                      "of library version " + "0.4.0")
 
 
 def parse():
@@ -469,10 +466,9 @@ def run_train(a):
     fwd_bytes = Q * 48 + 8 * sums[0].item() + 4 * (K - 1) * sums[1].item()
     bwd_bytes = Q * 48 + 8 * sums[0].item() + 8 * K * sums[2].item()
     # what THIS design's backward moves instead (it never re-reads records): per contributing
-    # sample the log entry (44 B) in, a 32-byte packet out and in again; per touched gradient
-    # element one read and one write; 96 B per ray of packed inputs
-    n_leaf_slots = int((tree.child[:tree.n_internal] == 0).sum().item())
-    replay_bytes = sums[2].item() * (44 + 32 + 32) + 2 * 4 * K * n_leaf_slots + Q * 96
+    # sample a 48-byte packet in; the gradient written once, its clearing included; 24 B per ray of
+    # upstream gradient and colours
+    replay_bytes = sums[2].item() * 48 + 4 * tree.data.numel() + Q * 24
 
     warm = max(a.warmup, 3)
     variants = {}
@@ -628,11 +624,10 @@ def run_train(a):
         # The backward replays the forward's item log.  `model_frac` divides the bytes of the
         # REFERENCE's backward (march again, re-read every record, accumulate the gradient once)
         # by this design's time: how much faster than that algorithm's roofline it runs.  The
-        # design's own traffic model (log in, packets out and in, touched gradient in and out)
-        # gives `achieved`, the bandwidth it really sustains.
+        # design's own traffic model (packets in, gradient out once) gives `achieved`, the
+        # bandwidth it really sustains.
         "roofline_backward": {"bound": "hbm",
-                              "kernel": "replay_bin_kernel + replay_scatter_kernel "
-                                        "(volume_render_backward)",
+                              "kernel": "replay_scatter_kernel (volume_render_backward)",
                               "achieved": replay_bytes / world / ms_bwd / 1e6, "peak": peak,
                               "unit": "GB/s", "frac": replay_bytes / world / ms_bwd / 1e6 / peak,
                               "bytes_of_this_design_per_launch": replay_bytes / world,
@@ -644,11 +639,11 @@ def run_train(a):
                           "achieved": (fwd_bytes + bwd_bytes) / ms_step / 1e6,
                           "frac": (fwd_bytes + bwd_bytes) / ms_step / 1e6 / (peak * world)},
         "e2e": e2e,
-        # per step: forward = annotate, leaf table, brick assign, brick fill, march; backward =
-        # prefix, ray pack, bin, scatter (one launch per part), and the five launches of the
-        # marching fallback, which return at once unless the log overflowed
-        "gpu_launches": (5 + 3 + (a.overlap_parts if best == "allreduce_inside_backward" else 1)
-                         + 5 + (1 if best == "allreduce_multicast" else 0)) * a.steps,
+        # per step: forward = leaf table, brick fill, march, ordering of the log; backward =
+        # scatter (one launch per part) and the marching fallback, which returns at once unless
+        # the log overflowed
+        "gpu_launches": (4 + (a.overlap_parts if best == "allreduce_inside_backward" else 1)
+                         + 1 + (1 if best == "allreduce_multicast" else 0)) * a.steps,
         "clocks": clocks,
     }
     if check is not None:
@@ -775,12 +770,12 @@ def run_query(a):
         "config": {"workload": workload_name(a), "points_per_gpu": n,
                    "parallelism": f"points cut into {world} slices, tree replicated, no collective",
                    "l2": "inputs larger than L2 (3.76 GB tree data, 3.3 GB of values)"},
-        "roofline": {"bound": "hbm", "kernel": "query_kernel<0> (query_vertical)",
+        "roofline": {"bound": "hbm", "kernel": "query_kernel (query_vertical)",
                      "achieved": fwd_bytes / ms_fwd / 1e6, "peak": peak, "unit": "GB/s",
                      "frac": fwd_bytes / ms_fwd / 1e6 / peak, "traffic": None,
                      "peak_source": peak_src, "ms_per_launch": ms_fwd,
                      "algorithmic_bytes_per_launch": fwd_bytes},
-        "roofline_backward": {"bound": "hbm", "kernel": "zero-fill + query_kernel<1> "
+        "roofline_backward": {"bound": "hbm", "kernel": "sorting + scatter_binned_rows_kernel "
                                                         "(query_vertical_backward)",
                               "achieved": (bwd_bytes + fill_bytes) / ms_bwd / 1e6, "peak": peak,
                               "unit": "GB/s",
@@ -788,7 +783,7 @@ def run_query(a):
                               "ms_per_launch": ms_bwd,
                               "algorithmic_bytes_per_launch": bwd_bytes,
                               "zero_fill_bytes": fill_bytes, "traffic": None},
-        "e2e": e2e, "gpu_launches": 4 * a.steps, "clocks": clocks,
+        "e2e": e2e, "gpu_launches": 5 * a.steps, "clocks": clocks,
     }
     if rank == 0 and world == 1 and not a.no_cpu_baseline:
         val, ms, info = cpu_arm(a, 2, 1, budget_s=20.0)
@@ -897,7 +892,7 @@ def run_image(a):
                      "frac": per_view / ms_view / 1e6 / peak, "traffic": None,
                      "peak_source": peak_src, "ms_per_launch": ms_view,
                      "algorithmic_bytes_per_launch": per_view},
-        "e2e": e2e, "gpu_launches": 5 * (hi - lo) * a.steps, "clocks": clocks,
+        "e2e": e2e, "gpu_launches": 3 * (hi - lo) * a.steps, "clocks": clocks,
     }
     if rank == 0 and world == 1 and not a.no_cpu_baseline:
         val, ms, info = cpu_arm(a, 2, 1, budget_s=20.0)
