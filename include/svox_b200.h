@@ -171,15 +171,15 @@ int svoxb_volume_render_image_backward(const svoxb_tree* tree, const svoxb_camer
 
 /* Rendering many views of a tree that does not change in between (no
  * counterpart in the reference).  The forward render needs an index of the
- * tree (density-annotated child array, leaf table, bricks) that depends on
+ * tree (a table of its upper levels and bricks below it) that depends on
  * child, data's densities, opt->sigma_thresh and opt->density_softplus; the
  * plain entry points rebuild it on every call because data may have changed.
  * Here the caller keeps it: svoxb_render_scratch_words int32 words of device
  * memory, filled once by svoxb_render_scratch_build and passed to any number
  * of svoxb_volume_render[_image]_prepared calls -- valid until the tree or those
- * two options change.  Octrees with three colour channels of 1, 4, 9, 16 or
- * 25 basis functions (SH, SG or ASG) only (else SVOXB_ERR_FORMAT: use the
- * plain entry points). */
+ * two options change.  Octrees with RGBA records of four floats or three
+ * colour channels of 1, 4, 9, 16 or 25 basis functions (SH, SG or ASG) only
+ * (else SVOXB_ERR_FORMAT: use the plain entry points). */
 int64_t svoxb_render_scratch_words(const svoxb_tree* tree);
 int svoxb_render_scratch_build(const svoxb_tree* tree, const svoxb_render_options* opt,
                                int32_t* scratch, void* stream);
@@ -200,8 +200,8 @@ int svoxb_volume_render_image_prepared(const svoxb_tree* tree, const svoxb_camer
  * instead of marching the rays and reading the leaf records again.  A forward
  * of many rays sorts its samples by leaf range, so that the gradient of a range
  * stays in L2 while it is reduced.
- * Only for octrees with three colour channels of 1, 4, 9, 16 or 25 basis
- * functions (SH, SG or ASG) and sigma_thresh =
+ * Only for octrees with RGBA records of four floats or three colour channels
+ * of 1, 4, 9, 16 or 25 basis functions (SH, SG or ASG) and sigma_thresh =
  * stop_thresh = 0 (else SVOXB_ERR_FORMAT / SVOXB_ERR_OPTION).  `data` must not change between the two calls.
  *
  * A log that was too small must not be replayed.  `chunks_used` says who
@@ -258,12 +258,11 @@ int svoxb_volume_render_image_backward_replay(const svoxb_tree* tree, const svox
  * 1111-1173): the diagonal of the Gauss-Newton matrix of the squared error
  * 1/2 sum (render - colour)^2, i.e. for every element of data the sum over rays
  * and channels of (d render / d element)^2.  Computed from the item log of a
- * logged forward like the replay backward (same restrictions, same scratch);
- * chunks_used must be the count read with svoxb_item_log_used (there is no
- * marching fallback for this result: 0 is refused with SVOXB_ERR_OPTION);
- * SVOXB_ERR_TOO_LARGE if the scratch cannot be had.  The first two results of
- * se_grad are the logged forward's output and the replay backward with
- * grad_output = render - colour. */
+ * logged forward like the replay backward (same restrictions); chunks_used
+ * must be the count read with svoxb_item_log_used (there is no marching
+ * fallback for this result alone: 0 is refused with SVOXB_ERR_OPTION).  The
+ * first two results of se_grad are the logged forward's output and the replay
+ * backward with grad_output = render - colour. */
 int svoxb_volume_render_hessdiag_replay(const svoxb_tree* tree, const svoxb_rays* rays,
                                         const svoxb_render_options* opt, const float* fwd_out,
                                         int32_t* log, int64_t capacity_chunks,
@@ -309,9 +308,9 @@ int svoxb_se_grad_image_march(const svoxb_tree* tree, const svoxb_camera* cam,
 
 /* The replay backward in steps, for callers that overlap the all-reduce of the
  * gradient with its computation (no counterpart in the reference).  _begin
- * sorts the logged samples by leaf range (arguments as for
- * svoxb_volume_render_backward_replay, chunks_used included;
- * SVOXB_ERR_TOO_LARGE if the scratch cannot be had) and returns a job.
+ * (arguments as for svoxb_volume_render_backward_replay, chunks_used included)
+ * returns a job.  (The samples of a log that the forward did not sort are all
+ * added with part 0.)
  * grad_data_out is the gradient buffer, zeroed by the caller: with
  * chunks_used = 0 the marching fallback for an overflowed log is enqueued here,
  * BEFORE the parts, so that a part's rows are final after its scatter
@@ -322,7 +321,7 @@ int svoxb_se_grad_image_march(const svoxb_tree* tree, const svoxb_camera* cam,
  * [begin, end) of a part, i.e. rows [begin*K, end*K) of the flat gradient.
  * svoxb_replay_scatter adds the gradient of one part into grad_data_out; with
  * reserve_sms > 0 it leaves that many SMs free for a collective kernel running
- * beside it.  svoxb_replay_end releases the scratch on `stream`. */
+ * beside it.  svoxb_replay_end releases the job. */
 int svoxb_replay_begin(const svoxb_tree* tree, const svoxb_rays* rays,
                        const svoxb_render_options* opt, const float* grad_output,
                        const float* fwd_out, int32_t* log, int64_t capacity_chunks,

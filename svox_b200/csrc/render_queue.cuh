@@ -3,29 +3,30 @@
 // forward with an item log, and backward in one or two marches.
 //
 //   G step  one lane = one ray.  Every iteration takes one SAMPLE per lane: the leaf is found
-//           by one table look-up, or one brick look-up below it (render_index.cuh), whose word
+//           by one table look-up, or one brick look-up below it (render_index.cuh), whose entry
 //           already holds the leaf's density, so the march itself reads L2-resident index
-//           words only.  A contributing sample is pushed as an ITEM (leaf slot, weight, ...)
-//           into the warp's queue in shared memory.
+//           entries only.  A contributing sample is pushed as an ITEM (leaf slot, step length,
+//           density, owner) into the warp's queue in shared memory.
 //   S step  one lane = one item.  When 32 items are queued their records are requested with
 //           cp.async (coalesced 16-byte words, global -> shared staging rows) and the warp
 //           goes on marching; the batch is evaluated when the next one is full, by which time
-//           the data has arrived.  Lane i evaluates item i (dot products with the owner ray's
-//           colour basis, sigmoids); then every owner folds the results of its own items into
-//           its ray's sums in march order, which keeps the reference's order of accumulation
+//           the data has arrived.  Lane i evaluates item i (attenuation, dot products with the
+//           owner ray's colour basis, sigmoids); then every owner folds the results of its own items into
+//           its ray's transmittance and sums in march order, which keeps the reference's order of accumulation
 //           (svox/csrc/rt_kernel.cu:282-295, 379-411, 442-471) whatever the batches are.  In
 //           the backward pass lane i forms the gradient of record i in its staging row and the
 //           warp flushes the rows with red.global.add.v4.f32, 16 bytes per lane.
 //
-// Bound: issue slots on scenes whose records stay in L2 (images: 65 % of the slots used), DRAM
-// where every sample's record misses (rays in random order: 14 GB for 2^20 rays of the 512^3
-// shell scene).  So the march is kept short: the position's bits come from one truncating
-// addition instead of conversions, the leaf's exit distance needs five operations per axis, the
-// index words of a sample are requested one iteration ahead so that the queue's work covers
-// their latency, and a block holds four warps so that shared memory and the L1 can be balanced
-// (kMarchBlocks).  Per 800x800 view of the shell scene with SH16 records 1.64 ms before, 1.11
-// after; logged forward of 2^20 rays, SH9, 4.10 -> 3.50 ms; 65536 rays of an RGBA tree, forward
-// and backward, 1.6 -> 0.3 ms (these went through the generic kernels).
+// Bound: issue slots where neighbouring rays share records (images: 63 % of the slots used), DRAM
+// too where every sample's record misses (rays in random order: 16 GB for 2^20 rays of the 512^3
+// shell scene).  So the march is kept short, 138 instructions per iteration and 259 per batch of
+// items: the position's bits come from one truncating addition instead of conversions, the leaf's
+// exit distance needs five operations per axis, lanes between samples compute along instead of
+// branching, what only items need is done where all lanes have one, the index entry of a sample
+// is requested one iteration ahead so that the queue's work covers its latency, and a block holds
+// four warps so that shared memory and the L1 can be balanced (kMarchBlocks).  Per 800x800 view of
+// the shell scene with SH16 records 1.64 -> 1.05 ms; logged forward of 2^20 rays, SH9, 4.09 -> 3.31;
+// 65536 rays of an RGBA tree, forward and backward, 1.6 -> 0.25 (they took the generic kernels).
 //
 // Lanes whose ray has ended wait until `refill` of them do; then the queue is drained, their
 // results are written and they take new rays from a block-wide ticket counter together (the
