@@ -645,6 +645,9 @@ PYBIND11_MODULE(_host, m) {
     m.def("render_node", [](const Tensor& data, py::handle tree, py::handle source, py::handle opt,
                             bool image, int64_t capacity, const optional<Tensor>& epoch) {
         auto call = std::make_shared<RenderCall>();
+        if (epoch && !(epoch->device().is_cpu() && epoch->scalar_type() == at::kLong &&
+                       epoch->numel() == 1))
+            fail("the tree's edit counter must be one int64 in host memory");
         call->tree = read_tree(tree);
         call->source = read_source(source, image, call->tree);
         call->options = read_options(opt);

@@ -88,9 +88,10 @@ class N3Tree(nn.Module):
             self.extra_data = None
 
         self._ver = 0
-        # counts the writes that go through ``data.data``; in a tensor so that the native
-        # autograd node can look at it
-        self._data_epoch = torch.zeros((), dtype=torch.int64)
+        # counts the writes that go through ``data.data``; in a tensor of host memory, whatever
+        # the default device, so that the native autograd node can look at it
+        with torch.inference_mode(False):
+            self._data_epoch = torch.zeros((), dtype=torch.int64, device="cpu")
         self._invalidate()
         self._lock_tree_structure = False
         self._weight_accum = None

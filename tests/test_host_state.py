@@ -1,0 +1,40 @@
+"""What the host side keeps between a forward and its backward, or from one call to the next: the
+tree's edit counter, the tensors a spec is packed from, leaf views, the item log's size."""
+import pytest
+import torch
+
+import svox_b200 as svox
+from svox_b200 import csrc
+
+needs_build = pytest.mark.skipif(not csrc.is_built(), reason="the native library is not built")
+
+
+@pytest.mark.parametrize("device", ["cpu", "meta"])
+def test_edit_counter_lives_in_host_memory(device):
+    # the native node reads it on the host in the backward
+    with torch.device(device):
+        tree = svox.N3Tree(data_format="SH1", init_refine=1, device="cpu")
+    assert tree.data.device.type == "cpu"
+    assert tree._data_epoch.device.type == "cpu" and tree._data_epoch.dtype == torch.int64
+    before = tree._spec().data_epoch()
+    tree[0, -1:] = 2.0
+    assert tree._spec().data_epoch() > before
+
+
+def test_edit_counter_of_a_tree_made_in_inference_mode():
+    with torch.inference_mode():
+        tree = svox.N3Tree(data_format="SH1")
+    before = int(tree._data_epoch)
+    tree._data_epoch += 1           # (an inference tensor refuses this outside that mode)
+    assert int(tree._data_epoch) == before + 1
+
+
+@needs_build
+@pytest.mark.parametrize("counter", [torch.zeros((), dtype=torch.int64, device="meta"),
+                                     torch.zeros((), dtype=torch.int32),
+                                     torch.zeros(2, dtype=torch.int64)])
+def test_native_node_refuses_a_counter_it_cannot_read(counter):
+    tree = svox.N3Tree(data_format="SH1")
+    opt = csrc.RenderOptions()
+    with pytest.raises(RuntimeError, match="edit counter"):
+        csrc.host().render_node(tree.data, tree._spec(), csrc.RaysSpec(), opt, False, 0, counter)
