@@ -444,6 +444,13 @@ def log_capacity(n_rays):
     return int(n_rays * _LogWatch.poll() / 32) + _LOG_SLACK_CHUNKS
 
 
+def log_words(capacity):
+    """int32 words of a log of ``capacity`` chunks."""
+    fn = library().svoxb_item_log_words
+    fn.restype = C.c_int64
+    return fn(C.c_int64(capacity))
+
+
 def log_is_sorted(tree, n_rays, image):
     """Whether a logged forward of this size sorts its samples, so that the replay clears the
     gradient on the way."""
@@ -564,6 +571,11 @@ def volume_render_backward_replay_parts(tree, rays_or_cam, opt, grad_output, fwd
         co = opt._pack()
         _check_input(grad_output, "grad_output")
         _check_input(fwd_out, "fwd_out")
+        n = n_rays_of(rays_or_cam, image)
+        if grad_output.numel() != 3 * n or fwd_out.numel() != 3 * n:
+            raise RuntimeError("grad_output and fwd_out must have the shape of the render")
+        if log.numel() < log_words(cap):
+            raise RuntimeError("the item log is smaller than its capacity")
         if image:
             cs = _pack_camera(rays_or_cam, dev)
             begin = lib.svoxb_replay_image_begin

@@ -94,10 +94,56 @@ struct Name {
 };
 #define SVOXB_NAME(id) static const Name id(#id);
 
+// A tree as a call sees it: the spec's tensors, and the pointers and sizes read from them.  A tensor
+// can be given another storage while a node waits for its backward (`data.data = x`, `tree.to()`),
+// which pins neither the old one nor counts as a version: `bind` is repeated there.
 struct Tree {
     Tensor data, child, offset, scaling, weight, extra;
+    bool weight_max = false;
     svoxb_tree c{};
+
+    void bind();
+    // Whether the records still lie where `other` was bound to them.
+    bool same_records(const svoxb_tree& other) const {
+        return c.data == other.data && c.M == other.M && c.N == other.N && c.K == other.K;
+    }
 };
+
+void Tree::bind() {
+    check_input(data, "data");
+    check_input(offset, "offset");
+    check_input(scaling, "scaling");
+    check_input(child, "child", at::kInt);
+    if (data.dim() != 5 || child.dim() != 4 || child.sizes() != data.sizes().slice(0, 4))
+        fail("data must be (M,N,N,N,K) and child (M,N,N,N)");
+    const auto dev = data.device();
+    if (child.device() != dev) fail("child must be on the same device as data");
+    if (offset.device() != dev) fail("offset must be on the same device as data");
+    if (scaling.device() != dev) fail("scaling must be on the same device as data");
+    c = svoxb_tree{};
+    if (weight.defined() && weight.numel()) {
+        check_input(weight, "_weight_accum");
+        if (weight.sizes() != child.sizes() || weight.device() != dev)
+            fail("_weight_accum must have the shape and device of child");
+        c.weight_accum = weight.data_ptr<float>();
+    }
+    c.weight_accum_max = weight_max;
+    if (extra.defined() && extra.numel()) {
+        check_input(extra, "extra_data");
+        if (extra.dim() != 2 || extra.device() != dev)
+            fail("extra_data must be (basis_dim, C) on the device of data");
+        c.extra_data = extra.data_ptr<float>();
+        c.extra_rows = (int32_t)extra.size(0);
+        c.extra_cols = (int32_t)extra.size(1);
+    }
+    c.data = data.data_ptr<float>();
+    c.child = child.data_ptr<int32_t>();
+    c.offset = offset.data_ptr<float>();
+    c.scaling = scaling.data_ptr<float>();
+    c.M = data.size(0);
+    c.N = (int32_t)data.size(1);
+    c.K = (int32_t)data.size(4);
+}
 
 Tree read_tree(py::handle spec) {
     SVOXB_NAME(data) SVOXB_NAME(child) SVOXB_NAME(offset) SVOXB_NAME(scaling)
@@ -107,45 +153,13 @@ Tree read_tree(py::handle spec) {
     t.child = tensor_of(child.of(spec), "child");
     t.offset = tensor_of(offset.of(spec), "offset");
     t.scaling = tensor_of(scaling.of(spec), "scaling");
-    check_input(t.data, "data");
-    check_input(t.offset, "offset");
-    check_input(t.scaling, "scaling");
-    check_input(t.child, "child", at::kInt);
-    if (t.data.dim() != 5 || t.child.dim() != 4 || t.child.sizes() != t.data.sizes().slice(0, 4))
-        fail("data must be (M,N,N,N,K) and child (M,N,N,N)");
-    const auto dev = t.data.device();
-    if (t.child.device() != dev) fail("child must be on the same device as data");
-    if (t.offset.device() != dev) fail("offset must be on the same device as data");
-    if (t.scaling.device() != dev) fail("scaling must be on the same device as data");
     py::object w = _weight_accum.of(spec), e = extra_data.of(spec);
     if (!w.is_none()) {
         t.weight = tensor_of(w, "_weight_accum");
-        if (t.weight.numel()) {
-            check_input(t.weight, "_weight_accum");
-            if (t.weight.sizes() != t.child.sizes() || t.weight.device() != dev)
-                fail("_weight_accum must have the shape and device of child");
-            t.c.weight_accum = t.weight.data_ptr<float>();
-        }
-        t.c.weight_accum_max = PyObject_IsTrue(_weight_accum_max.of(spec).ptr()) == 1;
+        t.weight_max = PyObject_IsTrue(_weight_accum_max.of(spec).ptr()) == 1;
     }
-    if (!e.is_none()) {
-        t.extra = tensor_of(e, "extra_data");
-        if (t.extra.numel()) {
-            check_input(t.extra, "extra_data");
-            if (t.extra.dim() != 2 || t.extra.device() != dev)
-                fail("extra_data must be (basis_dim, C) on the device of data");
-            t.c.extra_data = t.extra.data_ptr<float>();
-            t.c.extra_rows = (int32_t)t.extra.size(0);
-            t.c.extra_cols = (int32_t)t.extra.size(1);
-        }
-    }
-    t.c.data = t.data.data_ptr<float>();
-    t.c.child = t.child.data_ptr<int32_t>();
-    t.c.offset = t.offset.data_ptr<float>();
-    t.c.scaling = t.scaling.data_ptr<float>();
-    t.c.M = t.data.size(0);
-    t.c.N = (int32_t)t.data.size(1);
-    t.c.K = (int32_t)t.data.size(4);
+    if (!e.is_none()) t.extra = tensor_of(e, "extra_data");
+    t.bind();
     return t;
 }
 
@@ -177,6 +191,8 @@ struct Source {
     Tensor origins, dirs, vdirs, c2w;
     svoxb_rays rays{};
     svoxb_camera cam{};
+
+    void bind(const Tree& tree);      // repeated for a backward, as Tree::bind
     int64_t count() const { return image ? (int64_t)cam.width * cam.height : rays.Q; }
     std::vector<int64_t> shape(int64_t channels) const {
         if (image) return {cam.height, cam.width, channels};
@@ -184,41 +200,48 @@ struct Source {
     }
 };
 
-Source read_source(py::handle spec, bool image, const Tree& tree) {
-    SVOXB_NAME(origins) SVOXB_NAME(dirs) SVOXB_NAME(vdirs) SVOXB_NAME(c2w) SVOXB_NAME(fx)
-    SVOXB_NAME(fy) SVOXB_NAME(width) SVOXB_NAME(height)
-    Source s;
-    s.image = image;
+void Source::bind(const Tree& tree) {
     const auto dev = tree.data.device();
     if (image) {
-        s.c2w = tensor_of(c2w.of(spec), "c2w");
-        check_input(s.c2w, "c2w");
-        if (s.c2w.dim() != 2 || s.c2w.size(1) != 4 || (s.c2w.size(0) != 3 && s.c2w.size(0) != 4))
+        check_input(c2w, "c2w");
+        if (c2w.dim() != 2 || c2w.size(1) != 4 || (c2w.size(0) != 3 && c2w.size(0) != 4))
             fail("c2w must be (3, 4) or (4, 4)");
-        if (s.c2w.device() != dev) fail("c2w must be on the same device as the tree");
-        s.cam.c2w = s.c2w.data_ptr<float>();
-        s.cam.fx = (float)fx.number(spec);
-        s.cam.fy = (float)fy.number(spec);
-        s.cam.width = (int32_t)width.whole(spec);
-        s.cam.height = (int32_t)height.whole(spec);
-        return s;
+        if (c2w.device() != dev) fail("c2w must be on the same device as the tree");
+        cam.c2w = c2w.data_ptr<float>();
+        return;
     }
-    s.origins = tensor_of(origins.of(spec), "origins");
-    s.dirs = tensor_of(dirs.of(spec), "dirs");
-    s.vdirs = tensor_of(vdirs.of(spec), "vdirs");
     const std::array<std::pair<const Tensor*, const char*>, 3> all{
-        {{&s.origins, "origins"}, {&s.dirs, "dirs"}, {&s.vdirs, "vdirs"}}};
+        {{&origins, "origins"}, {&dirs, "dirs"}, {&vdirs, "vdirs"}}};
     for (const auto& [t, name] : all) {
         check_input(*t, name);
         if (t->dim() != 2 || t->size(1) != 3) fail(std::string(name) + " must be (Q, 3)");
         if (t->device() != dev) fail(std::string(name) + " must be on the same device as the tree");
     }
-    s.rays.Q = s.origins.size(0);
-    if (s.dirs.size(0) != s.rays.Q || s.vdirs.size(0) != s.rays.Q)
+    rays.Q = origins.size(0);
+    if (dirs.size(0) != rays.Q || vdirs.size(0) != rays.Q)
         fail("origins, dirs and vdirs must have the same length");
-    s.rays.origins = s.origins.data_ptr<float>();
-    s.rays.dirs = s.dirs.data_ptr<float>();
-    s.rays.vdirs = s.vdirs.data_ptr<float>();
+    rays.origins = origins.data_ptr<float>();
+    rays.dirs = dirs.data_ptr<float>();
+    rays.vdirs = vdirs.data_ptr<float>();
+}
+
+Source read_source(py::handle spec, bool image, const Tree& tree) {
+    SVOXB_NAME(origins) SVOXB_NAME(dirs) SVOXB_NAME(vdirs) SVOXB_NAME(c2w) SVOXB_NAME(fx)
+    SVOXB_NAME(fy) SVOXB_NAME(width) SVOXB_NAME(height)
+    Source s;
+    s.image = image;
+    if (image) {
+        s.c2w = tensor_of(c2w.of(spec), "c2w");
+        s.cam.fx = (float)fx.number(spec);
+        s.cam.fy = (float)fy.number(spec);
+        s.cam.width = (int32_t)width.whole(spec);
+        s.cam.height = (int32_t)height.whole(spec);
+    } else {
+        s.origins = tensor_of(origins.of(spec), "origins");
+        s.dirs = tensor_of(dirs.of(spec), "dirs");
+        s.vdirs = tensor_of(vdirs.of(spec), "vdirs");
+    }
+    s.bind(tree);
     return s;
 }
 
@@ -413,7 +436,15 @@ Tensor run_replay(const Tree& t, const Source& s, const svoxb_render_options& o,
                   int64_t used, const optional<Tensor>& zeroed) {
     check_input(grad_out, "grad_output");
     check_input(fwd, "fwd_out");
+    check_input(log, "log", at::kInt);
+    if (grad_out.numel() != 3 * s.count() || fwd.numel() != 3 * s.count())
+        fail("grad_output and fwd_out must have the shape of the render");
+    if (log.numel() < lib.item_log_words(capacity)) fail("the item log is smaller than its capacity");
     if (used > capacity) fail("the item log overflowed: it cannot be replayed");
+    if (zeroed) {
+        check_input(*zeroed, "zeroed");
+        if (zeroed->numel() != t.data.numel()) fail("zeroed must be like data");
+    }
     const c10::cuda::CUDAGuard guard(t.data.device());
     Tensor grad = zeroed ? *zeroed : at::empty(t.data.sizes(), t.data.options());
     const float *g = grad_out.data_ptr<float>(), *f = fwd.data_ptr<float>();
@@ -519,11 +550,17 @@ class RenderNode : public torch::autograd::Function<RenderNode> {
         if (!ctx->needs_input_grad(0)) return {Tensor(), Tensor()};
         RenderCall& c = *kept<std::shared_ptr<RenderCall>>(ctx);
         const Tensor grad_out = grads[0].contiguous();
+        const svoxb_tree then = c.tree.c;
+        c.tree.bind();
+        c.source.bind(c.tree);
         optional<Tensor> fwd;
         if (c.keeps_out) {
             const auto saved = ctx->get_saved_variables();
-            if (c.tree.data._version() == c.version_then && c.epoch_now() == c.epoch_then) {
-                if (saved[1].defined()) {
+            if (c.tree.data._version() == c.version_then && c.epoch_now() == c.epoch_then &&
+                c.tree.same_records(then)) {
+                // (a log of another size: a saved-tensor hook ran the forward again, and it was
+                // given another log by then)
+                if (saved[1].defined() && saved[1].numel() == lib.item_log_words(c.capacity)) {
                     optional<Tensor> zeroed;
                     if (auto z = std::move(c.zeroed)) zeroed = z->claim(0);
                     return {run_replay(c.tree, c.source, c.options, grad_out, saved[0], saved[1],
@@ -543,7 +580,7 @@ class RenderNode : public torch::autograd::Function<RenderNode> {
 struct QueryCall {
     Tree tree;
     Tensor ids;                // the leaves found, for as long as nobody writes to them or to
-    uint32_t ids_version = 0, child_version = 0;   // the tree's structure
+    uint32_t ids_version = 0, child_version = 0;   // the tree's structure, or replaces that
 };
 
 class QueryNode : public torch::autograd::Function<QueryNode> {
@@ -565,12 +602,16 @@ class QueryNode : public torch::autograd::Function<QueryNode> {
         if (!ctx->needs_input_grad(0)) return {Tensor(), Tensor(), Tensor()};
         QueryCall& c = *kept<std::shared_ptr<QueryCall>>(ctx);
         const Tensor indices = ctx->get_saved_variables()[0], grad_out = grads[0].contiguous();
-        if (c.ids._version() != c.ids_version || c.tree.child._version() != c.child_version)
+        const svoxb_tree then = c.tree.c;
+        c.tree.bind();
+        if (c.ids._version() != c.ids_version || c.tree.child._version() != c.child_version ||
+            c.tree.c.child != then.child || c.tree.c.M != then.M)
             return {run_query_backward(c.tree, indices, grad_out, {}), Tensor(), Tensor()};
         const c10::cuda::CUDAGuard guard(indices.device());
-        Tensor grad = at::empty(c.tree.data.sizes(), grad_out.options());
+        const int64_t Kg = grad_out.size(1);
+        Tensor grad = at::empty({then.M, then.N, then.N, then.N, Kg}, grad_out.options());
         check(lib.query_scatter(&c.tree.c, c.ids.data_ptr<int64_t>(), c.ids.numel(),
-                                grad_out.data_ptr<float>(), c.tree.c.K, grad.data_ptr<float>(), 1,
+                                grad_out.data_ptr<float>(), (int32_t)Kg, grad.data_ptr<float>(), 1,
                                 stream_of(indices)),
               "query_scatter");
         return {grad, Tensor(), Tensor()};

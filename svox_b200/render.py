@@ -97,6 +97,13 @@ def _single_march_ok(opt):
     return opt.sigma_thresh == 0.0 and opt.stop_thresh == 0.0
 
 
+def _data_state(tree):
+    """What tells whether ``data`` is what a forward saw: its edits, and where its records lie
+    (``data.data = x`` counts as no edit)."""
+    data = tree.data
+    return data._version, tree.data_epoch(), data.data_ptr(), data.shape
+
+
 def _forward(ctx, data, tree, src, opt, prepared, train, image):
     """Common forward of the two autograd Functions.
 
@@ -125,7 +132,7 @@ def _forward(ctx, data, tree, src, opt, prepared, train, image):
         out = _C.volume_render_image(tree, src, opt, prepared=prepared)
     else:
         out = _C.volume_render(tree, src, opt, prepared=prepared)
-    ctx.data_state = (data._version, tree.data_epoch())
+    ctx.data_state = _data_state(tree)
     ctx.keeps_out = train and _single_march_ok(opt)
     if ctx.keeps_out:
         ctx.save_for_backward(*((out,) if log is None else (out, log)))
@@ -142,10 +149,10 @@ def _backward(ctx, grad_out):
     fwd = log = None
     if ctx.keeps_out and not FORCE_TWO_MARCHES:
         saved = ctx.saved_tensors
-        unchanged = ctx.data_state == (ctx.tree.data._version, ctx.tree.data_epoch())
-        if unchanged:
+        if ctx.data_state == _data_state(ctx.tree):
             fwd = saved[0]
-            if len(saved) > 1:
+            # (a log of another size: a saved-tensor hook ran the forward again)
+            if len(saved) > 1 and saved[1].numel() == _C.log_words(ctx.log_capacity):
                 log = (saved[1], ctx.log_capacity)
     grad_out = grad_out.contiguous()
     if fwd is not None and log is not None:

@@ -2,6 +2,7 @@
 kept state no longer is what the forward saw."""
 import pytest
 import torch
+import torch.utils.checkpoint
 
 import svox_b200 as svox
 from svox_b200 import csrc
@@ -45,4 +46,96 @@ def test_training_step_under_a_default_device(cuda_device):
         got = _grad(tree, lambda: r(rays), up)
     want = _grad(want_tree, lambda: svox.VolumeRenderer(want_tree)(rays), up)
     assert got.is_cuda and _close(got, want)
+    csrc.check_device_status()
+
+
+def _refill(n_bytes, dev):
+    """Takes up memory that was just given back and writes to it."""
+    return [torch.full((n_bytes // 4,), float("nan"), device=dev) for _ in range(2)]
+
+
+@pytest.mark.parametrize("fast", [False, True])
+@pytest.mark.parametrize("fmt", ["SH4", "RGBA"])
+def test_storage_of_data_replaced_before_the_backward(fmt, fast, cuda_device):
+    # neither pinned by the node nor counted as an edit; the backward takes the new storage's
+    # values, as the reference does, from where they lie now
+    tree = _tree(cuda_device, fmt)
+    r = svox.VolumeRenderer(tree)
+    rays, up = _rays(300, cuda_device), torch.ones(300, 3, device=cuda_device)
+    c2w = W.look_at_cameras(1, torch.Generator().manual_seed(1), 1.6)[0].to(cuda_device)
+    image_up = torch.ones(12, 16, 3, device=cuda_device)
+
+    def image():
+        return r.render_persp(c2w, width=16, height=12, fx=22.0, fast=fast)
+    for call, grad_out in ((lambda: r(rays, fast=fast), up), (image, image_up)):
+        for change in (lambda d: d.clone(), lambda d: d * 0.5):
+            tree.data.grad = None
+            out = call()
+            tree.data.data = change(tree.data.data)
+            held = _refill(tree.data.numel() * 4, cuda_device)
+            out.backward(grad_out)
+            got = tree.data.grad
+            del held
+            assert _close(got, _grad(tree, call, grad_out))
+    csrc.check_device_status()
+
+
+def test_storage_of_data_replaced_before_the_backward_of_a_query(cuda_device):
+    tree = _tree(cuda_device)
+    pts = torch.rand(500, 3, device=cuda_device)
+    up = torch.ones(500, tree.data_dim, device=cuda_device)
+    tree.data.grad = None
+    out = tree(pts)
+    tree.data.data = tree.data.data.clone()
+    tree.child.data = tree.child.data.clone()
+    held = _refill(tree.data.numel() * 4, cuda_device)
+    out.backward(up)
+    got = tree.data.grad
+    del held
+    assert _close(got, _grad(tree, lambda: tree(pts), up))
+    csrc.check_device_status()
+
+
+@pytest.mark.parametrize("kind", ["rays", "rays_fast", "query"])
+def test_shape_of_data_changed_before_the_backward_is_refused(kind, cuda_device):
+    tree = _tree(cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(300, cuda_device)
+    pts = torch.rand(300, 3, device=cuda_device)
+    before = tree.data.data
+    for other in (before[:3].clone(), torch.cat((before, before)), before.cpu()):
+        out = tree(pts) if kind == "query" else r(rays, fast=kind == "rays_fast")
+        tree.data.data = other
+        with pytest.raises(RuntimeError):
+            out.sum().backward()
+        tree.data.data = before
+    csrc.check_device_status()
+
+
+def test_log_of_another_size_is_not_replayed(cuda_device):
+    # checkpointing runs the forward again in the backward, with a log sized by what has been
+    # learnt meanwhile
+    tree = _tree(cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(300, cuda_device)
+    up = torch.ones(300, 3, device=cuda_device)
+    want = _grad(tree, lambda: r(rays), up)
+    old = csrc._items_per_ray
+    csrc.log_estimate(wait=True)
+    for first, then in ((200.0, 20.0), (20.0, 200.0)):
+        tree.data.grad = None
+        csrc._items_per_ray = first
+        out = torch.utils.checkpoint.checkpoint(r, rays, use_reentrant=False,
+                                                determinism_check="none")
+        csrc.log_estimate(wait=True)
+        csrc._items_per_ray = then
+        out.backward(up)
+        assert _close(tree.data.grad, want)
+    spec, src, opt = tree._spec(), svox.render._rays_spec_from_rays(rays), r._get_options()
+    out, (log, cap) = csrc.volume_render_logged(spec, src, opt)
+    for bad in ((up, out.detach(), (log, cap + 1)), (up[:-1], out.detach(), (log, cap)),
+                (up, out.detach()[:-1], (log, cap))):
+        with pytest.raises(RuntimeError):
+            csrc.volume_render_backward_replay(spec, src, opt, *bad)
+        with pytest.raises(RuntimeError):
+            csrc.volume_render_backward_replay_parts(spec, src, opt, *bad, 2, lambda rows: None)
+    csrc._items_per_ray = old
     csrc.check_device_status()
