@@ -608,14 +608,23 @@ class N3Tree(nn.Module):
         """Pack the tensors for the native library (svox/svox.py:1084-1103)."""
         spec = _C.TreeSpec()
         spec._owner = weakref.ref(self)
-        buffers = self._buffers        # (attribute look-up on a Module goes through __getattr__)
-        data = spec.data = self._parameters["data"]
-        spec.child = buffers["child"]
-        spec.parent_depth = buffers["parent_depth"]
-        spec.extra_data = self.extra_data if "extra_data" in buffers else \
-            self.__dict__["extra_data"]
+        buffers = self._buffers
+        try:
+            # (look-up on a Module goes through __getattr__)
+            data = self._parameters["data"]
+            child, parent_depth = buffers["child"], buffers["parent_depth"]
+            offset, scaling = buffers["offset"], buffers["invradius"]
+            extra_data = buffers["extra_data"] if "extra_data" in buffers else \
+                self.__dict__["extra_data"]
+        except KeyError:
+            # parametrised, assigned as a plain tensor (a replica, a network that makes the
+            # data), a buffer that became a Parameter
+            data, child, parent_depth = self.data, self.child, self.parent_depth
+            offset, scaling, extra_data = self.offset, self.invradius, self.extra_data
+        spec.data, spec.child, spec.parent_depth = data, child, parent_depth
+        spec.extra_data = extra_data
         if world:
-            spec.offset, spec.scaling = buffers["offset"], buffers["invradius"]
+            spec.offset, spec.scaling = offset, scaling
         else:
             spec.offset = torch.zeros(3, dtype=data.dtype, device=data.device)
             spec.scaling = torch.ones(3, dtype=data.dtype, device=data.device)

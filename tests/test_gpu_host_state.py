@@ -139,3 +139,22 @@ def test_log_of_another_size_is_not_replayed(cuda_device):
             csrc.volume_render_backward_replay_parts(spec, src, opt, *bad, 2, lambda rows: None)
     csrc._items_per_ray = old
     csrc.check_device_status()
+
+
+def test_data_that_is_no_parameter(cuda_device):
+    tree = _tree(cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(300, cuda_device)
+    up = torch.ones(300, 3, device=cuda_device)
+    pts = torch.rand(200, 3, device=cuda_device)
+    rows = torch.ones(200, tree.data_dim, device=cuda_device)
+    want = _grad(tree, lambda: r(rays), up) * 2
+    want_query = _grad(tree, lambda: tree(pts), rows) * 2
+    half = (tree.data.detach() / 2).requires_grad_()
+    del tree.data
+    tree.data = half * 2                        # a network's output
+    r(rays).backward(up, retain_graph=True)
+    assert _close(half.grad, want)
+    half.grad = None
+    tree(pts).backward(rows)
+    assert _close(half.grad, want_query)
+    csrc.check_device_status()

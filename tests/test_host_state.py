@@ -2,6 +2,7 @@
 tree's edit counter, the tensors a spec is packed from, leaf views, the item log's size."""
 import pytest
 import torch
+import torch.nn.utils.parametrize
 
 import svox_b200 as svox
 from svox_b200 import csrc
@@ -38,3 +39,49 @@ def test_native_node_refuses_a_counter_it_cannot_read(counter):
     opt = csrc.RenderOptions()
     with pytest.raises(RuntimeError, match="edit counter"):
         csrc.host().render_node(tree.data, tree._spec(), csrc.RaysSpec(), opt, False, 0, counter)
+
+
+class _Doubled(torch.nn.Module):
+    def forward(self, x):
+        return 2 * x
+
+
+def test_spec_finds_tensors_wherever_the_module_keeps_them():
+    lobes = torch.rand(2, 4)
+    tree = svox.N3Tree(data_format="SG2", extra_data=lobes)
+    spec = tree._spec()
+    assert spec.data is tree.data and spec.child is tree.child and torch.equal(spec.extra_data, lobes)
+    del tree.extra_data
+    tree.extra_data = torch.nn.Parameter(lobes + 1)          # lobes that are trained elsewhere
+    assert tree._spec().extra_data is tree.extra_data
+    tree.offset = torch.nn.Parameter(tree.offset + 1)
+    assert tree._spec().offset is tree.offset
+    plain = svox.N3Tree(data_format="SH1")
+    assert plain._spec().extra_data is None
+    plain.extra_data = lobes                                 # a plain attribute
+    assert plain._spec().extra_data is lobes
+
+    tree = svox.N3Tree(data_format="SH1")
+    tree.data.data.fill_(1.5)
+    torch.nn.utils.parametrize.register_parametrization(tree, "data", _Doubled())
+    assert torch.equal(tree._spec().data, torch.full_like(tree.data, 3.0))
+
+    tree = svox.N3Tree(data_format="SH1")
+    made = tree.data * 2                     # what a replica, or a network that makes data, has
+    del tree.data
+    tree.data = made
+    assert tree._spec().data is made and tree._spec(world=False).data is made
+
+    tree = svox.N3Tree(data_format="SH1")
+    other = torch.ones_like(tree.data)
+    seen = []
+
+    class Call(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.tree = tree
+
+        def forward(self):
+            seen.append(self.tree._spec().data)
+    torch.func.functional_call(Call(), {"tree.data": other})
+    assert seen[0] is other
