@@ -343,9 +343,10 @@ int svoxb_replay_end(void* job, void* stream);
  * capacity means that it overflowed. */
 int svoxb_item_log_used(const int32_t* log, int64_t* chunks_used, void* stream);
 
-/* Enqueues the copy of {chunks asked for, samples} of a log into two int32 of
- * pinned host memory, for a caller that sizes its next log by them and looks
- * later whether they have arrived. */
+/* Enqueues the copy of {chunks asked for, samples / 32} of a log into two int32
+ * of pinned host memory, for a caller that sizes its next log by them and looks
+ * later whether they have arrived.  (The samples are rounded up per warp of the
+ * forward, at most 24 warps per multiprocessor.) */
 int svoxb_item_log_watch(const int32_t* log, int32_t* counts, void* stream);
 
 /* Forward ray render that allocates nothing (no counterpart in the

@@ -399,11 +399,11 @@ _items_per_ray = 80.0           # running estimate used to size the item log
 class _LogWatch:
     """Learns how large the item log has to be WITHOUT making the host wait for the device.
 
-    After a logged forward the number of chunks it asked for and of samples it wrote are copied
-    to pinned host memory, asynchronously (host.cpp); whenever the next log is sized, the counts
-    that have arrived by then adapt the per-ray estimate.  A log that was too small costs that
-    one step a marching backward (decided on the device, see ``volume_render_backward_replay``),
-    never a wrong gradient."""
+    After a logged forward the number of chunks it asked for and of samples it wrote (in units
+    of 32) are copied to pinned host memory, asynchronously (host.cpp); whenever the next log is
+    sized, the counts that have arrived by then adapt the per-ray estimate.  A log that was too
+    small costs that one step a marching backward (decided on the device, see
+    ``volume_render_backward_replay``), never a wrong gradient."""
     last_used = last_cap = 0
 
     @classmethod
@@ -413,11 +413,11 @@ class _LogWatch:
         if wait and host().logs_pending():
             for dev in range(torch.cuda.device_count()):
                 torch.cuda.synchronize(dev)
-        for used, items, n_rays, cap in host().poll_logs():
+        for used, batches, n_rays, cap in host().poll_logs():
             cls.last_used, cls.last_cap = used, cap
             if n_rays:
                 # items, or the chunks they took beyond the slack: keep 25 % head room
-                items = max(items, 32 * (used - _LOG_SLACK_CHUNKS))
+                items = 32 * max(batches, used - _LOG_SLACK_CHUNKS)
                 need = max(8.0, 1.25 * items / n_rays)
                 _items_per_ray = need if used > cap else max(need, 0.9 * _items_per_ray)
         return _items_per_ray

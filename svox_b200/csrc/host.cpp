@@ -266,7 +266,7 @@ void* stream_of(const Tensor& t) {
 // they arrive.
 class LogWatch {
   public:
-    struct Seen { int64_t used, items, rays, capacity; };
+    struct Seen { int64_t used, batches, rays, capacity; };
 
     void watch(const Tensor& log, int64_t capacity, int64_t rays) {
         std::lock_guard<std::mutex> lock(mutex_);
@@ -291,7 +291,7 @@ class LogWatch {
         for (int i = 0; i < kSlots; ++i) {
             if (pending_[i].capacity < 0 || all[2 * i] < 0 || all[2 * i + 1] < 0) continue;
             pending_[i].used = all[2 * i];
-            pending_[i].items = all[2 * i + 1];
+            pending_[i].batches = all[2 * i + 1];
             seen.push_back(pending_[i]);
             pending_[i].capacity = -1;
         }
@@ -740,7 +740,7 @@ PYBIND11_MODULE(_host, m) {
     m.def("poll_logs", [] {
         py::list out;
         for (const auto& s : log_watch().poll())
-            out.append(py::make_tuple(s.used, s.items, s.rays, s.capacity));
+            out.append(py::make_tuple(s.used, s.batches, s.rays, s.capacity));
         return out;
     });
     m.def("logs_pending", [] { return log_watch().waiting(); });

@@ -66,7 +66,8 @@ struct RecordShape {
 // Item log: what a logged forward leaves behind so that the backward pass can
 // replay the contributing samples without marching again and without reading
 // the leaf records a second time.  int32 words:
-//   [0] chunks asked for   [1] items   [2] bin shift   [3] number of bins
+//   [0] chunks asked for   [2] bin shift   [3] number of bins
+//   [1] items in units of 32, each warp's rounded up (items alone would outgrow a word)
 //   [kLogNext + p]         units taken of scatter part p, [kLogNext + kMaxParts + p] blocks done
 //   [kLogBins + b]         groups of bin b      [kLogCleared + b]  cleared units of bin b
 //   [kLogCounts + g]       items of group g (bits 0-7) and its bin (bits 8-)
@@ -805,7 +806,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         // groups taken but not used hold no items; the last group of a bin holds what it got
         for (int i = lane; i < log_left; i += 32)
             if (log_group + i < log_limit) log_counts[log_group + i] = 0;
-        if (lane == 0 && log_items > 0) atomicAdd(lg.log + 1, log_items);
+        if (lane == 0 && log_items > 0) atomicAdd(lg.log + 1, (log_items + 31) >> 5);
         if (SORTED) {
             __syncthreads();
             for (int b = threadIdx.x; b < lg.n_bins; b += BLOCK) {

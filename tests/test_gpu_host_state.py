@@ -158,3 +158,17 @@ def test_data_that_is_no_parameter(cuda_device):
     tree(pts).backward(rows)
     assert _close(half.grad, want_query)
     csrc.check_device_status()
+
+
+@pytest.mark.parametrize("n", [1, 700, 40000])
+def test_counts_that_size_the_log(n, cuda_device):
+    tree = _tree(cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(n, cuda_device)
+    src, opt = svox.render._rays_spec_from_rays(rays), r._get_options()
+    samples = int(csrc.march_stats(tree._spec(), src, opt)[2].sum())
+    _, (log, cap) = csrc.volume_render_logged(tree._spec(), src, opt)
+    warps = 24 * torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    assert samples <= 32 * int(log[1]) <= samples + 31 * min(warps, n)
+    assert int(log[0]) <= cap
+    csrc.log_estimate(wait=True)
+    assert csrc._LogWatch.last_used == int(log[0]) and csrc._LogWatch.last_cap == cap

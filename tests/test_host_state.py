@@ -85,3 +85,24 @@ def test_spec_finds_tensors_wherever_the_module_keeps_them():
             seen.append(self.tree._spec().data)
     torch.func.functional_call(Call(), {"tree.data": other})
     assert seen[0] is other
+
+
+class _Counts:
+    """Stands in for the native module: the counts of finished forwards."""
+
+    def __init__(self, *counts):
+        self.counts = list(counts)
+
+    def poll_logs(self):
+        counts, self.counts = self.counts, []
+        return counts
+
+
+@pytest.mark.parametrize("samples", [2 ** 31 - 32, 2 ** 31, 2 ** 33])
+def test_log_grows_for_any_number_of_samples(samples, monkeypatch):
+    # 2^24 rays with up to 512 samples each, through a log of 2^31 / 8 samples
+    rays, cap = 1 << 24, 1 << 23
+    monkeypatch.setattr(csrc, "_items_per_ray", 8.0)
+    monkeypatch.setattr(csrc, "host", lambda: _Counts((samples // 32, samples // 32, rays, cap)))
+    need = samples // 32
+    assert need <= csrc.log_capacity(rays) <= 1.25 * need + csrc._LOG_SLACK_CHUNKS + 1
