@@ -210,7 +210,7 @@ int svoxb_volume_render_image_prepared(const svoxb_tree* tree, const svoxb_camer
  *        device and do nothing if the forward asked for more chunks than
  *        `capacity_chunks`; a marching backward (as
  *        svoxb_volume_render_backward) is enqueued behind them that does its
- *        work only in that case.  No host synchronisation; the result is the
+ *        work only in that case, or if the forward gave the log up.  No host synchronisation; the result is the
  *        gradient either way.
  *   > 0  the caller read the count with svoxb_item_log_used (which
  *        synchronises) and found it <= capacity_chunks: no fallback is
@@ -340,7 +340,8 @@ int svoxb_replay_scatter(const void* job, int part, float* grad_data_out, int re
 int svoxb_replay_end(void* job, void* stream);
 
 /* Chunks the logged forward asked for (synchronises `stream`); more than the log's
- * capacity means that it overflowed. */
+ * capacity means that it overflowed.  INT64_MAX for a log that the forward had to
+ * give up for another reason than its size: it must not be replayed either. */
 int svoxb_item_log_used(const int32_t* log, int64_t* chunks_used, void* stream);
 
 /* Enqueues the copy of {chunks asked for, samples / 32} of a log into two int32

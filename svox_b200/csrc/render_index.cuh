@@ -25,15 +25,21 @@
 
 namespace svoxb {
 
-// A launch that is a FALLBACK for an overflowed item log: its kernels do their work only if
-// the logged forward needed more chunks than the log holds (word 0 of the log counts the
-// chunks it asked for), so the host can enqueue replay and fallback without knowing which of
-// the two applies.  `log` null: unconditional.
+// Whether an item log (render_queue.cuh) can be replayed: the forward did not ask for more chunks
+// than it holds (word 0), and did not give the log up (word kLogGivenUp).
+constexpr int kLogGivenUp = 4;
+__device__ __forceinline__ bool log_complete(const int32_t* log, int64_t capacity) {
+    return (int64_t)log[0] <= capacity && log[kLogGivenUp] == 0;
+}
+
+// A launch that is a FALLBACK for a log that cannot be replayed: its kernels do their work only
+// in that case, so the host can enqueue replay and fallback without knowing which of the two
+// applies.  `log` null: unconditional.
 struct LogGate {
     const int32_t* log = nullptr;
     int64_t capacity = 0;
     __device__ __forceinline__ bool closed() const {
-        return log != nullptr && (int64_t)__ldg(log) <= capacity;
+        return log != nullptr && log_complete(log, capacity);
     }
 };
 

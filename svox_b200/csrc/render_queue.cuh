@@ -68,6 +68,7 @@ struct RecordShape {
 // the leaf records a second time.  int32 words:
 //   [0] chunks asked for   [2] bin shift   [3] number of bins
 //   [1] items in units of 32, each warp's rounded up (items alone would outgrow a word)
+//   [kLogGivenUp] not 0: the log has holes and must not be replayed, whatever its size
 //   [kLogNext + p]         units taken of scatter part p, [kLogNext + kMaxParts + p] blocks done
 //   [kLogBins + b]         groups of bin b      [kLogCleared + b]  cleared units of bin b
 //   [kLogCounts + g]       items of group g (bits 0-7) and its bin (bits 8-)
@@ -276,7 +277,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     using Shape = RecordShape<K>;
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ unsigned s_next;
-    // backward with a log: the marching fallback of a replay, needed only if the log overflowed
+    // backward with a log: the marching fallback of a replay, for a log that is not complete
     if (BWD && LogGate{lg.log, lg.capacity}.closed()) return;
     if (threadIdx.x == 0) s_next = 0;
     // sorted log: items this block has put into each bin, and its last groups of the bin, each
@@ -538,7 +539,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                     }
                     group_id = (int)(v & 0xffffffu);
                     if ((v >> 24) != tag) {     // never seen: give the log up, march instead
-                        atomicMax(lg.log, 1 << 30);
+                        lg.log[kLogGivenUp] = 1;
                         group_id = 0x7fffffff;
                     }
                 }

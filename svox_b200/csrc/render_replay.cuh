@@ -36,7 +36,7 @@ __host__ __device__ inline int replay_part_first_bin(int p, int n_parts, int n_b
 __global__ void __launch_bounds__(256)
 order_groups_kernel(int32_t* __restrict__ log, int64_t capacity, int32_t* __restrict__ cursor) {
     __shared__ int s_first[kMaxBins], s_count[kMaxBins];
-    if (log[0] > capacity) return;               // overflowed: never replayed
+    if (!log_complete(log, capacity)) return;    // never replayed
     const int n = log[0] / kSortedChunks;
     const int n_bins = log[3] > kMaxBins ? kMaxBins : log[3];
     const int32_t* __restrict__ counts = log + kLogCounts;
@@ -103,13 +103,13 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
     const float d_rgb_pad = 1 + 2 * opt.rgb_padding;
     constexpr int WARPS = BLOCK / 32;
     __shared__ UnitShared s_units;
-    const bool overflow = (int64_t)log[0] > capacity;     // then no packet counts
+    const bool useless = !log_complete(log, capacity);    // then no packet counts
     const int n_bins = log[3] > kMaxBins ? kMaxBins : log[3];
     const bool sorted = n_bins > 1;
     const int lo_bin = sorted ? replay_part_first_bin(part, n_parts, n_bins) : 0,
               hi_bin = sorted ? replay_part_first_bin(part + 1, n_parts, n_bins) : 1;
     // batches of 32 packets a warp takes per unit, and per group
-    const int chunks = overflow || (!sorted && part != 0) ? 0 : log[0];
+    const int chunks = useless || (!sorted && part != 0) ? 0 : log[0];
     const int share = chunks / ((int)gridDim.x * WARPS * (sorted ? n_bins : 4));
     const int per_group = sorted ? kSortedChunks : 1;
     const int per_warp = share < 1 ? 1 : share > kScatterBatches ? kScatterBatches : share;
@@ -118,10 +118,10 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
     const int4* __restrict__ packets =
         reinterpret_cast<const int4*>(log + log_packets_at(capacity));
     int groups_before = 0;
-    for (int b = 0; b < lo_bin && !overflow; ++b) groups_before += log[kLogBins + b];
+    for (int b = 0; b < lo_bin && !useless; ++b) groups_before += log[kLogBins + b];
     const UnitCounters counters{log + kLogNext + part, log + kLogNext + kMaxParts + part,
                                 log + kLogCleared};
-    auto count = [&](int b) { return overflow ? 0 : sorted ? log[kLogBins + b] : chunks; };
+    auto count = [&](int b) { return useless ? 0 : sorted ? log[kLogBins + b] : chunks; };
     auto clear = [&](int64_t from, int64_t until) {
         const int4 none = make_int4(0, 0, 0, 0);
         for (int64_t i = from + 4 * threadIdx.x; i < until; i += 4 * BLOCK) {

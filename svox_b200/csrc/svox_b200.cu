@@ -41,7 +41,7 @@ struct RenderCall {
     // logged forward: buffers like `data` to clear on `clear_stream` beside the march
     float* clear[2] = {nullptr, nullptr};
     cudaStream_t clear_stream = nullptr;
-    // marching backward as the fallback of a replay: does its work only if this log overflowed
+    // marching backward as the fallback of a replay: does its work only if this log cannot be used
     LogGate gate{};
 };
 
@@ -1045,11 +1045,11 @@ int svoxb_replay_end(void* job, void*) {
 
 int svoxb_item_log_used(const int32_t* log, int64_t* chunks_used, void* stream) {
     if (!log || !chunks_used) return SVOXB_ERR_NULL;
-    int32_t used = 0;
-    SVOXB_CUDA(cudaMemcpyAsync(&used, log, sizeof(int32_t), cudaMemcpyDeviceToHost,
+    int32_t head[kLogGivenUp + 1] = {0};
+    SVOXB_CUDA(cudaMemcpyAsync(head, log, sizeof head, cudaMemcpyDeviceToHost,
                                (cudaStream_t)stream));
     SVOXB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    *chunks_used = used;
+    *chunks_used = head[kLogGivenUp] != 0 ? INT64_MAX : head[0];
     return SVOXB_OK;
 }
 

@@ -172,3 +172,28 @@ def test_counts_that_size_the_log(n, cuda_device):
     assert int(log[0]) <= cap
     csrc.log_estimate(wait=True)
     assert csrc._LogWatch.last_used == int(log[0]) and csrc._LogWatch.last_cap == cap
+
+
+@pytest.mark.parametrize("n", [300, 12000])
+def test_a_log_given_up_is_not_replayed(n, cuda_device):
+    gen = torch.Generator().manual_seed(5)
+    tree = W.shell_tree(4, 3, "SH9", gen, (5.0, 50.0), W._SHELL).to(cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(n, cuda_device)
+    up = torch.ones(n, 3, device=cuda_device)
+    want = _grad(tree, lambda: r(rays), up)
+    spec, src, opt = tree._spec(), svox.render._rays_spec_from_rays(rays), r._get_options()
+    assert csrc.log_is_sorted(spec, n, False) == (n == 12000)
+    out, (log, cap) = csrc.volume_render_logged(spec, src, opt)
+    used = csrc.log_chunks_used(log)
+    assert 0 < used <= cap
+    log[4] = 1                                   # the mark of a forward that gave its log up
+    assert csrc.log_chunks_used(log) > cap
+    got = csrc.volume_render_backward_replay(spec, src, opt, up, out, (log, cap))
+    assert _close(got, want)
+    parts = csrc.volume_render_backward_replay_parts(spec, src, opt, up, out, (log, cap), 3,
+                                                     lambda rows: None)
+    assert _close(parts, want)
+    # the counts that the next log is sized by are what they were
+    log[4] = 0
+    assert csrc.log_chunks_used(log) == used
+    csrc.check_device_status()

@@ -106,3 +106,11 @@ def test_log_grows_for_any_number_of_samples(samples, monkeypatch):
     monkeypatch.setattr(csrc, "host", lambda: _Counts((samples // 32, samples // 32, rays, cap)))
     need = samples // 32
     assert need <= csrc.log_capacity(rays) <= 1.25 * need + csrc._LOG_SLACK_CHUNKS + 1
+
+
+def test_a_log_given_up_does_not_size_the_next_one(monkeypatch):
+    # the head of such a log holds the chunks that were really asked for; the mark is a word of
+    # its own, which the host does not look at
+    monkeypatch.setattr(csrc, "_items_per_ray", 8.0)
+    monkeypatch.setattr(csrc, "host", lambda: _Counts((2000, 1500, 1000, 40000)))
+    assert csrc.log_capacity(1000) <= 2000 + csrc._LOG_SLACK_CHUNKS
