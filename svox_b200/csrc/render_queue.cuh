@@ -37,6 +37,7 @@
 #include "render.cuh"
 #include "render_index.cuh"
 #include "binned.cuh"
+#include "open_groups.h"
 
 namespace svoxb {
 
@@ -96,13 +97,6 @@ constexpr int kLogCounts = kLogCleared + kMaxBins;
 constexpr int kPacketWords = 12;
 constexpr int kLogGrab = 8;        // groups a warp takes at least per bump of the counter ...
 constexpr int kSortedGrab = 2;     // ... of a sorted log
-constexpr int kSortedChunks = 4;   // chunks per group of a sorted log
-constexpr int kSortedItems = 32 * kSortedChunks;
-// A block remembers this many of a bin's last groups.  A warp reads the id of its item's group
-// a few instructions after it has taken the item's place; a block has at most 24 * 32 items under
-// way, so their groups are among the last 7 (see the wait in `evaluate` for the rest).
-constexpr int kOpenGroups = 16;
-
 __host__ __device__ inline int64_t log_packets_at(int64_t capacity) {
     return (kLogCounts + capacity + 31) & ~(int64_t)31;
 }
@@ -230,7 +224,7 @@ constexpr int march_blocks_per_sm() {
 
 // A forward that sorts its log into bins runs as one block per SM, so that a bin has one open
 // group per SM and the lines being filled stay in L2 until they are full.
-constexpr size_t kBinSmem = (size_t)kMaxBins * (1 + kOpenGroups) * sizeof(uint32_t);
+constexpr size_t kBinSmem = (size_t)kMaxBins * (sizeof(uint32_t) + kOpenGroups * sizeof(uint64_t));
 template <int BD>
 constexpr int sorted_march_block() {
     const int fit = (int)((227 * 1024 - 1024 - kBinSmem) / sizeof(WarpQueue<BD, kModeForwardLogged>));
@@ -280,13 +274,14 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     // backward with a log: the marching fallback of a replay, for a log that is not complete
     if (BWD && LogGate{lg.log, lg.capacity}.closed()) return;
     if (threadIdx.x == 0) s_next = 0;
-    // sorted log: items this block has put into each bin, and its last groups of the bin, each
-    // as (1 + the group's number among them) mod 256 in the top byte and the group's id
+    // sorted log: items this block has put into each bin, and its last groups of the bin
     constexpr bool SORTED = LOG && BLOCK != kMarchBlock;
-    uint32_t* s_count = reinterpret_cast<uint32_t*>(s_raw + (BLOCK / 32) * sizeof(WQ));
-    uint32_t* s_open = s_count + lg.n_bins;
-    if (SORTED)
-        for (int i = threadIdx.x; i < lg.n_bins * (1 + kOpenGroups); i += BLOCK) s_count[i] = 0;
+    uint64_t* s_open = reinterpret_cast<uint64_t*>(s_raw + (BLOCK / 32) * sizeof(WQ));
+    uint32_t* s_count = reinterpret_cast<uint32_t*>(s_open + lg.n_bins * kOpenGroups);
+    if (SORTED) {
+        for (int i = threadIdx.x; i < lg.n_bins * kOpenGroups; i += BLOCK) s_open[i] = 0;
+        for (int i = threadIdx.x; i < lg.n_bins; i += BLOCK) s_count[i] = 0;
+    }
     if (LOG && blockIdx.x == 0 && threadIdx.x == 0) {
         lg.log[2] = lg.shift;
         lg.log[3] = lg.n_bins;
@@ -524,21 +519,19 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             if (opens && group_id < log_limit)
                 log_counts[group_id] = SORTED ? kSortedItems | (bin << 8) : nb;
             if (SORTED) {
-                volatile uint32_t* open = s_open + bin * kOpenGroups + (number & (kOpenGroups - 1));
-                const uint32_t tag = (number + 1u) & 0xffu;
-                if (opens)
-                    *open = (tag << 24) | (uint32_t)(group_id < 0xffffff ? group_id : 0xffffff);
+                volatile uint64_t* open = s_open + bin * kOpenGroups + open_group_place(number);
+                if (opens) *open = open_group_entry(number, group_id);
                 __syncwarp();
                 if (active && !opens) {
                     // another warp may be about to publish the group's id
-                    uint32_t v = *open;
+                    uint64_t v = *open;
                     int tries = 0;
-                    while ((v >> 24) != tag && ++tries < (1 << 14)) {
+                    while (!open_group_is(v, number) && ++tries < (1 << 14)) {
                         __nanosleep(32);
                         v = *open;
                     }
-                    group_id = (int)(v & 0xffffffu);
-                    if ((v >> 24) != tag) {     // never seen: give the log up, march instead
+                    group_id = open_group_id(v);
+                    if (!open_group_is(v, number)) {    // never seen: give the log up, march instead
                         lg.log[kLogGivenUp] = 1;
                         group_id = 0x7fffffff;
                     }
@@ -814,8 +807,10 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 const uint32_t n = s_count[b];
                 if (n == 0) continue;
                 const uint32_t last = (n - 1) / kSortedItems;
-                const int g = (int)(s_open[b * kOpenGroups + (last & (kOpenGroups - 1))] & 0xffffffu);
-                if (g < log_limit) log_counts[g] = (int)(n - kSortedItems * last) | (b << 8);
+                const uint64_t v = s_open[b * kOpenGroups + open_group_place(last)];
+                const int g = open_group_id(v);
+                if (!open_group_is(v, last)) lg.log[kLogGivenUp] = 1;   // overwritten by a late warp
+                else if (g < log_limit) log_counts[g] = (int)(n - kSortedItems * last) | (b << 8);
                 atomicAdd(lg.log + kLogBins + b, (int)last + 1);
             }
         }

@@ -114,3 +114,34 @@ def test_a_log_given_up_does_not_size_the_next_one(monkeypatch):
     monkeypatch.setattr(csrc, "_items_per_ray", 8.0)
     monkeypatch.setattr(csrc, "host", lambda: _Counts((2000, 1500, 1000, 40000)))
     assert csrc.log_capacity(1000) <= 2000 + csrc._LOG_SLACK_CHUNKS
+
+
+_DRIVER = r"""
+#include "open_groups.h"
+using namespace svoxb;
+// Looks in the entry that group `other` published for each of the groups lo .. hi - 1 that share
+// its place: how many take it for theirs without being `other`, or the other way round.
+extern "C" int mistaken(uint32_t lo, uint32_t hi, uint32_t other, int id) {
+    const uint64_t entry = open_group_entry(other, id);
+    int n_wrong = open_group_id(entry) != id;
+    for (uint32_t n = lo; n < hi; ++n)
+        if (open_group_place(n) == open_group_place(other))
+            n_wrong += open_group_is(entry, n) != (n == other) || open_group_is(0, n);
+    return n_wrong;
+}
+"""
+
+
+def test_open_groups_are_never_mistaken(tmp_path):
+    # whatever the group is that a late reader finds, or a late writer overwrites
+    import ctypes
+    import os
+    import subprocess
+    src, lib = tmp_path / "driver.cpp", tmp_path / "driver.so"
+    src.write_text(_DRIVER)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I",
+                    os.path.dirname(csrc.__file__), str(src), "-o", str(lib)], check=True)
+    mistaken = ctypes.CDLL(str(lib)).mistaken
+    for other in (0, 7, 8, 255, 256, 511, 4096, (1 << 25) - 1):
+        for id_ in (0, 0xffffff, 0x7fffffff):
+            assert mistaken(max(0, other - 5000), other + 5000, other, id_) == 0
