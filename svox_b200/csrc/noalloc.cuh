@@ -40,11 +40,7 @@ static int noalloc_scratch_address(int32_t** out) {
 
 static int launch_noalloc(const RenderCall& c, const RayBatch& src, int32_t* scratch) {
     const svoxb_tree* t = c.tree;
-    IndexLayout layout = IndexLayout::of(t->M, 0);
-    const int64_t left = kNoAllocWords - (int64_t)layout.words - 64;
-    int64_t bricks = left / (2 * kBrickCells + 1);
-    if (bricks > kMaxBricks) bricks = kMaxBricks;
-    layout = IndexLayout::of(t->M, (int)(bricks > 0 ? bricks : 0));
+    const IndexLayout layout = IndexLayout::within(t->M, kMaxBricks, kNoAllocWords);
     if ((int64_t)layout.words > kNoAllocWords) return SVOXB_ERR_TOO_LARGE;
     // Every part of the scratch is overwritten before it is read, so nothing left over from an
     // earlier call matters.

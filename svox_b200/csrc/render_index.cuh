@@ -132,10 +132,10 @@ build_table_kernel(const int32_t* __restrict__ child, const float* __restrict__ 
 __global__ void __launch_bounds__(256)
 fill_bricks_kernel(const int32_t* __restrict__ child, const float* __restrict__ data, int K,
                    int64_t M, int L, float thresh, int softplus, int cap,
-                   const int32_t* __restrict__ counter, const int32_t* __restrict__ roots,
+                   int32_t* __restrict__ counter, const int32_t* __restrict__ roots,
                    int2* __restrict__ bricks, LogGate gate) {
     if (gate.closed()) return;
-    int n = *counter;
+    int n = *(volatile int32_t*)counter;
     if (n > cap) n = cap;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)n * kBrickCells;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -160,10 +160,18 @@ fill_bricks_kernel(const int32_t* __restrict__ child, const float* __restrict__ 
         }
         bricks[i] = entry;
     }
+    if (gate.log != nullptr) {
+        // counter[1]: blocks that have read the count; the last one clears both for the next build
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(counter + 1, 1) == (int)gridDim.x - 1) counter[0] = counter[1] = 0;
+        }
+    }
 }
 
 // Grid of an index-building kernel over n items: enough blocks to fill the device, not one
-// per 256 items (a launch that finds its gate closed should cost next to nothing).
+// per 256 items.
 inline unsigned index_grid(int64_t n, int block, int sms) {
     const int64_t need = (n + block - 1) / block, most = (int64_t)sms * (2048 / block) * 2;
     return (unsigned)(need < most ? (need > 0 ? need : 1) : most);
@@ -206,20 +214,32 @@ struct IndexLayout {
         l.words = l.bricks + (size_t)l.cap * (2 * kBrickCells);
         return l;
     }
+    // The same with as many bricks as `room` words hold, at most max_bricks; `words` > room: there
+    // is not even room for the table.
+    static IndexLayout within(int64_t M, int max_bricks, int64_t room) {
+        const int64_t left = room - (int64_t)of(M, 0).words - 64;
+        const int64_t bricks = left / (2 * kBrickCells + 1);
+        return of(M, bricks < 0 ? 0 : bricks < max_bricks ? (int)bricks : max_bricks);
+    }
     TreeIndex view(const int32_t* mem) const {
         return TreeIndex{reinterpret_cast<const int2*>(mem), (uint32_t)(bricks / 2), level};
     }
 };
 
 // Launches the kernels that fill an index buffer.  `marks`: only the marked table cells get
-// bricks.
+// bricks.  With a gate nothing is launched that writes unless the gate is open: `counter` then is
+// two words that hold 0, and do so again afterwards.
 static int build_index(const svoxb_tree* t, const IndexLayout& l, float thresh, int softplus,
                        int32_t* mem, LogGate gate, cudaStream_t s,
-                       const uint8_t* marks = nullptr) {
-    const int sms = sm_count();
-    int32_t* counter = mem + l.counter;
+                       const uint8_t* marks = nullptr, int32_t* counter = nullptr) {
+    // (half as many blocks where the gate is hardly ever open: 8 per SM are launched and gone in
+    // some 2 us)
+    const int sms = gate.log ? sm_count() / 2 : sm_count();
     int32_t* roots = mem + l.roots;
-    if (l.cap > 0) SVOXB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int32_t), s));
+    if (!gate.log) {
+        counter = mem + l.counter;
+        if (l.cap > 0) SVOXB_CUDA(cudaMemsetAsync(counter, 0, sizeof(int32_t), s));
+    }
     build_table_kernel<<<index_grid(l.cells, 256, sms), 256, 0, s>>>(
         t->child, t->data, t->K, t->M, l.level, thresh, softplus, l.cap,
         reinterpret_cast<int2*>(mem), counter, roots, marks, gate);

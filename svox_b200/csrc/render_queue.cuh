@@ -70,6 +70,7 @@ struct RecordShape {
 //   [0] chunks asked for   [2] bin shift   [3] number of bins
 //   [1] items in units of 32, each warp's rounded up (items alone would outgrow a word)
 //   [kLogGivenUp] not 0: the log has holes and must not be replayed, whatever its size
+//   [kLogBricks], [.. + 1] counter of an index built in the log's memory (see fallback_index)
 //   [kLogNext + p]         units taken of scatter part p, [kLogNext + kMaxParts + p] blocks done
 //   [kLogBins + b]         groups of bin b      [kLogCleared + b]  cleared units of bin b
 //   [kLogCounts + g]       items of group g (bits 0-7) and its bin (bits 8-)
@@ -90,6 +91,7 @@ struct RecordShape {
 // group per bin, so that the backward can take the packets range by range and the gradient
 // stays in L2 meanwhile.
 constexpr int kMaxParts = 16;   // the scatter can run in up to 16 parts (bin ranges)
+constexpr int kLogBricks = 8;
 constexpr int kLogNext = 32;
 constexpr int kLogBins = kLogNext + 2 * kMaxParts;
 constexpr int kLogCleared = kLogBins + kMaxBins;

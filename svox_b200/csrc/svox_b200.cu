@@ -16,6 +16,11 @@ namespace svoxb {
 // Queue kernels: idle lanes of a warp before it drains its queue and refills (4 and 12 measure
 // within 1 % of 8 on ray batches and images).
 constexpr int kRefillLanes = 8;
+// Rays up to which the marching fallback of a replay walks the tree.  Measured (backward of an
+// overflowed log, 512^3 shell, SH9): 8192 rays 0.75 ms walking, 0.54 with an index, 65536 1.40 and
+// 0.92, 2^20 10.3 and 8.0.  At 4096 rays, 0.70 walking, a log hardly ever overflows (its slack alone
+// holds 256 samples for each ray), and a step of some 100 us would feel the two closed launches.
+constexpr int64_t kWalkRays = 4096;
 // Quarters of the leaf slots a batch has to touch for its log to be sorted.
 constexpr int kSortTouches = 1;
 // ... and warps per SM that a small batch is spread over before warps get 32 rays each.
@@ -357,24 +362,40 @@ struct ClearBeside {
     ~ClearBeside() { if (ready) cudaEventDestroy(ready); }
 };
 
+// The index for the marching fallback of a replay, which does its work only if the log turned out
+// to be of no use: built, in that case, in the log's own memory, with as many bricks as fit.  Up to
+// kWalkRays rays, or without room for the table, the march walks the tree instead (`mem` stays
+// null), which spares the two launches that hardly ever do anything.
+static int fallback_index(const RenderCall& c, IndexLayout* layout, const int32_t** mem) {
+    const int64_t capacity = c.gate.capacity, at = log_packets_at(capacity);
+    const int64_t room = log_words(capacity) - at;
+    *mem = nullptr;
+    if (c.Q <= kWalkRays) return SVOXB_OK;
+    *layout = IndexLayout::within(c.tree->M, g_tuning.render_bricks ? kMaxBricks : 0, room);
+    if ((int64_t)layout->words > room) return SVOXB_OK;
+    int32_t* log = const_cast<int32_t*>(c.gate.log);
+    const int st = build_index(c.tree, *layout, 0.f, c.opt.density_softplus, log + at, c.gate,
+                               c.stream, nullptr, log + kLogBricks);
+    if (st == SVOXB_OK) *mem = log + at;
+    return st;
+}
+
 template <class Source>
 static int launch_queue(const RenderCall& c, const Source& src) {
-    const IndexLayout layout = QueueScratch::layout(c.tree);
+    IndexLayout layout = QueueScratch::layout(c.tree);
     QueueScratch scratch;
     const int32_t* mem = c.prepared;
+    int st = SVOXB_OK;
     if (c.gate.log != nullptr) {
-        // the fallback of a replay hardly ever runs: one launch that walks the tree itself
-        mem = nullptr;
+        if ((st = fallback_index(c, &layout, &mem))) return st;
     } else if (mem == nullptr || c.backward) {
-        const int st = scratch.build(c, src, layout);
-        if (st) return st;
+        if ((st = scratch.build(c, src, layout))) return st;
         mem = scratch.mem;
     }
     TreeIndex index = layout.view(mem);
     if (mem == nullptr) index = TreeIndex{nullptr, 0, 1};
     ClearBeside clear{c};
-    int st = clear.index_built();
-    if (st) return st;
+    if ((st = clear.index_built())) return st;
     st = with_basis(c.opt, [&](auto basis) {
         constexpr int BD = decltype(basis)::value;
         if constexpr (BD > 0) {

@@ -197,3 +197,67 @@ def test_a_log_given_up_is_not_replayed(n, cuda_device):
     log[4] = 0
     assert csrc.log_chunks_used(log) == used
     csrc.check_device_status()
+
+
+@pytest.mark.parametrize("fmt", ["SH9", "RGBA"])
+@pytest.mark.parametrize("image", [False, True])
+def test_march_behind_a_log_that_was_too_small(fmt, image, cuda_device):
+    # its index is built in the log's memory: no room for the table, room for the table, for some
+    # of the bricks (about 4000), for all of them; and for few rays there is no index
+    gen = torch.Generator().manual_seed(5)
+    tree = W.shell_tree(4, 3, fmt, gen, (5.0, 50.0), W._SHELL).to(cuda_device)
+    r = svox.VolumeRenderer(tree)
+    spec, opt = tree._spec(), r._get_options()
+    if image:
+        c2w = W.look_at_cameras(1, gen, 1.6)[0].to(cuda_device)
+        # the image of this camera; rays: 4096 walk the tree, one more builds the index
+        srcs = [svox.render._make_camera_spec(c2w.contiguous(), w, 99, 140.0, 140.0)
+                for w in (41, 240)]
+    else:
+        srcs = [svox.render._rays_spec_from_rays(_rays(n, cuda_device))
+                for n in (4096, 4097, 20000)]
+    old = csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS
+    csrc.log_estimate(wait=True)
+    try:
+        for src in srcs:
+            n = csrc.n_rays_of(src, image)
+            for chunks in (2, 400, 3000, 9000):
+                csrc.log_estimate(wait=True)
+                csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS = 0.0, chunks
+                out, (log, cap) = csrc.volume_render_logged(spec, src, opt, image=image)
+                up = torch.linspace(-1, 1, out.numel(), device=cuda_device).view(out.shape)
+                want = csrc.host().volume_render_backward(spec, src, opt, image, up, out)
+                if csrc.log_chunks_used(log) <= cap:
+                    continue
+                for _ in range(2):               # the counters of the build are put back
+                    got = csrc.volume_render_backward_replay(spec, src, opt, up, out, (log, cap),
+                                                             image=image)
+                    assert _close(got, want), (n, chunks)
+                    got = csrc.volume_render_backward_replay_parts(
+                        spec, src, opt, up, out, (log, cap), 3, lambda rows: None, image=image)
+                    assert _close(got, want), (n, chunks)
+    finally:
+        csrc.log_estimate(wait=True)
+        csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS = old
+    csrc.check_device_status()
+
+
+def test_march_behind_a_log_sees_softplus_densities(cuda_device):
+    gen = torch.Generator().manual_seed(5)
+    tree = W.shell_tree(3, 2, "SH4", gen, (5.0, 50.0), W._SHELL).to(cuda_device)
+    r = svox.VolumeRenderer(tree, density_softplus=True)
+    src, opt, spec = svox.render._rays_spec_from_rays(_rays(6000, cuda_device)), r._get_options(), \
+        tree._spec()
+    old = csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS
+    csrc.log_estimate(wait=True)
+    try:
+        csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS = 0.0, 3000
+        out, logpair = csrc.volume_render_logged(spec, src, opt)
+    finally:
+        csrc.log_estimate(wait=True)
+        csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS = old
+    assert csrc.log_chunks_used(logpair[0]) > logpair[1]
+    up = torch.ones_like(out)
+    assert _close(csrc.volume_render_backward_replay(spec, src, opt, up, out, logpair),
+                  csrc.volume_render_backward(spec, src, opt, up, out))
+    csrc.check_device_status()
