@@ -496,13 +496,31 @@ def volume_render_backward_replay(tree, rays_or_cam, opt, grad_output, fwd_out, 
                                                     fwd_out, log, cap, used, zeroed)
 
 
+# Rays up to which nobody waits to learn whether a log of ``se_grad`` was large enough: its slack
+# alone holds 256 samples for each of them.
+_SE_GRAD_UNCHECKED = 4096
+
+
 def se_grad(tree, rays_or_cam, opt, colors, image=False):
     """-> (render, gradient, Gauss-Newton diagonal) of the squared error against ``colors``
-    (the reference's ``se_grad``) through the item log.  The host does not wait: a log that was
-    too small is noticed on the device, where a march enqueued behind the replay then takes
-    over."""
-    cap = log_capacity(n_rays_of(rays_or_cam, image))
-    return host().se_grad(tree, rays_or_cam, opt, image, colors, cap)
+    (the reference's ``se_grad``) through the item log.
+
+    A log that was too small: up to ``_SE_GRAD_UNCHECKED`` rays that is noticed on the device,
+    where a march enqueued behind the replay takes over.  With more rays that march would take
+    some 20 times as long as the call (it adds float by float), so the host looks, while the replay
+    runs, and repeats the call with a larger log."""
+    n = n_rays_of(rays_or_cam, image)
+    cap = log_capacity(n)
+    for attempt in range(4):
+        out, grad, hess, used = host().se_grad(tree, rays_or_cam, opt, image, colors, cap,
+                                               n > _SE_GRAD_UNCHECKED, attempt == 0)
+        if used <= cap:
+            return out, grad, hess
+        if used < 1 << 40:          # (more: given up, not for its size)
+            cap = used + used // 4 + _LOG_SLACK_CHUNKS
+    grad, hess = se_grad_march(tree, rays_or_cam, opt, out,
+                               colors.reshape(out.shape).contiguous(), image=image)
+    return out, grad, hess
 
 
 def se_grad_march(tree, rays_or_cam, opt, fwd_out, colors, image=False):

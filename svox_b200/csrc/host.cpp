@@ -34,6 +34,7 @@ struct Library {
     X(volume_render_image_backward) X(volume_render_logged) X(volume_render_image_logged)       \
     X(volume_render_backward_replay) X(volume_render_image_backward_replay)                     \
     X(se_grad_replay) X(se_grad_image_replay) X(item_log_words) X(item_log_watch)               \
+    X(item_log_used)                                                                            \
     X(volume_render_logged_clear) X(volume_render_image_logged_clear) X(log_is_sorted)          \
     X(strerror) X(last_cuda_error)
 #define SVOXB_MEMBER(name) decltype(&svoxb_##name) name = nullptr;
@@ -405,7 +406,8 @@ struct Zeroed {
 };
 
 std::pair<Tensor, Tensor> run_logged(const Tree& t, const Source& s, const svoxb_render_options& o,
-                                     int64_t capacity, Zeroed* zeroed = nullptr) {
+                                     int64_t capacity, Zeroed* zeroed = nullptr,
+                                     bool watch = true) {
     const c10::cuda::CUDAGuard guard(t.data.device());
     Tensor out = at::empty(s.shape(3), t.data.options());
     Tensor log = at::empty({lib.item_log_words(capacity)}, t.child.options());
@@ -426,7 +428,7 @@ std::pair<Tensor, Tensor> run_logged(const Tree& t, const Source& s, const svoxb
                      : lib.volume_render_logged(&t.c, &s.rays, &o, to, words, capacity, stream);
     }
     check(st, "volume_render_logged");
-    log_watch().watch(log, capacity, s.count());
+    if (watch) log_watch().watch(log, capacity, s.count());
     return {out, log};
 }
 
@@ -697,13 +699,19 @@ PYBIND11_MODULE(_host, m) {
         return unlocked([&] { return RenderNode::apply(data, std::move(call)); });
     });
 
+    // -> (render, gradient, diagonal, chunks the forward asked for).  `checked`: the host waits for
+    // the forward, while the replay runs, to learn whether the log was large enough; if it was not,
+    // gradient and diagonal are not filled and the call is for the caller to repeat.  Otherwise 0
+    // chunks are returned, and a march behind the replay covers a log that was too small.
     m.def("se_grad", [](py::handle tree, py::handle source, py::handle opt, bool image,
-                        const Tensor& colors, int64_t capacity) {
+                        const Tensor& colors, int64_t capacity, bool checked, bool watch) {
         const Tree t = read_tree(tree);
         const Source s = read_source(source, image, t);
         const svoxb_render_options o = read_options(opt);
         return unlocked([&] {
             const c10::cuda::CUDAGuard guard(t.data.device());
+            if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+                checked = false;                // nobody can wait for a stream that is captured
             Tensor grad, hess;
             const bool beside = fills_beside(t, s, capacity);
             optional<Zeroed> zeroed;
@@ -713,7 +721,9 @@ PYBIND11_MODULE(_host, m) {
                 grad = at::empty(t.data.sizes(), t.data.options());
                 hess = at::empty(t.data.sizes(), t.data.options());
             }
-            auto [out, log] = run_logged(t, s, o, capacity, beside ? &*zeroed : nullptr);
+            auto [out, log] = run_logged(t, s, o, capacity, beside ? &*zeroed : nullptr, watch);
+            at::cuda::CUDAEvent rendered;
+            if (checked) rendered.record(at::cuda::getCurrentCUDAStream(t.data.device().index()));
             const Tensor resid = at::sub(out, colors.reshape(out.sizes())).contiguous();
             check_input(resid, "colors");
             if (beside) {
@@ -723,13 +733,20 @@ PYBIND11_MODULE(_host, m) {
             const float *r = resid.data_ptr<float>(), *f = out.template data_ptr<float>();
             int32_t* words = log.template data_ptr<int32_t>();
             float *g = grad.data_ptr<float>(), *h = hess.data_ptr<float>();
+            const int64_t known = checked ? capacity : 0;
             void* stream = stream_of(t.data);
-            check(s.image ? lib.se_grad_image_replay(&t.c, &s.cam, &o, r, f, words, capacity, 0, g,
-                                                     h, !beside, stream)
-                          : lib.se_grad_replay(&t.c, &s.rays, &o, r, f, words, capacity, 0, g, h,
-                                               !beside, stream),
+            check(s.image ? lib.se_grad_image_replay(&t.c, &s.cam, &o, r, f, words, capacity, known,
+                                                     g, h, !beside, stream)
+                          : lib.se_grad_replay(&t.c, &s.rays, &o, r, f, words, capacity, known, g,
+                                               h, !beside, stream),
                   "se_grad_replay");
-            return std::make_tuple(out, grad, hess);
+            int64_t used = 0;
+            if (checked) {
+                const auto side = Zeroed::side_stream(t.data.device().index());
+                rendered.block(side);
+                check(lib.item_log_used(words, &used, side.stream()), "item_log_used");
+            }
+            return std::make_tuple(out, grad, hess, used);
         });
     });
 

@@ -145,3 +145,39 @@ def test_open_groups_are_never_mistaken(tmp_path):
     for other in (0, 7, 8, 255, 256, 511, 4096, (1 << 25) - 1):
         for id_ in (0, 0xffffff, 0x7fffffff):
             assert mistaken(max(0, other - 5000), other + 5000, other, id_) == 0
+
+
+def test_se_grad_repeats_with_a_larger_log_and_marches_at_last(monkeypatch):
+    calls = []
+
+    class Module:
+        def __init__(self, used):
+            self.used = list(used)
+
+        def poll_logs(self):
+            return []
+
+        def se_grad(self, tree, src, opt, image, colors, cap, checked, watch):
+            calls.append((cap, checked, watch))
+            return "out", "grad", "hess", self.used.pop(0)
+    rays = csrc.RaysSpec()
+    for n, checked in ((4096, False), (4097, True)):
+        rays.origins = torch.zeros(n, 3)
+        calls.clear()
+        module = Module([0])
+        monkeypatch.setattr(csrc, "host", lambda: module)
+        assert csrc.se_grad(None, rays, None, None) == ("out", "grad", "hess")
+        assert [c[1:] for c in calls] == [(checked, True)]
+    calls.clear()
+    module = Module([10 ** 6, 10 ** 6 - 1])
+    assert csrc.se_grad(None, rays, None, None) == ("out", "grad", "hess")
+    assert calls[0][0] < 10 ** 6 < calls[1][0] and [c[2] for c in calls] == [True, False]
+    calls.clear()
+    module = Module([2 ** 63 - 1] * 4)               # given up every time
+    out = torch.ones(n, 3)
+    monkeypatch.setattr(Module, "se_grad", lambda self, *a: (out, None, None, self.used.pop(0)))
+    seen = []
+    monkeypatch.setattr(csrc, "se_grad_march",
+                        lambda *a, **k: seen.append((a[3], a[4].shape)) or ("g", "h"))
+    got = csrc.se_grad(None, rays, None, torch.zeros(3 * n))
+    assert got[0] is out and got[1:] == ("g", "h") and seen == [(out, out.shape)]
