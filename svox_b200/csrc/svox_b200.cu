@@ -263,8 +263,10 @@ static int replay_scatter_block(const ReplayJob& job, int part, int reserve_sms,
     constexpr int K = RecordLength<BD>::K;
     const size_t smem = (size_t)(BLOCK / 32) * sizeof(ScatterSmem<K, HESS ? 2 : 1>);
     auto k = replay_scatter_kernel<BD, BLOCK, HESS, LOBES>;
+    // blocks for the clearing too, which few packets may come with
+    const int64_t clears = job.to.zero_slots * K / kZeroFloats * (BLOCK / 32);
     unsigned grid = 1;
-    int st = persistent_grid(k, BLOCK, smem, job.chunks, &grid);
+    int st = persistent_grid(k, BLOCK, smem, job.chunks > clears ? job.chunks : clears, &grid);
     if (st) return st;
     if (reserve_sms > 0) {
         const int sms = sm_count();
