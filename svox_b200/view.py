@@ -65,12 +65,15 @@ class N3TreeView:
         return tuple(k.to(dev) if torch.is_tensor(k) else k for k in self.key[:n])
 
     def _gather(self, arr):
-        if len(self.key) == 4 and arr.is_contiguous():
+        if len(self.key) == 4 and torch.is_tensor(arr) and arr.is_contiguous() and \
+                arr.shape[1:4] == self.tree.child.shape[1:]:
             # whole records: one packed id each instead of four coordinates, which for a view
             # of leaves lie in host memory (295 MB to copy for the 9.2 M leaves of a 512^3
             # scene: 26 of the 29.5 ms of a weight accumulation over two 800x800 views)
             slots = self._packed_ids
-            if slots is None and isinstance(self._leaf_key, slice):
+            # (the list of slots is that of the tree as it is: not for a view of an earlier one)
+            if slots is None and isinstance(self._leaf_key, slice) and \
+                    self._tree_ver == self.tree._ver:
                 slots = self.tree._leaf_slots()[self._leaf_key]
             if slots is not None and slots.device == arr.device:
                 return arr.view(-1, *arr.shape[4:])[slots]

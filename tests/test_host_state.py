@@ -181,3 +181,22 @@ def test_se_grad_repeats_with_a_larger_log_and_marches_at_last(monkeypatch):
                         lambda *a, **k: seen.append((a[3], a[4].shape)) or ("g", "h"))
     got = csrc.se_grad(None, rays, None, torch.zeros(3 * n))
     assert got[0] is out and got[1:] == ("g", "h") and seen == [(out, out.shape)]
+
+
+def test_aux_of_a_view_made_before_a_refine():
+    tree = svox.N3Tree(data_format="SH1", init_refine=1)
+    view, aux = tree[:], torch.rand(tree.child.shape)
+    want = aux[view.key]
+    assert torch.equal(view.aux(aux), want)
+    tree.refine(sel=(torch.tensor([3]), torch.tensor([0]), torch.tensor([1]), torch.tensor([0])))
+    assert torch.equal(view.aux(aux), want)              # the leaves it was made of
+    grown = torch.cat((aux, torch.rand(5, 2, 2, 2)))
+    assert torch.equal(view.aux(grown), want)
+    with pytest.raises(RuntimeError):
+        view.values
+    view = tree[:]
+    larger = torch.rand(tree.child.shape[0], 3, 3, 3)    # not of the tree's branching
+    assert torch.equal(view.aux(larger), larger[view.key])
+    assert (view.aux(larger.numpy()) == larger[view.key].numpy()).all()
+    with pytest.raises(IndexError):
+        view.aux(torch.rand(100))
