@@ -4,8 +4,9 @@ Same spec classes (``TreeSpec``, ``RaysSpec``, ``CameraSpec``,
 ``RenderOptions``) and the same functions with the same arguments and
 results as the reference's pybind11 module (svox/csrc/svox.cpp:63-122), but
 implemented by the C-ABI library ``libsvox_b200.so`` (hand-written sm_100a
-kernels) loaded with ctypes; the hot calls go through the extension ``_host``.  Tensors are allocated by PyTorch and handed to
-the library as raw device pointers together with the current CUDA stream.
+kernels) loaded with ctypes; the hot calls go through the extension ``_host``.
+Tensors are allocated by PyTorch and handed to the library as raw device
+pointers together with the current CUDA stream.
 
 There is no CPU implementation: if the library is missing or a tensor is
 not on a CUDA device, the call raises.
@@ -20,7 +21,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("SVOXB_LIBRARY") or os.path.join(_HERE, "libsvox_b200.so")
 
 FORMAT_RGBA, FORMAT_SH, FORMAT_SG, FORMAT_ASG = 0, 1, 2, 3
-ERR_TOO_LARGE = 8   # svoxb status: a size limit or the scratch allocation
+ERR_TOO_LARGE = 8   # svoxb status: a size limit
 
 
 class _CTree(C.Structure):
@@ -354,8 +355,8 @@ def calc_corners(tree, indexer):
 
 
 def render_scratch(tree, opt):
-    """The forward render's index of the tree (density-annotated child array, leaf table,
-    bricks) as an int32 tensor, for ``volume_render[_image](..., prepared=...)``: valid until
+    """The forward render's index of the tree (a table of its upper levels and bricks below it, 8
+    bytes per cell) as an int32 tensor, for ``volume_render[_image](..., prepared=...)``: valid until
     the tree, ``opt.sigma_thresh`` or ``opt.density_softplus`` change.  None if this tree /
     format renders through kernels that keep no such index."""
     lib = library()
@@ -488,7 +489,7 @@ def volume_render_backward_replay(tree, rays_or_cam, opt, grad_output, fwd_out, 
     ``used=0``: the host does not know whether the log was large enough and does not wait to
     find out -- the kernels check on the device, and a marching backward enqueued behind them
     takes over in that case.  ``used`` > 0: a count read with ``log_chunks_used`` that fits
-    the capacity (smaller scratch, no fallback enqueued).  ``zeroed``: a zero tensor like
+    the capacity (no fallback is enqueued).  ``zeroed``: a zero tensor like
     ``data`` to add the gradient into (else one is made here)."""
     log, cap = logpair
     with _timed("volume_render_backward"):
@@ -610,18 +611,6 @@ def volume_render_backward_replay_parts(tree, rays_or_cam, opt, grad_output, fwd
                        C.c_void_p(grad_output.data_ptr()), C.c_void_p(fwd_out.data_ptr()),
                        C.c_void_p(log.data_ptr()), C.c_int64(cap), C.c_int64(0),
                        C.c_int(n_parts), C.c_void_p(grad.data_ptr()), _stream(), C.byref(job))
-            if st == ERR_TOO_LARGE:
-                # no room for the sorted samples: march; the parts are then final at once
-                fn = lib.svoxb_volume_render_image_backward if image \
-                    else lib.svoxb_volume_render_backward
-                st = fn(C.byref(ct), C.byref(cs), C.byref(co),
-                        C.c_void_p(grad_output.data_ptr()), C.c_void_p(fwd_out.data_ptr()),
-                        C.c_void_p(grad.data_ptr()), C.c_int(0), _stream())
-                if st:
-                    _raise(st, "volume_render_backward")
-                for lo, hi in ranges:
-                    on_part(flat[lo * K:hi * K])
-                return grad
             if st:
                 _raise(st, "replay_begin")
             try:

@@ -232,8 +232,8 @@ class VolumeRenderer(nn.Module):
     def frozen_tree(self):
         """``with renderer.frozen_tree(): ...`` -- a promise that the tree (structure and
         data) is not modified inside the block.  Forward renders in the block then build the
-        render index of the tree (annotated child array, leaf table, bricks) once instead of
-        on every call, which is what many views of one scene want.  No counterpart in the
+        render index of the tree (a table of its upper levels, bricks below) once instead of on
+        every call, which is what many views of one scene want.  No counterpart in the
         reference; outside the block nothing is kept between calls, because ``tree.data`` can
         be changed through ``.data`` without any version counter noticing."""
         return _FrozenTree(self)
