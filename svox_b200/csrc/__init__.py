@@ -497,6 +497,39 @@ def volume_render_backward_replay(tree, rays_or_cam, opt, grad_output, fwd_out, 
                                                     fwd_out, log, cap, used, zeroed)
 
 
+def volume_render_hessdiag_replay(tree, rays_or_cam, opt, fwd_out, logpair, used, image=False):
+    """Gauss-Newton diagonal of the squared error alone, from the item log (third result of the
+    reference's ``se_grad``).  ``used``: the count from ``log_chunks_used`` (there is no
+    marching fallback for this result, so the caller has to know that the log was large
+    enough)."""
+    lib = library()
+    log, cap = logpair
+    dev = tree.data.device
+    if not 0 < used <= cap:
+        raise RuntimeError("the item log overflowed or its chunk count is not known")
+    with torch.cuda.device(dev):
+        ct = _pack_tree(tree)
+        co = opt._pack()
+        _check_input(fwd_out, "fwd_out")
+        if fwd_out.numel() != 3 * n_rays_of(rays_or_cam, image):
+            raise RuntimeError("fwd_out must have the shape of the render")
+        if log.numel() < log_words(cap):
+            raise RuntimeError("the item log is smaller than its capacity")
+        hess = torch.empty_like(tree.data, memory_format=torch.contiguous_format)
+        if image:
+            cs = _pack_camera(rays_or_cam, dev)
+            fn = lib.svoxb_volume_render_image_hessdiag_replay
+        else:
+            cs = _pack_rays(rays_or_cam, dev)
+            fn = lib.svoxb_volume_render_hessdiag_replay
+        st = fn(C.byref(ct), C.byref(cs), C.byref(co), C.c_void_p(fwd_out.data_ptr()),
+                C.c_void_p(log.data_ptr()), C.c_int64(cap), C.c_int64(used),
+                C.c_void_p(hess.data_ptr()), C.c_int(1), _stream())
+    if st:
+        _raise(st, "volume_render_hessdiag_replay")
+    return hess
+
+
 # Rays up to which nobody waits to learn whether a log of ``se_grad`` was large enough: its slack
 # alone holds 256 samples for each of them.
 _SE_GRAD_UNCHECKED = 4096

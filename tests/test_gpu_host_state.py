@@ -261,3 +261,30 @@ def test_march_behind_a_log_sees_softplus_densities(cuda_device):
     assert _close(csrc.volume_render_backward_replay(spec, src, opt, up, out, logpair),
                   csrc.volume_render_backward(spec, src, opt, up, out))
     csrc.check_device_status()
+
+
+@pytest.mark.parametrize("n", [300, 12000])
+@pytest.mark.parametrize("softplus", [False, True])
+def test_diagonal_alone_equals_that_of_se_grad(n, softplus, cuda_device):
+    gen = torch.Generator().manual_seed(5)
+    tree = W.shell_tree(4, 3, "SH9", gen, (5.0, 50.0), W._SHELL).to(cuda_device)
+    r, rays = svox.VolumeRenderer(tree, density_softplus=softplus), _rays(n, cuda_device)
+    spec, src, opt = tree._spec(), svox.render._rays_spec_from_rays(rays), r._get_options()
+    _, _, want = r.se_grad(rays, torch.zeros(n, 3, device=cuda_device))
+    csrc.log_estimate(wait=True)
+    out, (log, cap) = csrc.volume_render_logged(spec, src, opt)
+    used = csrc.log_chunks_used(log)
+    got = csrc.volume_render_hessdiag_replay(spec, src, opt, out, (log, cap), used)
+    assert _close(got, want)
+    for bad in (0, cap + 1):
+        with pytest.raises(RuntimeError):
+            csrc.volume_render_hessdiag_replay(spec, src, opt, out, (log, cap), bad)
+    c2w = W.look_at_cameras(1, gen, 1.6)[0].to(cuda_device)
+    cam = svox.render._make_camera_spec(c2w.contiguous(), 40, 30, 56.0, 56.0)
+    _, _, want = r.se_grad_persp(c2w, torch.zeros(30, 40, 3, device=cuda_device), width=40,
+                                 height=30, fx=56.0)
+    out, (log, cap) = csrc.volume_render_logged(spec, cam, opt, image=True)
+    got = csrc.volume_render_hessdiag_replay(spec, cam, opt, out, (log, cap),
+                                             csrc.log_chunks_used(log), image=True)
+    assert _close(got, want)
+    csrc.check_device_status()
