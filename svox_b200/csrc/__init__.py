@@ -11,6 +11,7 @@ pointers together with the current CUDA stream.
 There is no CPU implementation: if the library is missing or a tensor is
 not on a CUDA device, the call raises.
 """
+import copy
 import ctypes as C
 import os
 
@@ -546,6 +547,9 @@ def se_grad(tree, rays_or_cam, opt, colors, image=False):
     n = n_rays_of(rays_or_cam, image)
     cap = log_capacity(n)
     for attempt in range(4):
+        if attempt == 1 and tree._weight_accum is not None:     # the weights have been added
+            tree = copy.copy(tree)
+            tree._weight_accum = None
         out, grad, hess, used = host().se_grad(tree, rays_or_cam, opt, image, colors, cap,
                                                n > _SE_GRAD_UNCHECKED, attempt == 0)
         if used <= cap:

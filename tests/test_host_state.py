@@ -149,6 +149,8 @@ def test_open_groups_are_never_mistaken(tmp_path):
 
 def test_se_grad_repeats_with_a_larger_log_and_marches_at_last(monkeypatch):
     calls = []
+    tree = csrc.TreeSpec()
+    tree._weight_accum = torch.zeros(8)
 
     class Module:
         def __init__(self, used):
@@ -158,7 +160,7 @@ def test_se_grad_repeats_with_a_larger_log_and_marches_at_last(monkeypatch):
             return []
 
         def se_grad(self, tree, src, opt, image, colors, cap, checked, watch):
-            calls.append((cap, checked, watch))
+            calls.append((cap, checked, watch, tree._weight_accum))
             return "out", "grad", "hess", self.used.pop(0)
     rays = csrc.RaysSpec()
     for n, checked in ((4096, False), (4097, True)):
@@ -166,12 +168,14 @@ def test_se_grad_repeats_with_a_larger_log_and_marches_at_last(monkeypatch):
         calls.clear()
         module = Module([0])
         monkeypatch.setattr(csrc, "host", lambda: module)
-        assert csrc.se_grad(None, rays, None, None) == ("out", "grad", "hess")
-        assert [c[1:] for c in calls] == [(checked, True)]
+        assert csrc.se_grad(tree, rays, None, None) == ("out", "grad", "hess")
+        assert [c[1:3] for c in calls] == [(checked, True)]
     calls.clear()
     module = Module([10 ** 6, 10 ** 6 - 1])
-    assert csrc.se_grad(None, rays, None, None) == ("out", "grad", "hess")
+    assert csrc.se_grad(tree, rays, None, None) == ("out", "grad", "hess")
     assert calls[0][0] < 10 ** 6 < calls[1][0] and [c[2] for c in calls] == [True, False]
+    # weights are accumulated once
+    assert calls[0][3] is tree._weight_accum is not None and calls[1][3] is None
     calls.clear()
     module = Module([2 ** 63 - 1] * 4)               # given up every time
     out = torch.ones(n, 3)
@@ -179,7 +183,7 @@ def test_se_grad_repeats_with_a_larger_log_and_marches_at_last(monkeypatch):
     seen = []
     monkeypatch.setattr(csrc, "se_grad_march",
                         lambda *a, **k: seen.append((a[3], a[4].shape)) or ("g", "h"))
-    got = csrc.se_grad(None, rays, None, torch.zeros(3 * n))
+    got = csrc.se_grad(tree, rays, None, torch.zeros(3 * n))
     assert got[0] is out and got[1:] == ("g", "h") and seen == [(out, out.shape)]
 
 
