@@ -433,12 +433,15 @@ def log_estimate(wait=False):
 
 def log_eligible(tree, opt):
     """Whether the logged forward / replay backward pair applies to this call."""
-    K = tree.data.shape[4]
+    data = tree.data
+    M, N, K = data.shape[0], data.shape[1], data.shape[4]
     layout = K == 4 if opt.format == FORMAT_RGBA else \
         opt.basis_dim in (1, 4, 9, 16, 25) and K == 3 * opt.basis_dim + 1
-    return (layout and tree.data.shape[1] == 2
+    return (layout and N == 2 and M < 1 << 28
             and opt.sigma_thresh == 0.0 and opt.stop_thresh == 0.0
-            and tree.data.dtype == torch.float32)
+            and data.dtype == torch.float32
+            # records of whole 16-byte words are read as such
+            and (K % 4 != 0 or data.data_ptr() % 16 == 0))
 
 
 def log_capacity(n_rays):

@@ -292,10 +292,10 @@ class VolumeRenderer(nn.Module):
         -> ``colors (B, 3), grad (shape of tree.data), diag_hessian (shape of tree.data)``.
         The diagonal is the squared norm of the Jacobian's columns, as in the reference
         (with ``density_softplus`` plus the reference's own second-order term for the density).
-        Octrees with three colour channels of 1, 4, 9, 16 or 25 basis functions (SH, SG or
-        ASG) take the route through the item log; every other layout with at most four
-        output channels (RGBA, N != 2, other basis sizes) is marched twice (the forward,
-        then gradient and diagonal together).
+        Octrees with RGBA records of four floats or three colour channels of 1, 4, 9, 16 or 25
+        basis functions (SH, SG or ASG) take the route through the item log; every other layout
+        with at most four output channels (N != 2, other basis sizes, records at odd addresses)
+        is marched twice (the forward, then gradient and diagonal together).
         """
         self._require_cuda(True)
         return self._se_grad(_rays_spec_from_rays(rays), colors, False)
@@ -316,8 +316,7 @@ class VolumeRenderer(nn.Module):
         with torch.no_grad():
             colors = colors.to(device=self.tree.data.device, dtype=self.tree.data.dtype)
             if not _C.log_eligible(tree, opt):
-                # any other layout (RGBA, N != 2, other basis sizes): the forward, then one
-                # more march for gradient and diagonal
+                # any other layout: the forward, then one more march for gradient and diagonal
                 out = (_C.volume_render_image if image else _C.volume_render)(tree, src, opt)
                 grad, hess = _C.se_grad_march(tree, src, opt, out,
                                               colors.reshape(out.shape).contiguous(),

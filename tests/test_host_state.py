@@ -204,3 +204,19 @@ def test_aux_of_a_view_made_before_a_refine():
     assert (view.aux(larger.numpy()) == larger[view.key].numpy()).all()
     with pytest.raises(IndexError):
         view.aux(torch.rand(100))
+
+
+@pytest.mark.parametrize("fmt,floats", [("RGBA", 4), ("SH1", 4), ("SH9", 28), ("SH4", 13)])
+def test_records_that_cannot_be_read_in_words_are_not_logged(fmt, floats):
+    # they are rendered and differentiated by the kernels for any alignment
+    opt = csrc.RenderOptions()
+    opt.format = csrc.FORMAT_RGBA if fmt == "RGBA" else csrc.FORMAT_SH
+    opt.basis_dim = (floats - 1) // 3 if fmt != "RGBA" else -1
+    tree = csrc.TreeSpec()
+    flat = torch.zeros(8 * floats + 4)
+    for shift in range(4):
+        tree.data = flat[shift:shift + 8 * floats].view(1, 2, 2, 2, floats)
+        whole = tree.data.data_ptr() % 16 == 0
+        assert csrc.log_eligible(tree, opt) == (whole or floats % 4 != 0)
+    tree.data = torch.empty(1 << 28, 2, 2, 2, floats, device="meta")
+    assert not csrc.log_eligible(tree, opt)              # more nodes than the log has bits for
