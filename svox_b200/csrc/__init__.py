@@ -16,6 +16,7 @@ import ctypes as C
 import os
 
 import torch
+from torch.autograd import forward_ad as _fwd
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # SVOXB_LIBRARY: load another build of the library (e.g. one compiled with other flags)
@@ -447,6 +448,13 @@ def log_eligible(tree, opt):
 def log_capacity(n_rays):
     """Chunks of the next log for ``n_rays`` rays."""
     return int(n_rays * _LogWatch.poll() / 32) + _LOG_SLACK_CHUNKS
+
+
+def refuse_tangent(data):
+    """Raises for a ``data`` that carries a forward-mode tangent: there is no derivative of that
+    kind here, and the calls that make no autograd node would drop it."""
+    if _fwd._current_level >= 0 and _fwd.unpack_dual(data).tangent is not None:
+        raise NotImplementedError("svox_b200 has no forward-mode derivatives")
 
 
 def log_words(capacity):

@@ -265,6 +265,7 @@ class VolumeRenderer(nn.Module):
         opt = self._get_options(fast)
         tree = self.tree._spec()
         data = tree.data
+        _C.refuse_tangent(data)
         train = data.requires_grad and torch.is_grad_enabled()
         if not train and _C._timing is None:
             render = _C.volume_render_image if image else _C.volume_render

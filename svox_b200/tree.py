@@ -39,6 +39,7 @@ class _QueryVerticalFunction:
     def apply(data, tree_spec, indices):
         # (clearing the gradient buffer on a second stream beside the forward query, as the
         # renderer does, was measured: no gain, both are bound by DRAM)
+        _C.refuse_tangent(data)
         if data.requires_grad and torch.is_grad_enabled():
             return _C.host().query_node(data, tree_spec, indices)
         return _C.query_vertical(tree_spec, indices)

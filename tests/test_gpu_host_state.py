@@ -320,3 +320,19 @@ def test_records_at_any_address(fmt, cuda_device):
         # test_se_grad_through_either_log_and_without)
         assert (a - b).abs().max() <= 3e-4 * b.abs().max()
     csrc.check_device_status()
+
+
+def test_forward_mode_tangents_are_refused(cuda_device):
+    from torch.autograd import forward_ad
+    tree = _tree(cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(10, cuda_device)
+    pts = torch.rand(10, 3, device=cuda_device)
+    data = tree.data.detach()
+    del tree.data
+    with forward_ad.dual_level():
+        tree.data = forward_ad.make_dual(data, torch.ones_like(data))
+        for call in (lambda: r(rays), lambda: tree(pts)):
+            with pytest.raises(NotImplementedError):
+                call()
+        tree.data = data
+        assert r(rays).shape == (10, 3) and tree(pts).shape == (10, tree.data_dim)

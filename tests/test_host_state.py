@@ -220,3 +220,18 @@ def test_records_that_cannot_be_read_in_words_are_not_logged(fmt, floats):
         assert csrc.log_eligible(tree, opt) == (whole or floats % 4 != 0)
     tree.data = torch.empty(1 << 28, 2, 2, 2, floats, device="meta")
     assert not csrc.log_eligible(tree, opt)              # more nodes than the log has bits for
+
+
+def test_forward_mode_tangents_are_refused():
+    from torch.autograd import forward_ad
+    from svox_b200.tree import _QueryVerticalFunction
+    data = torch.zeros(1, 2, 2, 2, 4)
+    csrc.refuse_tangent(data)
+    with forward_ad.dual_level():
+        csrc.refuse_tangent(data)
+        dual = forward_ad.make_dual(data, torch.ones_like(data))
+        with pytest.raises(NotImplementedError):
+            csrc.refuse_tangent(dual)
+        with pytest.raises(NotImplementedError):
+            _QueryVerticalFunction.apply(dual, None, torch.zeros(1, 3))
+    csrc.refuse_tangent(data)
