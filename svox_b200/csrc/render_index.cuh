@@ -232,8 +232,7 @@ struct IndexLayout {
 static int build_index(const svoxb_tree* t, const IndexLayout& l, float thresh, int softplus,
                        int32_t* mem, LogGate gate, cudaStream_t s,
                        const uint8_t* marks = nullptr, int32_t* counter = nullptr) {
-    // (half as many blocks where the gate is hardly ever open: 8 per SM are launched and gone in
-    // some 2 us)
+    // (half as many blocks where the gate is hardly ever open: launched and gone in 4 us)
     const int sms = gate.log ? sm_count() / 2 : sm_count();
     int32_t* roots = mem + l.roots;
     if (!gate.log) {

@@ -18,9 +18,10 @@ namespace svoxb {
 constexpr int kRefillLanes = 8;
 // Rays up to which the marching fallback of a replay walks the tree.  Measured (backward of an
 // overflowed log, 512^3 shell, SH9): 8192 rays 0.75 ms walking, 0.54 with an index, 65536 1.40 and
-// 0.92, 2^20 10.3 and 8.0.  At 4096 rays, 0.70 walking, a log hardly ever overflows (its slack alone
-// holds 256 samples for each ray), and a step of some 100 us would feel the two closed launches.
-constexpr int64_t kWalkRays = 4096;
+// 0.92, 2^18 3.19 and 2.32, 2^20 10.3 and 8.0.  The index would pay earlier, if the log overflowed
+// at every call; but its two closed launches take 8 us of every other call (3 % of a step with
+// 65536 rays of an RGBA tree, 0.5 % with 2^18 of the shell).
+constexpr int64_t kWalkRays = 1 << 17;
 // Quarters of the leaf slots a batch has to touch for its log to be sorted.
 constexpr int kSortTouches = 1;
 // ... and warps per SM that a small batch is spread over before warps get 32 rays each.
@@ -367,7 +368,7 @@ struct ClearBeside {
 // The index for the marching fallback of a replay, which does its work only if the log turned out
 // to be of no use: built, in that case, in the log's own memory, with as many bricks as fit.  Up to
 // kWalkRays rays, or without room for the table, the march walks the tree instead (`mem` stays
-// null), which spares the two launches that hardly ever do anything.
+// null).
 static int fallback_index(const RenderCall& c, IndexLayout* layout, const int32_t** mem) {
     const int64_t capacity = c.gate.capacity, at = log_packets_at(capacity);
     const int64_t room = log_words(capacity) - at;

@@ -210,18 +210,18 @@ def test_march_behind_a_log_that_was_too_small(fmt, image, cuda_device):
     spec, opt = tree._spec(), r._get_options()
     if image:
         c2w = W.look_at_cameras(1, gen, 1.6)[0].to(cuda_device)
-        # the image of this camera; rays: 4096 walk the tree, one more builds the index
-        srcs = [svox.render._make_camera_spec(c2w.contiguous(), w, 99, 140.0, 140.0)
-                for w in (41, 240)]
+        # 2^17 pixels (or rays) walk the tree, more build the index
+        srcs = [svox.render._make_camera_spec(c2w.contiguous(), 512, h, 700.0, 700.0)
+                for h in (20, 256, 257)]
     else:
         srcs = [svox.render._rays_spec_from_rays(_rays(n, cuda_device))
-                for n in (4096, 4097, 20000)]
+                for n in (5000, 1 << 17, (1 << 17) + 1)]
     old = csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS
     csrc.log_estimate(wait=True)
     try:
         for src in srcs:
             n = csrc.n_rays_of(src, image)
-            for chunks in (2, 400, 3000, 9000):
+            for chunks in (2, 400, 3000, 20000):
                 csrc.log_estimate(wait=True)
                 csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS = 0.0, chunks
                 out, (log, cap) = csrc.volume_render_logged(spec, src, opt, image=image)
@@ -246,7 +246,7 @@ def test_march_behind_a_log_sees_softplus_densities(cuda_device):
     gen = torch.Generator().manual_seed(5)
     tree = W.shell_tree(3, 2, "SH4", gen, (5.0, 50.0), W._SHELL).to(cuda_device)
     r = svox.VolumeRenderer(tree, density_softplus=True)
-    src, opt, spec = svox.render._rays_spec_from_rays(_rays(6000, cuda_device)), r._get_options(), \
+    src, opt, spec = svox.render._rays_spec_from_rays(_rays(140000, cuda_device)), r._get_options(), \
         tree._spec()
     old = csrc._items_per_ray, csrc._LOG_SLACK_CHUNKS
     csrc.log_estimate(wait=True)
