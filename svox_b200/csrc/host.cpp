@@ -261,6 +261,10 @@ void* stream_of(const Tensor& t) {
     return at::cuda::getCurrentCUDAStream(t.device().index()).stream();
 }
 
+bool capturing() {      // on the current stream of the current device
+    return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+}
+
 // ---------------------------------------------------------------------------
 // How large the item log has to be, learnt without making the host wait: after a logged forward
 // the counts at the head of its log are copied to a slot of pinned memory that holds -1 until
@@ -270,6 +274,9 @@ class LogWatch {
     struct Seen { int64_t used, batches, rays, capacity; };
 
     void watch(const Tensor& log, int64_t capacity, int64_t rays) {
+        // a forward that is captured would write to its slot at every replay, also when the slot
+        // has long been another forward's
+        if (capturing()) return;
         std::lock_guard<std::mutex> lock(mutex_);
         if (!slots_.defined())
             slots_ = torch::full({kSlots, 2}, -1, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
@@ -710,8 +717,7 @@ PYBIND11_MODULE(_host, m) {
         const svoxb_render_options o = read_options(opt);
         return unlocked([&] {
             const c10::cuda::CUDAGuard guard(t.data.device());
-            if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-                checked = false;                // nobody can wait for a stream that is captured
+            if (capturing()) checked = false;       // nobody can wait for a captured stream
             Tensor grad, hess;
             const bool beside = fills_beside(t, s, capacity);
             optional<Zeroed> zeroed;

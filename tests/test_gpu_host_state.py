@@ -336,3 +336,41 @@ def test_forward_mode_tangents_are_refused(cuda_device):
                 call()
         tree.data = data
         assert r(rays).shape == (10, 3) and tree(pts).shape == (10, tree.data_dim)
+
+
+@pytest.mark.parametrize("n", [300, 12000])
+def test_training_step_in_a_graph(n, cuda_device):
+    # the counts of a captured forward are nobody's: its slot would be written at every replay
+    gen = torch.Generator().manual_seed(5)
+    tree = W.shell_tree(4, 3, "SH9", gen, (5.0, 50.0), W._SHELL).to(cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(n, cuda_device)
+    up = torch.ones(n, 3, device=cuda_device)
+    want = _grad(tree, lambda: r(rays), up).clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(3):
+            _grad(tree, lambda: r(rays), up)
+    torch.cuda.current_stream().wait_stream(side)
+    csrc.log_estimate(wait=True)
+    assert not csrc.host().logs_pending()
+    tree.data.grad = None
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        r(rays).backward(up)
+    assert not csrc.host().logs_pending()
+    got = tree.data.grad
+    for _ in range(2):
+        got.fill_(7.0)                      # the step writes the whole gradient anew
+        graph.replay()
+        torch.cuda.synchronize()
+        assert _close(got, want)
+    before = csrc.log_estimate()
+    few = svox.Rays(*[t[:10].contiguous() for t in rays])
+    for _ in range(20):                     # takes every slot there is
+        graph.replay()
+        _grad(tree, lambda: r(few), up[:10].contiguous())
+        graph.replay()
+        csrc.log_estimate(wait=True)
+    assert csrc.log_estimate() <= max(before, 1000.0)
+    csrc.check_device_status()
