@@ -56,14 +56,14 @@ METRICS = {
     "image5": "Mrays/s render_persp forward (SH deg 3, three shells at 1024^3, 1920x1080 views)",
 }
 # DRAM bytes (read + write) of one launch of the training step's kernels: the logged march from an
-# ncu capture of a 2^17-ray launch (1.657 GB read + 0.381 GB written), scaled by 8 because its
+# ncu capture of a 2^17-ray launch (1.658 GB read + 0.383 GB written), scaled by 8 because its
 # traffic grows with the rays; the scatter's does not (the gradient is written once whatever the
 # number of rays), so no scaled figure is given for it.  Printed only together with
 # `traffic_source`, which names the capture.
-NCU_TRAFFIC = {"forward": 8 * (1.657470e9 + 0.381325e9), "backward": None}
+NCU_TRAFFIC = {"forward": 8 * (1.658214e9 + 0.382567e9), "backward": None}
 NCU_TRAFFIC_SOURCE = ("ncu --set full of render_queue_kernel<9,2,768> at 2^17 rays x 8 "
                       "(profiles/training_step_rays131072_ncu_full.md); valid for the kernel as "
-                      "of library version " + "0.4.0")
+                      "of library version " + "0.4.1")
 
 
 def parse():
@@ -640,10 +640,10 @@ def run_train(a):
                           "frac": (fwd_bytes + bwd_bytes) / ms_step / 1e6 / (peak * world)},
         "e2e": e2e,
         # per step: forward = leaf table, brick fill, march, ordering of the log; backward =
-        # scatter (one launch per part) and the marching fallback, which returns at once unless
-        # the log overflowed
+        # scatter (one launch per part) and the marching fallback with, from 2^17 rays on, table
+        # and brick fill of its own, which return at once unless the log overflowed
         "gpu_launches": (4 + (a.overlap_parts if best == "allreduce_inside_backward" else 1)
-                         + 1 + (1 if best == "allreduce_multicast" else 0)) * a.steps,
+                         + (3 if n_local > 1 << 17 else 1) + (1 if best == "allreduce_multicast" else 0)) * a.steps,
         "clocks": clocks,
     }
     if check is not None:

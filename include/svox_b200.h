@@ -202,7 +202,10 @@ int svoxb_volume_render_image_prepared(const svoxb_tree* tree, const svoxb_camer
  * stays in L2 while it is reduced.
  * Only for octrees with RGBA records of four floats or three colour channels
  * of 1, 4, 9, 16 or 25 basis functions (SH, SG or ASG) and sigma_thresh =
- * stop_thresh = 0 (else SVOXB_ERR_FORMAT / SVOXB_ERR_OPTION).  `data` must not change between the two calls.
+ * stop_thresh = 0 (else SVOXB_ERR_FORMAT / SVOXB_ERR_OPTION).  `data` must not
+ * change between the two calls.  The replay counts in the log's head, and its
+ * fallback (below) uses the memory of a log that is of no use: a log can be
+ * replayed several times, but by one call at a time.
  *
  * A log that was too small must not be replayed.  `chunks_used` says who
  * checks that:
@@ -210,12 +213,12 @@ int svoxb_volume_render_image_prepared(const svoxb_tree* tree, const svoxb_camer
  *        device and do nothing if the forward asked for more chunks than
  *        `capacity_chunks`; a marching backward (as
  *        svoxb_volume_render_backward) is enqueued behind them that does its
- *        work only in that case, or if the forward gave the log up.  No host synchronisation; the result is the
- *        gradient either way.
+ *        work only in that case, or if the forward gave the log up.  No host
+ *        synchronisation; the result is the gradient either way.
  *   > 0  the caller read the count with svoxb_item_log_used (which
  *        synchronises) and found it <= capacity_chunks: no fallback is
- *        enqueued.  With a larger
- *        count the caller must call svoxb_volume_render_backward instead.
+ *        enqueued.  With a larger count the caller must call
+ *        svoxb_volume_render_backward instead.
  */
 int64_t svoxb_item_log_words(int64_t capacity_chunks);
 /* 1 if a logged forward of n_rays rays (image != 0: pixels) sorts its samples.

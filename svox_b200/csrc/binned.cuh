@@ -60,10 +60,10 @@ struct UnitShared {
 //
 // Units are taken by blocks in order from one counter, so that the grid works within a window
 // much smaller than a bin (with a fixed assignment the blocks drift apart and several bins compete
-// for the L2: 2.9 ms for the scatter of 2^20 rays instead of 1.7; with a unit per warp the counter
-// itself is the bound, some 6 ns per unit).  A unit may have to wait for the clearing of its bin:
-// those units were all taken before it, and a block works on its units in order, so the oldest
-// unit that is not done never waits.
+// for the L2: 2.9 ms for the scatter of 2^20 rays against 1.7 in this order, then; with a unit per
+// warp the counter itself is the bound, some 6 ns per unit).  A unit may have to wait for the
+// clearing of its bin: those units were all taken before it, and a block works on its units in
+// order, so the oldest unit that is not done never waits.
 template <int BLOCK, class Count, class Clear, class Work>
 __device__ __forceinline__ void ordered_units(UnitShared& s, const UnitCounters& counters, int lo,
                                               int hi, int before, int per_unit, int64_t bin_floats,

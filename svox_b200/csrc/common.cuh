@@ -149,8 +149,8 @@ struct TopScratch {
     ~TopScratch() { if (cells) cudaFreeAsync(cells, stream); }
 };
 
-// Gradient MB one log bin spans.  Measured on the scatter of the training step: 32 -> 1.49 ms,
-// 64 -> 1.62, 128 -> 2.39, 256 -> 3.40, unsorted 4.50.
+// Gradient MB one log bin spans.  Measured on the scatter of the training step while it still found
+// its gradient cleared: 32 -> 1.49 ms, 64 -> 1.62, 128 -> 2.39, 256 -> 3.40, unsorted 4.50.
 constexpr int kReplayBinMB = 32;
 
 // The two switches the tests flip to show that an index or a bin size changes no result

@@ -11,7 +11,7 @@
 // HBM roofline per point: 12 B in + K*4 B gathered + K*4 B written + 8 B id
 // (+ one 4-B child entry per level below the jump table, L2 resident).  2^24 points over 256^3
 // leaves of 49 floats, 268 of the 196 bytes per record read (64-byte pieces): 1.75 -> 1.63 ms.
-// Backward: 3.43 ms (clear, then reductions at random) -> 2.77 ms (binned, see below).
+// Backward: 3.43 ms (clear, then reductions at random) -> 2.63 ms (binned, see below).
 #pragma once
 
 #include "common.cuh"

@@ -20,7 +20,7 @@
 // Bound: issue slots where neighbouring rays share records (images: 63 % of the slots used), DRAM
 // too where every sample's record misses (rays in random order: 16 GB for 2^20 rays of the 512^3
 // shell scene).  So the march is kept short, 138 instructions per iteration and 259 per batch of
-// items: the position's bits come from one truncating addition instead of conversions, the leaf's
+// items with SH9 records (some 540 with SH16): the position's bits come from one truncating addition instead of conversions, the leaf's
 // exit distance needs five operations per axis, lanes between samples compute along instead of
 // branching, what only items need is done where all lanes have one, the index entry of a sample
 // is requested one iteration ahead so that the queue's work covers its latency, and a block holds

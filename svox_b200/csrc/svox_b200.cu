@@ -13,8 +13,8 @@
 
 namespace svoxb {
 
-// Queue kernels: idle lanes of a warp before it drains its queue and refills (4 and 12 measure
-// within 1 % of 8 on ray batches and images).
+// Queue kernels: idle lanes of a warp before it drains its queue and refills (5 measured level on
+// ray batches and 2 % slower on 1080p views, 12 1 % slower on both).
 constexpr int kRefillLanes = 8;
 // Rays up to which the marching fallback of a replay walks the tree.  Measured (backward of an
 // overflowed log, 512^3 shell, SH9): 8192 rays 0.75 ms walking, 0.54 with an index, 65536 1.40 and
@@ -161,7 +161,7 @@ static int replay_bins(int64_t M, int K) {
 
 // Whether a logged forward sorts its items into bins: when the gradient outgrows a bin and a
 // good part of it is touched (64 contributing samples per ray of a random batch, 24 per pixel,
-// against the leaf slots).  Then the scatter finds the gradient in L2 and clears it on the way.
+// against the leaf slots: the averages of the 512^3 shell scene, the only one measured).  Then the scatter finds the gradient in L2 and clears it on the way.
 // (A log of 2^26 chunks, 100 GB, or more is not sorted: no such size has been run.)
 static bool sorts_log(const svoxb_tree* t, int64_t rays, bool image, int64_t capacity) {
     if (capacity / kSortedChunks >= 0xffffff || replay_bins(t->M, t->K) < 2) return false;
@@ -1161,7 +1161,7 @@ int svoxb_allreduce_multimem(float* multicast, int64_t n_floats, int rank, int w
     return SVOXB_OK;
 }
 
-const char* svoxb_version(void) { return "0.4.0"; }
+const char* svoxb_version(void) { return "0.4.1"; }
 
 // Test hook (include/svox_b200_testing.h): key 5 = MB of gradient one replay bin spans,
 // key 7 = bricks below the render leaf table on / off.
