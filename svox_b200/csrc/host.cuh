@@ -42,21 +42,22 @@ int blocks_per_sm(const void* kernel, int block, size_t smem, int* per_sm) {
     static std::vector<Known> all;
     int dev = 0;
     SVOXB_CUDA(cudaGetDevice(&dev));
-    {
-        std::lock_guard<std::mutex> lock(mutex);
-        for (const Known& k : all)
-            if (k.kernel == kernel && k.dev == dev && k.block == block && k.smem == smem) {
-                *per_sm = k.per_sm;
-                return SVOXB_OK;
-            }
+    std::lock_guard<std::mutex> lock(mutex);
+    size_t limit = 20 * 1024;    // the 48 KB a kernel gets without asking, less its static share
+    for (const Known& k : all) {
+        if (k.kernel != kernel || k.dev != dev) continue;
+        if (k.block == block && k.smem == smem) {
+            *per_sm = k.per_sm;
+            return SVOXB_OK;
+        }
+        if (k.smem > limit) limit = k.smem;
     }
-    // the 48 KB a kernel gets without asking cover its static shared memory too (up to 4 KB here)
-    if (smem > 40 * 1024)
+    // (raised only: an earlier call's size stays good)
+    if (smem > limit)
         SVOXB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem));
     SVOXB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, block, smem));
     if (*per_sm < 1) *per_sm = 1;
-    std::lock_guard<std::mutex> lock(mutex);
     all.push_back(Known{kernel, smem, block, dev, *per_sm});
     return SVOXB_OK;
 }

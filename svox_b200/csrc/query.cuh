@@ -11,11 +11,13 @@
 // HBM roofline per point: 12 B in + K*4 B gathered + K*4 B written + 8 B id
 // (+ one 4-B child entry per level below the jump table, L2 resident).  2^24 points over 256^3
 // leaves of 49 floats, 268 of the 196 bytes per record read (64-byte pieces): 1.75 -> 1.63 ms.
-// Backward: 3.43 ms (clear, then reductions at random) -> 2.63 ms (binned, see below).
+// Backward: 3.43 ms (clear, then reductions at random) -> 2.57 (binned) -> 2.0 (summed by tiles, see
+// below).
 #pragma once
 
 #include "common.cuh"
 #include "binned.cuh"
+#include "tiles.cuh"
 
 namespace svoxb {
 
@@ -371,6 +373,242 @@ scatter_binned_rows_kernel(int64_t Q, const float* __restrict__ rows, int K,
                                [&](int i) { return b.count[i]; }, clear, work);
 }
 
+// Long rows into a gradient far larger than the L2: the points are sorted by tile of the gradient, and
+// a block adds up the rows of a tile's points (tiles.cuh).
+constexpr int kPlaceBlock = 512;
+constexpr int kPlaceEach = 16;       // points a thread places at a time
+
+// Items per tile of the points.
+template <bool SHARED>
+__global__ void __launch_bounds__(kPlaceBlock)
+count_tiles_kernel(const int64_t* __restrict__ ids, int64_t Q, TileLists t) {
+    extern __shared__ int s_count[];
+    if (SHARED) {
+        for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock) s_count[i] = 0;
+        __syncthreads();
+    }
+    for (int64_t i = (int64_t)blockIdx.x * kPlaceBlock + threadIdx.x; i < Q;
+         i += (int64_t)gridDim.x * kPlaceBlock) {
+        const int64_t slot = ids[i];
+        if (slot >= 0 && slot < t.n_rows)
+            atomicAdd((SHARED ? s_count : t.count) + (int)(slot >> t.shift), 1);
+    }
+    if (!SHARED) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock)
+        if (s_count[i]) atomicAdd(t.count + i, s_count[i]);
+}
+
+// Lists the points {slot, row} tile by tile.  0.19 ms for 2^24 points and 4681 tiles, the same with
+// 256 to 1024 threads.
+template <bool SHARED>
+__global__ void __launch_bounds__(kPlaceBlock)
+place_tiles_kernel(const int64_t* __restrict__ ids, int64_t Q, TileLists t, int2* __restrict__ pair,
+                  int K, float* __restrict__ grad) {
+    extern __shared__ int s_count[];
+    clear_hot_tiles(t, K, grad);
+    constexpr int EACH = SHARED ? kPlaceEach : 1;
+    for (int64_t tile = blockIdx.x; tile * (EACH * kPlaceBlock) < Q; tile += gridDim.x) {
+        if (SHARED) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock) s_count[i] = 0;
+            __syncthreads();
+        }
+        int slot[EACH], rank[EACH];
+#pragma unroll
+        for (int j = 0; j < EACH; ++j) {
+            const int64_t i = tile * (EACH * kPlaceBlock) + kPlaceBlock * j + threadIdx.x;
+            const int64_t s = i < Q ? ids[i] : -1;
+            slot[j] = s >= 0 && s < t.n_rows ? (int)s : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < EACH; ++j)
+            rank[j] = slot[j] >= 0
+                          ? atomicAdd((SHARED ? s_count : t.end) + (slot[j] >> t.shift), 1) : 0;
+        if (SHARED) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock)
+                if (s_count[i] > 0) s_count[i] = atomicAdd(t.end + i, s_count[i]);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int j = 0; j < EACH; ++j)
+            if (slot[j] >= 0)
+                pair[rank[j] + (SHARED ? s_count[slot[j] >> t.shift] : 0)] = make_int2(
+                    slot[j], (int)(tile * (EACH * kPlaceBlock) + kPlaceBlock * j + threadIdx.x));
+    }
+}
+
+// A 16-byte word into shared memory, asynchronously, in 64-byte pieces of L2 lines.
+__device__ __forceinline__ void copy_word(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global.L2::64B [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+
+constexpr int kStageWords = 104;     // 16-byte words of rows a warp has under way per stage
+
+// Warps take equal shares of a tile's sorted items; lane e of a warp holds columns e, e + 32, ... of
+// the row being summed (N of them; further columns in further passes).  Rows come in as the 16-byte
+// words that cover them, a stage of some rows ahead of the one being summed; finished rows, and
+// zeros between them, leave through a StreamWriter.  2^24 rows of 49 floats into 3.76 GB: 2.41 ms
+// with the gradient cleared and added to bin by bin, 1.78 so.  Bound: issue slots (82 % used, 77
+// instructions per row); without the stores it takes 0.95 ms, and 2.05 with a row's floats stored
+// one by one; unrolled by the row it outgrew the instruction cache (4.6 ms).
+template <int N>
+__global__ void __launch_bounds__(kOwnBlock, 2)
+own_rows_kernel(const float* __restrict__ rows, uint32_t last_id, int K,
+                float* __restrict__ grad, TileLists t, const int2* __restrict__ pair) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ float s_carry[kOwnWarps * 32 * N];
+    __shared__ int s_state[kOwnWarps];
+    const TileSort sorted(s_raw, t.shift);
+    // (through a shuffle, so that the compiler knows it to be the same in a warp: loops over a warp's
+    // items then need no code for divergence)
+    const int me = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), e = threadIdx.x & 31;
+    float* const stages = reinterpret_cast<float*>(s_raw + TileSort::bytes(t.shift));
+    float* const stage = stages + me * (2 * 4 * kStageWords);
+    StreamWriter writer;
+    writer.buf = stages + kOwnWarps * (2 * 4 * kStageWords) + me * (2 * StreamWriter::kPiece);
+    writer.clear();
+    const uint32_t pitch = 4u * (uint32_t)K;
+    const bool one_pass = K <= 32 * N && (reinterpret_cast<uintptr_t>(grad) & 15) == 0;
+    owned_units(t, 0, t.n_tiles, [&](int tile, int first, int last, bool hot) {
+        const int64_t row0 = (int64_t)tile << t.shift;
+        const int n_rows = (int)(t.n_rows - row0 < (1 << t.shift) ? t.n_rows - row0
+                                                                  : (int64_t)1 << t.shift);
+        float* __restrict__ out = grad + row0 * K;
+        bool store = !hot;          // rows are written, else added to
+        do {
+            const int n = last - first < kOwnItems ? last - first : kOwnItems;
+            sorted.sort(n, t.shift, [&](int i) {
+                const int2 p = __ldg(pair + first + i);
+                return make_int2(p.x - (int)row0, p.y);
+            });
+            const bool stream = store && one_pass && n > 0;
+            if (store && !stream) sorted.clear_empty(n_rows, K, out);
+            const int lo = n * me / kOwnWarps, hi = n * (me + 1) / kOwnWarps;
+            for (int base = 0; base < K; base += 32 * N) {
+                const int cols = K - base < 32 * N ? K - base : 32 * N;
+                const uintptr_t src = reinterpret_cast<uintptr_t>(rows + base);
+                // words per row; whether a row may not need its last one; rows per stage; the
+                // lane's words of a stage
+                const bool same = K % 4 == 0;
+                const int words = same ? ((int)(src >> 2 & 3) + cols + 3) / 4 : (cols + 6) / 4;
+                const bool loose = !same && cols % 4 != 1;
+                const int per = kStageWords / words < 32 ? kStageWords / words : 32;
+                constexpr int COPIES = (kStageWords + 31) / 32;
+                int at_item[COPIES], at_word[COPIES];
+#pragma unroll
+                for (int p = 0; p < COPIES; ++p) {
+                    const int w = 32 * p + e;
+                    at_item[p] = w < per * words ? w / words : 1 << 16;
+                    at_word[p] = 16 * (w % words);
+                }
+                float acc[N];
+#pragma unroll
+                for (int j = 0; j < N; ++j) acc[j] = 0.f;
+                auto issue = [&](int i, float* to) {
+#pragma unroll
+                    for (int p = 0; p < COPIES; ++p) {
+                        const int k = i + at_item[p];
+                        if (k < hi) {
+                            const uint32_t id = sorted.item[k];
+                            const uintptr_t a =
+                                ((src + (uint64_t)id * pitch) & ~(uintptr_t)15) + at_word[p];
+                            if (loose && id == last_id && a >= src + (uint64_t)id * pitch + 4 * cols)
+                                continue;                        // beyond the buffer
+                            copy_word(to + 4 * (32 * p + e), reinterpret_cast<const void*>(a));
+                        }
+                    }
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                };
+                auto hand_on = [&](int state) {
+                    if (e == 0) s_state[me] = state;
+#pragma unroll
+                    for (int j = 0; j < N; ++j) s_carry[me * (32 * N) + e + j * 32] = acc[j];
+                };
+                auto flush = [&](int r) {
+                    if (stream) {
+                        writer.skip_to(r * K);
+                        writer.append<N>(acc, K);
+                    } else {
+                        float* const to = out + (r * K + base + e);
+#pragma unroll
+                        for (int j = 0; j < N; ++j) {
+                            if (e + 32 * j < cols) {
+                                if (store) to[32 * j] = acc[j];
+                                else atomicAdd(to + 32 * j, acc[j]);
+                            }
+                        }
+                    }
+                };
+                if (e == 0) s_state[me] = lo < hi ? kCarryNone : kCarrySkip;
+                // the first run began with an earlier warp
+                const int before = lo > 0 ? sorted.row[lo - 1] : -1;
+                writer.begin(out, (before + 1) * K);
+                bool head = lo > 0 && lo < hi && before == sorted.row[lo];
+                issue(lo, stage);
+                int buf = 0;
+                for (int i = lo; i < hi; i += per, buf ^= 1) {
+                    issue(i + per, stage + (buf ^ 1) * (4 * kStageWords));
+                    const int k = i + e, m = hi - i < per ? hi - i : per;
+                    bool ends = false;
+                    int at_row = 0;
+                    if (e < m) {
+                        ends = k + 1 == n || sorted.row[k + 1] != sorted.row[k];
+                        at_row = e * words * 4 +
+                                 ((int)((src + (uint64_t)sorted.item[k] * pitch) >> 2) & 3);
+                    }
+                    unsigned mask = __ballot_sync(0xffffffffu, ends);
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                    __syncwarp();
+                    const float* const in = stage + buf * (4 * kStageWords) + e;
+                    for (int a = 0;;) {
+                        const int stop = mask != 0u ? __ffs(mask) : m;
+#pragma unroll 1
+                        for (; a < stop; ++a) {
+                            // (lanes beyond the row's columns add what lies there and drop it)
+                            const float* const row = in + __shfl_sync(0xffffffffu, at_row, a);
+#pragma unroll
+                            for (int j = 0; j < N; ++j) acc[j] += row[32 * j];
+                        }
+                        if (mask == 0u) break;
+                        mask &= mask - 1u;                               // a run ends here
+                        if (head) hand_on(kCarryEnds);
+                        else flush(sorted.row[i + a - 1]);
+                        head = false;
+#pragma unroll
+                        for (int j = 0; j < N; ++j) acc[j] = 0.f;
+                    }
+                    __syncwarp();
+                }
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                // the last run goes on with the next warp
+                const bool open = lo < hi && hi < n && sorted.row[hi - 1] == sorted.row[hi];
+                if (open && head) hand_on(kCarryThrough);
+                __syncthreads();
+                if (open && !head) {
+                    for (int w = me + 1; w < kOwnWarps; ++w) {
+                        const int state = s_state[w];
+                        if (state == kCarrySkip) continue;
+#pragma unroll
+                        for (int j = 0; j < N; ++j) acc[j] += s_carry[w * (32 * N) + e + j * 32];
+                        if (state != kCarryThrough) break;
+                    }
+                    flush(sorted.row[hi - 1]);
+                }
+                if (stream) {
+                    if (lo < hi && hi == n) writer.skip_to(n_rows * K);
+                    writer.finish();
+                }
+                __syncthreads();
+            }
+            store = false;                   // what follows is added
+            first += n;
+        } while (first < last);
+    });
+}
+
 // Calls f with the lanes per row that suit K floats.
 template <int N>
 struct Lanes { static constexpr int value = N; };
@@ -389,6 +627,86 @@ static int zero_rows(float* grad, int64_t n_floats, cudaStream_t stream) {
     return SVOXB_OK;
 }
 
+// Calls f with the columns per lane that suit K floats.
+template <class F>
+static int with_columns(int K, F f) {
+    if (K <= 32) return f(Lanes<1>{});
+    if (K <= 64) return f(Lanes<2>{});
+    return f(Lanes<4>{});
+}
+
+// log2 of the rows of a tile: as many as bring a block nine tenths of the items that it sorts at a
+// time, at most `most`.
+static int tile_shift(int64_t items, int64_t n_rows, int most) {
+    int shift = most;
+    while (shift > kMinTileShift &&
+           (double)items / (double)n_rows * (double)(1LL << shift) > 0.9 * kOwnItems)
+        --shift;
+    return shift;
+}
+
+static int launch_tiled(const int64_t* ids, int64_t Q, const float* rows, int K, float* grad,
+                        int64_t n_slots, cudaStream_t stream) {
+    int st;
+    if ((st = keep_pool_cached())) return st;
+    TileLists t{};
+    t.n_rows = n_slots;
+    t.shift = tile_shift(Q, n_slots, 12);
+    t.n_tiles = (int)(((n_slots - 1) >> t.shift) + 1);
+    const size_t words = TileLists::words(t.n_tiles, Q);
+    int32_t* mem = nullptr;
+    SVOXB_CUDA(cudaMallocAsync((void**)&mem, (words + 2 * (size_t)Q) * sizeof(int32_t), stream));
+    t.place_in(mem, Q);
+    int2* pair = reinterpret_cast<int2*>(mem + words);
+    st = [&] {
+        SVOXB_CUDA(cudaMemsetAsync(mem, 0, t.zero_words() * sizeof(int32_t), stream));
+        const int sms = sm_count();
+        const bool shared = t.n_tiles <= kMaxSharedTiles;
+        const size_t smem = shared ? (size_t)t.n_tiles * sizeof(int32_t) : 0;
+        auto grid_of = [&](auto kernel, int block, size_t smem, int64_t need, unsigned* grid) {
+            int per_sm = 0;
+            const int s2 = blocks_per_sm(reinterpret_cast<const void*>(kernel), block, smem, &per_sm);
+            const int64_t most = (int64_t)sms * per_sm;
+            *grid = (unsigned)(need < most ? need : most);
+            return s2;
+        };
+        unsigned grid = 1;
+        auto count = shared ? count_tiles_kernel<true> : count_tiles_kernel<false>;
+        int s2 = grid_of(count, kPlaceBlock, smem, (Q + kPlaceBlock * 16 - 1) / (kPlaceBlock * 16),
+                         &grid);
+        if (s2) return s2;
+        count<<<grid, kPlaceBlock, smem, stream>>>(ids, Q, t);
+        scan_tiles_kernel<<<1, 1024, 0, stream>>>(t);
+        auto place = shared ? place_tiles_kernel<true> : place_tiles_kernel<false>;
+        const int64_t each = kPlaceBlock * (shared ? kPlaceEach : 1);
+        if ((s2 = grid_of(place, kPlaceBlock, smem, (Q + each - 1) / each, &grid))) return s2;
+        place<<<grid, kPlaceBlock, smem, stream>>>(ids, Q, t, pair, K, grad);
+        return with_columns(K, [&](auto columns) {
+            auto own = own_rows_kernel<decltype(columns)::value>;
+            const size_t bytes = TileSort::bytes(t.shift) +
+                                 kOwnWarps * (2 * 16 * kStageWords + 8 * StreamWriter::kPiece);
+            const int s3 = grid_of(own, kOwnBlock, bytes, (int64_t)t.n_tiles + Q / kOwnItems, &grid);
+            if (s3) return s3;
+            own<<<grid, kOwnBlock, bytes, stream>>>(rows, (uint32_t)(Q - 1), K, grad, t, pair);
+            SVOXB_CUDA(cudaGetLastError());
+            return (int)SVOXB_OK;
+        });
+    }();
+    cudaFreeAsync(mem, stream);
+    return st;
+}
+
+// Which of the two a large gradient takes.  Summing by tiles costs 77 instructions per row whatever
+// its length and writes the gradient once; adding bin by bin costs a reduction per 16 bytes and
+// writes it twice into the L2.  Measured (us, bins / tiles): K = 4, 732 MB, 16 M points 790 / 1742;
+// K = 13, 524 MB, 2.7 M 375 / 401; K = 28, 127 MB, 0.3 M 82 / 135; 255 MB, 0.6 M 150 / 137, 4.2 M
+// 354 / 371; 1.13 GB, 2.7 M 589 / 476, 4.2 M 675 / 611; K = 49, 447 MB, 0.6 M 227 / 172, 4.2 M 502 /
+// 440; 3.58 GB, 5 M 1680 / 1082; K = 100, 914 MB, 1 M 497 / 319; K = 200, 909 MB, 0.5 M 491 / 478.
+static bool sums_by_tiles(int64_t n_floats, int K) {
+    const int64_t mb = n_floats >> 18;
+    return K > 32 ? mb >= 384 : K > 20 && mb >= 768;
+}
+
 static int launch_scatter(const svoxb_tree* tree, const int64_t* ids, int64_t Q, const float* rows,
                           int K, float* grad, bool zero_first, cudaStream_t stream) {
     const int64_t n_slots = tree->M * tree->N * tree->N * tree->N, n_floats = n_slots * K;
@@ -398,6 +716,7 @@ static int launch_scatter(const svoxb_tree* tree, const int64_t* ids, int64_t Q,
                         Q < (1LL << 31) - kBinRows && n_slots < (1LL << 31) &&
                         reinterpret_cast<uintptr_t>(grad) % 16 == 0;
     int st;
+    if (binned && sums_by_tiles(n_floats, K)) return launch_tiled(ids, Q, rows, K, grad, n_slots, stream);
     if (!binned) {
         if (zero_first && (st = zero_rows(grad, n_floats, stream))) return st;
         if (Q == 0) return SVOXB_OK;

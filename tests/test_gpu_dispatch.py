@@ -183,6 +183,43 @@ def test_query_backward_binned(K, Q, cuda_device):
     csrc.check_device_status()
 
 
+@pytest.mark.parametrize("K", [4, 28, 33, 49, 64, 65, 130])
+@pytest.mark.parametrize("how", ["even", "dense", "hot", "ends"])
+def test_query_gradient_by_tiles(K, how, cuda_device):
+    # a gradient of 400 MB (or, for short rows, 800; K = 4: bins), rows summed tile by tile: tiles without points, with a chunk of
+    # them, with several chunks, and rows so often hit that their tile is shared out among blocks;
+    # ids that are no row are left out
+    import ctypes as C
+    M = -(-((400 if K > 32 else 800) << 20) // (32 * K))
+    n = 8 * M
+    Q = {"even": n // 3, "dense": 2 * n if K > 8 else n // 2, "hot": n // 3 + 70001, "ends": n // 3}[how]
+    gen = torch.Generator(cuda_device).manual_seed(K)
+    ids = torch.randint(0, n, (Q,), generator=gen, device=cuda_device)
+    if how == "hot":
+        ids[:70001] = 5 + 3 * (torch.arange(70001, device=cuda_device) % 3)
+    elif how == "ends":
+        ids = torch.where(ids % 2 == 0, torch.full_like(ids, n - 1), ids % 7)
+        ids[::3] = n // 2 + ids[::3] % 2
+    ids[17], ids[18] = -1, n
+    rows = torch.randint(-8, 9, (Q, K), generator=gen, device=cuda_device).float()
+    none = torch.zeros(3, device=cuda_device)
+    ok = (ids >= 0) & (ids < n)
+    want = torch.zeros(n, K, dtype=torch.float64, device=cuda_device)
+    want.index_add_(0, ids[ok], rows[ok].double())
+    # whole numbers whose sums stay below 2^24: exact in any order
+    assert want.abs().max().item() < 1 << 24
+    for shift in (0, 1):                 # 16-byte aligned gradient, and not
+        grad = torch.full((n * K + shift,), float("nan"), device=cuda_device)[shift:]
+        t = csrc._CTree(grad.data_ptr(), none.data_ptr(), none.data_ptr(), none.data_ptr(), M, 2, K)
+        st = csrc.library().svoxb_query_scatter(
+            C.byref(t), C.c_void_p(ids.data_ptr()), C.c_int64(Q), C.c_void_p(rows.data_ptr()),
+            C.c_int32(K), C.c_void_p(grad.data_ptr()), C.c_int(1),
+            C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == 0
+        assert torch.equal(grad.view(n, K).double(), want)
+    csrc.check_device_status()
+
+
 def test_query_backward_after_the_ids_were_written_to(cuda_device):
     tree, _ = W.config1()
     tree = tree.to(cuda_device)
