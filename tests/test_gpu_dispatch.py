@@ -168,6 +168,33 @@ def test_query_rows_of_any_length(K, N, cuda_device):
     csrc.check_device_status()
 
 
+@pytest.mark.parametrize("K", [4, 12, 28, 32, 36, 76, 128, 132, 224, 225])
+def test_query_values_through_shared_memory(K, cuda_device):
+    # records that are copied as 16-byte words, longer ones as floats, and those that go row by row;
+    # into results that lie on a 16-byte boundary and beside one
+    import ctypes as C
+    tree = svox.N3Tree(data_dim=K, data_format=None, init_refine=2, device=cuda_device)
+    gen = torch.Generator(cuda_device).manual_seed(K)
+    tree.data.data.normal_(generator=gen)
+    spec = tree._spec()
+    for Q in (1, 5, 33, 1000):
+        pts = torch.rand(Q, 3, generator=gen, device=cuda_device)
+        ids, _ = _query_reference(tree, pts, torch.zeros(Q, 1, device=cuda_device))
+        want = tree.data.data.view(-1, K)[ids]
+        for shift in (0, 1):
+            out = torch.full((Q * K + 8,), -7.0, device=cuda_device)
+            t = csrc._CTree(spec.data.data_ptr(), spec.child.data_ptr(), spec.offset.data_ptr(),
+                            spec.scaling.data_ptr(), tree.data.shape[0], 2, K)
+            st = csrc.library().svoxb_query_vertical(
+                C.byref(t), C.c_void_p(pts.data_ptr()), C.c_int64(Q),
+                C.c_void_p(out.data_ptr() + 4 * shift), C.c_void_p(0),
+                C.c_void_p(torch.cuda.current_stream().cuda_stream))
+            assert st == 0
+            assert torch.equal(out[shift:shift + Q * K].view(Q, K), want)
+            assert (out[:shift] == -7).all() and (out[shift + Q * K:] == -7).all()
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("K", [97, 100])
 @pytest.mark.parametrize("Q", [74000, 75000, 300001])
 def test_query_backward_binned(K, Q, cuda_device):
