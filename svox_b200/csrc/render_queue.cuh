@@ -168,18 +168,18 @@ struct alignas(16) WarpQueue {
     using Shape = RecordShape<K>;
     // three batches: items being collected, what spills over, and the batch in flight
     static constexpr int CAP = 96;
-    // per ray: colour basis, upstream gradient or view direction, delta_scale; read as 16-byte
-    // words, an odd number of them (no bank conflicts)
+    // per ray: colour basis, upstream gradient or view direction, delta_scale; odd stride: no
+    // bank conflicts
     static constexpr int SCALE = BD + (BWD || LOG ? 3 : 0);
-    static constexpr int RAYQ = (SCALE + 4) / 4 | 1;
+    static constexpr int RAYW = (SCALE + 1) | 1;
     // Staging rows (cp.async targets).  After lane i has read row i it reuses the
     // row's first words for the item's results.
     alignas(16) float rows[32 * Shape::STRIDE];
-    // items: slot, step length, density, owner (bits 0-4: lane, bit 7: accumulation march); one
-    // 16-byte word each, so that a push is one store
-    int4 item[CAP];
-    alignas(16) float rayv[32][4 * RAYQ];
-    unsigned mine[32];                 // per lane: its items of the batch being evaluated
+    uint32_t slot[CAP];
+    float dt[CAP];                     // step length
+    float sigma[CAP];
+    unsigned char owner[CAP];          // bits 0-4 owner lane, bit 7 accumulation march
+    float rayv[32][RAYW];
 };
 
 // Marks the table cells that the rays pass, at points a quarter of a cell apart: for a few rays
@@ -322,9 +322,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     bool in_brick = false;             // ... from the brick `cur_brick`, else from the table
     // queue: ring of three batches; `qn` items collected from ring position `head` on
     int head = 0, qn = 0;
+    unsigned mine = 0u, mine_next = 0u, mine_fly = 0u;  // my items: first 32, spilled, in flight
     int fly = 0;                       // items in flight, in the batch before `head`
-    // items are numbered through: the first one not folded in yet, and the lane's last one
-    unsigned folded_items = 0u, my_last = 0u - 1u;
     // logged forward: groups the warp has taken from the log but not used, items written
     int log_group = 0, log_left = 0, log_items = 0;
     const int log_limit = SORTED ? (int)(lg.capacity / kSortedChunks) : (int)lg.capacity;
@@ -360,7 +359,10 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     // Takes the first n (<= 32) collected items as the batch in flight and requests their
     // records: consecutive lanes copy consecutive 16-byte words, asynchronously.
     auto request = [&](int n) {
-        const uint32_t slot = lane < n ? (uint32_t)q.item[head + lane].x : 0u;
+        const uint32_t slot = lane < n ? q.slot[head + lane] : 0u;
+        mine_fly = mine;
+        mine = mine_next;
+        mine_next = 0u;
         fly = n;
         head = head == 64 ? 0 : head + 32;
         qn = qn > 32 ? qn - 32 : 0;
@@ -388,17 +390,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         const int nb = fly;
         const bool active = lane < nb;
         const int at = (head == 0 ? 64 : head - 32) + lane;     // item of this lane
-        const int4 it4 = q.item[at];
-        const uint32_t b_slot = (uint32_t)it4.x;
-        const int b_own = it4.w;
-        // every owner learns which items are its own
-        q.mine[lane] = 0u;
-        __syncwarp();
-        {
-            const unsigned same = __match_any_sync(0xffffffffu, active ? b_own & 31 : 32);
-            if (active) q.mine[b_own & 31] = same;
-        }
-        folded_items += nb;
+        const uint32_t b_slot = q.slot[at];
+        const int b_own = q.owner[at];
         float* row = q.rows + lane * Shape::STRIDE;
         const int off = record_offset<K>(tr.data, b_slot);
         const int own = b_own & 31;
@@ -406,15 +399,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         float sg[3] = {0.f, 0.f, 0.f}, col[3] = {0.f, 0.f, 0.f};
         float raw_sigma = 0.f, att = 0.f, b_dd = 0.f;
         if (active) {
-            // the owner's basis and scale, by 16-byte words
-            float ray_q[4 * WQ::RAYQ];
-#pragma unroll
-            for (int w = 0; w < (WQ::SCALE + 4) / 4; ++w) {
-                const float4 x = reinterpret_cast<const float4*>(q.rayv[own])[w];
-                ray_q[4 * w] = x.x; ray_q[4 * w + 1] = x.y; ray_q[4 * w + 2] = x.z; ray_q[4 * w + 3] = x.w;
-            }
-            const float delta_t = __int_as_float(it4.y), sigma = __int_as_float(it4.z),
-                        delta_scale = ray_q[WQ::SCALE];
+            const float delta_t = q.dt[at], sigma = q.sigma[at],
+                        delta_scale = q.rayv[own][WQ::SCALE];
             b_dd = delta_t * delta_scale;
             att = BWD ? expf(-delta_t * sigma * delta_scale)
                       : expf(-delta_t * delta_scale * sigma);
@@ -426,7 +412,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             } else {
                 float bs[BD > 0 ? BD : 1];
 #pragma unroll
-                for (int i = 0; i < BD; ++i) bs[i] = ray_q[i];
+                for (int i = 0; i < BD; ++i) bs[i] = q.rayv[own][i];
                 if (Shape::ALIGNED) {
 #pragma unroll
                     for (int w = 0; w < K / 4; ++w) {
@@ -467,7 +453,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         }
         __syncwarp();
         // every owner folds in its items, in march order
-        for (unsigned m = q.mine[lane]; m != 0u; m &= m - 1u) {
+        for (unsigned m = mine_fly; m != 0u; m &= m - 1u) {
             float4* res = reinterpret_cast<float4*>(q.rows + (__ffs(m) - 1) * Shape::STRIDE);
             const float4 x = *res;
             if (!BWD) {
@@ -495,6 +481,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 }
             }
         }
+        mine_fly = 0u;
         fly = 0;
         __syncwarp();
         if (!BWD && tr.weight_accum != nullptr && active)
@@ -632,7 +619,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         unsigned marching = __ballot_sync(0xffffffffu, state == kMarching);
         const unsigned waiting = alive & ~marching;
         if (marching == 0u || __popc(waiting) >= shape.refill) {
-            if (__any_sync(0xffffffffu, state == kEnded && (int)(my_last - folded_items) >= 0)) {
+            if (__any_sync(0xffffffffu, state == kEnded && (mine | mine_next | mine_fly) != 0u)) {
                 __syncwarp();
                 if (fly > 0) evaluate();
                 while (qn > 0) {
@@ -682,7 +669,6 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                         march_ready(r);
                         state = kMarching;
                         t = r.tmin; light = ahead = 1.f; it = 0; stopped = false;
-                        my_last = folded_items - 1u;
                         q.rayv[lane][WQ::SCALE] = r.delta_scale;
                         place_cursor();
                         request_words();
@@ -732,41 +718,36 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             cur_brick = index.bricks + (uint32_t)(entry.x & 0x7fffffff) * kBrickCells;
             on = false;
         }
+        int depth = (int)((uint32_t)entry.y >> 28) + (in_brick ? L : 0);
         uint32_t slot = (uint32_t)entry.y & 0x0fffffffu;
         float sigma = __int_as_float(entry.x);
         bool item = on && entry.x <= kWordInf;      // the leaf passes the density test
         bool done = false;
-        // side of the leaf's cube, 2^-depth
-        float inv_cube = __int_as_float((127 << 23) - (int)((uint32_t)entry.y >> 28 << 23));
-        float fine = 0.f;
+        uint32_t ux = bits(px), uy = bits(py), uz = bits(pz);
         if (on && entry.x >= kWordFetch) {
             // seldom: a tree deeper than the index, a density that is not in the word
             float raw = 0.f;
             if (entry.x == kWordWalk) {
                 const float big = (float)(1 << 24);
-                const int depth = (int)((uint32_t)entry.y >> 28);
                 const Walked f = walk_to_leaf(
                     tr.child, tr.data, K, tr.M, depth > L ? (int64_t)slot : 0,
                     depth > L ? depth - 1 : 0, (int)(px * big), (int)(py * big), (int)(pz * big));
                 done = !f.ok;
                 slot = f.slot;
-                inv_cube = __int_as_float((127 - (f.ok ? f.depth : 1)) << 23);
+                depth = f.ok ? f.depth : 1;
                 raw = f.raw;
-                // 2^-24 leaves: a float resolves them below 1/2, where the sum below would not
-                if (f.ok && f.depth > kPosBits) fine = 1.f;
             } else {
                 raw = __ldg(tr.data + (size_t)slot * K + (K - 1));
             }
             sigma = opt.density_softplus ? softplus_m1(raw) : raw;
             item = !done && sigma > (BWD ? 0.f : opt.sigma_thresh);
         }
-        // Lower corner of the leaf: a number whose last place is the leaf's side takes in the
-        // position's multiples of it and drops the rest.
-        const float coarse = __int_as_float(__float_as_int(inv_cube) + (kPosBits << 23));
-        float cx = __fsub_rn(__fadd_rz(px, coarse), coarse);
-        float cy = __fsub_rn(__fadd_rz(py, coarse), coarse);
-        float cz = __fsub_rn(__fadd_rz(pz, coarse), coarse);
-        if (fine != 0.f) {
+        // lower corner of the leaf, offset of the sample from it
+        const uint32_t keep = 0xffffffffu << (kPosBits - (depth < kPosBits ? depth : kPosBits));
+        float cx = __fsub_rn(__uint_as_float(ux & keep), 1.0f);
+        float cy = __fsub_rn(__uint_as_float(uy & keep), 1.0f);
+        float cz = __fsub_rn(__uint_as_float(uz & keep), 1.0f);
+        if (depth > kPosBits) {                     // 2^-24 leaves: a float resolves them below 1/2
             const float big = (float)(1 << 24);
             cx = truncf(px * big) * (1.f / big);
             cy = truncf(py * big) * (1.f / big);
@@ -776,6 +757,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         // scale).  The point lies inside, so the entry distance is 0 and per axis the larger of
         // t1 = -f*inv and t1 + inv is t1 + max(inv, 0); powers of two commute with rounding, so
         // everything can be done at the tree's scale.
+        const float inv_cube = __int_as_float((127 - depth) << 23);  // 2^-depth
         const float ex = __fmaf_rn(fmaxf(r.ix, 0.f), inv_cube, __fmul_rn(__fsub_rn(cx, px), r.ix));
         const float ey = __fmaf_rn(fmaxf(r.iy, 0.f), inv_cube, __fmul_rn(__fsub_rn(cy, py), r.iy));
         const float ez = __fmaf_rn(fmaxf(r.iz, 0.f), inv_cube, __fmul_rn(__fsub_rn(cz, pz), r.iz));
@@ -801,9 +783,13 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         if (item) {
             const int n = qn + __popc(pushed & ((1u << lane) - 1u));
             const int pos = head + n < WQ::CAP ? head + n : head + n - WQ::CAP;
-            q.item[pos] = make_int4((int)slot, __float_as_int(delta_t), __float_as_int(sigma),
-                                    lane | ((BWD && phase == 0) ? 0x80 : 0));
-            my_last = folded_items + (unsigned)(fly + n);
+            q.slot[pos] = slot;
+            q.dt[pos] = delta_t;
+            q.sigma[pos] = sigma;
+            q.owner[pos] = (unsigned char)(lane | ((BWD && phase == 0) ? 0x80 : 0));
+            const unsigned bit = 1u << (n & 31);
+            if (n < 32) mine |= bit;
+            else mine_next |= bit;
         }
         qn += __popc(pushed);
         if (qn >= 32) {
