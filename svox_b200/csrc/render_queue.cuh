@@ -19,13 +19,14 @@
 //
 // Bound: issue slots where neighbouring rays share records (images: 63 % of the slots used), DRAM
 // too where every sample's record misses (rays in random order: 16 GB for 2^20 rays of the 512^3
-// shell scene).  So the march is kept short, 138 instructions per iteration and 259 per batch of
-// items with SH9 records (some 540 with SH16): the position's bits come from one truncating addition instead of conversions, the leaf's
+// shell scene).  So the march is kept short (138 instructions per iteration and 259 per batch of
+// items with SH9 records, some 540 with SH16, before the leaf's corner took one such addition too):
+// the position's bits come from one truncating addition instead of conversions, the leaf's
 // exit distance needs five operations per axis, lanes between samples compute along instead of
 // branching, what only items need is done where all lanes have one, the index entry of a sample
 // is requested one iteration ahead so that the queue's work covers its latency, and a block holds
 // four warps so that shared memory and the L1 can be balanced (kMarchBlocks).  Per 800x800 view of
-// the shell scene with SH16 records 1.64 -> 1.05 ms; logged forward of 2^20 rays, SH9, 4.09 -> 3.31;
+// the shell scene with SH16 records 1.64 -> 1.01 ms; logged forward of 2^20 rays, SH9, 4.09 -> 3.31;
 // 65536 rays of an RGBA tree, forward and backward, 1.6 -> 0.25 (they took the generic kernels).
 //
 // Lanes whose ray has ended wait until `refill` of them do; then the queue is drained, their
@@ -166,8 +167,10 @@ struct alignas(16) WarpQueue {
     static constexpr bool BWD = MODE == kModeBackward;
     static constexpr bool LOG = MODE == kModeForwardLogged;
     using Shape = RecordShape<K>;
-    // three batches: items being collected, what spills over, and the batch in flight
-    static constexpr int CAP = 96;
+    // two batches: items being collected, and what spills over (the batch in flight lies in
+    // registers; a queue of 96 items left the SH16 forward 28 KB of L1 instead of 60, 1.10 ms per
+    // 800x800 view instead of 1.05)
+    static constexpr int CAP = 64;
     // per ray: colour basis, upstream gradient or view direction, delta_scale; odd stride: no
     // bank conflicts
     static constexpr int SCALE = BD + (BWD || LOG ? 3 : 0);
@@ -217,6 +220,13 @@ constexpr int kMarchBlock = 128;
 // rays, SH9: 8 blocks (64 registers, no L1 left beside 213 KB of queues) 5.0 ms, 7 blocks 3.6,
 // 6 blocks 3.5, 5 blocks 3.7.
 constexpr int kMarchBlocks = 6;
+
+// A batch of few rays (march_shape leaves no more than kSpreadWarps warps per SM with work) goes
+// through blocks of this size, compiled for 16 warps per SM and thus 128 registers: 65536 rays of
+// an RGBA tree 175 -> 157, 4096 rays of the 512^3 shell 237 -> 204 us.
+constexpr int kFewBlock = 64;
+constexpr int kSpreadWarps = 16;
+
 template <int BD, int MODE>
 constexpr int march_blocks_per_sm() {
     const size_t smem = (kMarchBlock / 32) * sizeof(WarpQueue<BD, MODE>) + 1024;
@@ -224,14 +234,29 @@ constexpr int march_blocks_per_sm() {
     return fit > kMarchBlocks ? kMarchBlocks : fit < 1 ? 1 : fit;
 }
 
+template <int BD, int MODE>
+constexpr int few_blocks_per_sm() {
+    const int most = kSpreadWarps / (kFewBlock / 32);
+    const int fit = (int)(227 * 1024 / ((kFewBlock / 32) * sizeof(WarpQueue<BD, MODE>) + 1024));
+    return fit < most ? fit : most;
+}
+
 // A forward that sorts its log into bins runs as one block per SM, so that a bin has one open
 // group per SM and the lines being filled stay in L2 until they are full.
-constexpr size_t kBinSmem = (size_t)kMaxBins * (sizeof(uint32_t) + kOpenGroups * sizeof(uint64_t));
+constexpr size_t bin_smem(int n_bins) {
+    return (size_t)n_bins * (sizeof(uint32_t) + kOpenGroups * sizeof(uint64_t));
+}
+constexpr size_t kBinSmem = bin_smem(kMaxBins);
 template <int BD>
 constexpr int sorted_march_block() {
-    const int fit = (int)((227 * 1024 - 1024 - kBinSmem) / sizeof(WarpQueue<BD, kModeForwardLogged>));
+    // If it costs no more than a warp, within 196 KB, the next smaller split of an SM's memory,
+    // which leaves 60 KB of L1 instead of 28 (SH16: 19 warps instead of 20, logged 800x800 view 1.26
+    // -> 1.21 ms; SH25 stays at 15 warps, 13 took 417 us instead of 387 for a 640x640 view).
+    constexpr size_t one = sizeof(WarpQueue<BD, kModeForwardLogged>);
     const int warps = 4 * march_blocks_per_sm<BD, kModeForwardLogged>();
-    return 32 * (fit < warps ? fit : warps);
+    int most = (int)((227 * 1024 - 1024 - kBinSmem) / one), fit = (int)((196 * 1024 - 1024 - kBinSmem / 2) / one);
+    if (most > warps) most = warps;
+    return 32 * (fit < most - 1 ? most : fit < most ? fit : most);
 }
 
 // clamp01's upper bound
@@ -261,7 +286,8 @@ struct MarchShape {
 
 template <int BD, int MODE, int BLOCK, class Source>
 __global__ void
-__launch_bounds__(BLOCK, BLOCK == kMarchBlock ? march_blocks_per_sm<BD, MODE>() : 1)
+__launch_bounds__(BLOCK, BLOCK == kMarchBlock ? march_blocks_per_sm<BD, MODE>()
+                         : BLOCK == kFewBlock ? few_blocks_per_sm<BD, MODE>() : 1)
 render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex index,
                     int64_t tickets, float* __restrict__ out,
                     const float* __restrict__ grad_out, const float* __restrict__ fwd_out,
@@ -277,7 +303,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     if (BWD && LogGate{lg.log, lg.capacity}.closed()) return;
     if (threadIdx.x == 0) s_next = 0;
     // sorted log: items this block has put into each bin, and its last groups of the bin
-    constexpr bool SORTED = LOG && BLOCK != kMarchBlock;
+    constexpr bool SORTED = LOG && BLOCK > kMarchBlock;
     uint64_t* s_open = reinterpret_cast<uint64_t*>(s_raw + (BLOCK / 32) * sizeof(WQ));
     uint32_t* s_count = reinterpret_cast<uint32_t*>(s_open + lg.n_bins * kOpenGroups);
     if (SORTED) {
@@ -308,6 +334,9 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     r.hit = false;
     int64_t ray = 0;
     int state = lane < shape.lanes ? kNeedRay : kExhausted;
+    // max(1 / direction, 0), where registers allow (1 % of an image's march; the logged kernels spill)
+    constexpr bool MAXES = MODE == kModeForward;
+    float mx = 0.f, my = 0.f, mz = 0.f;
     float t = 0.f, light = 1.f, ahead = 1.f;   // transmittance after the items folded / pushed
     float a0 = 0.f, a1 = 0.f, a2 = 0.f;  // forward: colour sums; backward: a0 = accum
     bool stopped = false;
@@ -320,10 +349,13 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     int2 entry = make_int2(0, 0);
     uint32_t cell = 0;                 // ... and its table cell
     bool in_brick = false;             // ... from the brick `cur_brick`, else from the table
-    // queue: ring of three batches; `qn` items collected from ring position `head` on
+    // queue: ring of two batches; `qn` items collected from ring position `head` on
     int head = 0, qn = 0;
     unsigned mine = 0u, mine_next = 0u, mine_fly = 0u;  // my items: first 32, spilled, in flight
-    int fly = 0;                       // items in flight, in the batch before `head`
+    int fly = 0;                       // items in flight; this lane's:
+    uint32_t fly_slot = 0u;
+    float fly_dt = 0.f, fly_sigma = 0.f;
+    int fly_own = 0;
     // logged forward: groups the warp has taken from the log but not used, items written
     int log_group = 0, log_left = 0, log_items = 0;
     const int log_limit = SORTED ? (int)(lg.capacity / kSortedChunks) : (int)lg.capacity;
@@ -359,12 +391,16 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     // Takes the first n (<= 32) collected items as the batch in flight and requests their
     // records: consecutive lanes copy consecutive 16-byte words, asynchronously.
     auto request = [&](int n) {
-        const uint32_t slot = lane < n ? q.slot[head + lane] : 0u;
+        fly_slot = q.slot[head + lane];
+        fly_dt = q.dt[head + lane];
+        fly_sigma = q.sigma[head + lane];
+        fly_own = q.owner[head + lane];
+        const uint32_t slot = lane < n ? fly_slot : 0u;
         mine_fly = mine;
         mine = mine_next;
         mine_next = 0u;
         fly = n;
-        head = head == 64 ? 0 : head + 32;
+        head ^= 32;
         qn = qn > 32 ? qn - 32 : 0;
         const int sub = lane / Shape::GROUP, w = lane % Shape::GROUP;
         const float* base = tr.data + 4 * w;
@@ -381,6 +417,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+        __syncwarp();        // the items' places are free again
     };
 
     // Waits for the records of the batch in flight and evaluates it.
@@ -389,9 +426,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         __syncwarp();
         const int nb = fly;
         const bool active = lane < nb;
-        const int at = (head == 0 ? 64 : head - 32) + lane;     // item of this lane
-        const uint32_t b_slot = q.slot[at];
-        const int b_own = q.owner[at];
+        const uint32_t b_slot = fly_slot;
+        const int b_own = fly_own;
         float* row = q.rows + lane * Shape::STRIDE;
         const int off = record_offset<K>(tr.data, b_slot);
         const int own = b_own & 31;
@@ -399,7 +435,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         float sg[3] = {0.f, 0.f, 0.f}, col[3] = {0.f, 0.f, 0.f};
         float raw_sigma = 0.f, att = 0.f, b_dd = 0.f;
         if (active) {
-            const float delta_t = q.dt[at], sigma = q.sigma[at],
+            const float delta_t = fly_dt, sigma = fly_sigma,
                         delta_scale = q.rayv[own][WQ::SCALE];
             b_dd = delta_t * delta_scale;
             att = BWD ? expf(-delta_t * sigma * delta_scale)
@@ -412,7 +448,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             } else {
                 float bs[BD > 0 ? BD : 1];
 #pragma unroll
-                for (int i = 0; i < BD; ++i) bs[i] = q.rayv[own][i];
+                for (int i = 0; i < BD; ++i)
+                    if (Shape::ALIGNED) bs[i] = q.rayv[own][i];
                 if (Shape::ALIGNED) {
 #pragma unroll
                     for (int w = 0; w < K / 4; ++w) {
@@ -428,12 +465,30 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                         }
                     }
                 } else {
-                    const float* rec = row + off;
+                    // The row's 16-byte words as they are: float j of the row is coefficient j - off,
+                    // so basis function (j - off) mod BD takes it, which is one register for all
+                    // three channels; only the first three of a channel's places depend on `off`.  (A
+                    // 49-float record as single floats met three bank conflicts a read: 1.03 ms per
+                    // 800x800 view instead of 1.01.)
+                    constexpr int B = BD > 0 ? BD : 1;
 #pragma unroll
-                    for (int e = 0; e < K - 1; ++e)
-                        tmp[e / (BD > 0 ? BD : 1)] = __fmaf_rn(
-                            bs[e % (BD > 0 ? BD : 1)], rec[e], tmp[e / (BD > 0 ? BD : 1)]);
-                    raw_sigma = rec[K - 1];
+                    for (int m = 0; m < B; ++m)
+                        bs[m] = q.rayv[own][m >= 3 || m >= off ? m - off : m - off + B];
+#pragma unroll
+                    for (int w = 0; w < Shape::WORDS; ++w) {
+                        const float4 x = reinterpret_cast<const float4*>(row)[w];
+                        const float v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int j = 4 * w + i, m = j % B, c = j / B;
+                            if (m >= 3 || m >= off) {
+                                if (c < 3) tmp[c < 3 ? c : 0] = __fmaf_rn(bs[m], v[i], tmp[c < 3 ? c : 0]);
+                                else if (m == off) raw_sigma = v[i];
+                            } else if (c > 0) {
+                                tmp[c > 0 ? c - 1 : 0] = __fmaf_rn(bs[m], v[i], tmp[c > 0 ? c - 1 : 0]);
+                            }
+                        }
+                    }
                 }
             }
 #pragma unroll
@@ -669,6 +724,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                         march_ready(r);
                         state = kMarching;
                         t = r.tmin; light = ahead = 1.f; it = 0; stopped = false;
+                        mx = fmaxf(r.ix, 0.f); my = fmaxf(r.iy, 0.f); mz = fmaxf(r.iz, 0.f);
                         q.rayv[lane][WQ::SCALE] = r.delta_scale;
                         place_cursor();
                         request_words();
@@ -718,36 +774,41 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             cur_brick = index.bricks + (uint32_t)(entry.x & 0x7fffffff) * kBrickCells;
             on = false;
         }
-        int depth = (int)((uint32_t)entry.y >> 28) + (in_brick ? L : 0);
         uint32_t slot = (uint32_t)entry.y & 0x0fffffffu;
         float sigma = __int_as_float(entry.x);
         bool item = on && entry.x <= kWordInf;      // the leaf passes the density test
         bool done = false;
-        uint32_t ux = bits(px), uy = bits(py), uz = bits(pz);
+        // side of the leaf's cube, 2^-depth
+        float inv_cube = __int_as_float((127 << 23) - (int)((uint32_t)entry.y >> 28 << 23));
+        float fine = 0.f;
         if (on && entry.x >= kWordFetch) {
             // seldom: a tree deeper than the index, a density that is not in the word
             float raw = 0.f;
             if (entry.x == kWordWalk) {
                 const float big = (float)(1 << 24);
+                const int depth = (int)((uint32_t)entry.y >> 28);
                 const Walked f = walk_to_leaf(
                     tr.child, tr.data, K, tr.M, depth > L ? (int64_t)slot : 0,
                     depth > L ? depth - 1 : 0, (int)(px * big), (int)(py * big), (int)(pz * big));
                 done = !f.ok;
                 slot = f.slot;
-                depth = f.ok ? f.depth : 1;
+                inv_cube = __int_as_float((127 - (f.ok ? f.depth : 1)) << 23);
                 raw = f.raw;
+                // 2^-24 leaves: a float resolves them below 1/2, where the sum below would not
+                if (f.ok && f.depth > kPosBits) fine = 1.f;
             } else {
                 raw = __ldg(tr.data + (size_t)slot * K + (K - 1));
             }
             sigma = opt.density_softplus ? softplus_m1(raw) : raw;
             item = !done && sigma > (BWD ? 0.f : opt.sigma_thresh);
         }
-        // lower corner of the leaf, offset of the sample from it
-        const uint32_t keep = 0xffffffffu << (kPosBits - (depth < kPosBits ? depth : kPosBits));
-        float cx = __fsub_rn(__uint_as_float(ux & keep), 1.0f);
-        float cy = __fsub_rn(__uint_as_float(uy & keep), 1.0f);
-        float cz = __fsub_rn(__uint_as_float(uz & keep), 1.0f);
-        if (depth > kPosBits) {                     // 2^-24 leaves: a float resolves them below 1/2
+        // Lower corner of the leaf: a number whose last place is the leaf's side takes in the
+        // position's multiples of it and drops the rest.
+        const float coarse = __int_as_float(__float_as_int(inv_cube) + (kPosBits << 23));
+        float cx = __fsub_rn(__fadd_rz(px, coarse), coarse);
+        float cy = __fsub_rn(__fadd_rz(py, coarse), coarse);
+        float cz = __fsub_rn(__fadd_rz(pz, coarse), coarse);
+        if (fine != 0.f) {
             const float big = (float)(1 << 24);
             cx = truncf(px * big) * (1.f / big);
             cy = truncf(py * big) * (1.f / big);
@@ -757,10 +818,9 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         // scale).  The point lies inside, so the entry distance is 0 and per axis the larger of
         // t1 = -f*inv and t1 + inv is t1 + max(inv, 0); powers of two commute with rounding, so
         // everything can be done at the tree's scale.
-        const float inv_cube = __int_as_float((127 - depth) << 23);  // 2^-depth
-        const float ex = __fmaf_rn(fmaxf(r.ix, 0.f), inv_cube, __fmul_rn(__fsub_rn(cx, px), r.ix));
-        const float ey = __fmaf_rn(fmaxf(r.iy, 0.f), inv_cube, __fmul_rn(__fsub_rn(cy, py), r.iy));
-        const float ez = __fmaf_rn(fmaxf(r.iz, 0.f), inv_cube, __fmul_rn(__fsub_rn(cz, pz), r.iz));
+        const float ex = __fmaf_rn(MAXES ? mx : fmaxf(r.ix, 0.f), inv_cube, __fmul_rn(__fsub_rn(cx, px), r.ix));
+        const float ey = __fmaf_rn(MAXES ? my : fmaxf(r.iy, 0.f), inv_cube, __fmul_rn(__fsub_rn(cy, py), r.iy));
+        const float ez = __fmaf_rn(MAXES ? mz : fmaxf(r.iz, 0.f), inv_cube, __fmul_rn(__fsub_rn(cz, pz), r.iz));
         const float delta_t = __fadd_rn(fminf(ex, fminf(ey, ez)), opt.step_size);
         if (on) {
             t = __fadd_rn(t, delta_t);
@@ -782,7 +842,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         const unsigned pushed = __ballot_sync(0xffffffffu, item);
         if (item) {
             const int n = qn + __popc(pushed & ((1u << lane) - 1u));
-            const int pos = head + n < WQ::CAP ? head + n : head + n - WQ::CAP;
+            const int pos = (head + n) & (WQ::CAP - 1);
             q.slot[pos] = slot;
             q.dt[pos] = delta_t;
             q.sigma[pos] = sigma;

@@ -24,8 +24,6 @@ constexpr int kRefillLanes = 8;
 constexpr int64_t kWalkRays = 1 << 17;
 // Quarters of the leaf slots a batch has to touch for its log to be sorted.
 constexpr int kSortTouches = 1;
-// ... and warps per SM that a small batch is spread over before warps get 32 rays each.
-constexpr int kSpreadWarps = 16;
 
 struct RenderCall {
     const svoxb_tree* tree;
@@ -175,7 +173,10 @@ static bool sorts_log(const svoxb_tree* t, int64_t rays, bool image, int64_t cap
 static MarchShape march_shape(int64_t tickets, int64_t warps) {
     MarchShape m{32, 5, kRefillLanes};
     while (m.lanes > 4 && tickets <= warps * (m.lanes / 2)) m.lanes /= 2;
-    if (m.lanes == 4) m.granule_shift = 4;
+    // as many as two warps take, so that the blocks get alike shares (20 000 rays, SH16, 19 warps of 8
+    // lanes per block: granules of 32 left some blocks with more rays than lanes, 154 us instead of
+    // 135; granules of one warp: 4096 rays of a toy scene 31.5 instead of 28.8)
+    while ((1 << m.granule_shift) > 2 * m.lanes) --m.granule_shift;
     if (m.lanes < 32) m.refill = m.lanes / 4;
     return m;
 }
@@ -184,10 +185,10 @@ template <int BD, int MODE, int BLOCK, class Source>
 static int launch_march(const RenderCall& c, const Source& src, const TreeIndex& index,
                         LogArgs log) {
     const size_t smem = (BLOCK / 32) * sizeof(WarpQueue<BD, MODE>) +
-                        (BLOCK == kMarchBlock ? 0 : kBinSmem);
+                        (BLOCK > kMarchBlock ? bin_smem(log.n_bins) : 0);
     const int64_t tickets = Source::tickets(src, c.Q);
     const MarchShape shape = march_shape(
-        tickets, (int64_t)sm_count() * (BLOCK == kMarchBlock ? kSpreadWarps : BLOCK / 32));
+        tickets, (int64_t)sm_count() * (BLOCK > kMarchBlock ? BLOCK / 32 : kSpreadWarps));
     auto k = render_queue_kernel<BD, MODE, BLOCK, Source>;
     unsigned grid = 1;
     const int64_t granules = (tickets + (1 << shape.granule_shift) - 1) >> shape.granule_shift;
@@ -211,12 +212,16 @@ static int launch_mode(const RenderCall& c, const Source& src, const TreeIndex& 
         log.capacity = c.gate.capacity;
         return launch_march<BD, kModeBackward, kMarchBlock>(c, src, index, log);
     }
-    if (c.log == nullptr) return launch_march<BD, kModeForward, kMarchBlock>(c, src, index, log);
+    const bool few = Source::tickets(src, c.Q) <= (int64_t)sm_count() * kSpreadWarps * 32;
+    if (c.log == nullptr)
+        return few ? launch_march<BD, kModeForward, kFewBlock>(c, src, index, log)
+                   : launch_march<BD, kModeForward, kMarchBlock>(c, src, index, log);
     log.log = c.log;
     log.capacity = c.log_capacity;
     log.shift = replay_bin_shift(c.tree->M, c.tree->K);
     if (!sorts_log(c.tree, c.Q, Source::kImage, c.log_capacity))
-        return launch_march<BD, kModeForwardLogged, kMarchBlock>(c, src, index, log);
+        return few ? launch_march<BD, kModeForwardLogged, kFewBlock>(c, src, index, log)
+                   : launch_march<BD, kModeForwardLogged, kMarchBlock>(c, src, index, log);
     log.n_bins = replay_bins(c.tree->M, c.tree->K);
     const int st = launch_march<BD, kModeForwardLogged, sorted_march_block<BD>()>(c, src, index, log);
     if (st) return st;

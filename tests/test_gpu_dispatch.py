@@ -52,6 +52,19 @@ def test_bricks_where_a_few_rays_pass(n, big_tree, cuda_device):
     csrc.check_device_status()
 
 
+@pytest.mark.parametrize("fmt", ["RGBA", "SH4", "SH9", "SH16"])
+def test_few_rays_and_many_give_the_same(fmt, cuda_device):
+    # up to 16 warps of rays per SM go through smaller blocks, compiled for fewer of them
+    r = svox.VolumeRenderer(_shell(fmt, 3, 2, cuda_device))
+    few = torch.cuda.get_device_properties(cuda_device).multi_processor_count * 512
+    rays = _rays(few + 33, cuda_device)
+    with torch.no_grad():
+        every = r(rays)
+        for n in (few, 4097, 33):
+            assert torch.equal(r(svox.Rays(*[t[:n].contiguous() for t in rays])), every[:n])
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("fmt,refine,n_rays", [("RGBA", 5, 50000), ("SH9", 4, 12000),
                                                ("SH16", 4, 12000)])
 @pytest.mark.parametrize("image", [False, True])
