@@ -56,7 +56,10 @@ struct UnitShared {
 // through from `before` on; a unit is up to `per_unit` of a bin's items, handed to
 // `work(first, end)` by all threads of the block.  With `clear_floats` > 0 (the length of the
 // outputs) bin b + 1, `bin_floats` floats, is cleared by `clear(from, until)` in units that come
-// before the items of bin b, the first bin before all.
+// before the items of bin b, the first bin before all; with `spread` they are spread over the first
+// two thirds of the bin's units instead, so that clearing and adding run side by side (scatter of 2^20
+// rays 1.90 -> 1.84 ms; where units are small they then hold up the next bin, `se_grad` of 100 000
+// rays 1.12 -> 1.28, an 800x800 view 1.26 -> 1.29).
 //
 // Units are taken by blocks in order from one counter, so that the grid works within a window
 // much smaller than a bin (with a fixed assignment the blocks drift apart and several bins compete
@@ -67,8 +70,8 @@ struct UnitShared {
 template <int BLOCK, class Count, class Clear, class Work>
 __device__ __forceinline__ void ordered_units(UnitShared& s, const UnitCounters& counters, int lo,
                                               int hi, int before, int per_unit, int64_t bin_floats,
-                                              int64_t clear_floats, Count count, Clear clear,
-                                              Work work) {
+                                              int64_t clear_floats, bool spread, Count count,
+                                              Clear clear, Work work) {
     for (int b = threadIdx.x; b <= kMaxBins; b += BLOCK) {
         const int64_t left = clear_floats - b * bin_floats;
         s.zero[b] = clear_floats > 0 && b < hi && left > 0
@@ -101,16 +104,27 @@ __device__ __forceinline__ void ordered_units(UnitShared& s, const UnitCounters&
                 bin = at_bin;
                 u = taken - s.start[bin];
                 z = s.zero[bin + 1];
-                if (u < z) {
+                int before = u < z ? u : z, upto = u < z ? u + 1 : z;    // units of clearing
+                if (spread && z > 0) {
+                    const int n = s.start[bin + 1] - s.start[bin];
+                    const int64_t num = 3 * z < 2 * n ? 3 * z : 2 * n;
+                    before = (int)min((int64_t)z, u * num / (2 * n));
+                    upto = (int)min((int64_t)z, (u + 1) * num / (2 * n));
+                }
+                if (before < upto) {
                     ++bin;
-                } else if (clear_floats > 0 && bin != ready) {
-                    int tries = 0;
-                    while (*(volatile int32_t*)(counters.cleared + bin) < s.zero[bin] &&
-                           ++tries < (1 << 22))
-                        __nanosleep(64);
-                    if (tries == (1 << 22)) report(SVOXB_ERR_CUDA);
-                    __threadfence();
-                    ready = bin;
+                    u = before;
+                } else {
+                    z = before;
+                    if (clear_floats > 0 && bin != ready) {
+                        int tries = 0;
+                        while (*(volatile int32_t*)(counters.cleared + bin) < s.zero[bin] &&
+                               ++tries < (1 << 22))
+                            __nanosleep(64);
+                        if (tries == (1 << 22)) report(SVOXB_ERR_CUDA);
+                        __threadfence();
+                        ready = bin;
+                    }
                 }
             }
             s.unit = taken;

@@ -453,7 +453,7 @@ scatter_binned_rows_kernel(int64_t Q, const float* __restrict__ rows, int K,
         }
     };
     ordered_units<kQueryBlock>(s_units, b.units, 0, b.n_bins, 0, kQueryBlock * per_warp,
-                               ((int64_t)1 << b.shift) * K, n_slots * K,
+                               ((int64_t)1 << b.shift) * K, n_slots * K, false,
                                [&](int i) { return b.count[i]; }, clear, work);
 }
 

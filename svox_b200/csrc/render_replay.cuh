@@ -32,7 +32,8 @@ __host__ __device__ inline int replay_part_first_bin(int p, int n_parts, int n_b
     return (int)(((int64_t)p * n_bins) / n_parts);
 }
 
-// Lists the groups of a sorted log bin by bin.  `cursor`: kMaxBins zeroed words.
+// Lists the groups of a sorted log bin by bin, with their items in the upper 8 bits (there are fewer
+// than 2^24 groups).  `cursor`: kMaxBins zeroed words.
 __global__ void __launch_bounds__(256)
 order_groups_kernel(int32_t* __restrict__ log, int64_t capacity, int32_t* __restrict__ cursor) {
     __shared__ int s_first[kMaxBins], s_count[kMaxBins];
@@ -50,12 +51,13 @@ order_groups_kernel(int32_t* __restrict__ log, int64_t capacity, int32_t* __rest
         __syncthreads();
         if (threadIdx.x < kMaxBins) s_count[threadIdx.x] = 0;
         __syncthreads();
-        int bin[kOrderTile / 256], rank[kOrderTile / 256];
+        int bin[kOrderTile / 256], rank[kOrderTile / 256], items[kOrderTile / 256];
 #pragma unroll
         for (int j = 0; j < kOrderTile / 256; ++j) {
             const int64_t g = tile * kOrderTile + 256 * j + threadIdx.x;
             const int32_t w = g < n ? counts[g] : 0;
-            bin[j] = (w & 0xff) != 0 ? w >> 8 : -1;          // groups without items are left out
+            items[j] = w & 0xff;
+            bin[j] = items[j] != 0 ? w >> 8 : -1;            // groups without items are left out
             rank[j] = bin[j] >= 0 ? atomicAdd(&s_count[bin[j]], 1) : 0;
         }
         __syncthreads();
@@ -66,14 +68,16 @@ order_groups_kernel(int32_t* __restrict__ log, int64_t capacity, int32_t* __rest
 #pragma unroll
         for (int j = 0; j < kOrderTile / 256; ++j)
             if (bin[j] >= 0)
-                order[s_count[bin[j]] + rank[j]] = (int)(tile * kOrderTile + 256 * j + threadIdx.x);
+                order[s_count[bin[j]] + rank[j]] =
+                    (int)((uint32_t)(tile * kOrderTile + 256 * j + threadIdx.x) |
+                          (uint32_t)items[j] << 24);
     }
 }
 
-template <int K, int OUTS>
+template <int K>
 struct alignas(16) ScatterSmem {
     using Shape = RecordShape<K>;
-    alignas(16) float rows[32 * Shape::STRIDE * OUTS];
+    alignas(16) float rows[32 * Shape::STRIDE];
 };
 
 // What a scatter adds into.  HESS kernels: the Gauss-Newton diagonal of the squared error (the
@@ -95,7 +99,7 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
                       int64_t capacity, ScatterOut to, int part, int n_parts) {
     constexpr int K = RecordLength<BD>::K;
     using Shape = RecordShape<K>;
-    using SM = ScatterSmem<K, HESS ? 2 : 1>;
+    using SM = ScatterSmem<K>;
     extern __shared__ __align__(16) unsigned char s_raw[];
     const int lane = threadIdx.x & 31;
     SM& sm = *reinterpret_cast<SM*>(s_raw + (size_t)(threadIdx.x >> 5) * sizeof(SM));
@@ -137,10 +141,11 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
             const int batch = (threadIdx.x >> 5) * per_warp + lane;
             const int i = first + batch / per_group;
             if (lane < per_warp && i < end) {
-                const int g = sorted ? __ldg(order + i) : i;
+                const uint32_t g =
+                    sorted ? (uint32_t)__ldg(order + i) : (uint32_t)__ldg(counts + i) << 24;
                 const int sub = batch % per_group;
-                at = ((int64_t)g * per_group + sub) * 32;
-                len = (__ldg(counts + g) & 0xff) - 32 * sub;
+                at = ((int64_t)(sorted ? g & 0xffffffu : (uint32_t)i) * per_group + sub) * 32;
+                len = (int)(g >> 24) - 32 * sub;
                 len = len < 0 ? 0 : len > 32 ? 32 : len;
             }
         }
@@ -161,6 +166,9 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
             if (n == 0) continue;
             uint32_t slot = 0;
             int off = 0, hoff = 0;
+            float f[3] = {0.f, 0.f, 0.f}, fh[3] = {0.f, 0.f, 0.f}, gs = 0.f, hs = 0.f;
+            float basis[BD > 0 ? BD : 1] = {};
+            const bool want_grad = !HESS || to.grad != nullptr;
             if (lane < n) {
                 slot = (uint32_t)pa.x;
                 const int64_t ray = pa.y;
@@ -169,8 +177,7 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
                 const float h[3] = {__int_as_float(pb.y), __int_as_float(pb.z),
                                     __int_as_float(pb.w)};
                 const float dd = __int_as_float(pc.x);
-                float f[3] = {0.f, 0.f, 0.f}, fh[3], gs = 0.f, hs = 0.f, one_minus_s = 0.f;
-                const bool want_grad = !HESS || to.grad != nullptr;
+                float one_minus_s = 0.f;
                 // Gauss-Newton diagonal with a softplus density: the reference adds, per
                 // channel, (d out / d raw)^2 + (d out / d density) * softplus'' with its own
                 // formula for the second term (svox/csrc/rt_kernel.cu:683-693); dd already
@@ -197,7 +204,6 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
                 // 16-byte word), zeros around it
                 off = record_offset<K>(to.grad, slot);
                 hoff = HESS ? record_offset<K>(to.hess, slot) : 0;
-                float basis[BD > 0 ? BD : 1];
                 if constexpr (BD > 0) {
                     const float vdir[3] = {__int_as_float(pc.y), __int_as_float(pc.z),
                                            __int_as_float(pc.w)};
@@ -206,40 +212,39 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
                     for (int k = 0; k < BD; ++k)
                         if (k < opt.min_comp || k > opt.max_comp) basis[k] = 0.f;
                 }
-                float* row = sm.rows + lane * Shape::STRIDE;
-                auto expand = [&](float* __restrict__ r, int o, bool square) {
-                    float v[K];
+            }
+            float* row = sm.rows + lane * Shape::STRIDE;
+            auto expand = [&](float* __restrict__ r, int o, bool square) {
+                float v[K];
 #pragma unroll
-                    for (int ch = 0; ch < 3; ++ch) {
-                        if constexpr (BD == 0) {
-                            v[ch] = square ? fh[ch] * fh[ch] : f[ch];
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < BD; ++k) {
-                                const float w = basis[k] * (square ? fh[ch] : f[ch]);
-                                v[ch * BD + k] = square ? w * w : w;
-                            }
-                        }
-                    }
-                    v[K - 1] = square ? hs : gs;
-                    if (Shape::ALIGNED) {
-#pragma unroll
-                        for (int w = 0; w < K / 4; ++w)
-                            reinterpret_cast<float4*>(r)[w] =
-                                make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
+                for (int ch = 0; ch < 3; ++ch) {
+                    if constexpr (BD == 0) {
+                        v[ch] = square ? fh[ch] * fh[ch] : f[ch];
                     } else {
 #pragma unroll
-                        for (int i = 0; i < 3; ++i) {
-                            if (i < o) r[i] = 0.f;
-                            if (o + K + i < 4 * Shape::WORDS) r[o + K + i] = 0.f;
+                        for (int k = 0; k < BD; ++k) {
+                            const float w = basis[k] * (square ? fh[ch] : f[ch]);
+                            v[ch * BD + k] = square ? w * w : w;
                         }
-#pragma unroll
-                        for (int w = 0; w < K; ++w) r[o + w] = v[w];
                     }
-                };
-                if (want_grad) expand(row, off, false);
-                if constexpr (HESS) expand(row + 32 * Shape::STRIDE, hoff, true);
-            }
+                }
+                v[K - 1] = square ? hs : gs;
+                if (Shape::ALIGNED) {
+#pragma unroll
+                    for (int w = 0; w < K / 4; ++w)
+                        reinterpret_cast<float4*>(r)[w] =
+                            make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        if (i < o) r[i] = 0.f;
+                        if (o + K + i < 4 * Shape::WORDS) r[o + K + i] = 0.f;
+                    }
+#pragma unroll
+                    for (int w = 0; w < K; ++w) r[o + w] = v[w];
+                }
+            };
+            if (lane < n && want_grad) expand(row, off, false);
             __syncwarp();
             // groups of lanes add consecutive 16-byte words of a record
             auto flush = [&](float* __restrict__ out, const float* rows, int offset) {
@@ -256,14 +261,19 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
                                       vec_ok, pol_keep);
                 }
             };
-            if (!HESS || to.grad != nullptr) flush(to.grad, sm.rows, off);
-            if constexpr (HESS) flush(to.hess, sm.rows + 32 * Shape::STRIDE, hoff);
+            if (want_grad) flush(to.grad, sm.rows, off);
             __syncwarp();
+            if constexpr (HESS) {       // through the same rows
+                if (lane < n) expand(row, hoff, true);
+                __syncwarp();
+                flush(to.hess, sm.rows, hoff);
+                __syncwarp();
+            }
         }
     };
     ordered_units<BLOCK>(s_units, counters, lo_bin, hi_bin, groups_before,
                          WARPS * per_warp / per_group, ((int64_t)1 << log[2]) * K,
-                         sorted ? to.zero_slots * K : 0, count, clear, work);
+                         sorted ? to.zero_slots * K : 0, per_warp >= 4, count, clear, work);
 }
 
 }  // namespace svoxb

@@ -267,13 +267,20 @@ template <int BD, int BLOCK, bool HESS, bool LOBES>
 static int replay_scatter_block(const ReplayJob& job, int part, int reserve_sms,
                                 cudaStream_t stream) {
     constexpr int K = RecordLength<BD>::K;
-    const size_t smem = (size_t)(BLOCK / 32) * sizeof(ScatterSmem<K, HESS ? 2 : 1>);
+    const size_t smem = (size_t)(BLOCK / 32) * sizeof(ScatterSmem<K>);
     auto k = replay_scatter_kernel<BD, BLOCK, HESS, LOBES>;
     // blocks for the clearing too, which few packets may come with
     const int64_t clears = job.to.zero_slots * K / kZeroFloats * (BLOCK / 32);
     unsigned grid = 1;
     int st = persistent_grid(k, BLOCK, smem, job.chunks > clears ? job.chunks : clears, &grid);
     if (st) return st;
+    // Two outputs to clear: with more than two blocks per SM the units of adding come round to a bin
+    // before it is cleared, and wait (`se_grad` of 100 000 rays, 1 / 2 / 3 / 4 / 6 blocks: 1.07, 1.00,
+    // 1.11, 1.12, 1.56 ms; one output: the 2^20-ray step 3.05, 2.05, 1.90, 1.90, 2.34).
+    if (HESS && job.to.grad != nullptr && job.to.zero_slots > 0) {
+        const int64_t most = 2LL * (sm_count() - g_reserved_sms);
+        if ((int64_t)grid > most && most > 0) grid = (unsigned)most;
+    }
     if (reserve_sms > 0) {
         const int sms = sm_count();
         const int64_t per_sm = ((int64_t)grid + sms - 1) / sms;
