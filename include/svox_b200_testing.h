@@ -18,6 +18,10 @@ extern "C" {
  * key 7 changes.  Unknown keys return SVOXB_ERR_OPTION. */
 int svoxb_test_knob(int key, int value);
 
+/* Launch configurations (kernel, block, shared memory, device) whose occupancy the library has
+ * looked up so far and keeps. */
+int svoxb_test_known_launches(void);
+
 #ifdef __cplusplus
 }
 #endif

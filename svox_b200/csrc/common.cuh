@@ -129,6 +129,8 @@ __device__ __forceinline__ bool descendN(const int32_t* __restrict__ child, int6
 int set_cuda_error(cudaError_t e);  // records the text, returns SVOXB_ERR_CUDA
 int sm_count();                     // multiprocessors of the current device
 int blocks_per_sm(const void* kernel, int block, size_t smem, int* per_sm);
+// A count that follows the data, rounded up to a step, for the size of a launch's shared memory.
+constexpr size_t stepped(size_t n, size_t step) { return (n + step - 1) / step * step; }
 
 #define SVOXB_CUDA(call)                                              \
     do {                                                              \

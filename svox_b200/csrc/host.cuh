@@ -34,17 +34,20 @@ int sm_count() {
 }
 
 // Resident blocks per SM of a kernel on the current device, after raising its shared memory
-// limit where that is needed; asked of the runtime once per kernel and device (a microsecond or
-// two of the host's time per launch otherwise).
+// limit where that is needed; asked of the runtime once per kernel, size and device (a microsecond
+// or two of the host's time per launch otherwise).  Every launch looks through what is known, so
+// a size that follows the data (a tree that grows) comes rounded up to a few steps.
+struct KnownLaunch { const void* kernel; size_t smem; int block, dev, per_sm; };
+static std::mutex g_known_mutex;
+static std::vector<KnownLaunch> g_known;
+
 int blocks_per_sm(const void* kernel, int block, size_t smem, int* per_sm) {
-    struct Known { const void* kernel; size_t smem; int block, dev, per_sm; };
-    static std::mutex mutex;
-    static std::vector<Known> all;
+    auto& all = g_known;
     int dev = 0;
     SVOXB_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mutex);
+    std::lock_guard<std::mutex> lock(g_known_mutex);
     size_t limit = 20 * 1024;    // the 48 KB a kernel gets without asking, less its static share
-    for (const Known& k : all) {
+    for (const KnownLaunch& k : all) {
         if (k.kernel != kernel || k.dev != dev) continue;
         if (k.block == block && k.smem == smem) {
             *per_sm = k.per_sm;
@@ -58,7 +61,7 @@ int blocks_per_sm(const void* kernel, int block, size_t smem, int* per_sm) {
                                         (int)smem));
     SVOXB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, block, smem));
     if (*per_sm < 1) *per_sm = 1;
-    all.push_back(Known{kernel, smem, block, dev, *per_sm});
+    all.push_back(KnownLaunch{kernel, smem, block, dev, *per_sm});
     return SVOXB_OK;
 }
 

@@ -746,7 +746,7 @@ static int launch_tiled(const int64_t* ids, int64_t Q, const float* rows, int K,
         SVOXB_CUDA(cudaMemsetAsync(mem, 0, t.zero_words() * sizeof(int32_t), stream));
         const int sms = sm_count();
         const bool shared = t.n_tiles <= kMaxSharedTiles;
-        const size_t smem = shared ? (size_t)t.n_tiles * sizeof(int32_t) : 0;
+        const size_t smem = shared ? stepped(t.n_tiles, 2048) * sizeof(int32_t) : 0;
         auto grid_of = [&](auto kernel, int block, size_t smem, int64_t need, unsigned* grid) {
             int per_sm = 0;
             const int s2 = blocks_per_sm(reinterpret_cast<const void*>(kernel), block, smem, &per_sm);

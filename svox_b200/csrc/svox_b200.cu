@@ -185,7 +185,7 @@ template <int BD, int MODE, int BLOCK, class Source>
 static int launch_march(const RenderCall& c, const Source& src, const TreeIndex& index,
                         LogArgs log) {
     const size_t smem = (BLOCK / 32) * sizeof(WarpQueue<BD, MODE>) +
-                        (BLOCK > kMarchBlock ? bin_smem(log.n_bins) : 0);
+                        (BLOCK > kMarchBlock ? bin_smem((int)stepped(log.n_bins, kBinStep)) : 0);
     const int64_t tickets = Source::tickets(src, c.Q);
     const MarchShape shape = march_shape(
         tickets, (int64_t)sm_count() * (BLOCK > kMarchBlock ? BLOCK / 32 : kSpreadWarps));
@@ -1186,6 +1186,11 @@ int svoxb_test_knob(int key, int value) {
             return SVOXB_OK;
     }
     return SVOXB_ERR_OPTION;
+}
+
+int svoxb_test_known_launches(void) {
+    std::lock_guard<std::mutex> lock(g_known_mutex);
+    return (int)g_known.size();
 }
 
 }  // extern "C"

@@ -208,6 +208,44 @@ def test_query_values_through_shared_memory(K, cuda_device):
     csrc.check_device_status()
 
 
+def test_launches_known_do_not_grow_with_the_trees(cuda_device):
+    # gradients of many sizes, and logs of many numbers of bins, share a few launch configurations
+    import ctypes as C
+    lib = csrc.library()
+    K, Q = 49, 800000
+    gen = torch.Generator(cuda_device).manual_seed(3)
+    rows = torch.zeros(Q, K, device=cuda_device)
+    none = torch.zeros(3, device=cuda_device)
+    grad = torch.empty(8 * 400000 * K, device=cuda_device)
+
+    def backward(M):
+        ids = torch.randint(0, 8 * M, (Q,), generator=gen, device=cuda_device)
+        t = csrc._CTree(grad.data_ptr(), none.data_ptr(), none.data_ptr(), none.data_ptr(), M, 2, K)
+        assert lib.svoxb_query_scatter(
+            C.byref(t), C.c_void_p(ids.data_ptr()), C.c_int64(Q), C.c_void_p(rows.data_ptr()),
+            C.c_int32(K), C.c_void_p(grad.data_ptr()), C.c_int(1),
+            C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+
+    tree = _shell("SH4", 4, 2, cuda_device)
+    tree.data.requires_grad_(True)
+    r = svox.VolumeRenderer(tree)
+    rays = _rays(20000, cuda_device)
+    backward(270000)
+    r(rays).sum().backward()
+    before = lib.svoxb_test_known_launches()
+    for M in range(270000, 390000, 4000):
+        backward(M)
+    try:
+        for mb in range(1, 13):
+            assert lib.svoxb_test_knob(5, mb) == 0
+            r(rays).sum().backward()
+    finally:
+        lib.svoxb_test_knob(5, 32)
+    # two kernels count tiles, one fills bins; each has at most a dozen steps
+    assert lib.svoxb_test_known_launches() - before <= 12
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("K", [97, 100])
 @pytest.mark.parametrize("Q", [74000, 75000, 300001])
 def test_query_backward_binned(K, Q, cuda_device):
