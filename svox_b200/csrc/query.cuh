@@ -462,64 +462,75 @@ scatter_binned_rows_kernel(int64_t Q, const float* __restrict__ rows, int K,
 constexpr int kPlaceBlock = 512;
 constexpr int kPlaceEach = 16;       // points a thread places at a time
 
-// Items per tile of the points.
-template <bool SHARED>
+// Items per range of rows of the points.
 __global__ void __launch_bounds__(kPlaceBlock)
-count_tiles_kernel(const int64_t* __restrict__ ids, int64_t Q, TileLists t) {
+count_ranges_kernel(const int64_t* __restrict__ ids, TileLists t) {
     extern __shared__ int s_count[];
-    if (SHARED) {
-        for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock) s_count[i] = 0;
-        __syncthreads();
-    }
-    for (int64_t i = (int64_t)blockIdx.x * kPlaceBlock + threadIdx.x; i < Q;
+    for (int i = threadIdx.x; i < t.n_ranges; i += kPlaceBlock) s_count[i] = 0;
+    __syncthreads();
+    for (int64_t i = (int64_t)blockIdx.x * kPlaceBlock + threadIdx.x; i < t.n_items;
          i += (int64_t)gridDim.x * kPlaceBlock) {
         const int64_t slot = ids[i];
-        if (slot >= 0 && slot < t.n_rows)
-            atomicAdd((SHARED ? s_count : t.count) + (int)(slot >> t.shift), 1);
+        if (slot >= 0 && slot < t.n_rows) atomicAdd(s_count + (int)(slot >> t.shift), 1);
     }
-    if (!SHARED) return;
     __syncthreads();
-    for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock)
+    for (int i = threadIdx.x; i < t.n_ranges; i += kPlaceBlock)
+        if (s_count[i]) atomicAdd(t.in_range + i, s_count[i]);
+    if (last_block(t.head + 4)) cut_ranges<kPlaceBlock>(t);
+}
+
+// Items per tile of the points, where these are not the ranges.
+__global__ void __launch_bounds__(kPlaceBlock)
+count_tiles_kernel(const int64_t* __restrict__ ids, TileLists t) {
+    extern __shared__ int s_count[];
+    const int n_tiles = t.head[3];
+    if (n_tiles == t.n_ranges) return;
+    for (int i = threadIdx.x; i < n_tiles; i += kPlaceBlock) s_count[i] = 0;
+    __syncthreads();
+    for (int64_t i = (int64_t)blockIdx.x * kPlaceBlock + threadIdx.x; i < t.n_items;
+         i += (int64_t)gridDim.x * kPlaceBlock) {
+        const int64_t slot = ids[i];
+        if (slot >= 0 && slot < t.n_rows) atomicAdd(s_count + t.tile_of(slot), 1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_tiles; i += kPlaceBlock)
         if (s_count[i]) atomicAdd(t.count + i, s_count[i]);
+    if (last_block(t.head + 5)) list_tiles<kPlaceBlock>(t, t.count);
 }
 
 // Lists the points {slot, row} tile by tile.  0.19 ms for 2^24 points and 4681 tiles, the same with
 // 256 to 1024 threads.
-template <bool SHARED>
 __global__ void __launch_bounds__(kPlaceBlock)
-place_tiles_kernel(const int64_t* __restrict__ ids, int64_t Q, TileLists t, int2* __restrict__ pair,
-                  int K, float* __restrict__ grad) {
+place_tiles_kernel(const int64_t* __restrict__ ids, TileLists t, int2* __restrict__ pair, int K,
+                   float* __restrict__ grad) {
     extern __shared__ int s_count[];
     clear_hot_tiles(t, K, grad);
-    constexpr int EACH = SHARED ? kPlaceEach : 1;
-    for (int64_t tile = blockIdx.x; tile * (EACH * kPlaceBlock) < Q; tile += gridDim.x) {
-        if (SHARED) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock) s_count[i] = 0;
-            __syncthreads();
-        }
-        int slot[EACH], rank[EACH];
+    const int n_tiles = t.head[3];
+    constexpr int64_t each = kPlaceEach * kPlaceBlock;
+    for (int64_t first = blockIdx.x * each; first < t.n_items; first += gridDim.x * each) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < n_tiles; i += kPlaceBlock) s_count[i] = 0;
+        __syncthreads();
+        int slot[kPlaceEach], rank[kPlaceEach];
 #pragma unroll
-        for (int j = 0; j < EACH; ++j) {
-            const int64_t i = tile * (EACH * kPlaceBlock) + kPlaceBlock * j + threadIdx.x;
-            const int64_t s = i < Q ? ids[i] : -1;
+        for (int j = 0; j < kPlaceEach; ++j) {
+            const int64_t i = first + kPlaceBlock * j + threadIdx.x;
+            const int64_t s = i < t.n_items ? ids[i] : -1;
             slot[j] = s >= 0 && s < t.n_rows ? (int)s : -1;
         }
 #pragma unroll
-        for (int j = 0; j < EACH; ++j)
-            rank[j] = slot[j] >= 0
-                          ? atomicAdd((SHARED ? s_count : t.end) + (slot[j] >> t.shift), 1) : 0;
-        if (SHARED) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < t.n_tiles; i += kPlaceBlock)
-                if (s_count[i] > 0) s_count[i] = atomicAdd(t.end + i, s_count[i]);
-            __syncthreads();
+        for (int j = 0; j < kPlaceEach; ++j) {
+            rank[j] = slot[j] >= 0 ? atomicAdd(s_count + t.tile_of(slot[j]), 1) : 0;
         }
+        __syncthreads();
+        for (int i = threadIdx.x; i < n_tiles; i += kPlaceBlock)
+            if (s_count[i] > 0) s_count[i] = atomicAdd(t.end + i, s_count[i]);
+        __syncthreads();
 #pragma unroll
-        for (int j = 0; j < EACH; ++j)
+        for (int j = 0; j < kPlaceEach; ++j)
             if (slot[j] >= 0)
-                pair[rank[j] + (SHARED ? s_count[slot[j] >> t.shift] : 0)] = make_int2(
-                    slot[j], (int)(tile * (EACH * kPlaceBlock) + kPlaceBlock * j + threadIdx.x));
+                pair[rank[j] + s_count[t.tile_of(slot[j])]] =
+                    make_int2(slot[j], (int)(first + kPlaceBlock * j + threadIdx.x));
     }
 }
 
@@ -529,6 +540,9 @@ __device__ __forceinline__ void copy_word(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global.L2::64B [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
 
+// Items of a tile from which its rows, and the zeros between them, leave through StreamWriter:
+// fewer items leave most of the tile to few of the warps.
+constexpr int kStreamItems = 32;
 constexpr int kStageWords = 104;     // 16-byte words of rows a warp has under way per stage
 
 // Warps take equal shares of a tile's sorted items; lane e of a warp holds columns e, e + 32, ... of
@@ -545,30 +559,32 @@ own_rows_kernel(const float* __restrict__ rows, uint32_t last_id, int K,
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ float s_carry[kOwnWarps * 32 * N];
     __shared__ int s_state[kOwnWarps];
-    const TileSort sorted(s_raw, t.shift);
+    const TileSort sorted(s_raw);
     // (through a shuffle, so that the compiler knows it to be the same in a warp: loops over a warp's
     // items then need no code for divergence)
     const int me = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), e = threadIdx.x & 31;
-    float* const stages = reinterpret_cast<float*>(s_raw + TileSort::bytes(t.shift));
+    float* const stages = reinterpret_cast<float*>(s_raw + TileSort::kBytes);
     float* const stage = stages + me * (2 * 4 * kStageWords);
     StreamWriter writer;
     writer.buf = stages + kOwnWarps * (2 * 4 * kStageWords) + me * (2 * StreamWriter::kPiece);
     writer.clear();
     const uint32_t pitch = 4u * (uint32_t)K;
     const bool one_pass = K <= 32 * N && (reinterpret_cast<uintptr_t>(grad) & 15) == 0;
-    owned_units(t, 0, t.n_tiles, [&](int tile, int first, int last, bool hot) {
-        const int64_t row0 = (int64_t)tile << t.shift;
-        const int n_rows = (int)(t.n_rows - row0 < (1 << t.shift) ? t.n_rows - row0
-                                                                  : (int64_t)1 << t.shift);
+    owned_units(t, [&](int tile, int first, int last, bool hot) {
+        const int64_t row0 = t.first_row(tile);
+        const int shift = t.tile_shift(tile);
+        if (row0 >= t.n_rows) return;            // the last range may reach beyond the buffer
+        const int n_rows = (int)(t.n_rows - row0 < (1 << shift) ? t.n_rows - row0
+                                                                : (int64_t)1 << shift);
         float* __restrict__ out = grad + row0 * K;
         bool store = !hot;          // rows are written, else added to
         do {
             const int n = last - first < kOwnItems ? last - first : kOwnItems;
-            sorted.sort(n, t.shift, [&](int i) {
+            sorted.sort(n, shift, [&](int i) {
                 const int2 p = __ldg(pair + first + i);
                 return make_int2(p.x - (int)row0, p.y);
             });
-            const bool stream = store && one_pass && n > 0;
+            const bool stream = store && one_pass && n >= kStreamItems;
             if (store && !stream) sorted.clear_empty(n_rows, K, out);
             const int lo = n * me / kOwnWarps, hi = n * (me + 1) / kOwnWarps;
             for (int base = 0; base < K; base += 32 * N) {
@@ -719,34 +735,19 @@ static int with_columns(int K, F f) {
     return f(Lanes<4>{});
 }
 
-// log2 of the rows of a tile: as many as bring a block nine tenths of the items that it sorts at a
-// time, at most `most`.
-static int tile_shift(int64_t items, int64_t n_rows, int most) {
-    int shift = most;
-    while (shift > kMinTileShift &&
-           (double)items / (double)n_rows * (double)(1LL << shift) > 0.9 * kOwnItems)
-        --shift;
-    return shift;
-}
-
-static int launch_tiled(const int64_t* ids, int64_t Q, const float* rows, int K, float* grad,
-                        int64_t n_slots, cudaStream_t stream) {
+static int launch_tiled(const int64_t* ids, const float* rows, int K, float* grad, TileLists t,
+                        cudaStream_t stream) {
     int st;
     if ((st = keep_pool_cached())) return st;
-    TileLists t{};
-    t.n_rows = n_slots;
-    t.shift = tile_shift(Q, n_slots, 12);
-    t.n_tiles = (int)(((n_slots - 1) >> t.shift) + 1);
-    const size_t words = TileLists::words(t.n_tiles, Q);
+    const int64_t Q = t.n_items;
+    const size_t words = t.words();
     int32_t* mem = nullptr;
     SVOXB_CUDA(cudaMallocAsync((void**)&mem, (words + 2 * (size_t)Q) * sizeof(int32_t), stream));
-    t.place_in(mem, Q);
+    t.place_in(mem);
     int2* pair = reinterpret_cast<int2*>(mem + words);
     st = [&] {
         SVOXB_CUDA(cudaMemsetAsync(mem, 0, t.zero_words() * sizeof(int32_t), stream));
         const int sms = sm_count();
-        const bool shared = t.n_tiles <= kMaxSharedTiles;
-        const size_t smem = shared ? stepped(t.n_tiles, 2048) * sizeof(int32_t) : 0;
         auto grid_of = [&](auto kernel, int block, size_t smem, int64_t need, unsigned* grid) {
             int per_sm = 0;
             const int s2 = blocks_per_sm(reinterpret_cast<const void*>(kernel), block, smem, &per_sm);
@@ -754,22 +755,24 @@ static int launch_tiled(const int64_t* ids, int64_t Q, const float* rows, int K,
             *grid = (unsigned)(need < most ? need : most);
             return s2;
         };
+        auto blocks = [&](int each) { return (Q + kPlaceBlock * each - 1) / (kPlaceBlock * each); };
         unsigned grid = 1;
-        auto count = shared ? count_tiles_kernel<true> : count_tiles_kernel<false>;
-        int s2 = grid_of(count, kPlaceBlock, smem, (Q + kPlaceBlock * 16 - 1) / (kPlaceBlock * 16),
-                         &grid);
-        if (s2) return s2;
-        count<<<grid, kPlaceBlock, smem, stream>>>(ids, Q, t);
-        scan_tiles_kernel<<<1, 1024, 0, stream>>>(t);
-        auto place = shared ? place_tiles_kernel<true> : place_tiles_kernel<false>;
-        const int64_t each = kPlaceBlock * (shared ? kPlaceEach : 1);
-        if ((s2 = grid_of(place, kPlaceBlock, smem, (Q + each - 1) / each, &grid))) return s2;
-        place<<<grid, kPlaceBlock, smem, stream>>>(ids, Q, t, pair, K, grad);
+        int s2;
+        size_t smem = stepped(t.n_ranges, 2048) * sizeof(int32_t);
+        if ((s2 = grid_of(count_ranges_kernel, kPlaceBlock, smem, blocks(4), &grid)))
+            return s2;
+        count_ranges_kernel<<<grid, kPlaceBlock, smem, stream>>>(ids, t);
+        smem = stepped(t.max_tiles, 2048) * sizeof(int32_t);
+        if ((s2 = grid_of(count_tiles_kernel, kPlaceBlock, smem, blocks(4), &grid))) return s2;
+        count_tiles_kernel<<<grid, kPlaceBlock, smem, stream>>>(ids, t);
+        if ((s2 = grid_of(place_tiles_kernel, kPlaceBlock, smem, blocks(kPlaceEach), &grid)))
+            return s2;
+        place_tiles_kernel<<<grid, kPlaceBlock, smem, stream>>>(ids, t, pair, K, grad);
         return with_columns(K, [&](auto columns) {
             auto own = own_rows_kernel<decltype(columns)::value>;
-            const size_t bytes = TileSort::bytes(t.shift) +
+            const size_t bytes = TileSort::kBytes +
                                  kOwnWarps * (2 * 16 * kStageWords + 8 * StreamWriter::kPiece);
-            const int s3 = grid_of(own, kOwnBlock, bytes, (int64_t)t.n_tiles + Q / kOwnItems, &grid);
+            const int s3 = grid_of(own, kOwnBlock, bytes, (int64_t)t.max_tiles + Q / kOwnItems, &grid);
             if (s3) return s3;
             own<<<grid, kOwnBlock, bytes, stream>>>(rows, (uint32_t)(Q - 1), K, grad, t, pair);
             SVOXB_CUDA(cudaGetLastError());
@@ -800,7 +803,10 @@ static int launch_scatter(const svoxb_tree* tree, const int64_t* ids, int64_t Q,
                         Q < (1LL << 31) - kBinRows && n_slots < (1LL << 31) &&
                         reinterpret_cast<uintptr_t>(grad) % 16 == 0;
     int st;
-    if (binned && sums_by_tiles(n_floats, K)) return launch_tiled(ids, Q, rows, K, grad, n_slots, stream);
+    if (binned && sums_by_tiles(n_floats, K)) {
+        const TileLists t(n_slots, Q);
+        if (t.max_tiles <= kMaxTiles) return launch_tiled(ids, rows, K, grad, t, stream);
+    }
     if (!binned) {
         if (zero_first && (st = zero_rows(grad, n_floats, stream))) return st;
         if (Q == 0) return SVOXB_OK;

@@ -7,8 +7,15 @@
 // once for the zeros, and the L2 takes 46 G reductions of a 112-byte row a second (5.2 TB/s, measured
 // with all of them hits); here the buffer is written once and only the items are read.
 //
-//   count    items per tile
-//   scan     where each tile's items begin; tiles with very many items (HOT) become several units
+// Items are spread unevenly: coarse leaves are hit more often than fine ones, points lie near a
+// surface.  So the buffer is first divided into equal RANGES of 2^shift rows, and each is cut into 1,
+// 2, 4 .. tiles, as many as bring a block no more than it can sort at a time.  (Cut by the average
+// alone, 14.7 M uniform points into a 1024^3 tree of three shells, 56 M rows of 28 floats, made tiles of
+// 33 000 items: 5.95 ms, now 2.22; 1.4 M points around one place of 400 MB of 76 floats: 0.84 -> 0.29.)
+//
+//   count    items per range; the last block cuts the ranges into tiles
+//   recount  items per tile, if any range was cut; the last block lists where each tile's begin, and
+//            the tiles that have very many all the same (HOT), which become several units of work
 //   place    the items' references, tile by tile; hot tiles are cleared
 //   own      (the caller's kernel) a block per unit, through TileSort
 #pragma once
@@ -19,96 +26,182 @@ namespace svoxb {
 
 constexpr int kOwnBlock = 512;
 constexpr int kOwnWarps = kOwnBlock / 32;
-constexpr int kOwnItems = 4096;                // items a block sorts at a time
-constexpr int kHotItems = 8 * kOwnItems;       // a tile with more is shared out, see scan_tiles_kernel
-constexpr int kMinTileShift = 6;
-// Tiles up to which a block counts in shared memory.
-constexpr int kMaxSharedTiles = 12288;
+// Items a block sorts at a time; with two blocks per SM there is room for 4840.  (4096 left half of the
+// tiles of 2^24 uniform points in a 256^3 tree, 4096 +- 64 items each, a second turn for a few items:
+// 2.07 ms, 2.00 with 4608 or 4800.)
+constexpr int kOwnItems = 4800;
+// A tile with more than kOwnItems is shared out, see list_tiles, if its rows have this many on
+// average, or if it would take one block more than kHotTurns turns.
+constexpr int kHotRow = 16, kHotTurns = 8;
+constexpr int kMinTileShift = 6, kMaxTileShift = 12;
+// Tiles that a block counts in shared memory; buffers that need more are not summed by tiles.
+constexpr int kMaxTiles = 24576;
 
 // Lists of items by tile, in one allocation.
 struct TileLists {
-    int32_t* head;       // [0] next unit  [1] hot units  [2] hot tiles
-    int32_t* count;      // [n_tiles] items of a tile
-    int32_t* end;        // [n_tiles] end of those placed so far; after `place` of all
+    int32_t* head;       // [0] next unit  [1] hot units  [2] hot tiles  [3] tiles
+                         // [4], [5] blocks that are done with counting, recounting
+    int32_t* in_range;   // [n_ranges] items of a range
+    int32_t* count;      // [max_tiles] items of a tile
+    int32_t* end;        // [max_tiles] end of those placed so far; after `place` of all
+    uint32_t* cut;       // [n_ranges] first tile; bits 28-31: log2 of the range's tiles
+    uint32_t* where;     // [max_tiles] first row / 2^kMinTileShift; bits 28-31: log2 of the tile's
+                         // rows, less kMinTileShift
     int2* hot_unit;      // {tile, first item within the tile}
     int32_t* hot_tile;
-    int shift;           // log2 of a tile's rows
-    int n_tiles;
-    int64_t n_rows;
+    int shift;           // log2 of a range's rows
+    int n_ranges, max_tiles;
+    int64_t n_rows, n_items;
 
-    // Hot units and tiles that `items` items can make.
-    static int64_t most_hot(int64_t items) { return items / kOwnItems * 5 / 4 + 2; }
-    static size_t words(int n_tiles, int64_t items) {
-        return (32 + 2 * (size_t)n_tiles + 3 + 3 * (size_t)most_hot(items)) & ~(size_t)1;
-    }
+    static constexpr size_t up4(size_t n) { return (n + 3) & ~(size_t)3; }
+    // Hot units and tiles that the items can make.
+    int64_t most_hot() const { return 2 * n_items / kOwnItems + 2; }
     // Words that are zero before `count`.
-    size_t zero_words() const { return 32 + (size_t)n_tiles; }
-    void place_in(int32_t* mem, int64_t items) {
+    size_t zero_words() const { return 32 + up4(n_ranges) + up4(max_tiles); }
+    size_t words() const {
+        return zero_words() + 2 * up4(max_tiles) + up4(n_ranges) + up4(3 * (size_t)most_hot());
+    }
+    TileLists(int64_t rows, int64_t items) : n_rows(rows), n_items(items) {
+        shift = kMaxTileShift;
+        n_ranges = (int)(((rows - 1) >> shift) + 1);
+        // A range is cut into 2^n tiles, n > 0, only with more than 2^(n-1) * kOwnItems items.
+        const int64_t most = n_ranges + 2 * items / kOwnItems + 1;
+        max_tiles = most < INT32_MAX ? (int)most : INT32_MAX;
+    }
+    void place_in(int32_t* mem) {
         head = mem;
-        count = mem + 32;
-        end = count + n_tiles;
-        hot_unit = reinterpret_cast<int2*>(mem + ((32 + 2 * (size_t)n_tiles + 1) & ~(size_t)1));
-        hot_tile = reinterpret_cast<int32_t*>(hot_unit + most_hot(items));
+        in_range = mem + 32;
+        count = in_range + up4(n_ranges);
+        end = count + up4(max_tiles);
+        where = reinterpret_cast<uint32_t*>(end + up4(max_tiles));
+        cut = where + up4(max_tiles);
+        hot_unit = reinterpret_cast<int2*>(cut + up4(n_ranges));
+        hot_tile = reinterpret_cast<int32_t*>(hot_unit + most_hot());
+    }
+    // Tile of a row.
+    __device__ __forceinline__ int tile_of(int64_t row) const {
+        const uint32_t c = __ldg(cut + (row >> shift));
+        return (int)(c & 0x0fffffffu) +
+               (int)(((uint32_t)row & ((1u << shift) - 1u)) >> (shift - (int)(c >> 28)));
+    }
+    __device__ __forceinline__ bool is_hot(int tile, int items) const {
+        return items > kOwnItems &&
+               (items > kHotTurns * kOwnItems || items >= kHotRow << tile_shift(tile));
+    }
+    __device__ __forceinline__ int64_t first_row(int tile) const {
+        return (int64_t)(where[tile] & 0x0fffffffu) << kMinTileShift;
+    }
+    __device__ __forceinline__ int tile_shift(int tile) const {
+        return (int)(where[tile] >> 28) + kMinTileShift;
     }
 };
 
-// One block.  A tile's items are one unit of work, unless there are more than kHotItems of them
-// (rows that very many items hit: the leaf that a camera stands in): then every kOwnItems of them
-// are, so that the device shares in them, and what they add goes into a cleared tile.
-__global__ void __launch_bounds__(1024) scan_tiles_kernel(TileLists t) {
-    __shared__ int s_sum[32];
-    __shared__ int s_carry;
-    const int tid = threadIdx.x, lane = tid & 31;
-    if (tid == 0) s_carry = 0;
+// Sum of n over the threads before this one; *total: over all.  `s_sum`: BLOCK / 32 words.
+template <int BLOCK>
+__device__ __forceinline__ int sum_before(int n, int* s_sum, int* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = n;
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+        const int y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    if (lane == 31) s_sum[warp] = x;
     __syncthreads();
-    for (int base = 0; base < t.n_tiles; base += 1024) {
-        const int i = base + tid;
-        const int n = i < t.n_tiles ? t.count[i] : 0;
-        int x = n;
+    int before = 0, all = 0;
 #pragma unroll
-        for (int d = 1; d < 32; d *= 2) {
-            const int y = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= d) x += y;
-        }
-        if (lane == 31) s_sum[tid >> 5] = x;
-        __syncthreads();
-        if (tid < 32) {
-            int w = s_sum[tid];
+    for (int w = 0; w < BLOCK / 32; ++w) {
+        const int v = s_sum[w];
+        if (w < warp) before += v;
+        all += v;
+    }
+    __syncthreads();
+    *total = all;
+    return before + x - n;
+}
+
+// Whether this block is the last one of the grid to come here; it then sees what the others wrote
+// before.  All threads.
+__device__ __forceinline__ bool last_block(int32_t* done) {
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last != 0;
+}
+
+// Lists where the tiles' items begin; one block.  A tile's items are one unit of work, unless it is
+// HOT: then every kOwnItems of them are, so that the device shares in them, and what they add goes
+// into a cleared tile.  `counted`: items per tile.  With many items per row (the leaf that a camera stands in) the reductions for
+// that are few; else it is the lesser evil.
+template <int BLOCK>
+__device__ __forceinline__ void list_tiles(const TileLists& t, const int32_t* counted) {
+    __shared__ int s_sum[BLOCK / 32];
+    const int n_tiles = t.head[3];
+    int run = 0;
+    for (int base = 0; base < n_tiles; base += 4 * BLOCK) {
+        const int i = base + 4 * (int)threadIdx.x;
+        int n[4];
 #pragma unroll
-            for (int d = 1; d < 32; d *= 2) {
-                const int y = __shfl_up_sync(0xffffffffu, w, d);
-                if (lane >= d) w += y;
-            }
-            s_sum[tid] = w;
+        for (int j = 0; j < 4; ++j) n[j] = i + j < n_tiles ? __ldcg(counted + i + j) : 0;
+        int total;
+        int first = run + sum_before<BLOCK>(n[0] + n[1] + n[2] + n[3], s_sum, &total);
+        run += total;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (i + j >= n_tiles) break;
+            if (counted != t.count) t.count[i + j] = n[j];
+            t.end[i + j] = first;
+            first += n[j];
+            if (!t.is_hot(i + j, n[j])) continue;
+            const int units = (n[j] + kOwnItems - 1) / kOwnItems;
+            const int at = atomicAdd(t.head + 1, units);
+            for (int u = 0; u < units; ++u) t.hot_unit[at + u] = make_int2(i + j, u * kOwnItems);
+            t.hot_tile[atomicAdd(t.head + 2, 1)] = i + j;
         }
-        __syncthreads();
-        const int first = s_carry + (tid >= 32 ? s_sum[(tid >> 5) - 1] : 0) + x - n;
-        if (i < t.n_tiles) {
-            t.end[i] = first;
-            if (n > kHotItems) {
-                const int units = (n + kOwnItems - 1) / kOwnItems;
-                const int at = atomicAdd(t.head + 1, units);
-                for (int u = 0; u < units; ++u) t.hot_unit[at + u] = make_int2(i, u * kOwnItems);
-                t.hot_tile[atomicAdd(t.head + 2, 1)] = i;
-            }
-        }
-        __syncthreads();
-        if (tid == 0) s_carry += s_sum[31];
-        __syncthreads();
     }
 }
 
-// Clears the rows of the hot tiles; all threads of the grid.
+// Cuts the ranges into tiles, and lists these if they are the ranges; one block.
+template <int BLOCK>
+__device__ __forceinline__ void cut_ranges(const TileLists& t) {
+    __shared__ int s_sum[BLOCK / 32];
+    int run = 0;
+    for (int base = 0; base < t.n_ranges; base += BLOCK) {
+        const int r = base + (int)threadIdx.x;
+        int levels = 0;
+        if (r < t.n_ranges) {
+            const int64_t items = __ldcg(t.in_range + r);
+            while (levels < t.shift - kMinTileShift && items > (int64_t)kOwnItems << levels) ++levels;
+        }
+        int total;
+        const int first = run + sum_before<BLOCK>(r < t.n_ranges ? 1 << levels : 0, s_sum, &total);
+        run += total;
+        if (r < t.n_ranges) {
+            t.cut[r] = (uint32_t)first | (uint32_t)levels << 28;
+            const int shift = t.shift - levels;
+            const uint32_t row0 = (uint32_t)(((int64_t)r << t.shift) >> kMinTileShift);
+            for (int j = 0; j < 1 << levels; ++j)
+                t.where[first + j] = (row0 + ((uint32_t)j << (shift - kMinTileShift))) |
+                                     (uint32_t)(shift - kMinTileShift) << 28;
+        }
+    }
+    if (threadIdx.x == 0) t.head[3] = run;
+    __syncthreads();
+    if (run == t.n_ranges) list_tiles<BLOCK>(t, t.in_range);
+}
+
+// Clears the rows of the hot tiles; all blocks of the grid.
 __device__ __forceinline__ void clear_hot_tiles(const TileLists& t, int K, float* __restrict__ out) {
-    const int n = *(volatile int32_t*)(t.head + 2);
-    for (int h = 0; h < n; ++h) {
-        const int64_t first = (int64_t)t.hot_tile[h] << t.shift;
-        const int64_t left = t.n_rows - first, rows = (int64_t)1 << t.shift;
+    const int n = t.head[2];
+    for (int h = blockIdx.x; h < n; h += gridDim.x) {
+        const int64_t first = t.first_row(t.hot_tile[h]);
+        const int64_t left = t.n_rows - first, rows = (int64_t)1 << t.tile_shift(t.hot_tile[h]);
         float* __restrict__ to = out + first * K;
         const int64_t floats = (left < rows ? left : rows) * K;
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < floats;
-             i += (int64_t)gridDim.x * blockDim.x)
-            to[i] = 0.f;
+        for (int64_t i = threadIdx.x; i < floats; i += blockDim.x) to[i] = 0.f;
     }
 }
 
@@ -119,20 +212,18 @@ struct TileSort {
     uint32_t* item;
     uint16_t* row;
 
-    static __host__ __device__ size_t bytes(int shift) {
-        return ((size_t)2 << shift) + (size_t)kOwnItems * 6;
-    }
-    __device__ __forceinline__ explicit TileSort(unsigned char* smem, int shift) {
+    static constexpr size_t kBytes = ((size_t)2 << kMaxTileShift) + (size_t)kOwnItems * 6;
+    __device__ __forceinline__ explicit TileSort(unsigned char* smem) {
         end = reinterpret_cast<uint32_t*>(smem);
-        item = end + (1 << (shift - 1));
+        item = end + (1 << (kMaxTileShift - 1));
         row = reinterpret_cast<uint16_t*>(item + kOwnItems);
     }
     // Number of the items in rows up to `r` of the tile.
     __device__ __forceinline__ int upto(int r) const {
         return r < 0 ? 0 : reinterpret_cast<const uint16_t*>(end)[r];
     }
-    // Sorts n <= kOwnItems items, `get(i)` = {row within the tile, item}, by row.  All threads;
-    // ends with a barrier.
+    // Sorts n <= kOwnItems items, `get(i)` = {row within the tile, item}, by row of a tile of 2^shift.
+    // All threads; ends with a barrier.
     template <class Get>
     __device__ __forceinline__ void sort(int n, int shift, Get get) const {
         __shared__ int s_sum[kOwnWarps];
@@ -277,10 +368,10 @@ enum { kCarryNone = 0, kCarryEnds = 1, kCarryThrough = 2, kCarrySkip = 3 };
 // Units of a launch: hot units first, then the tiles that are not hot, handed out in order.
 // `work(tile, first, last, hot)` by all threads, items [first, last) of the sorted list.
 template <class Work>
-__device__ __forceinline__ void owned_units(const TileLists& t, int lo_tile, int hi_tile, Work work) {
+__device__ __forceinline__ void owned_units(const TileLists& t, Work work) {
     __shared__ int s_unit;
     const int n_hot = *(volatile int32_t*)(t.head + 1);
-    const int all = n_hot + hi_tile - lo_tile;
+    const int all = n_hot + *(volatile int32_t*)(t.head + 3);
     int next = 0;
     if (threadIdx.x == 0) next = atomicAdd(t.head, 1);
     for (;;) {
@@ -296,14 +387,13 @@ __device__ __forceinline__ void owned_units(const TileLists& t, int lo_tile, int
             tile = h.x;
             from = h.y;
         } else {
-            tile = lo_tile + u - n_hot;
+            tile = u - n_hot;
         }
         const int n = t.count[tile];
         const int first = t.end[tile] - n;
         if (hot) {
-            if (tile >= lo_tile && tile < hi_tile)
-                work(tile, first + from, first + (n < from + kOwnItems ? n : from + kOwnItems), true);
-        } else if (n <= kHotItems) {
+            work(tile, first + from, first + (n < from + kOwnItems ? n : from + kOwnItems), true);
+        } else if (!t.is_hot(tile, n)) {
             work(tile, first, first + n, false);
         }
         __syncthreads();

@@ -264,9 +264,10 @@ def test_query_backward_binned(K, Q, cuda_device):
 @pytest.mark.parametrize("K", [4, 28, 33, 49, 64, 65, 130])
 @pytest.mark.parametrize("how", ["even", "dense", "hot", "ends"])
 def test_query_gradient_by_tiles(K, how, cuda_device):
-    # a gradient of 400 MB (or, for short rows, 800; K = 4: bins), rows summed tile by tile: tiles without points, with a chunk of
-    # them, with several chunks, and rows so often hit that their tile is shared out among blocks;
-    # ids that are no row are left out
+    # a gradient of 400 MB (or, for short rows, 800; K = 4: bins), rows summed tile by tile: tiles
+    # without points, with as many as a block takes in one turn, and rows so often hit that their
+    # tile is shared out among blocks; ids that are no row are left out.  (A gradient beside a 16-byte
+    # boundary is added to point by point.)
     import ctypes as C
     M = -(-((400 if K > 32 else 800) << 20) // (32 * K))
     n = 8 * M
@@ -296,6 +297,100 @@ def test_query_gradient_by_tiles(K, how, cuda_device):
         assert st == 0
         assert torch.equal(grad.view(n, K).double(), want)
     csrc.check_device_status()
+
+
+def _scatter(M, K, ids, rows, grad):
+    import ctypes as C
+    none = torch.zeros(3, device=ids.device)
+    t = csrc._CTree(grad.data_ptr(), none.data_ptr(), none.data_ptr(), none.data_ptr(), M, 2, K)
+    assert csrc.library().svoxb_query_scatter(
+        C.byref(t), C.c_void_p(ids.data_ptr()), C.c_int64(ids.numel()),
+        C.c_void_p(rows.data_ptr()), C.c_int32(K), C.c_void_p(grad.data_ptr()), C.c_int(1),
+        C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+
+
+def _scatter_is_exact(M, K, ids, rows):
+    """Rows of small whole numbers: their sums are exact in any order."""
+    n = 8 * M
+    want = torch.zeros(n, K, device=ids.device).index_add_(0, ids, rows)
+    assert want.abs().max().item() < 1 << 24
+    grad = torch.full((n, K), float("nan"), device=ids.device)
+    _scatter(M, K, ids, rows, grad)
+    assert torch.equal(grad, want)
+    csrc.check_device_status()
+
+
+@pytest.mark.parametrize("K", [33, 49, 76, 130])
+@pytest.mark.parametrize("how", ["steep", "turns", "run", "end", "sparse"])
+def test_query_gradient_of_clustered_points(K, how, cuda_device):
+    # ranges of 4096 rows are cut into tiles where points lie densely; tiles that still have more
+    # points than a block sorts at a time are written in a first turn and added to in others; a row's
+    # points may fill several warps; the last range reaches beyond the buffer; few points in a tile
+    M = -(-(400 << 20) // (32 * K))
+    n = 8 * M
+    gen = torch.Generator(cuda_device).manual_seed(K)
+    base = n + n // 4 if K > 128 else n // 3
+    ids = torch.randint(0, n, (base,), generator=gen, device=cuda_device)
+
+    def near(first, rows, points):
+        return first + torch.randint(0, rows, (points,), generator=gen, device=cuda_device)
+
+    if how == "steep":
+        ids = (n * 0.6 + n * 0.01 * torch.randn(base, generator=gen, device=cuda_device)).long()
+    elif how == "turns":
+        more = [near(20 * 4096 + 1024 * q, 1024, 3 * p) for q, p in ((1, 4000), (3, 1700))]
+        ids = torch.cat([ids, *more, near(33 * 4096, 2048, 5000)])
+    elif how == "run":
+        ids = torch.cat([ids, near(7 * 4096 + 5, 1, 3000), near(8 * 4096 - 1, 1, 900)])
+    elif how == "end":
+        ids = torch.cat([ids, near(n - 300, 300, 60000)])
+    else:
+        # a few points in most ranges, the others (without which they would be too few to be sorted
+        # at all) on one row
+        few = torch.arange(n // 4096, device=cuda_device) % 70
+        at = torch.repeat_interleave(torch.arange(n // 4096, device=cuda_device) * 4096, few)
+        at += torch.randint(0, 4096, (at.numel(),), generator=gen, device=cuda_device)
+        ids = torch.cat([at, near(n // 2, 1, base)])
+    ids = ids.clamp(0, n - 1)
+    lim = 2 if how == "sparse" else 9
+    rows = torch.randint(1 - lim, lim, (ids.numel(), K), generator=gen, device=cuda_device).float()
+    _scatter_is_exact(M, K, ids, rows)
+
+
+@pytest.mark.parametrize("K", [36, 49, 64, 66, 76, 130])
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_query_gradient_of_rows_at_any_address(K, offset, cuda_device):
+    # rows are copied as the 16-byte words that cover them; the last row ends with its buffer
+    M = -(-(400 << 20) // (32 * K))
+    n = 8 * M
+    gen = torch.Generator(cuda_device).manual_seed(K)
+    Q = n + 5 if K > 128 else n // 3 + 5
+    ids = torch.randint(0, n, (Q,), generator=gen, device=cuda_device)
+    rows = torch.randint(-8, 9, (Q * K + offset,), generator=gen, device=cuda_device).float()
+    _scatter_is_exact(M, K, ids, rows[offset:].view(Q, K))
+
+
+def test_query_gradient_of_clustered_points_takes_no_longer(cuda_device):
+    # (tiles cut by the average density: three times as long as for points spread evenly)
+    K = 76
+    M = (400 << 20) // (32 * K)
+    n = 8 * M
+    gen = torch.Generator(cuda_device).manual_seed(1)
+    rows = torch.randn(n // 2, K, generator=gen, device=cuda_device)
+    grad = torch.empty(n, K, device=cuda_device)
+    even = torch.randint(0, n, (n // 2,), generator=gen, device=cuda_device)
+    near = n * 0.55 + n * 0.02 * torch.randn(n // 2, generator=gen, device=cuda_device)
+    near = near.long().clamp(0, n - 1)
+    best = {"even": 1e9, "near": 1e9}
+    for _ in range(12):
+        for name, ids in (("even", even), ("near", near)):
+            a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+            a.record()
+            _scatter(M, K, ids, rows, grad)
+            b.record()
+            b.synchronize()
+            best[name] = min(best[name], a.elapsed_time(b))
+    assert best["near"] < 2 * best["even"], best
 
 
 def test_query_backward_after_the_ids_were_written_to(cuda_device):
