@@ -804,7 +804,7 @@ static int launch_scatter(const svoxb_tree* tree, const int64_t* ids, int64_t Q,
                         reinterpret_cast<uintptr_t>(grad) % 16 == 0;
     int st;
     if (binned && sums_by_tiles(n_floats, K)) {
-        const TileLists t(n_slots, Q);
+        const TileLists t(n_slots, Q, sm_count());
         if (t.max_tiles <= kMaxTiles) return launch_tiled(ids, rows, K, grad, t, stream);
     }
     if (!binned) {

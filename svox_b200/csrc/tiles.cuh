@@ -11,7 +11,7 @@
 // surface.  So the buffer is first divided into equal RANGES of 2^shift rows, and each is cut into 1,
 // 2, 4 .. tiles, as many as bring a block no more than it can sort at a time.  (Cut by the average
 // alone, 14.7 M uniform points into a 1024^3 tree of three shells, 56 M rows of 28 floats, made tiles of
-// 33 000 items: 5.95 ms, now 2.22; 1.4 M points around one place of 400 MB of 76 floats: 0.84 -> 0.29.)
+// 33 000 items: 5.95 ms, now 2.22; 0.7 M points around one place of 400 MB of 76 floats: 0.84 -> 0.23.)
 //
 //   count    items per range; the last block cuts the ranges into tiles
 //   recount  items per tile, if any range was cut; the last block lists where each tile's begin, and
@@ -61,8 +61,14 @@ struct TileLists {
     size_t words() const {
         return zero_words() + 2 * up4(max_tiles) + up4(n_ranges) + up4(3 * (size_t)most_hot());
     }
-    TileLists(int64_t rows, int64_t items) : n_rows(rows), n_items(items) {
+    // Ranges have 2^kMaxTileShift rows, or fewer where the `sms` processors would not come to about two
+    // rounds of two blocks each with them: 0.5 M points into 1.05 M rows of 100 floats (256 ranges of
+    // 4096 rows) 295 us, 190 with 1024 ranges; 0.1 M into 0.21 M rows of 1000 floats 1254, 314; 0.5 M
+    // into 2.05 M of 128 (500 ranges) 424, 290.  From there on more ranges cost more than they gain (0.6 M
+    // into 2.4 M of 49: 585 ranges 178, 1170 ranges 192).
+    TileLists(int64_t rows, int64_t items, int sms) : n_rows(rows), n_items(items) {
         shift = kMaxTileShift;
+        while (shift > kMinTileShift && (rows >> shift) < 4 * (int64_t)sms - sms / 4) --shift;
         n_ranges = (int)(((rows - 1) >> shift) + 1);
         // A range is cut into 2^n tiles, n > 0, only with more than 2^(n-1) * kOwnItems items.
         const int64_t most = n_ranges + 2 * items / kOwnItems + 1;

@@ -370,6 +370,20 @@ def test_query_gradient_of_rows_at_any_address(K, offset, cuda_device):
     _scatter_is_exact(M, K, ids, rows[offset:].view(Q, K))
 
 
+def _fastest(calls):
+    """Shortest device time of each call, taken in turn."""
+    best = [float("inf")] * len(calls)
+    for _ in range(12):
+        for i, call in enumerate(calls):
+            a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            best[i] = min(best[i], a.elapsed_time(b))
+    return best
+
+
 def test_query_gradient_of_clustered_points_takes_no_longer(cuda_device):
     # (tiles cut by the average density: three times as long as for points spread evenly)
     K = 76
@@ -381,16 +395,25 @@ def test_query_gradient_of_clustered_points_takes_no_longer(cuda_device):
     even = torch.randint(0, n, (n // 2,), generator=gen, device=cuda_device)
     near = n * 0.55 + n * 0.02 * torch.randn(n // 2, generator=gen, device=cuda_device)
     near = near.long().clamp(0, n - 1)
-    best = {"even": 1e9, "near": 1e9}
-    for _ in range(12):
-        for name, ids in (("even", even), ("near", near)):
-            a, b = torch.cuda.Event(True), torch.cuda.Event(True)
-            a.record()
-            _scatter(M, K, ids, rows, grad)
-            b.record()
-            b.synchronize()
-            best[name] = min(best[name], a.elapsed_time(b))
-    assert best["near"] < 2 * best["even"], best
+    t_even, t_near = _fastest([lambda: _scatter(M, K, even, rows, grad),
+                               lambda: _scatter(M, K, near, rows, grad)])
+    assert t_near < 2 * t_even
+
+
+def test_query_gradient_of_half_the_size_takes_less_time(cuda_device):
+    # (with tiles of 4096 rows, too few for the device, nine tenths of it)
+    K = 100
+    gen = torch.Generator(cuda_device).manual_seed(1)
+    calls = []
+    for mb in (400, 800):
+        M = (mb << 20) // (32 * K)
+        Q = 4 * M
+        ids = torch.randint(0, 8 * M, (Q,), generator=gen, device=cuda_device)
+        rows = torch.randn(Q, K, generator=gen, device=cuda_device)
+        grad = torch.empty(8 * M, K, device=cuda_device)
+        calls.append(lambda M=M, ids=ids, rows=rows, grad=grad: _scatter(M, K, ids, rows, grad))
+    half, whole = _fastest(calls)
+    assert half < 0.8 * whole
 
 
 def test_query_backward_after_the_ids_were_written_to(cuda_device):
