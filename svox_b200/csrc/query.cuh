@@ -783,15 +783,38 @@ static int launch_tiled(const int64_t* ids, const float* rows, int K, float* gra
     return st;
 }
 
-// Which of the two a large gradient takes.  Summing by tiles costs 77 instructions per row whatever
-// its length and writes the gradient once; adding bin by bin costs a reduction per 16 bytes and
-// writes it twice into the L2.  Measured (us, bins / tiles): K = 4, 732 MB, 16 M points 790 / 1742;
-// K = 13, 524 MB, 2.7 M 375 / 401; K = 28, 127 MB, 0.3 M 82 / 135; 255 MB, 0.6 M 150 / 137, 4.2 M
-// 354 / 371; 1.13 GB, 2.7 M 589 / 476, 4.2 M 675 / 611; K = 49, 447 MB, 0.6 M 227 / 172, 4.2 M 502 /
-// 440; 3.58 GB, 5 M 1680 / 1082; K = 100, 914 MB, 1 M 497 / 319; K = 200, 909 MB, 0.5 M 491 / 478.
-static bool sums_by_tiles(int64_t n_floats, int K) {
-    const int64_t mb = n_floats >> 18;
-    return K > 32 ? mb >= 384 : K > 20 && mb >= 768;
+// Which of the two a large gradient takes.  Summing by tiles writes the gradient once, and costs
+// instructions per row of points (77 for 49 floats); adding bin by bin clears and adds in the L2, and
+// costs a reduction per 16 bytes, which eight lanes share for rows of up to 29 floats and sixteen from
+// there on.  So tiles need long rows, and points that fall on many different rows; the fewer points
+// per row and the larger the gradient, the shorter rows may be.  Measured (us, bins / tiles; points
+// spread over 7/8 of the rows, then 93 % of them in 3 % of the rows, as uniform points in a tree of
+// coarse and fine leaves, then around one place, +- 8 % of the rows):
+//
+//   floats, MB   0.26 points a row            0.5                          1                           2
+//   24, 1130     594/527  429/470  486/503    773/754  610/600  643/684    1116/1203 937/906 950/1023  1633/1873 1472/1476 1464/1604
+//   28,  400     224/199  170/208  188/248    282/277  222/235  243/295    390/423   317/331 322/393   549/617   495/513   483/558
+//   28,  800     435/347  304/329  350/365    538/485  414/415  451/485    758/783   629/586 641/668   1089/1184 991/970   973/1064
+//   28, 2050     1067/822 740/771  850/795    1339/1176 1056/986 1123/1090 1920/1885 1604/1455 1645/1612  2888/3076 2532/2529 2539/2710
+//   32,  400     200/194  190/176  183/243    248/267  244/213  234/284    358/381   357/289 342/351   579/558   586/442   554/501
+//   32, 1130     530/436  438/412  436/444    654/637  623/516  587/587    973/988   987/728 901/829   1600/1475 1626/1157 1497/1286
+//   49,  256     135/132  133/167  129/173    179/149  155/193  157/193    230/195   209/284 213/233   335/326   319/350   312/305
+//   49,  400     211/180  178/196  178/188    261/215  217/228  220/242    339/292   303/285 302/301   502/474   476/415   459/437
+//   49, 1130     585/385  385/412  434/413    692/487  520/518  548/501    879/746   805/663 789/692   1383/1131 1312/1049 1260/1082
+//   76,  400     218/157  183/238  183/212    266/187  222/239  226/243    359/243   313/269 311/286   510/415   496/365   477/382
+//  200,  400     184/151  188/209  166/156    244/175  238/208  228/202    328/227   292/252 290/292   462/317   402/413   410/415
+//  200,  800     371/251  310/271  304/273    475/307  370/331  385/367    639/409   492/462 529/496   885/603   753/599   779/645
+//  300,  400     189/156  222/265  175/185    271/189  227/260  224/242    357/242   305/338 309/352   500/333   424/453   431/462
+//
+// Around one place of +- 2 % tiles of up to 128 floats take at most 1.4 times as long as bins (400 MB, 0.26
+// points a row, 162 / 207), longer rows, which do not fit a warp's registers at once, more below 768 MB
+// (200 floats, 400 MB, 196 / 363; 2 GB 753 / 728).
+static bool sums_by_tiles(int64_t n_slots, int K, int64_t Q) {
+    const int64_t mb = n_slots * K >> 18;
+    if (K <= 24) return false;
+    if (K <= 29) return mb >= 768 && Q <= n_slots;
+    if (K <= 32) return mb >= 768;
+    return mb >= (K <= 128 || Q >= n_slots ? 384 : 768);
 }
 
 static int launch_scatter(const svoxb_tree* tree, const int64_t* ids, int64_t Q, const float* rows,
@@ -803,7 +826,7 @@ static int launch_scatter(const svoxb_tree* tree, const int64_t* ids, int64_t Q,
                         Q < (1LL << 31) - kBinRows && n_slots < (1LL << 31) &&
                         reinterpret_cast<uintptr_t>(grad) % 16 == 0;
     int st;
-    if (binned && sums_by_tiles(n_floats, K)) {
+    if (binned && sums_by_tiles(n_slots, K, Q)) {
         const TileLists t(n_slots, Q, sm_count());
         if (t.max_tiles <= kMaxTiles) return launch_tiled(ids, rows, K, grad, t, stream);
     }

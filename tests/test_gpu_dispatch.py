@@ -370,6 +370,19 @@ def test_query_gradient_of_rows_at_any_address(K, offset, cuda_device):
     _scatter_is_exact(M, K, ids, rows[offset:].view(Q, K))
 
 
+@pytest.mark.parametrize("K,mb", [(24, 768), (25, 767), (25, 768), (29, 768), (30, 767), (30, 768),
+                                  (33, 383), (33, 384), (128, 384), (129, 384), (129, 768)])
+@pytest.mark.parametrize("more", [0, 1])
+def test_query_gradient_where_the_rule_changes(K, mb, more, cuda_device):
+    # bins and tiles meet at these lengths and sizes, and at one point per row
+    M = -(-(mb << 20) // (32 * K))
+    gen = torch.Generator(cuda_device).manual_seed(K)
+    Q = 8 * M + more if K > 128 or K < 30 else 2 * M + more
+    ids = torch.randint(0, 8 * M, (Q,), generator=gen, device=cuda_device)
+    rows = torch.randint(-8, 9, (Q, K), generator=gen, device=cuda_device).float()
+    _scatter_is_exact(M, K, ids, rows)
+
+
 def _fastest(calls):
     """Shortest device time of each call, taken in turn."""
     best = [float("inf")] * len(calls)
