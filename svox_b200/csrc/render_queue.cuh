@@ -247,7 +247,6 @@ constexpr size_t bin_smem(int n_bins) {
     return (size_t)n_bins * (sizeof(uint32_t) + kOpenGroups * sizeof(uint64_t));
 }
 constexpr size_t kBinSmem = bin_smem(kMaxBins);
-constexpr int kBinStep = 16;      // the shared memory of a launch is for a multiple of so many bins
 template <int BD>
 constexpr int sorted_march_block() {
     // If it costs no more than a warp, within 196 KB, the next smaller split of an SM's memory,

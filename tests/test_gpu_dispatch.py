@@ -241,7 +241,7 @@ def test_launches_known_do_not_grow_with_the_trees(cuda_device):
             r(rays).sum().backward()
     finally:
         lib.svoxb_test_knob(5, 32)
-    # two kernels count tiles, one fills bins; each has at most a dozen steps
+    # three kernels count tiles, each in at most a dozen steps; one fills bins
     assert lib.svoxb_test_known_launches() - before <= 12
     csrc.check_device_status()
 
