@@ -57,9 +57,9 @@ struct UnitShared {
 // `work(first, end)` by all threads of the block.  With `clear_floats` > 0 (the length of the
 // outputs) bin b + 1, `bin_floats` floats, is cleared by `clear(from, until)` in units that come
 // before the items of bin b, the first bin before all; with `spread` they are spread over the first
-// two thirds of the bin's units instead, so that clearing and adding run side by side (scatter of 2^20
-// rays 1.90 -> 1.84 ms; where units are small they then hold up the next bin, `se_grad` of 100 000
-// rays 1.12 -> 1.28, an 800x800 view 1.26 -> 1.29).
+// two thirds of the bin's units instead, so that clearing and adding run side by side: worth while
+// where units are large, in the middle of the lengths that were tried, see the call in
+// render_replay.cuh.
 //
 // Units are taken by blocks in order from one counter, so that the grid works within a window
 // much smaller than a bin (with a fixed assignment the blocks drift apart and several bins compete

@@ -271,9 +271,14 @@ replay_scatter_kernel(TreeArgs tr, svoxb_render_options opt, int32_t* __restrict
             }
         }
     };
+    // Clearing is spread between the units of adding where these are large, and for records of up to 28
+    // floats.  Scatter alone (512^3 shell, us, before / between): 2^20 rays RGBA 935 / 938, SH4 1729 / 1719,
+    // SH9 1931 / 1891; views of 1000x1000 and 1600x1600 pixels, SH9, 915 / 887 and 1668 / 1635; but 2^19
+    // rays SH16 2156 / 2182, a view of 1200x1200 2183 / 2216.  Small units then hold up the next bin:
+    // 2^18 rays SH9 746 / 792, `se_grad` of 100 000 rays 1.12 / 1.28 ms.
     ordered_units<BLOCK>(s_units, counters, lo_bin, hi_bin, groups_before,
                          WARPS * per_warp / per_group, ((int64_t)1 << log[2]) * K,
-                         sorted ? to.zero_slots * K : 0, per_warp >= 4, count, clear, work);
+                         sorted ? to.zero_slots * K : 0, K <= 28 && per_warp >= 4, count, clear, work);
 }
 
 }  // namespace svoxb
