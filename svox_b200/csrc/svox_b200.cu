@@ -279,10 +279,18 @@ static int replay_scatter_block(const ReplayJob& job, int part, int reserve_sms,
     int st = persistent_grid(k, BLOCK, smem, job.chunks > clears ? job.chunks : clears, &grid);
     if (st) return st;
     // Two outputs to clear: with more than two blocks per SM the units of adding come round to a bin
-    // before it is cleared, and wait (`se_grad` of 100 000 rays, 1 / 2 / 3 / 4 / 6 blocks: 1.07, 1.00,
-    // 1.11, 1.12, 1.56 ms; one output: the 2^20-ray step 3.05, 2.05, 1.90, 1.90, 2.34).
+    // before it is cleared, and wait.  Measured (`se_grad`, 512^3 shell, 10.5 M records, ms with 2 / 3 / as
+    // many blocks as fit; 1 block is slower everywhere but for 45 000 rays of SH16, 1.86 against 1.91):
+    //            45 000 rays         100 000             300 000             2^20
+    //     RGBA   0.57 / 0.59 / 0.59  0.75 / 0.76 / 0.76  1.60 / 1.59 / 1.60  4.78 / 4.73 / 4.75
+    //     SH4    0.84 / 0.90 / 0.92  1.11 / 1.12 / 1.16  2.20 / 2.21 / 2.21  6.53 / 6.39 / 6.40
+    //     SH9    1.20 / 1.43 / 1.43  1.58 / 1.70 / 1.70  2.98 / 2.98 / 2.98  7.76 / 7.84 / 7.86
+    //     SH16   1.91 / 1.91 / 1.91  2.50 / 2.50 / 2.50  4.40 / 4.40 / 4.40
+    // So two, or three where many samples (64 a ray) come to a short record.  One output: the 2^20-ray
+    // step with 1 / 2 / 3 / 4 / 6 blocks 3.05, 2.05, 1.90, 1.90, 2.34.
     if (HESS && job.to.grad != nullptr && job.to.zero_slots > 0) {
-        const int64_t most = 2LL * (sm_count() - g_reserved_sms);
+        const bool many = K <= 13 && 32 * job.chunks > 4 * job.to.zero_slots;
+        const int64_t most = (many ? 3LL : 2LL) * (sm_count() - g_reserved_sms);
         if ((int64_t)grid > most && most > 0) grid = (unsigned)most;
     }
     if (reserve_sms > 0) {
