@@ -12,9 +12,9 @@
 //            kWordWalk                  the tree goes deeper here: walk `child`
 //            negative (table only)      kWordBrick | brick id
 //   word 1   bits 28-31: the leaf's depth; bits 0-27: its slot.  kWordWalk: the node to walk on
-//            from, in bits 28-31 the depth of its children, or 0: walk from the root.  (Trees of 34 M nodes or more, which get no bricks, and cells
-//            beyond the last brick; 200 000 rays through 34.2 M nodes: 9.2 ms if all walk from
-//            the root.)
+//            from, in bits 28-31 the depth of its children, or 0: walk from the root.  (Trees
+//            of 34 M nodes or more, which get no bricks, and cells beyond the last brick;
+//            200 000 rays through 34.2 M nodes: 9.2 ms if all walk from the root.)
 // so that one 8-byte load per sample brings all that the march needs of a leaf.
 //
 // Built per call (`data` can change between any two): one thread per table cell, then one per

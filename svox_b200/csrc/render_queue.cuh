@@ -222,8 +222,18 @@ constexpr int kMarchBlock = 128;
 constexpr int kMarchBlocks = 6;
 
 // A batch of few rays (march_shape leaves no more than kSpreadWarps warps per SM with work) goes
-// through blocks of this size, compiled for 16 warps per SM and thus 128 registers: 65536 rays of
-// an RGBA tree 175 -> 157, 4096 rays of the 512^3 shell 237 -> 204 us.
+// through blocks of this size, compiled for 16 warps per SM and thus 128 registers; the march of 4096
+// rays of the 512^3 shell, SH9, takes 204 us instead of 237.  The whole call, us, blocks of 128 / of 64
+// (512^3 shell, rendering alone; the line is at 75 776 rays):
+//            4096 rays   20 000      50 000      75 000      100 000     140 000
+//     RGBA   280 / 273   310 / 298   334 / 335   349 / 345   379 / 358   454 / 469
+//     SH4    306 / 298   343 / 331   383 / 373   400 / 381   413 / 495   552 / 536
+//     SH9    325 / 313   373 / 354   404 / 385   425 / 398   461 / 531   608 / 636
+//     SH16   338 / 322   394 / 359   456 / 417   487 / 467   630 / 614   724 / 734
+// Beyond the line a warp's 32 lanes all have rays and 16 warps are too few of them; up to it all
+// formats gain, images too (224x224 to 272x272 pixels 1 to 2 %).  Logged, with the backward: SH4
+// and SH9 7 to 10 % (128^3), SH16 level to 6 %, SH25 level to 2 %, whose kernel has 121 to 128 registers
+// either way: there the smaller blocks only share rays out more evenly.
 constexpr int kFewBlock = 64;
 constexpr int kSpreadWarps = 16;
 
@@ -249,12 +259,14 @@ constexpr size_t bin_smem(int n_bins) {
 constexpr size_t kBinSmem = bin_smem(kMaxBins);
 template <int BD>
 constexpr int sorted_march_block() {
-    // If it costs no more than a warp, within 196 KB, the next smaller split of an SM's memory,
-    // which leaves 60 KB of L1 instead of 28 (SH16: 19 warps instead of 20, logged 800x800 view 1.26
-    // -> 1.21 ms; SH25 stays at 15 warps, 13 took 417 us instead of 387 for a 640x640 view).
+    // If it costs no more than a warp, within 196 KB with half of the bins, the next smaller split of an
+    // SM's memory, which leaves 60 KB of L1 instead of 28 (SH16 with 62 bins: 19 warps instead of 20,
+    // logged 800x800 view 1.26 -> 1.21 ms; SH25 stays at 15 warps, 13 took 417 us instead of 387 for a
+    // 640x640 view).
     constexpr size_t one = sizeof(WarpQueue<BD, kModeForwardLogged>);
     const int warps = 4 * march_blocks_per_sm<BD, kModeForwardLogged>();
-    int most = (int)((227 * 1024 - 1024 - kBinSmem) / one), fit = (int)((196 * 1024 - 1024 - kBinSmem / 2) / one);
+    int most = (int)((227 * 1024 - 1024 - kBinSmem) / one);
+    const int fit = (int)((196 * 1024 - 1024 - kBinSmem / 2) / one);
     if (most > warps) most = warps;
     return 32 * (fit < most - 1 ? most : fit < most ? fit : most);
 }
@@ -818,9 +830,12 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         // scale).  The point lies inside, so the entry distance is 0 and per axis the larger of
         // t1 = -f*inv and t1 + inv is t1 + max(inv, 0); powers of two commute with rounding, so
         // everything can be done at the tree's scale.
-        const float ex = __fmaf_rn(MAXES ? mx : fmaxf(r.ix, 0.f), inv_cube, __fmul_rn(__fsub_rn(cx, px), r.ix));
-        const float ey = __fmaf_rn(MAXES ? my : fmaxf(r.iy, 0.f), inv_cube, __fmul_rn(__fsub_rn(cy, py), r.iy));
-        const float ez = __fmaf_rn(MAXES ? mz : fmaxf(r.iz, 0.f), inv_cube, __fmul_rn(__fsub_rn(cz, pz), r.iz));
+        const float ex = __fmaf_rn(MAXES ? mx : fmaxf(r.ix, 0.f), inv_cube,
+                                   __fmul_rn(__fsub_rn(cx, px), r.ix));
+        const float ey = __fmaf_rn(MAXES ? my : fmaxf(r.iy, 0.f), inv_cube,
+                                   __fmul_rn(__fsub_rn(cy, py), r.iy));
+        const float ez = __fmaf_rn(MAXES ? mz : fmaxf(r.iz, 0.f), inv_cube,
+                                   __fmul_rn(__fsub_rn(cz, pz), r.iz));
         const float delta_t = __fadd_rn(fminf(ex, fminf(ey, ez)), opt.step_size);
         if (on) {
             t = __fadd_rn(t, delta_t);

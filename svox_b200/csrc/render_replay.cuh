@@ -11,9 +11,9 @@
 //
 // Where every leaf is touched several times by rays far apart in time, each touch would miss L2
 // and cost a read and a write of DRAM (20 GB for 2^20 rays of the 512^3 shell scene, 4.5 ms
-// against 1.87 with the clearing, see below).  There the forward sorts its packets into BINS, ranges of leaf slots whose
-// gradient spans some tens of MB, and `order` lists the groups of packets bin by bin: all SMs
-// work on the same few bins at a time.  The kernel then also clears the gradient, one bin ahead
+// against 1.87 with the clearing, see below).  There the forward sorts its packets into BINS, ranges
+// of leaf slots whose gradient spans some tens of MB, and `order` lists the groups of packets bin by
+// bin: all SMs work on the same few bins at a time.  The kernel then also clears the gradient, one bin ahead
 // of the scatter: the zeros are still in L2 when the packets are added, so a gradient line is
 // written to DRAM once and never read (clearing first costs another write, and a read of every
 // line touched).  Bound then: L2 atomics, 4.5 sectors per 112-byte record.

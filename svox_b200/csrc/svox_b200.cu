@@ -159,7 +159,8 @@ static int replay_bins(int64_t M, int K) {
 
 // Whether a logged forward sorts its items into bins: when the gradient outgrows a bin and a
 // good part of it is touched (64 contributing samples per ray of a random batch, 24 per pixel,
-// against the leaf slots: the averages of the 512^3 shell scene, the only one measured).  Then the scatter finds the gradient in L2 and clears it on the way.
+// against the leaf slots: the averages of the 512^3 shell scene, the only one measured).  Then the
+// scatter finds the gradient in L2 and clears it on the way.
 // (A log of 2^26 chunks, 100 GB, or more is not sorted: no such size has been run.)
 static bool sorts_log(const svoxb_tree* t, int64_t rays, bool image, int64_t capacity) {
     if (capacity / kSortedChunks >= 0xffffff || replay_bins(t->M, t->K) < 2) return false;

@@ -140,8 +140,8 @@ __device__ __forceinline__ bool last_block(int32_t* done) {
 
 // Lists where the tiles' items begin; one block.  A tile's items are one unit of work, unless it is
 // HOT: then every kOwnItems of them are, so that the device shares in them, and what they add goes
-// into a cleared tile.  `counted`: items per tile.  With many items per row (the leaf that a camera stands in) the reductions for
-// that are few; else it is the lesser evil.
+// into a cleared tile.  With many items per row (the leaf that a camera stands in) the reductions for
+// that are few; else it is the lesser evil.  `counted`: items per tile.
 template <int BLOCK>
 __device__ __forceinline__ void list_tiles(const TileLists& t, const int32_t* counted) {
     __shared__ int s_sum[BLOCK / 32];
@@ -279,15 +279,14 @@ struct TileSort {
         }
         __syncthreads();
     }
-    // Writes zeros to the rows [0, n_rows) of `out` that have no item.
+    // Writes zeros to the rows [0, n_rows) of `out`, 16-byte aligned, that have no item.
     __device__ __forceinline__ void clear_empty(int n_rows, int K, float* __restrict__ out) const {
         const int lane = threadIdx.x & 31;
-        const bool vec_ok = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
         for (int r0 = threadIdx.x & ~31; r0 < n_rows; r0 += kOwnBlock) {
             const int r = r0 + lane;
             unsigned none = __ballot_sync(0xffffffffu, r < n_rows && upto(r) == upto(r - 1));
             float* __restrict__ to = out + (int64_t)r0 * K;
-            if (none == 0xffffffffu && vec_ok) {
+            if (none == 0xffffffffu) {
                 for (int i = lane; i < 8 * K; i += 32)
                     reinterpret_cast<float4*>(to)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             } else {
