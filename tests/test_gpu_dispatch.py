@@ -134,6 +134,38 @@ def test_se_grad_through_either_log_and_without(fmt, n, cuda_device):
     csrc.check_device_status()
 
 
+@pytest.mark.parametrize("fmt", ["SH4", "SH16"])
+@pytest.mark.parametrize("n", [200, 30000])
+@pytest.mark.parametrize("at", [(0, 0), (0, 1), (2, 0), (3, 1)])
+def test_se_grad_into_buffers_of_different_alignment(fmt, n, at, cuda_device):
+    # both results are expanded through the same rows of shared memory, shifted to their words
+    # (records of whole 16-byte words have to lie on them: SVOXB_ERR_FORMAT)
+    import ctypes as C
+    tree = _shell(fmt, 4, 3, cuda_device)
+    r, rays = svox.VolumeRenderer(tree), _rays(n, cuda_device)
+    spec, src, opt = tree._spec(), _render._rays_spec_from_rays(rays), r._get_options()
+    resid = torch.randn(n, 3, generator=torch.Generator(cuda_device).manual_seed(3),
+                        device=cuda_device)
+    r.se_grad(rays, resid)
+    csrc.log_estimate(wait=True)            # the next log is large enough
+    out, (log, cap) = csrc.volume_render_logged(spec, src, opt)
+    used = csrc.log_chunks_used(log)
+    assert used <= cap
+    want = r.se_grad(rays, out - resid)[1:]
+    size = tree.data.numel()
+    got = [torch.full((size + 8,), float("nan"), device=cuda_device) for _ in at]
+    ct, cr, co = csrc._pack_tree(spec), csrc._pack_rays(src, tree.data.device), opt._pack()
+    assert csrc.library().svoxb_se_grad_replay(
+        C.byref(ct), C.byref(cr), C.byref(co), C.c_void_p(resid.data_ptr()),
+        C.c_void_p(out.data_ptr()), C.c_void_p(log.data_ptr()), C.c_int64(cap), C.c_int64(used),
+        *[C.c_void_p(g.data_ptr() + 4 * k) for g, k in zip(got, at)], C.c_int(1),
+        C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    for g, k, w in zip(got, at, want):
+        assert _close(g[k:k + size], w.reshape(-1))
+        assert g[:k].isnan().all() and g[k + size:].isnan().all()
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("n", [40, 12000])
 def test_backward_twice_over_one_forward(n, cuda_device):
     # a gradient cleared beside the forward is handed out once; a sorted log is replayed twice
