@@ -138,10 +138,15 @@ query_kernel(TreeArgs tr, TopTable top, const float* __restrict__ pts, int64_t Q
 
 // The same for records of up to kStagedRow floats, through shared memory: `per` rows of a warp at a
 // time are requested with cp.async, as 16-byte words where records are aligned (VEC), else as
-// floats, and leave as one stretch in 16-byte words.  All rows of a warp are under way at once, and a
-// quarter of the requests are made.  Measured (2^22 points, us; row by row / staged): 28 floats 300 /
-// 253, 76 floats 484 / 480, 101 floats 1130 / 657, 200 floats 1510 / 1253; as single floats 49 floats
-// 344 / 395, 13 floats 136 / 144: those go row by row.
+// floats, and leave as one stretch in 16-byte words.  `per` rows of a warp are under way at once, 32 up
+// to 28 floats and 4 of more than 112, and as 16-byte words a quarter of the requests are made.
+// Measured (2^22 points, us; row by row / staged):
+//   words    8 floats 99 / 103, 12: 130 / 127, 16: 142 / 132, 20: 266 / 174, 28: 304 / 251, 76: 483 / 478,
+//            100: 1050 / 606, 128: 685 / 606; 4 (RGBA) 76 / 78
+//   floats   13 floats 136 / 144, 49: 344 / 395, 97: 1202 / 730, 129: 1477 / 840, 144: 939 / 888, 160: 893
+//            / 950, 192: 1101 / 1099, 200: 1512 / 1255, 208: 1424 / 1280, 223: 2752 / 1378, 224: 1304 / 1338
+// So records up to 8 floats, unaligned ones up to 96, and long ones of a multiple of 32 floats, which
+// fill every request of a warp, go row by row.
 constexpr int kStagedRow = 224;
 constexpr int kStagedFloats = 896;       // per warp
 template <int G, int STEPS, bool VEC>
@@ -298,11 +303,11 @@ static int launch_query(const svoxb_tree* tree, const float* indices, int64_t Q,
     if (rows != nullptr)
         assign_kernel<<<grid, kQueryBlock, 0, stream>>>(tree_args(tree), tt, indices, Q, rows,
                                                         data_out, Kv);
-    else if (values_out == nullptr || K > kStagedRow) forward(query_kernel<32, 0>);
-    else if (vec && K <= 4) staged(query_staged_kernel<1, 1, true>);
-    else if (vec && K <= 16) staged(query_staged_kernel<4, 1, true>);
-    else if (vec && K <= 32) staged(query_staged_kernel<8, 1, true>);
-    else if (vec && K <= 128) staged(query_staged_kernel<32, 1, true>);
+    else if (values_out == nullptr || K > kStagedRow || (K > 128 && K % 32 == 0))
+        forward(query_kernel<32, 0>);
+    else if (vec && K > 8 && K <= 16) staged(query_staged_kernel<4, 1, true>);
+    else if (vec && K > 16 && K <= 32) staged(query_staged_kernel<8, 1, true>);
+    else if (vec && K > 32 && K <= 128) staged(query_staged_kernel<32, 1, true>);
     else if (K <= 2) forward(query_kernel<2, 1>);
     else if (K <= 4) forward(query_kernel<4, 1>);
     else if (K <= 8) forward(query_kernel<8, 1>);

@@ -213,7 +213,7 @@ def test_query_rows_of_any_length(K, N, cuda_device):
     csrc.check_device_status()
 
 
-@pytest.mark.parametrize("K", [4, 12, 28, 32, 36, 76, 128, 132, 224, 225])
+@pytest.mark.parametrize("K", [4, 8, 12, 28, 32, 36, 76, 128, 132, 160, 220, 224, 225])
 def test_query_values_through_shared_memory(K, cuda_device):
     # records that are copied as 16-byte words, longer ones as floats, and those that go row by row;
     # into results that lie on a 16-byte boundary and beside one
