@@ -56,14 +56,14 @@ METRICS = {
     "image5": "Mrays/s render_persp forward (SH deg 3, three shells at 1024^3, 1920x1080 views)",
 }
 # DRAM bytes (read + write) of one launch of the training step's kernels: the logged march from an
-# ncu capture of a 2^17-ray launch (1.658 GB read + 0.383 GB written), scaled by 8 because its
+# ncu capture of a 2^17-ray launch (1.661 GB read + 0.383 GB written), scaled by 8 because its
 # traffic grows with the rays; the scatter's does not (the gradient is written once whatever the
 # number of rays), so no scaled figure is given for it.  Printed only together with
 # `traffic_source`, which names the capture.
-NCU_TRAFFIC = {"forward": 8 * (1.658214e9 + 0.382567e9), "backward": None}
-NCU_TRAFFIC_SOURCE = ("ncu --set full of render_queue_kernel<9,2,768> at 2^17 rays x 8 "
+NCU_TRAFFIC = {"forward": 8 * (1.661109e9 + 0.382764e9), "backward": None}
+NCU_TRAFFIC_SOURCE = ("ncu of render_queue_kernel<9,2,768> at 2^17 rays x 8 "
                       "(profiles/training_step_rays131072_ncu_full.md); valid for the kernel as "
-                      "of library version " + "0.4.1")
+                      "of library version " + "0.4.3")
 
 
 def parse():
@@ -775,7 +775,7 @@ def run_query(a):
                      "frac": fwd_bytes / ms_fwd / 1e6 / peak, "traffic": None,
                      "peak_source": peak_src, "ms_per_launch": ms_fwd,
                      "algorithmic_bytes_per_launch": fwd_bytes},
-        "roofline_backward": {"bound": "hbm", "kernel": "sorting + scatter_binned_rows_kernel "
+        "roofline_backward": {"bound": "hbm", "kernel": "sorting + own_rows_kernel "
                                                         "(query_vertical_backward)",
                               "achieved": (bwd_bytes + fill_bytes) / ms_bwd / 1e6, "peak": peak,
                               "unit": "GB/s",
@@ -783,7 +783,8 @@ def run_query(a):
                               "ms_per_launch": ms_bwd,
                               "algorithmic_bytes_per_launch": bwd_bytes,
                               "zero_fill_bytes": fill_bytes, "traffic": None},
-        "e2e": e2e, "gpu_launches": 5 * a.steps, "clocks": clocks,
+        # table, query; count, recount (returns at once where no range was cut), place, sums
+        "e2e": e2e, "gpu_launches": 6 * a.steps, "clocks": clocks,
     }
     if rank == 0 and world == 1 and not a.no_cpu_baseline:
         val, ms, info = cpu_arm(a, 2, 1, budget_s=20.0)

@@ -553,8 +553,8 @@ constexpr int kStageWords = 104;     // 16-byte words of rows a warp has under w
 // the row being summed (N of them; further columns in further passes).  Rows come in as the 16-byte
 // words that cover them, a stage of some rows ahead of the one being summed; finished rows, and
 // zeros between them, leave through a StreamWriter.  2^24 rows of 49 floats into 3.76 GB: 2.41 ms
-// with the gradient cleared and added to bin by bin, 1.78 so.  Bound: issue slots (82 % used, 77
-// instructions per row); without the stores it takes 0.95 ms, and 2.05 with a row's floats stored
+// with the gradient cleared and added to bin by bin, 1.78 so.  Bound: issue slots (79 % used, 69
+// instructions per row in a capture of 2^22 rows); without the stores it takes 0.95 ms, and 2.05 with a row's floats stored
 // one by one; unrolled by the row it outgrew the instruction cache (4.6 ms).
 template <int N>
 __global__ void __launch_bounds__(kOwnBlock, 2)
@@ -788,7 +788,7 @@ static int launch_tiled(const int64_t* ids, const float* rows, int K, float* gra
 }
 
 // Which of the two a large gradient takes.  Summing by tiles writes the gradient once, and costs
-// instructions per row of points (77 for 49 floats); adding bin by bin clears and adds in the L2, and
+// instructions per row of points (69 for 49 floats); adding bin by bin clears and adds in the L2, and
 // costs a reduction per 16 bytes, which eight lanes share for rows of up to 29 floats and sixteen from
 // there on.  So tiles need long rows, and points that fall on many different rows; the fewer points
 // per row and the larger the gradient, the shorter rows may be.  Measured (us, bins / tiles; points

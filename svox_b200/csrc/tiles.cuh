@@ -11,7 +11,7 @@
 // surface.  So the buffer is first divided into equal RANGES of 2^shift rows, and each is cut into 1,
 // 2, 4 .. tiles, as many as bring a block no more than it can sort at a time.  (Cut by the average
 // alone, 14.7 M uniform points into a 1024^3 tree of three shells, 56 M rows of 28 floats, made tiles of
-// 33 000 items: 5.95 ms, now 2.22; 0.7 M points around one place of 400 MB of 76 floats: 0.84 -> 0.23.)
+// 33 000 items: 5.95 ms, now 2.22; 0.7 M points around one place of 400 MB of 76 floats: 0.84 -> 0.25.)
 //
 //   count    items per range; the last block cuts the ranges into tiles
 //   recount  items per tile, if any range was cut; the last block lists where each tile's begin, and
