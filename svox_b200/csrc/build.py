@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "svox_b200.cu")
 LIB = os.path.join(HERE, "libsvox_b200.so")
 DEPS = ["svox_b200.cu", "common.cuh", "arith.cuh", "host.cuh", "binned.cuh", "tiles.cuh", "query.cuh", "render.cuh", "render_index.cuh",
-        "render_queue.cuh", "render_replay.cuh", "noalloc.cuh", "collective.cuh", "open_groups.h",
+        "render_queue.cuh", "render_back.cuh", "render_replay.cuh", "noalloc.cuh", "collective.cuh", "open_groups.h",
         os.path.join("..", "..", "include", "svox_b200.h")]
 
 

@@ -205,6 +205,10 @@ struct RayBatch {  // render_ray_kernel's inputs (svox/csrc/rt_kernel.cu:717-733
 
     // The order in which the queue kernels take the rays: ticket -> ray, for `tickets` tickets.
     static int64_t tickets(const RayBatch&, int64_t n_rays) { return n_rays; }
+    // Makes the compiler take the arguments as new, so that it computes from them in place.
+    __device__ __forceinline__ void pin() {
+        asm volatile("" : "+l"(origins), "+l"(dirs), "+l"(vdirs));
+    }
     __device__ __forceinline__ int64_t pick(int64_t ticket) const { return ticket; }
 
     __device__ __forceinline__ void load(int64_t i, const TreeArgs& tr,
@@ -232,6 +236,9 @@ struct PixelRays {  // render_image_kernel's inputs (svox/csrc/rt_kernel.cu:758-
     // words.  Tickets of a tile that hang over the image's edge yield no ray (-1).
     static int64_t tickets(const PixelRays& p, int64_t) {
         return 32 * (int64_t)((p.width + 7) / 8) * ((p.height + 3) / 4);
+    }
+    __device__ __forceinline__ void pin() {
+        asm volatile("" : "+l"(c2w), "+f"(fx), "+f"(fy), "+r"(width), "+r"(height));
     }
     __device__ __forceinline__ int64_t pick(int64_t ticket) const {
         const int64_t tile = ticket >> 5;

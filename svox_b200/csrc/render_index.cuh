@@ -66,6 +66,16 @@ struct TreeIndex {
     const int2* table = nullptr;      // (2^level)^3 entries, z fastest, at the start
     uint32_t bricks = 0;              // from this entry on: kBrickCells per brick
     int level = 0;
+    // What a march needs of the level, worked out here once: a number whose last place is the side
+    // of a brick's cell, the place of a table cell among such cells, and the table's row length.
+    float fine = 0.f;
+    uint32_t cell_mask = 0, row = 0;
+
+    static TreeIndex at(const int2* table, uint32_t bricks, int level) {
+        const int finest = level + kBrickLevels;
+        return TreeIndex{table, bricks, level, (float)(1 << (kPosBits - finest)),
+                         ((1u << level) - 1u) << kBrickLevels, 1u << level};
+    }
 };
 
 // One density out of its record.  Without the 64-byte hint the L2 fetched 128 bytes for each of
@@ -221,7 +231,7 @@ struct IndexLayout {
         return of(M, bricks < 0 ? 0 : bricks < max_bricks ? (int)bricks : max_bricks);
     }
     TreeIndex view(const int32_t* mem) const {
-        return TreeIndex{reinterpret_cast<const int2*>(mem), (uint32_t)(bricks / 2), level};
+        return TreeIndex::at(reinterpret_cast<const int2*>(mem), (uint32_t)(bricks / 2), level);
     }
 };
 

@@ -1,34 +1,42 @@
 // Queue-based warp-cooperative volume rendering for octrees (N = 2) whose records hold three
-// colour channels: K = 3 * basis_dim + 1 floats, or RGBA with K = 4 (BD = 0 here).  Forward,
-// forward with an item log, and backward in one or two marches.
+// colour channels: K = 3 * basis_dim + 1 floats, or RGBA with K = 4 (BD = 0 here).  Forward, and
+// forward with an item log (the marching backward: render_back.cuh).
 //
 //   G step  one lane = one ray.  Every iteration takes one SAMPLE per lane: the leaf is found
 //           by one table look-up, or one brick look-up below it (render_index.cuh), whose entry
 //           already holds the leaf's density, so the march itself reads L2-resident index
-//           entries only.  A contributing sample is pushed as an ITEM (leaf slot, step length,
-//           density, owner) into the warp's queue in shared memory.
+//           entries only.  A contributing sample is pushed as an ITEM (leaf slot, optical depth,
+//           owner) into the warp's queue in shared memory.
 //   S step  one lane = one item.  When 32 items are queued their records are requested with
 //           cp.async (coalesced 16-byte words, global -> shared staging rows) and the warp
 //           goes on marching; the batch is evaluated when the next one is full, by which time
 //           the data has arrived.  Lane i evaluates item i (attenuation, dot products with the
 //           owner ray's colour basis, sigmoids); then every owner folds the results of its own items into
 //           its ray's transmittance and sums in march order, which keeps the reference's order of accumulation
-//           (svox/csrc/rt_kernel.cu:282-295, 379-411, 442-471) whatever the batches are.  In
-//           the backward pass lane i forms the gradient of record i in its staging row and the
-//           warp flushes the rows with red.global.add.v4.f32, 16 bytes per lane.
+//           (svox/csrc/rt_kernel.cu:282-295) whatever the batches are.
 //
-// Bound: issue slots where neighbouring rays share records (images: 63 % of the slots used), DRAM
+// Bound: issue slots where neighbouring rays share records (images: 60 % of the slots used), DRAM
 // too where every sample's record misses (rays in random order: 16 GB for 2^20 rays of the 512^3
 // shell scene).  So the march is kept short: an 800x800 view of the shell scene with SH16 records takes
-// 0.583 G warp instructions for 2.28 M iterations and 0.49 M batches of items (0.603 G with the leaf's
-// corner from masks, when an iteration was 138 of them, a batch 540, and 259 with SH9).  The
-// position's bits and the leaf's corner come from truncating additions instead of conversions, the leaf's
-// exit distance needs five operations per axis, lanes between samples compute along instead of
-// branching, what only items need is done where all lanes have one, the index entry of a sample
-// is requested one iteration ahead so that the queue's work covers its latency, and a block holds
-// four warps so that shared memory and the L1 can be balanced (kMarchBlocks).  Per 800x800 view of
-// the shell scene with SH16 records 1.64 -> 1.01 ms; logged forward of 2^20 rays, SH9, 4.09 -> 3.31;
-// 65536 rays of an RGBA tree, forward and backward, 1.6 -> 0.25 (they took the generic kernels).
+// 0.500 G warp instructions for 2.28 M iterations and 0.49 M batches of items.  The leaf's corner
+// comes from truncating additions, its exit distance from five operations per axis, two axes to
+// an instruction; lanes between samples compute along instead of branching; the index entry of a
+// sample is requested one iteration ahead so that the queue's work covers its latency; and a block holds
+// four warps so that shared memory and the L1 can be balanced (kMarchBlocks).
+//
+// What the march's instructions were, and what became of them (0.583 G before; a tenth of them were
+// branches and their reconvergence, another tenth constants and addresses worked out again):
+//  - the early stop summed as optical depth, where it was an exponential and a branch per sample;
+//  - one word for a lane's state and the samples it has left; seldom cases behind one vote;
+//  - items in one or two stores; the product of length and density formed by the march's lanes;
+//  - index entries addressed in bytes, by masks that the host works out;
+//  - nothing of a ray's set-up or of the log's layout kept in registers through the march (the
+//    compiler moved it out of the loop, then spilled: the logged SH9 march 16 % slower), and the
+//    lane, the queue's place and the policy not worked out again.
+// us before and after, whole call: 800x800 view, SH16 1145 and 1052, SH4 858 and 765, SH9 with
+// thresholds 761 and 671; 65536 RGBA rays with gradient 234 and 213; 2^20 SH9 rays with gradient
+// 5743 and 5583 (bound by memory); four 1080p views of the 1024^3 scene 20.4 and 19.0 ms.  (Dot
+// products with two coefficients per instruction: level for SH9 to SH25, 9 % slower for RGBA.)
 //
 // Lanes whose ray has ended wait until `refill` of them do; then the queue is drained, their
 // results are written and they take new rays from a block-wide ticket counter together (the
@@ -44,7 +52,6 @@
 namespace svoxb {
 
 constexpr int kModeForward = 0;
-constexpr int kModeBackward = 1;
 constexpr int kModeForwardLogged = 2;  // forward that also records its items for the backward
 
 // Floats per record of a colour basis size (0: RGBA).
@@ -136,6 +143,16 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, uint64_
                  "l"(gmem), "l"(pol)
                  : "memory");
 }
+// a - b, both halves in one instruction.
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, d;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+        "sub.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
 // Adds the 16-byte word `word` of a gradient row to its place.  The row holds the record's K
 // floats from offset `off` on, zeros around them; `rec` is the record's first float.  With a
 // gradient buffer that is not 16-byte aligned the record's floats go one by one.
@@ -165,25 +182,53 @@ __device__ __forceinline__ int record_offset(const float* base, uint32_t slot) {
 template <int BD, int MODE>
 struct alignas(16) WarpQueue {
     static constexpr int K = RecordLength<BD>::K;
-    static constexpr bool BWD = MODE == kModeBackward;
     static constexpr bool LOG = MODE == kModeForwardLogged;
     using Shape = RecordShape<K>;
     // two batches: items being collected, and what spills over (the batch in flight lies in
     // registers; a queue of 96 items left the SH16 forward 28 KB of L1 instead of 60, 1.10 ms per
     // 800x800 view instead of 1.05)
     static constexpr int CAP = 64;
-    // per ray: colour basis, upstream gradient or view direction, delta_scale; odd stride: no
-    // bank conflicts
-    static constexpr int SCALE = BD + (BWD || LOG ? 3 : 0);
-    static constexpr int RAYW = (SCALE + 1) | 1;
+    // per ray: colour basis and, for the log, the view direction; odd stride: no bank conflicts
+    // among different owners (which 16-byte reads of the basis would have)
+    static constexpr int RAYW = (BD + (LOG ? 3 : 0)) | 1;
+    // An item in words: slot, optical depth (step length * delta_scale * density), owner lane and, for
+    // the log, step length * delta_scale.  With the latter it goes as one 16-byte word, else as an
+    // 8-byte and a 4-byte one (with 16 bytes the SH16 forward's five blocks would no longer leave
+    // 60 KB of L1).  For 25 logged functions the owner is a byte: with more a fourth block would
+    // not fit the SM.
+    static constexpr bool BYTE = LOG && BD == 25;
+    static constexpr bool WIDE = LOG && !BYTE;
+    struct Item {
+        uint32_t slot;
+        float depth, length;
+        int owner;
+    };
     // Staging rows (cp.async targets).  After lane i has read row i it reuses the
     // row's first words for the item's results.
     alignas(16) float rows[32 * Shape::STRIDE];
-    uint32_t slot[CAP];
-    float dt[CAP];                     // step length
-    float sigma[CAP];
-    unsigned char owner[CAP];          // bits 0-4 owner lane, bit 7 accumulation march
+    alignas(16) uint32_t items[CAP * (WIDE ? 4 : 3)];
+    unsigned char owners[BYTE ? CAP : 1];
     float rayv[32][RAYW];
+
+    __device__ __forceinline__ void put(int i, const Item& x) {
+        const uint32_t depth = __float_as_uint(x.depth), length = __float_as_uint(x.length);
+        if (WIDE) {
+            reinterpret_cast<uint4*>(items)[i] = make_uint4(x.slot, depth, length, x.owner);
+        } else {
+            reinterpret_cast<uint2*>(items)[i] = make_uint2(x.slot, depth);
+            items[2 * CAP + i] = BYTE ? length : x.owner;
+            if (BYTE) owners[i] = (unsigned char)x.owner;
+        }
+    }
+    __device__ __forceinline__ Item get(int i) const {
+        if (WIDE) {
+            const uint4 w = reinterpret_cast<const uint4*>(items)[i];
+            return {w.x, __uint_as_float(w.y), __uint_as_float(w.z), (int)w.w};
+        }
+        const uint2 w = reinterpret_cast<const uint2*>(items)[i];
+        const uint32_t v = items[2 * CAP + i];
+        return {w.x, __uint_as_float(w.y), BYTE ? __uint_as_float(v) : 0.f, BYTE ? owners[i] : (int)v};
+    }
 };
 
 // Marks the table cells that the rays pass, at points a quarter of a cell apart: for a few rays
@@ -212,7 +257,8 @@ mark_cells_kernel(TreeArgs tr, Source src, svoxb_render_options opt, int64_t tic
     }
 }
 
-enum { kNeedRay = 0, kMarching = 1, kEnded = 2, kExhausted = 3 };
+// State of a lane: the samples its ray may still take (marching), or one of these.
+enum { kMarching = 1, kCapped = 0, kNeedRay = -1, kEnded = -2, kExhausted = -3 };
 
 constexpr int kMarchBlock = 128;
 
@@ -302,18 +348,13 @@ __global__ void
 __launch_bounds__(BLOCK, BLOCK == kMarchBlock ? march_blocks_per_sm<BD, MODE>()
                          : BLOCK == kFewBlock ? few_blocks_per_sm<BD, MODE>() : 1)
 render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex index,
-                    int64_t tickets, float* __restrict__ out,
-                    const float* __restrict__ grad_out, const float* __restrict__ fwd_out,
-                    float* __restrict__ grad_data, LogArgs lg, MarchShape shape) {
+                    int64_t tickets, float* __restrict__ out, LogArgs lg, MarchShape shape) {
     constexpr int K = RecordLength<BD>::K;
-    constexpr bool BWD = MODE == kModeBackward;
     constexpr bool LOG = MODE == kModeForwardLogged;
     using WQ = WarpQueue<BD, MODE>;
     using Shape = RecordShape<K>;
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ unsigned s_next;
-    // backward with a log: the marching fallback of a replay, for a log that is not complete
-    if (BWD && LogGate{lg.log, lg.capacity}.closed()) return;
     if (threadIdx.x == 0) s_next = 0;
     // sorted log: items this block has put into each bin, and its last groups of the bin
     constexpr bool SORTED = LOG && BLOCK > kMarchBlock;
@@ -327,53 +368,51 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         lg.log[2] = lg.shift;
         lg.log[3] = lg.n_bins;
     }
-    const int lane = threadIdx.x & 31;
-    WQ& q = *reinterpret_cast<WQ*>(s_raw + (size_t)(threadIdx.x >> 5) * sizeof(WQ));
+    // Kept in registers: left to itself the compiler works these three out again at every use.
+    int lane = threadIdx.x & 31;
+    uint32_t place = (uint32_t)__cvta_generic_to_shared(s_raw) + (threadIdx.x >> 5) * (uint32_t)sizeof(WQ);
+    unsigned below = (1u << lane) - 1u;
+    asm volatile("" : "+r"(lane), "+r"(place), "+r"(below));
+    WQ& q = *reinterpret_cast<WQ*>(__cvta_shared_to_generic(place));
+    const uint64_t pol_stream = l2_policy_stream();
     __syncthreads();
     const float d_rgb_pad = 1 + 2 * opt.rgb_padding;
-    const bool single = BWD && fwd_out != nullptr;
     const float bg = opt.background_brightness;
-    const int L = index.level;
-    const uint32_t side = (1u << L) - 1u;
-    const uint64_t pol_keep = l2_policy_keep(), pol_stream = l2_policy_stream();
-    const bool vec_ok = (reinterpret_cast<uintptr_t>(grad_data) & 15) == 0;
-    // Only an early stop needs the transmittance while marching (with a threshold of 0 a ray
-    // stops where it is exactly 0, after which nothing contributes); otherwise items are
-    // evaluated 32 at a time, where all lanes have one, and folded into the ray in order.
-    const bool early = !BWD && opt.stop_thresh > 0.f;
+    // Items are evaluated 32 at a time, where all lanes have one, and folded into the ray in order;
+    // there it is decided whether the ray stops early.  The march itself only has to notice in time:
+    // it ends a ray once its summed optical depth is beyond that of the threshold by more than
+    // the roundings of 2^16 factors can amount to, and items past the stop count for nothing.
+    float deep = __int_as_float(0x7f800000);
+    if (MODE == kModeForward && opt.stop_thresh > 0.f) {
+        deep = -logf(opt.stop_thresh);
+        deep += 0.0625f + fmaxf(deep, 0.f) * 0.015625f;
+    }
 
     // ---- per-lane state -------------------------------------------------------
-    Ray r;
-    r.hit = false;
+    Ray r{};        // (lanes without a ray look up entries too)
     int64_t ray = 0;
     int state = lane < shape.lanes ? kNeedRay : kExhausted;
-    // max(1 / direction, 0), where registers allow (1 % of an image's march; the logged kernels spill)
+    // max(1 / direction, 0), where registers allow (1 % of an image's march)
     constexpr bool MAXES = MODE == kModeForward;
     float mx = 0.f, my = 0.f, mz = 0.f;
-    float t = 0.f, light = 1.f, ahead = 1.f;   // transmittance after the items folded / pushed
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;  // forward: colour sums; backward: a0 = accum
+    float t = 0.f, light = 1.f;          // transmittance after the items folded
+    float depth = 0.f;                   // optical depth of the items pushed
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f;  // colour sums
     bool stopped = false;
-    int phase = 1;  // backward: 0 = accumulation march (reference PASS 1), 1 = scatter march
-    int it = 0;
     uint32_t cur_cell = 0xffffffffu;   // table cell of the brick used last ...
     uint32_t cur_brick = 0;            // ... and where the brick lies in the index
     // cursor: the position of the lane's next sample, and the index words requested for it
     float px = 0.f, py = 0.f, pz = 0.f;
     int2 entry = make_int2(0, 0);
     uint32_t cell = 0;                 // ... and its table cell
-    bool in_brick = false;             // ... from the brick `cur_brick`, else from the table
     // queue: ring of two batches; `qn` items collected from ring position `head` on
     int head = 0, qn = 0;
-    unsigned mine = 0u, mine_next = 0u, mine_fly = 0u;  // my items: first 32, spilled, in flight
-    int fly = 0;                       // items in flight; this lane's:
-    uint32_t fly_slot = 0u;
-    float fly_dt = 0.f, fly_sigma = 0.f;
-    int fly_own = 0;
+    // my items, the first in the highest bit: first 32, spilled, in flight
+    unsigned mine = 0u, mine_next = 0u, mine_fly = 0u;
+    int fly = 0;                       // items in flight, and this lane's
+    typename WQ::Item fly_item{0u, 0.f, 0.f, 0};
     // logged forward: groups the warp has taken from the log but not used, items written
     int log_group = 0, log_left = 0, log_items = 0;
-    const int log_limit = SORTED ? (int)(lg.capacity / kSortedChunks) : (int)lg.capacity;
-    int32_t* const log_counts = lg.log + kLogCounts;
-    int4* const packets = reinterpret_cast<int4*>(lg.log + log_packets_at(lg.capacity));
 
     // Places the cursor at parameter t and requests the index words there, to be consumed one
     // iteration later: the brick's, if the ray is still in the table cell whose brick it used
@@ -383,39 +422,33 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         py = fminf(__saturatef(mad_site<FC_POS>(t, r.dy, r.oy)), kPosMax);
         pz = fminf(__saturatef(mad_site<FC_POS>(t, r.dz, r.oz)), kPosMax);
     };
-    // 1 + floor(p * 2^23) / 2^23, exactly: the low 23 bits are the position's bits
-    auto bits = [](float p) { return __float_as_uint(__fadd_rz(p, 1.0f)); };
     auto request_words = [&]() {
-        const uint32_t ux = bits(px), uy = bits(py), uz = bits(pz);
-        if (BWD && index.table == nullptr) {       // fallback march: no index was built
-            entry = make_int2(kWordWalk, 0);
-            in_brick = false;
-            return;
-        }
-        cell = ((ux >> (kPosBits - 3 * L)) & (side << (2 * L))) |
-               ((uy >> (kPosBits - 2 * L)) & (side << L)) | ((uz >> (kPosBits - L)) & side);
-        in_brick = cell == cur_cell;
-        const int s3 = kPosBits - kBrickLevels - L;
-        const uint32_t c = ((ux >> (s3 - 6)) & 0x1c0u) | ((uy >> (s3 - 3)) & 0x38u) |
-                           ((uz >> s3) & 7u);
-        entry = ld_keep(index.table + (in_brick ? cur_brick + c : cell), pol_keep);
+        // the sums' low bits: the position in cells of a brick, exactly
+        const float2 xy = __fadd2_rz(make_float2(px, py), make_float2(index.fine, index.fine));
+        const uint32_t ux = __float_as_uint(xy.x), uy = __float_as_uint(xy.y),
+                       uz = __float_as_uint(__fadd_rz(pz, index.fine));
+        // places in bytes: an entry has 2^kBrickLevels of them
+        cell = ((ux & index.cell_mask) * index.row + (uy & index.cell_mask)) * index.row +
+               (uz & index.cell_mask);
+        const uint32_t c = ((ux & 7u) << 9) | ((uy & 7u) << 6) | ((uz & 7u) << 3);
+        const uint32_t at = cell == cur_cell ? cur_brick + c : cell;
+        entry = __ldg(reinterpret_cast<const int2*>(reinterpret_cast<const char*>(index.table) + at));
     };
 
     // Takes the first n (<= 32) collected items as the batch in flight and requests their
     // records: consecutive lanes copy consecutive 16-byte words, asynchronously.
     auto request = [&](int n) {
-        fly_slot = q.slot[head + lane];
-        fly_dt = q.dt[head + lane];
-        fly_sigma = q.sigma[head + lane];
-        fly_own = q.owner[head + lane];
-        const uint32_t slot = lane < n ? fly_slot : 0u;
+        fly_item = q.get(head + lane);
+        const uint32_t slot = fly_item.slot;
         mine_fly = mine;
         mine = mine_next;
         mine_next = 0u;
         fly = n;
         head ^= 32;
         qn = qn > 32 ? qn - 32 : 0;
-        const int sub = lane / Shape::GROUP, w = lane % Shape::GROUP;
+        int l = lane;
+        asm volatile("" : "+r"(l));
+        const int sub = l / Shape::GROUP, w = l % Shape::GROUP;
         const float* base = tr.data + 4 * w;
         float* row = q.rows + sub * Shape::STRIDE + 4 * w;
 #pragma unroll
@@ -439,67 +472,59 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         __syncwarp();
         const int nb = fly;
         const bool active = lane < nb;
-        const uint32_t b_slot = fly_slot;
-        const int b_own = fly_own;
+        const uint32_t b_slot = fly_item.slot;
         float* row = q.rows + lane * Shape::STRIDE;
         const int off = record_offset<K>(tr.data, b_slot);
-        const int own = b_own & 31;
-        const bool acc_item = BWD && (b_own & 0x80) != 0;
-        float sg[3] = {0.f, 0.f, 0.f}, col[3] = {0.f, 0.f, 0.f};
-        float raw_sigma = 0.f, att = 0.f, b_dd = 0.f;
-        if (active) {
-            const float delta_t = fly_dt, sigma = fly_sigma,
-                        delta_scale = q.rayv[own][WQ::SCALE];
-            b_dd = delta_t * delta_scale;
-            att = BWD ? expf(-delta_t * sigma * delta_scale)
-                      : expf(-delta_t * delta_scale * sigma);
+        const int own = fly_item.owner & 31;
+        // (a lane without an item computes along on what its row and place held before)
+        float sg[3], col[3], raw_sigma = 0.f;
+        const float att = expf(-fly_item.depth);
+        {
             float tmp[3] = {0.f, 0.f, 0.f};
+            const float* ray_basis = q.rayv[own];
             if (BD == 0) {
                 const float4 x = *reinterpret_cast<const float4*>(row);
                 tmp[0] = x.x; tmp[1] = x.y; tmp[2] = x.z;
                 raw_sigma = x.w;
-            } else {
-                float bs[BD > 0 ? BD : 1];
+            } else if (Shape::ALIGNED) {
+                constexpr int B = BD > 0 ? BD : 1;
+                float bs[B];
 #pragma unroll
-                for (int i = 0; i < BD; ++i)
-                    if (Shape::ALIGNED) bs[i] = q.rayv[own][i];
-                if (Shape::ALIGNED) {
+                for (int i = 0; i < B; ++i) bs[i] = ray_basis[i];
 #pragma unroll
-                    for (int w = 0; w < K / 4; ++w) {
-                        const float4 x = reinterpret_cast<const float4*>(row)[w];
-                        const float v[4] = {x.x, x.y, x.z, x.w};
+                for (int w = 0; w < K / 4; ++w) {
+                    const float4 x = reinterpret_cast<const float4*>(row)[w];
+                    const float v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int e = 4 * w + i;
-                            if (e < K - 1)
-                                tmp[e / (BD > 0 ? BD : 1)] = __fmaf_rn(
-                                    bs[e % (BD > 0 ? BD : 1)], v[i], tmp[e / (BD > 0 ? BD : 1)]);
-                            else raw_sigma = v[i];
-                        }
+                    for (int i = 0; i < 4; ++i) {
+                        const int e = 4 * w + i;
+                        if (e < K - 1) tmp[e / B] = __fmaf_rn(bs[e % B], v[i], tmp[e / B]);
+                        else raw_sigma = v[i];
                     }
-                } else {
-                    // The row's 16-byte words as they are: float j of the row is coefficient j - off,
-                    // so basis function (j - off) mod BD takes it, which is one register for all
-                    // three channels; only the first three of a channel's places depend on `off`.  (A
-                    // 49-float record as single floats met three bank conflicts a read: 1.03 ms per
-                    // 800x800 view instead of 1.01.)
-                    constexpr int B = BD > 0 ? BD : 1;
+                }
+            } else {
+                // The row's 16-byte words as they are: float j of the row is coefficient j - off,
+                // so basis function (j - off) mod BD takes it, which is one register for all
+                // three channels; only the first three of a channel's places depend on `off`.  (A
+                // 49-float record as single floats met three bank conflicts a read: 1.03 ms per
+                // 800x800 view instead of 1.01.)
+                constexpr int B = BD > 0 ? BD : 1;
+                float bs[B];
 #pragma unroll
-                    for (int m = 0; m < B; ++m)
-                        bs[m] = q.rayv[own][m >= 3 || m >= off ? m - off : m - off + B];
+                for (int m = 0; m < B; ++m)
+                    bs[m] = ray_basis[m >= 3 || m >= off ? m - off : m - off + B];
 #pragma unroll
-                    for (int w = 0; w < Shape::WORDS; ++w) {
-                        const float4 x = reinterpret_cast<const float4*>(row)[w];
-                        const float v[4] = {x.x, x.y, x.z, x.w};
+                for (int w = 0; w < Shape::WORDS; ++w) {
+                    const float4 x = reinterpret_cast<const float4*>(row)[w];
+                    const float v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int j = 4 * w + i, m = j % B, c = j / B;
-                            if (m >= 3 || m >= off) {
-                                if (c < 3) tmp[c < 3 ? c : 0] = __fmaf_rn(bs[m], v[i], tmp[c < 3 ? c : 0]);
-                                else if (m == off) raw_sigma = v[i];
-                            } else if (c > 0) {
-                                tmp[c > 0 ? c - 1 : 0] = __fmaf_rn(bs[m], v[i], tmp[c > 0 ? c - 1 : 0]);
-                            }
+                    for (int i = 0; i < 4; ++i) {
+                        const int j = 4 * w + i, m = j % B, c = j / B;
+                        if (m >= 3 || m >= off) {
+                            if (c < 3) tmp[c < 3 ? c : 0] = __fmaf_rn(bs[m], v[i], tmp[c < 3 ? c : 0]);
+                            else if (m == off) raw_sigma = v[i];
+                        } else if (c > 0) {
+                            tmp[c > 0 ? c - 1 : 0] = __fmaf_rn(bs[m], v[i], tmp[c > 0 ? c - 1 : 0]);
                         }
                     }
                 }
@@ -509,52 +534,40 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 sg[ch] = sigmoid_ref(tmp[ch]);
                 col[ch] = sg[ch] * d_rgb_pad - opt.rgb_padding;
             }
-            if (!BWD) {
-                *reinterpret_cast<float4*>(row) = make_float4(col[0], col[1], col[2], att);
-            } else {
-                float total_color = 0.f;
-#pragma unroll
-                for (int ch = 0; ch < 3; ++ch) total_color += col[ch] * q.rayv[own][BD + ch];
-                *reinterpret_cast<float4*>(row) =
-                    make_float4(total_color, att, acc_item ? 1.f : 0.f, b_dd);
-            }
+            *reinterpret_cast<float4*>(row) = make_float4(col[0], col[1], col[2], att);
         }
         __syncwarp();
         // every owner folds in its items, in march order
-        for (unsigned m = mine_fly; m != 0u; m &= m - 1u) {
-            float4* res = reinterpret_cast<float4*>(q.rows + (__ffs(m) - 1) * Shape::STRIDE);
+        for (unsigned m = mine_fly; m != 0u;) {
+            const int first = __clz(m);
+            m &= ~(0x80000000u >> first);
+            float4* res = reinterpret_cast<float4*>(q.rows + first * Shape::STRIDE);
             const float4 x = *res;
-            if (!BWD) {
-                // res->w: the transmittance before the item, 0 where the ray has stopped
-                const float before = stopped ? 0.f : light;
-                const float weight = before * (1.f - x.w);
-                if (!stopped) {
-                    a0 = __fmaf_rn(weight, x.x, a0);
-                    a1 = __fmaf_rn(weight, x.y, a1);
-                    a2 = __fmaf_rn(weight, x.z, a2);
-                    light = light * x.w;
-                    stopped = light <= opt.stop_thresh;
-                }
-                if (LOG) *res = make_float4(a0, a1, a2, before);
-                else if (tr.weight_accum != nullptr) res->w = before;
-            } else {
-                const float weight = light * (1.f - x.y);
-                light = light * x.y;
-                if (x.z != 0.f) {
-                    a0 += weight * x.x;
-                } else {
-                    a0 -= weight * x.x;
-                    res->x = x.w * (x.x * light - a0);    // density gradient
-                    res->y = weight;
-                }
+            // res->w: the transmittance before the item, 0 where the ray has stopped
+            const float before = stopped ? 0.f : light;
+            const float weight = before * (1.f - x.w);
+            if (!stopped) {
+                a0 = __fmaf_rn(weight, x.x, a0);
+                a1 = __fmaf_rn(weight, x.y, a1);
+                a2 = __fmaf_rn(weight, x.z, a2);
+                light = light * x.w;
+                stopped = light <= opt.stop_thresh;
             }
+            if (LOG) *res = make_float4(a0, a1, a2, before);
+            else res->w = before;
         }
         mine_fly = 0u;
         fly = 0;
         __syncwarp();
-        if (!BWD && tr.weight_accum != nullptr && active)
+        if (tr.weight_accum != nullptr && active)
             accumulate_weight(tr, b_slot, row[3] * (1.f - att));
         if (LOG) {
+            int32_t* log = lg.log;                   // (computed from here, not kept)
+            int64_t capacity = lg.capacity;
+            asm volatile("" : "+l"(log), "+l"(capacity));
+            const int log_limit = SORTED ? (int)(capacity / kSortedChunks) : (int)capacity;
+            int32_t* const log_counts = log + kLogCounts;
+            int4* const packets = reinterpret_cast<int4*>(log + log_packets_at(capacity));
             // lane i writes the packet of item i, now that its ray's colour sums are known: to
             // place i of the batch's chunk, or to the next place of its bin
             const int ray_id = __shfl_sync(0xffffffffu, (int)ray, own);
@@ -570,14 +583,14 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             const bool opens = SORTED ? active && place == 0 : lane == 0;
             const unsigned opening = __ballot_sync(0xffffffffu, opens);
             const int n_open = __popc(opening);
-            const int mine_open = __popc(opening & ((1u << lane) - 1u));
+            const int mine_open = __popc(opening & below);
             int group_id = log_group + mine_open;
             if (n_open > log_left) {
                 constexpr int GRAB = SORTED ? kSortedGrab : kLogGrab;
                 constexpr int UNIT = SORTED ? kSortedChunks : 1;
                 const int more = n_open - log_left > GRAB ? n_open - log_left : GRAB;
                 int c = 0;
-                if (lane == 0) c = atomicAdd(lg.log, more * UNIT) / UNIT;
+                if (lane == 0) c = atomicAdd(log, more * UNIT) / UNIT;
                 c = __shfl_sync(0xffffffffu, c, 0);
                 if (mine_open >= log_left) group_id = c + mine_open - log_left;
                 log_group = c + n_open - log_left;
@@ -602,7 +615,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                     }
                     group_id = open_group_id(v);
                     if (!open_group_is(v, number)) {    // never seen: give the log up, march instead
-                        lg.log[kLogGivenUp] = 1;
+                        log[kLogGivenUp] = 1;
                         group_id = 0x7fffffff;
                     }
                 }
@@ -615,15 +628,19 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 const float b_w = sums.w * (1.f - att), b_T = sums.w * att;
                 // the step length carries d softplus / d raw density, the one factor the
                 // density gradient needs from the raw value (svox/csrc/rt_kernel.cu:469-470)
+                float b_dd = fly_item.length;
                 if (opt.density_softplus) b_dd *= sigmoid_ref(raw_sigma - 1);
                 int qf[3];
 #pragma unroll
-                for (int ch = 0; ch < 3; ++ch)
-                    qf[ch] = __float_as_int((float)(b_w * sg[ch] * (1.0 - sg[ch])));
+                for (int ch = 0; ch < 3; ++ch) {
+                    // w sg (1 - sg), the product with 1 - sg rounded once
+                    const float part = b_w * sg[ch];
+                    qf[ch] = __float_as_int(__fmaf_rn(-part, sg[ch], part));
+                }
                 const float* vd = &q.rayv[own][BD];
                 int4* to = packets + ((int64_t)group_id * (SORTED ? kSortedItems : 32) + place) *
                                          (kPacketWords / 4);
-                const uint64_t pol = SORTED ? pol_keep : pol_stream;
+                const uint64_t pol = SORTED ? l2_policy_keep() : pol_stream;
                 st_hint16(to, make_int4((int)b_slot, ray_id, qf[0], qf[1]), pol);
                 st_hint16(to + 1, make_int4(qf[2], __float_as_int(__fmaf_rn(col[0], b_T, sums.x)),
                                             __float_as_int(__fmaf_rn(col[1], b_T, sums.y)),
@@ -634,93 +651,52 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             log_items += nb;
             __syncwarp();
         }
-        if (BWD) {
-            // lane i forms the gradient of record i in its staging row
-            const int goff = record_offset<K>(grad_data, b_slot);
-            if (active && !acc_item) {
-                const float gs = row[0], b_w = row[1];
-                float v[K];
-#pragma unroll
-                for (int ch = 0; ch < 3; ++ch) {
-                    const float tmp2 = b_w * sg[ch] * (1.0 - sg[ch]) * q.rayv[own][BD + ch] *
-                                       d_rgb_pad;
-                    if (BD == 0) v[ch] = tmp2;
-#pragma unroll
-                    for (int i = 0; i < BD; ++i) v[ch * BD + i] = q.rayv[own][i] * tmp2;
-                }
-                v[K - 1] = gs * (opt.density_softplus ? sigmoid_ref(raw_sigma - 1) : 1);
-                if (Shape::ALIGNED) {
-#pragma unroll
-                    for (int w = 0; w < K / 4; ++w)
-                        reinterpret_cast<float4*>(row)[w] =
-                            make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {       // the row's places around the record
-                        if (i < goff) row[i] = 0.f;
-                        if (goff + K + i < 4 * Shape::WORDS) row[goff + K + i] = 0.f;
-                    }
-#pragma unroll
-                    for (int w = 0; w < K; ++w) row[goff + w] = v[w];
-                }
-            }
-            __syncwarp();
-            const int sub = lane / Shape::GROUP, w = lane % Shape::GROUP;
-            const int meta = goff | (acc_item ? 8 : 0);
-#pragma unroll
-            for (int p = 0; p < Shape::GROUP; ++p) {
-                const int k = p * Shape::RPP + sub;
-                const uint32_t s = __shfl_sync(0xffffffffu, b_slot, k);
-                const int m = __shfl_sync(0xffffffffu, meta, k);
-                if (k < nb && w < Shape::WORDS && m < 8)
-                    flush_word<K>(grad_data + (size_t)s * K, m & 3, w,
-                                  reinterpret_cast<const float4*>(q.rows + k * Shape::STRIDE)[w],
-                                  vec_ok, pol_stream);
-            }
-            __syncwarp();
-        }
     };
 
-    unsigned alive = __ballot_sync(0xffffffffu, state != kExhausted);
+    // marching lanes at which the others are refilled: at none at the latest
+    auto refill_line = [&]() {
+        const int alive = __popc(__ballot_sync(0xffffffffu, state != kExhausted));
+        return alive > shape.refill ? alive - shape.refill : 0;
+    };
+    int refill_at = refill_line();
     for (;;) {
         // ---- lanes that are not marching: finish, refill, termination ---------------------
-        unsigned marching = __ballot_sync(0xffffffffu, state == kMarching);
-        const unsigned waiting = alive & ~marching;
-        if (marching == 0u || __popc(waiting) >= shape.refill) {
+        int marching_lanes = __popc(__ballot_sync(0xffffffffu, state >= kMarching));
+        if (marching_lanes <= refill_at) {
+            if (state == kCapped) {
+                report(SVOXB_ERR_MARCH);
+                state = kEnded;
+            }
             if (__any_sync(0xffffffffu, state == kEnded && (mine | mine_next | mine_fly) != 0u)) {
                 __syncwarp();
-                if (fly > 0) evaluate();
-                while (qn > 0) {
-                    request(qn < 32 ? qn : 32);
-                    evaluate();
+                while (fly > 0 || qn > 0) {
+                    if (fly > 0) evaluate();
+                    if (qn > 0) request(qn < 32 ? qn : 32);
                 }
             }
             if (state == kEnded) {
                 state = kNeedRay;
-                if (!BWD) {
-                    if (stopped) {
-                        const float scale = 1.0 / (1.0 - light);
-                        out[3 * ray + 0] = a0 * scale;
-                        out[3 * ray + 1] = a1 * scale;
-                        out[3 * ray + 2] = a2 * scale;
-                    } else {
-                        out[3 * ray + 0] = a0 + light * bg;
-                        out[3 * ray + 1] = a1 + light * bg;
-                        out[3 * ray + 2] = a2 + light * bg;
-                    }
-                } else if (phase == 0) {
-                    // tail of the reference's PASS 1 (rt_kernel.cu:415-418), then march again
-                    const float* g = &q.rayv[lane][BD];
-                    const float total_grad = g[0] + g[1] + g[2];
-                    a0 += light * bg * total_grad;
-                    phase = 1;
-                    t = r.tmin; light = 1.f; it = 0;
-                    state = kMarching;
-                    place_cursor();
-                    request_words();
+                if (stopped) {
+                    const float scale = 1.0 / (1.0 - light);
+                    out[3 * ray + 0] = a0 * scale;
+                    out[3 * ray + 1] = a1 * scale;
+                    out[3 * ray + 2] = a2 * scale;
+                } else {
+                    out[3 * ray + 0] = a0 + light * bg;
+                    out[3 * ray + 1] = a1 + light * bg;
+                    out[3 * ray + 2] = a2 + light * bg;
                 }
             }
             if (state == kNeedRay) {
+                // What a ray's set-up derives from the call's arguments is not to be kept in registers
+                // through the march.
+                Source rays = src;
+                TreeArgs tree = tr;
+                svoxb_render_options how = opt;
+                rays.pin();
+                asm volatile("" : "+l"(tree.offset), "+l"(tree.scaling), "+l"(tree.extra));
+                asm volatile("" : "+r"(how.ndc_width), "+r"(how.ndc_height), "+f"(how.ndc_focal),
+                                  "+r"(how.min_comp), "+r"(how.max_comp));
                 const unsigned ticket = atomicAdd(&s_next, 1u);
                 const int gs = shape.granule_shift;
                 const int64_t first =
@@ -728,153 +704,141 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 const int64_t place = first + (ticket & ((1u << gs) - 1u));
                 if (first >= tickets) {
                     state = kExhausted;
-                } else if (place < tickets && (ray = src.pick(place)) >= 0) {
-                    src.load(ray, tr, opt, r);
-                    ray_setup(r, tr.scaling);
+                } else if (place < tickets && (ray = rays.pick(place)) >= 0) {
+                    rays.load(ray, tree, how, r);
+                    ray_setup(r, tree.scaling);
                     if (!r.hit || !(r.tmin < r.tmax)) {
-                        if (!BWD) { out[3 * ray + 0] = bg; out[3 * ray + 1] = bg; out[3 * ray + 2] = bg; }
+                        out[3 * ray + 0] = bg; out[3 * ray + 1] = bg; out[3 * ray + 2] = bg;
                     } else {
                         march_ready(r);
-                        state = kMarching;
-                        t = r.tmin; light = ahead = 1.f; it = 0; stopped = false;
+                        state = kMaxSteps;
+                        t = r.tmin; light = 1.f; depth = 0.f; stopped = false;
                         mx = fmaxf(r.ix, 0.f); my = fmaxf(r.iy, 0.f); mz = fmaxf(r.iz, 0.f);
-                        q.rayv[lane][WQ::SCALE] = r.delta_scale;
                         place_cursor();
                         request_words();
                         if (BD > 0) {
                             float basis[BD > 0 ? BD : 1];
-                            colour_basis<(BD > 0 ? BD : 1), Source::kLobes>(tr, opt, r.vdir, basis);
+                            colour_basis<(BD > 0 ? BD : 1), Source::kLobes>(tree, how, r.vdir, basis);
 #pragma unroll
                             for (int i = 0; i < BD; ++i)
                                 q.rayv[lane][i] =
-                                    (i < opt.min_comp || i > opt.max_comp) ? 0.f : basis[i];
+                                    (i < how.min_comp || i > how.max_comp) ? 0.f : basis[i];
                         }
                         if (LOG) {
 #pragma unroll
                             for (int i = 0; i < 3; ++i) q.rayv[lane][BD + i] = r.vdir[i];
                         }
                         a0 = a1 = a2 = 0.f;
-                        if (BWD) {
-                            const float g0 = __ldg(grad_out + 3 * ray), g1 = __ldg(grad_out + 3 * ray + 1),
-                                        g2 = __ldg(grad_out + 3 * ray + 2);
-                            float* g = &q.rayv[lane][BD];
-                            g[0] = g0; g[1] = g1; g[2] = g2;
-                            phase = single ? 1 : 0;
-                            if (single) {
-                                a0 = __ldg(fwd_out + 3 * ray) * g0;
-                                a0 += __ldg(fwd_out + 3 * ray + 1) * g1;
-                                a0 += __ldg(fwd_out + 3 * ray + 2) * g2;
-                            }
-                        }
                     }
                 }
             }
             __syncwarp();
-            marching = __ballot_sync(0xffffffffu, state == kMarching);
-            alive = __ballot_sync(0xffffffffu, state != kExhausted);
-            if (marching == 0u) {
-                if (alive == 0u) break;
+            refill_at = refill_line();
+            if (!__any_sync(0xffffffffu, state >= kMarching)) {
+                if (!__any_sync(0xffffffffu, state != kExhausted)) break;
                 continue;
             }
         }
 
         // ---- G step: every lane consumes the words requested one iteration ago --------------
         // (without branches but for the rare cases: lanes that have nothing to do compute along)
-        bool on = state == kMarching;
-        if (on && !in_brick && entry.x < 0) {
+        const bool to_brick = entry.x < 0;
+        if (to_brick) {
             // the table cell has a brick: the sample is looked up there
             cur_cell = cell;
-            cur_brick = index.bricks + (uint32_t)(entry.x & 0x7fffffff) * kBrickCells;
-            on = false;
+            cur_brick = (index.bricks + (uint32_t)entry.x * kBrickCells) * 8;    // (drops the sign)
         }
+        const bool on = state >= kMarching && !to_brick;
         uint32_t slot = (uint32_t)entry.y & 0x0fffffffu;
         float sigma = __int_as_float(entry.x);
         bool item = on && entry.x <= kWordInf;      // the leaf passes the density test
         bool done = false;
         // side of the leaf's cube, 2^-depth
         float inv_cube = __int_as_float((127 << 23) - (int)((uint32_t)entry.y >> 28 << 23));
-        float fine = 0.f;
-        if (on && entry.x >= kWordFetch) {
-            // seldom: a tree deeper than the index, a density that is not in the word
-            float raw = 0.f;
-            if (entry.x == kWordWalk) {
-                const float big = (float)(1 << 24);
-                const int depth = (int)((uint32_t)entry.y >> 28);
-                const Walked f = walk_to_leaf(
-                    tr.child, tr.data, K, tr.M, depth > L ? (int64_t)slot : 0,
-                    depth > L ? depth - 1 : 0, (int)(px * big), (int)(py * big), (int)(pz * big));
-                done = !f.ok;
-                slot = f.slot;
-                inv_cube = __int_as_float((127 - (f.ok ? f.depth : 1)) << 23);
-                raw = f.raw;
-                // 2^-24 leaves: a float resolves them below 1/2, where the sum below would not
-                if (f.ok && f.depth > kPosBits) fine = 1.f;
-            } else {
-                raw = __ldg(tr.data + (size_t)slot * K + (K - 1));
-            }
-            sigma = opt.density_softplus ? softplus_m1(raw) : raw;
-            item = !done && sigma > (BWD ? 0.f : opt.sigma_thresh);
-        }
         // Lower corner of the leaf: a number whose last place is the leaf's side takes in the
         // position's multiples of it and drops the rest.
-        const float coarse = __int_as_float(__float_as_int(inv_cube) + (kPosBits << 23));
-        float cx = __fsub_rn(__fadd_rz(px, coarse), coarse);
-        float cy = __fsub_rn(__fadd_rz(py, coarse), coarse);
+        float coarse = __int_as_float(__float_as_int(inv_cube) + (kPosBits << 23));
+        const float2 pxy = make_float2(px, py), coarse2 = make_float2(coarse, coarse);
+        float2 cxy = sub2(__fadd2_rz(pxy, coarse2), coarse2);
         float cz = __fsub_rn(__fadd_rz(pz, coarse), coarse);
-        if (fine != 0.f) {
-            const float big = (float)(1 << 24);
-            cx = truncf(px * big) * (1.f / big);
-            cy = truncf(py * big) * (1.f / big);
-            cz = truncf(pz * big) * (1.f / big);
+        const bool rare = on && entry.x >= kWordFetch;
+        if (__any_sync(0xffffffffu, rare)) {
+            // seldom: a tree deeper than the index, a density that is not in the word
+            if (rare) {
+                float raw = 0.f;
+                if (entry.x == kWordWalk) {
+                    const float big = (float)(1 << 24);
+                    const int level = (int)((uint32_t)entry.y >> 28);
+                    const int ix = (int)(px * big), iy = (int)(py * big), iz = (int)(pz * big);
+                    const Walked f = walk_to_leaf(tr.child, tr.data, K, tr.M,
+                                                  level > index.level ? (int64_t)slot : 0,
+                                                  level > index.level ? level - 1 : 0, ix, iy, iz);
+                    done = !f.ok;
+                    slot = f.slot;
+                    inv_cube = __int_as_float((127 - (f.ok ? f.depth : 1)) << 23);
+                    raw = f.raw;
+                    coarse = __int_as_float(__float_as_int(inv_cube) + (kPosBits << 23));
+                    cxy.x = __fsub_rn(__fadd_rz(px, coarse), coarse);
+                    cxy.y = __fsub_rn(__fadd_rz(py, coarse), coarse);
+                    cz = __fsub_rn(__fadd_rz(pz, coarse), coarse);
+                    // 2^-24 leaves: a float resolves them below 1/2, where the sums would not
+                    if (f.ok && f.depth > kPosBits) {
+                        cxy.x = (float)ix * (1.f / big);
+                        cxy.y = (float)iy * (1.f / big);
+                        cz = (float)iz * (1.f / big);
+                    }
+                } else {
+                    raw = __ldg(tr.data + (size_t)slot * K + (K - 1));
+                }
+                sigma = opt.density_softplus ? softplus_m1(raw) : raw;
+                item = !done && sigma > opt.sigma_thresh;
+            }
         }
         // Exit distance of the leaf (_dda_unit, svox/csrc/rt_kernel.cu:203-220, in the leaf's own
         // scale).  The point lies inside, so the entry distance is 0 and per axis the larger of
         // t1 = -f*inv and t1 + inv is t1 + max(inv, 0); powers of two commute with rounding, so
         // everything can be done at the tree's scale.
-        const float ex = __fmaf_rn(MAXES ? mx : fmaxf(r.ix, 0.f), inv_cube,
-                                   __fmul_rn(__fsub_rn(cx, px), r.ix));
-        const float ey = __fmaf_rn(MAXES ? my : fmaxf(r.iy, 0.f), inv_cube,
-                                   __fmul_rn(__fsub_rn(cy, py), r.iy));
+        const float2 exy = __ffma2_rn(MAXES ? make_float2(mx, my)
+                                            : make_float2(fmaxf(r.ix, 0.f), fmaxf(r.iy, 0.f)),
+                                      make_float2(inv_cube, inv_cube),
+                                      __fmul2_rn(sub2(cxy, pxy), make_float2(r.ix, r.iy)));
         const float ez = __fmaf_rn(MAXES ? mz : fmaxf(r.iz, 0.f), inv_cube,
                                    __fmul_rn(__fsub_rn(cz, pz), r.iz));
-        const float delta_t = __fadd_rn(fminf(ex, fminf(ey, ez)), opt.step_size);
+        const float delta_t = __fadd_rn(fminf(exy.x, fminf(exy.y, ez)), opt.step_size);
+        const float length = __fmul_rn(delta_t, r.delta_scale);
+        const float thick = __fmul_rn(length, sigma);
         if (on) {
             t = __fadd_rn(t, delta_t);
-            if (!(t < r.tmax)) done = true;
-            if (early && item) {
-                ahead *= expf(-delta_t * r.delta_scale * sigma);
-                if (ahead <= opt.stop_thresh) done = true;
-            }
-            if (++it > kMaxSteps) {
-                report(SVOXB_ERR_MARCH);
-                done = true;
-            }
-            if (done) state = kEnded;
+            --state;
+            if (MODE == kModeForward && item) depth += thick;
+            if (done || !(t < r.tmax) || (MODE == kModeForward && item && depth > deep))
+                state = kEnded;
         }
         place_cursor();
-        if (state == kMarching) request_words();
+        request_words();
 
         // ---- push items --------------------------------------------------------------
         const unsigned pushed = __ballot_sync(0xffffffffu, item);
-        if (item) {
-            const int n = qn + __popc(pushed & ((1u << lane) - 1u));
-            const int pos = (head + n) & (WQ::CAP - 1);
-            q.slot[pos] = slot;
-            q.dt[pos] = delta_t;
-            q.sigma[pos] = sigma;
-            q.owner[pos] = (unsigned char)(lane | ((BWD && phase == 0) ? 0x80 : 0));
-            const unsigned bit = 1u << (n & 31);
-            if (n < 32) mine |= bit;
-            else mine_next |= bit;
-        }
-        qn += __popc(pushed);
-        if (qn >= 32) {
-            __syncwarp();
-            if (fly > 0) evaluate();
-            request(32);
+        if (pushed != 0u) {
+            const int n = qn + __popc(pushed & below);
+            if (item) {
+                q.put((head + n) & (WQ::CAP - 1),
+                      typename WQ::Item{slot, thick, length, lane});
+                const unsigned bit = 0x80000000u >> (n & 31);
+                if (n < 32) mine |= bit;
+                else mine_next |= bit;
+            }
+            qn += __popc(pushed);
+            if (qn >= 32) {
+                __syncwarp();
+                if (fly > 0) evaluate();
+                request(32);
+            }
         }
     }
     if (LOG) {
+        const int log_limit = SORTED ? (int)(lg.capacity / kSortedChunks) : (int)lg.capacity;
+        int32_t* const log_counts = lg.log + kLogCounts;
         // groups taken but not used hold no items; the last group of a bin holds what it got
         for (int i = lane; i < log_left; i += 32)
             if (log_group + i < log_limit) log_counts[log_group + i] = 0;

@@ -6,6 +6,7 @@
 #include "query.cuh"
 #include "render.cuh"
 #include "render_queue.cuh"
+#include "render_back.cuh"
 #include "render_replay.cuh"
 #include "collective.cuh"
 #include <initializer_list>
@@ -200,23 +201,34 @@ static int launch_march(const RenderCall& c, const Source& src, const TreeIndex&
     int st = persistent_grid(k, BLOCK, queues + (SORTED ? kBinSmem : 0), granules * (BLOCK / 32), &grid);
     if (st) return st;
     const size_t smem = queues + (SORTED ? bin_smem(log.n_bins) : 0);
-    const bool single = MODE == kModeBackward && c.fwd_out != nullptr && c.opt.sigma_thresh == 0.f &&
-                        c.opt.stop_thresh == 0.f;
-    k<<<grid, BLOCK, smem, c.stream>>>(tree_args(c.tree), src, c.opt, index, tickets, c.out,
-                                       c.grad_out, single ? c.fwd_out : nullptr, c.grad_data, log,
+    k<<<grid, BLOCK, smem, c.stream>>>(tree_args(c.tree), src, c.opt, index, tickets, c.out, log,
                                        shape);
     SVOXB_CUDA(cudaGetLastError());
     return SVOXB_OK;
 }
 
 template <int BD, class Source>
+static int launch_back(const RenderCall& c, const Source& src, const TreeIndex& index) {
+    constexpr size_t queues = (kMarchBlock / 32) * sizeof(BackQueue<BD>);
+    const int64_t tickets = Source::tickets(src, c.Q);
+    const MarchShape shape = march_shape(tickets, (int64_t)sm_count() * kSpreadWarps);
+    auto k = render_back_kernel<BD, Source>;
+    unsigned grid = 1;
+    const int64_t granules = (tickets + (1 << shape.granule_shift) - 1) >> shape.granule_shift;
+    const int st = persistent_grid(k, kMarchBlock, queues, granules * (kMarchBlock / 32), &grid);
+    if (st) return st;
+    const bool single = c.fwd_out != nullptr && c.opt.sigma_thresh == 0.f && c.opt.stop_thresh == 0.f;
+    k<<<grid, kMarchBlock, queues, c.stream>>>(tree_args(c.tree), src, c.opt, index, tickets,
+                                               c.grad_out, single ? c.fwd_out : nullptr, c.grad_data,
+                                               c.gate, shape);
+    SVOXB_CUDA(cudaGetLastError());
+    return SVOXB_OK;
+}
+
+template <int BD, class Source>
 static int launch_mode(const RenderCall& c, const Source& src, const TreeIndex& index) {
+    if (c.backward) return launch_back<BD>(c, src, index);
     LogArgs log;
-    if (c.backward) {
-        log.log = const_cast<int32_t*>(c.gate.log);
-        log.capacity = c.gate.capacity;
-        return launch_march<BD, kModeBackward, kMarchBlock>(c, src, index, log);
-    }
     const bool few = Source::tickets(src, c.Q) <= (int64_t)sm_count() * kSpreadWarps * 32;
     if (c.log == nullptr)
         return few ? launch_march<BD, kModeForward, kFewBlock>(c, src, index, log)
@@ -421,7 +433,7 @@ static int launch_queue(const RenderCall& c, const Source& src) {
         mem = scratch.mem;
     }
     TreeIndex index = layout.view(mem);
-    if (mem == nullptr) index = TreeIndex{nullptr, 0, 1};
+    if (mem == nullptr) index = TreeIndex::at(nullptr, 0, 1);
     ClearBeside clear{c};
     if ((st = clear.index_built())) return st;
     st = with_basis(c.opt, [&](auto basis) {

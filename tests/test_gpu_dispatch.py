@@ -65,6 +65,28 @@ def test_few_rays_and_many_give_the_same(fmt, cuda_device):
     csrc.check_device_status()
 
 
+@pytest.mark.parametrize("thresh", [1e-40, 1e-30, 1e-2, 0.5, 0.97, 1.0, 3.0, float("inf")])
+@pytest.mark.parametrize("fmt", ["RGBA", "SH9"])
+def test_early_stop_against_the_kernel_that_multiplies_as_it_goes(fmt, thresh, cuda_device):
+    # The march ends a ray by its summed optical depth, the evaluation by the product of its
+    # attenuations; records at odd addresses take the one-thread-per-ray kernel, which stops by the
+    # same product.  Many rays cross empty space first, where nothing may stop them.
+    tree = _shell(fmt, 3, 3, cuda_device)
+    tree.data.data[..., -1] *= 8.0
+    tree.data.requires_grad_(False)
+    rays = _rays(5003, cuda_device)
+    r = svox.VolumeRenderer(tree)
+    r.stop_thresh = thresh
+    out = r(rays)
+    odd = torch.empty(tree.data.numel() + 1, device=cuda_device)[1:].view(tree.data.shape)
+    odd.copy_(tree.data)
+    tree.data.data = odd
+    want = r(rays)
+    # (rounding of the colours' sums: the stop itself is the same bits)
+    assert (out - want).abs().max().item() <= 1e-5
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("fmt,refine,n_rays", [("RGBA", 5, 50000), ("SH9", 4, 12000),
                                                ("SH16", 4, 12000)])
 @pytest.mark.parametrize("image", [False, True])
