@@ -126,7 +126,8 @@ struct LogArgs {
 };
 
 // The index (tens of MB, re-read hundreds of times per launch) must stay in L2 while the leaf
-// records and gradients (GBs, touched a few times each) stream through it.
+// records and gradients (GBs, touched a few times each) stream through it.  (Without the hint 300 rays
+// with gradient take 354 us instead of 302, 4096 467 instead of 459; calls that fill the device level.)
 __device__ __forceinline__ int2 ld_keep(const int2* a, uint64_t pol) {
     int2 v;
     asm volatile("ld.global.nc.L2::cache_hint.v2.s32 {%0, %1}, [%2], %3;"
@@ -374,7 +375,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     unsigned below = (1u << lane) - 1u;
     asm volatile("" : "+r"(lane), "+r"(place), "+r"(below));
     WQ& q = *reinterpret_cast<WQ*>(__cvta_shared_to_generic(place));
-    const uint64_t pol_stream = l2_policy_stream();
+    const uint64_t pol_stream = l2_policy_stream(), pol_keep = l2_policy_keep();
     __syncthreads();
     const float d_rgb_pad = 1 + 2 * opt.rgb_padding;
     const float bg = opt.background_brightness;
@@ -432,7 +433,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                (uz & index.cell_mask);
         const uint32_t c = ((ux & 7u) << 9) | ((uy & 7u) << 6) | ((uz & 7u) << 3);
         const uint32_t at = cell == cur_cell ? cur_brick + c : cell;
-        entry = __ldg(reinterpret_cast<const int2*>(reinterpret_cast<const char*>(index.table) + at));
+        entry = ld_keep(reinterpret_cast<const int2*>(reinterpret_cast<const char*>(index.table) + at), pol_keep);
     };
 
     // Takes the first n (<= 32) collected items as the batch in flight and requests their
@@ -807,7 +808,19 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         const float delta_t = __fadd_rn(fminf(exy.x, fminf(exy.y, ez)), opt.step_size);
         const float length = __fmul_rn(delta_t, r.delta_scale);
         const float thick = __fmul_rn(length, sigma);
-        if (on) {
+        // The same twice: branches here cost long records registers and time, their absence short
+        // ones instructions (800x800 view, us, with / without: SH4 772 / 794, SH9 with thresholds 674 /
+        // 669, SH16 1054 / 1041, SH25 1328 / 1221; 65536 RGBA rays with gradient 213 / 216).
+        if constexpr (BD >= 9) {
+            const float next_t = __fadd_rn(t, delta_t);
+            bool end = done | !(next_t < r.tmax);
+            if (MODE == kModeForward) {
+                depth += item ? thick : 0.f;
+                end |= item & (depth > deep);
+            }
+            t = on ? next_t : t;
+            state = on ? (end ? kEnded : state - 1) : state;
+        } else if (on) {
             t = __fadd_rn(t, delta_t);
             --state;
             if (MODE == kModeForward && item) depth += thick;
@@ -815,7 +828,9 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 state = kEnded;
         }
         place_cursor();
-        request_words();
+        // (lanes without a ray load along, which saves a branch: 1 to 2 % of a view; not beside the 28 KB
+        // of L1 that 25 functions leave: 100 000 such rays 778 us, 721 without)
+        if (BD != 25 || state >= kMarching) request_words();
 
         // ---- push items --------------------------------------------------------------
         const unsigned pushed = __ballot_sync(0xffffffffu, item);
