@@ -56,14 +56,14 @@ METRICS = {
     "image5": "Mrays/s render_persp forward (SH deg 3, three shells at 1024^3, 1920x1080 views)",
 }
 # DRAM bytes (read + write) of one launch of the training step's kernels: the logged march from an
-# ncu capture of a 2^17-ray launch (1.661 GB read + 0.383 GB written), scaled by 8 because its
+# ncu capture of a 2^17-ray launch (1.658 GB read + 0.382 GB written), scaled by 8 because its
 # traffic grows with the rays; the scatter's does not (the gradient is written once whatever the
 # number of rays), so no scaled figure is given for it.  Printed only together with
 # `traffic_source`, which names the capture.
-NCU_TRAFFIC = {"forward": 8 * (1.661109e9 + 0.382764e9), "backward": None}
+NCU_TRAFFIC = {"forward": 8 * (1.657777e9 + 0.381872e9), "backward": None}
 NCU_TRAFFIC_SOURCE = ("ncu of render_queue_kernel<9,2,768> at 2^17 rays x 8 "
                       "(profiles/training_step_rays131072_ncu_full.md); valid for the kernel as "
-                      "of library version " + "0.4.3")
+                      "of library version " + "0.4.4")
 
 
 def parse():

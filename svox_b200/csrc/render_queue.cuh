@@ -18,7 +18,7 @@
 // Bound: issue slots where neighbouring rays share records (images: 60 % of the slots used), DRAM
 // too where every sample's record misses (rays in random order: 16 GB for 2^20 rays of the 512^3
 // shell scene).  So the march is kept short: an 800x800 view of the shell scene with SH16 records takes
-// 0.500 G warp instructions for 2.28 M iterations and 0.49 M batches of items.  The leaf's corner
+// 0.512 G warp instructions for 2.28 M iterations and 0.49 M batches of items.  The leaf's corner
 // comes from truncating additions, its exit distance from five operations per axis, two axes to
 // an instruction; lanes between samples compute along instead of branching; the index entry of a
 // sample is requested one iteration ahead so that the queue's work covers its latency; and a block holds
@@ -33,9 +33,9 @@
 //  - nothing of a ray's set-up or of the log's layout kept in registers through the march (the
 //    compiler moved it out of the loop, then spilled: the logged SH9 march 16 % slower), and the
 //    lane, the queue's place and the policy not worked out again.
-// us before and after, whole call: 800x800 view, SH16 1145 and 1052, SH4 858 and 765, SH9 with
-// thresholds 761 and 671; 65536 RGBA rays with gradient 234 and 213; 2^20 SH9 rays with gradient
-// 5743 and 5583 (bound by memory); four 1080p views of the 1024^3 scene 20.4 and 19.0 ms.  (Dot
+// us before and after, whole call: 800x800 view, SH16 1135 and 1040, SH4 858 and 758, SH9 with
+// thresholds 760 and 671; 65536 RGBA rays with gradient 233 and 216; 2^20 SH9 rays with gradient
+// 5712 and 5560 (bound by memory); four 1080p views of the 1024^3 scene 20.2 and 18.8 ms.  (Dot
 // products with two coefficients per instruction: level for SH9 to SH25, 9 % slower for RGBA.)
 //
 // Lanes whose ray has ended wait until `refill` of them do; then the queue is drained, their
