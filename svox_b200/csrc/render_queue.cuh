@@ -560,7 +560,8 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         mine_fly = 0u;
         fly = 0;
         __syncwarp();
-        if (tr.weight_accum != nullptr && active)
+        // (nothing of an item that its ray did not reach, whatever its density)
+        if (tr.weight_accum != nullptr && active && row[3] != 0.f)
             accumulate_weight(tr, b_slot, row[3] * (1.f - att));
         if (LOG) {
             int32_t* log = lg.log;                   // (computed from here, not kept)

@@ -87,6 +87,34 @@ def test_early_stop_against_the_kernel_that_multiplies_as_it_goes(fmt, thresh, c
     csrc.check_device_status()
 
 
+@pytest.mark.parametrize("op", ["sum", "max"])
+def test_weights_of_rays_that_stop_early(op, cuda_device):
+    # samples that the march still took behind a ray's stop leave no weight
+    tree = _shell("RGBA", 3, 3, cuda_device)
+    tree.data.data[..., -1] *= 8.0
+    tree.data.requires_grad_(False)
+    rays = _rays(5003, cuda_device)
+    r = svox.VolumeRenderer(tree)
+    r.stop_thresh = 0.3
+
+    def weights():
+        with tree.accumulate_weights(op=op) as accum:
+            r(rays)
+        return accum()
+
+    out = weights()
+    odd = torch.empty(tree.data.numel() + 1, device=cuda_device)[1:].view(tree.data.shape)
+    odd.copy_(tree.data)
+    tree.data.data = odd                 # (the one-thread-per-ray kernel)
+    want = weights()
+    # a largest weight is the same product; sums of up to some hundred weights in another order
+    if op == "max":
+        assert torch.equal(out, want)
+    else:
+        assert _close(out, want)
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("fmt,refine,n_rays", [("RGBA", 5, 50000), ("SH9", 4, 12000),
                                                ("SH16", 4, 12000)])
 @pytest.mark.parametrize("image", [False, True])
