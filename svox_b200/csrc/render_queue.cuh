@@ -258,7 +258,8 @@ mark_cells_kernel(TreeArgs tr, Source src, svoxb_render_options opt, int64_t tic
     }
 }
 
-// State of a lane: the samples its ray may still take (marching), or one of these.
+// State of a lane: the samples its ray may still take (marching), or one of these.  (A ray that met a
+// damaged node ends like any other, its tmax no number.)
 enum { kMarching = 1, kCapped = 0, kNeedRay = -1, kEnded = -2, kExhausted = -3 };
 
 constexpr int kMarchBlock = 128;
@@ -380,11 +381,13 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     const float d_rgb_pad = 1 + 2 * opt.rgb_padding;
     const float bg = opt.background_brightness;
     // Items are evaluated 32 at a time, where all lanes have one, and folded into the ray in order;
-    // there it is decided whether the ray stops early.  The march itself only has to notice in time:
-    // it ends a ray once its summed optical depth is beyond that of the threshold by more than
-    // the roundings of 2^16 factors can amount to, and items past the stop count for nothing.
+    // there it is decided whether the ray stops early, and the march is told.  Before that it ends a
+    // ray once its summed optical depth is beyond that of the threshold by more than the
+    // roundings of 2^16 factors can amount to.  What it takes behind the stop counts for nothing,
+    // a damaged node there and the sample cap too.
+    const bool early = MODE == kModeForward && opt.stop_thresh > 0.f;
     float deep = __int_as_float(0x7f800000);
-    if (MODE == kModeForward && opt.stop_thresh > 0.f) {
+    if (early) {
         deep = -logf(opt.stop_thresh);
         deep += 0.0625f + fmaxf(deep, 0.f) * 0.015625f;
     }
@@ -559,6 +562,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         }
         mine_fly = 0u;
         fly = 0;
+        if (early && stopped && state >= kMarching) state = kEnded;
         __syncwarp();
         // (nothing of an item that its ray did not reach, whatever its density)
         if (tr.weight_accum != nullptr && active && row[3] != 0.f)
@@ -665,18 +669,17 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         // ---- lanes that are not marching: finish, refill, termination ---------------------
         int marching_lanes = __popc(__ballot_sync(0xffffffffu, state >= kMarching));
         if (marching_lanes <= refill_at) {
-            if (state == kCapped) {
-                report(SVOXB_ERR_MARCH);
-                state = kEnded;
-            }
-            if (__any_sync(0xffffffffu, state == kEnded && (mine | mine_next | mine_fly) != 0u)) {
+            if (__any_sync(0xffffffffu, state < kMarching && (mine | mine_next | mine_fly) != 0u)) {
                 __syncwarp();
                 while (fly > 0 || qn > 0) {
                     if (fly > 0) evaluate();
                     if (qn > 0) request(qn < 32 ? qn : 32);
                 }
             }
-            if (state == kEnded) {
+            if (state == kEnded || state == kCapped) {
+                const int fault = state == kCapped ? SVOXB_ERR_MARCH
+                                  : r.tmax != r.tmax ? SVOXB_ERR_TREE : 0;
+                if (fault != 0 && !(early && stopped)) report(fault);
                 state = kNeedRay;
                 if (stopped) {
                     const float scale = 1.0 / (1.0 - light);
@@ -754,7 +757,6 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         uint32_t slot = (uint32_t)entry.y & 0x0fffffffu;
         float sigma = __int_as_float(entry.x);
         bool item = on && entry.x <= kWordInf;      // the leaf passes the density test
-        bool done = false;
         // side of the leaf's cube, 2^-depth
         float inv_cube = __int_as_float((127 << 23) - (int)((uint32_t)entry.y >> 28 << 23));
         // Lower corner of the leaf: a number whose last place is the leaf's side takes in the
@@ -775,7 +777,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                     const Walked f = walk_to_leaf(tr.child, tr.data, K, tr.M,
                                                   level > index.level ? (int64_t)slot : 0,
                                                   level > index.level ? level - 1 : 0, ix, iy, iz);
-                    done = !f.ok;
+                    if (!f.ok) r.tmax = __int_as_float(0x7fffffff);     // ends the ray
                     slot = f.slot;
                     inv_cube = __int_as_float((127 - (f.ok ? f.depth : 1)) << 23);
                     raw = f.raw;
@@ -793,7 +795,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                     raw = __ldg(tr.data + (size_t)slot * K + (K - 1));
                 }
                 sigma = opt.density_softplus ? softplus_m1(raw) : raw;
-                item = !done && sigma > opt.sigma_thresh;
+                item = r.tmax == r.tmax && sigma > opt.sigma_thresh;
             }
         }
         // Exit distance of the leaf (_dda_unit, svox/csrc/rt_kernel.cu:203-220, in the leaf's own
@@ -814,7 +816,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
         // 669, SH16 1054 / 1041, SH25 1328 / 1221; 65536 RGBA rays with gradient 213 / 216).
         if constexpr (BD >= 9) {
             const float next_t = __fadd_rn(t, delta_t);
-            bool end = done | !(next_t < r.tmax);
+            bool end = !(next_t < r.tmax);
             if (MODE == kModeForward) {
                 depth += item ? thick : 0.f;
                 end |= item & (depth > deep);
@@ -825,7 +827,7 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
             t = __fadd_rn(t, delta_t);
             --state;
             if (MODE == kModeForward && item) depth += thick;
-            if (done || !(t < r.tmax) || (MODE == kModeForward && item && depth > deep))
+            if (!(t < r.tmax) || (MODE == kModeForward && item && depth > deep))
                 state = kEnded;
         }
         place_cursor();

@@ -115,6 +115,45 @@ def test_weights_of_rays_that_stop_early(op, cuda_device):
     csrc.check_device_status()
 
 
+def _eight_leaves(fmt, sigma, dev):
+    """A tree of one node; density of the half x > 1/2."""
+    tree = svox.N3Tree(N=2, data_format=fmt, init_refine=0, device=dev)
+    tree.data.data.fill_(0.3)
+    tree.data.data[..., -1] = 0.0
+    tree.data.data[0, 1, :, :, -1] = sigma
+    return tree
+
+
+def _along_x(n, sign, dev, seed=3):
+    """Parallel rays along the axis x through both halves of the unit cube."""
+    yz = torch.rand(n, 2, generator=torch.Generator().manual_seed(seed)) * 0.4 + 0.05
+    origins = torch.cat((torch.full((n, 1), 0.5 - 2.0 * sign), yz), 1).to(dev)
+    dirs = torch.tensor([[float(sign), 0.0, 0.0]]).expand(n, 3).contiguous().to(dev)
+    return svox.Rays(origins, dirs, dirs.clone())
+
+
+@pytest.mark.parametrize("what,code", [("damaged", 6), ("stuck", 7)])
+@pytest.mark.parametrize("fmt", ["RGBA", "SH9", "SH25"])
+def test_nothing_behind_an_early_stop_is_reported(fmt, what, code, cuda_device):
+    # The first half has an optical depth of 0.72: exp(-0.72) = 0.487.  Behind it lies a node that
+    # does not exist, or (step size 0) the rays do not get off its far side, which has an extent
+    # of 0 in their direction.
+    tree = _eight_leaves(fmt, 1.44, cuda_device)
+    tree.data.requires_grad_(False)
+    if what == "damaged":
+        tree.child[0, 0, 0, 0] = 1_000_000
+    r = svox.VolumeRenderer(tree, step_size=1e-3 if what == "damaged" else 0.0)
+    rays = _along_x(37, -1, cuda_device)
+    r.stop_thresh = 0.5
+    out = r(rays)
+    assert csrc.device_status(clear=True) == 0
+    if fmt == "RGBA":                       # the colour of what was met, whatever its weight
+        assert (out - torch.sigmoid(torch.tensor(0.3))).abs().max().item() < 1e-5
+    r.stop_thresh = 0.48                    # not reached
+    r(rays)
+    assert csrc.device_status(clear=True) == code
+
+
 @pytest.mark.parametrize("fmt,refine,n_rays", [("RGBA", 5, 50000), ("SH9", 4, 12000),
                                                ("SH16", 4, 12000)])
 @pytest.mark.parametrize("image", [False, True])
