@@ -48,6 +48,7 @@
 #include "render_index.cuh"
 #include "binned.cuh"
 #include "open_groups.h"
+#include <cfloat>
 
 namespace svoxb {
 
@@ -383,11 +384,13 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     // Items are evaluated 32 at a time, where all lanes have one, and folded into the ray in order;
     // there it is decided whether the ray stops early, and the march is told.  Before that it ends a
     // ray once its summed optical depth is beyond that of the threshold by more than the
-    // roundings of 2^16 factors can amount to.  What it takes behind the stop counts for nothing,
-    // a damaged node there and the sample cap too.
+    // roundings of 2^16 factors can amount to (only where no density is negative, which would make the
+    // two part further, and where the product does not run into denormal numbers before the
+    // threshold).  What it takes behind the stop counts for nothing, a damaged node there and the sample
+    // cap too.
     const bool early = MODE == kModeForward && opt.stop_thresh > 0.f;
     float deep = __int_as_float(0x7f800000);
-    if (early) {
+    if (early && opt.sigma_thresh >= 0.f && opt.stop_thresh >= FLT_MIN) {
         deep = -logf(opt.stop_thresh);
         deep += 0.0625f + fmaxf(deep, 0.f) * 0.015625f;
     }

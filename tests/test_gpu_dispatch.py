@@ -154,6 +154,42 @@ def test_nothing_behind_an_early_stop_is_reported(fmt, what, code, cuda_device):
     assert csrc.device_status(clear=True) == code
 
 
+def _at_odd_addresses(tree):
+    """The tree's records where only the one-thread-per-ray kernels take them."""
+    odd = torch.empty(tree.data.numel() + 1, device=tree.data.device)[1:].view(tree.data.shape)
+    odd.copy_(tree.data)
+    tree.data.data = odd
+
+
+def _largest_weights(tree, renderer, rays):
+    with torch.no_grad(), tree.accumulate_weights(op="max") as accum:
+        renderer(rays)
+    return accum()
+
+
+def test_early_stop_among_negative_densities(cuda_device):
+    # Four leaves in a row, of depth -89, 45, 46 and 1.  The transmittance overflows in the first and is
+    # infinite from there on, so the ray never stops, although the depths' sum passes the
+    # threshold in the third.
+    tree = svox.N3Tree(N=2, data_format="RGBA", init_refine=1, device=cuda_device)
+    tree.data.requires_grad_(False)
+    x = torch.tensor([0.875, 0.625, 0.375, 0.125], device=cuda_device)
+    depth = torch.tensor([-89.0, 45.0, 46.0, 1.0], device=cuda_device)
+    points = torch.cartesian_prod(x, x, x)
+    _, ids = tree(points, want_node_ids=True)
+    tree.data.data.view(-1, 4)[ids, -1] = depth.repeat_interleave(16) / 0.251
+    r = svox.VolumeRenderer(tree)
+    r.sigma_thresh, r.stop_thresh = -1e9, 0.5
+    rays = _along_x(37, -1, cuda_device)
+    out = _largest_weights(tree, r, rays)
+    _at_odd_addresses(tree)
+    want = _largest_weights(tree, r, rays)
+    last = ids[points[:, 0] == 0.125]
+    assert torch.isinf(want.view(-1)[last]).any()
+    assert torch.equal(out, want)
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("fmt,refine,n_rays", [("RGBA", 5, 50000), ("SH9", 4, 12000),
                                                ("SH16", 4, 12000)])
 @pytest.mark.parametrize("image", [False, True])
