@@ -387,10 +387,11 @@ render_back_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex 
             if (entry.x == kWordWalk) {
                 const float big = (float)(1 << 24);
                 const int depth = (int)((uint32_t)entry.y >> 28);
-                const Walked f = walk_to_leaf<true>(
+                const Walked f = walk_to_leaf(
                     tr.child, tr.data, K, tr.M, depth > L ? (int64_t)slot : 0,
                     depth > L ? depth - 1 : 0, (int)(px * big), (int)(py * big), (int)(pz * big));
                 done = !f.ok;
+                if (done) report(SVOXB_ERR_TREE);
                 slot = f.slot;
                 inv_cube = __int_as_float((127 - (f.ok ? f.depth : 1)) << 23);
                 raw = f.raw;

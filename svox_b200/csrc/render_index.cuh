@@ -268,10 +268,7 @@ struct Walked {
 };
 
 // Walks `child` from `node` at level `lvl` (root: 0) to the leaf that holds the position given
-// by its coordinates floor(x * 2^24).  `ok` false: the tree is damaged there, reported here or left to the
-// caller.  (Reported by the marching backward itself, its registers fell out worse: a view with SH16
-// records 2.55 ms instead of 2.20, 65 536 RGBA rays 166 us instead of 150.)
-template <bool REPORT>
+// by its coordinates floor(x * 2^24).  `ok` false: the tree is damaged there, for the caller to report.
 __device__ __noinline__ Walked walk_to_leaf(const int32_t* __restrict__ child,
                                             const float* __restrict__ data, int K, int64_t M,
                                             int64_t node, int lvl, int ix, int iy, int iz) {
@@ -284,7 +281,6 @@ __device__ __noinline__ Walked walk_to_leaf(const int32_t* __restrict__ child,
         node += e;
         if (node < 0 || node >= M) break;
     }
-    if (REPORT) report(SVOXB_ERR_TREE);
     return {false, 0u, 0, 0.f};
 }
 

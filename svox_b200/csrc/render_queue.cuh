@@ -777,9 +777,9 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                     const float big = (float)(1 << 24);
                     const int level = (int)((uint32_t)entry.y >> 28);
                     const int ix = (int)(px * big), iy = (int)(py * big), iz = (int)(pz * big);
-                    const Walked f = walk_to_leaf<false>(
-                        tr.child, tr.data, K, tr.M, level > index.level ? (int64_t)slot : 0,
-                        level > index.level ? level - 1 : 0, ix, iy, iz);
+                    const Walked f = walk_to_leaf(tr.child, tr.data, K, tr.M,
+                                                  level > index.level ? (int64_t)slot : 0,
+                                                  level > index.level ? level - 1 : 0, ix, iy, iz);
                     if (!f.ok) r.tmax = __int_as_float(0x7fffffff);     // ends the ray
                     slot = f.slot;
                     inv_cube = __int_as_float((127 - (f.ok ? f.depth : 1)) << 23);
