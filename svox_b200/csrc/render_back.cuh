@@ -63,8 +63,7 @@ render_back_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex 
     const bool vec_ok = (reinterpret_cast<uintptr_t>(grad_data) & 15) == 0;
 
     // ---- per-lane state -------------------------------------------------------
-    Ray r;
-    r.hit = false;
+    Ray r{};        // (lanes without a ray compute along)
     int64_t ray = 0;
     int state = lane < shape.lanes ? kNeedRay : kExhausted;
     float t = 0.f, light = 1.f;   // transmittance after the items folded

@@ -230,6 +230,28 @@ def test_sorted_log_unsorted_log_and_march_agree(fmt, refine, n_rays, image, cud
     csrc.check_device_status()
 
 
+@pytest.mark.parametrize("two", [False, True])
+@pytest.mark.parametrize("n", [1, 37, 4097])
+@pytest.mark.parametrize("fmt", ["RGBA", "SH9", "SH16"])
+def test_marching_backward_with_lanes_that_have_no_ray(fmt, n, two, cuda_device):
+    # warps with fewer rays than lanes, and rays that miss the cube among them: those lanes compute along
+    tree = _shell(fmt, 3, 2, cuda_device)
+    r = svox.VolumeRenderer(tree)
+    origins, dirs, views = _rays(n, cuda_device)
+    origins[1::5] += 40.0
+    rays = svox.Rays(origins, dirs, views)
+    up = torch.randn(n, 3, generator=torch.Generator().manual_seed(2)).to(cuda_device)
+    a = _grad(r, lambda: r(rays), up)
+    _render.USE_ITEM_LOG, _render.FORCE_TWO_MARCHES = False, two
+    try:
+        b = _grad(r, lambda: r(rays), up)
+    finally:
+        _render.USE_ITEM_LOG, _render.FORCE_TWO_MARCHES = True, False
+    assert b.abs().max().item() > 0
+    assert _close(b, a)
+    csrc.check_device_status()
+
+
 @pytest.mark.parametrize("fmt", ["RGBA", "SH4"])
 @pytest.mark.parametrize("n", [50, 30000])
 def test_se_grad_through_either_log_and_without(fmt, n, cuda_device):
