@@ -82,7 +82,8 @@ def test_early_stop_against_the_kernel_that_multiplies_as_it_goes(fmt, thresh, c
     odd.copy_(tree.data)
     tree.data.data = odd
     want = r(rays)
-    # (rounding of the colours' sums: the stop itself is the same bits)
+    # (rounding of the colours' sums: the stop itself is the same bits.  What the small thresholds leave
+    # changes no colour: test_early_stop_leaf_by_leaf tells where those stop.)
     assert (out - want).abs().max().item() <= 1e-5
     csrc.check_device_status()
 
@@ -188,6 +189,47 @@ def test_early_stop_among_negative_densities(cuda_device):
     assert torch.isinf(want.view(-1)[last]).any()
     assert torch.equal(out, want)
     csrc.check_device_status()
+
+
+@pytest.mark.parametrize("thresh", [1e-40, 1e-30, 1e-2, 0.5])
+@pytest.mark.parametrize("fmt", ["RGBA", "SH9"])
+def test_early_stop_leaf_by_leaf(fmt, thresh, cuda_device):
+    # 32 leaves of depth 3 to 5 in every row, each met by rays that have come through the same
+    # ones: the leaves with a weight are the leaves before the stop, however small the threshold
+    tree = svox.N3Tree(N=2, data_format=fmt, init_refine=4, device=cuda_device)
+    tree.data.requires_grad_(False)
+    gen = torch.Generator().manual_seed(4)
+    sigma = (3.0 + 2.0 * torch.rand(tree.data.shape[:-1], generator=gen)) / (1 / 32 + 1e-3)
+    tree.data.data[..., -1] = sigma.to(cuda_device)
+    r = svox.VolumeRenderer(tree)
+    rays = _along_x(2000, -1, cuda_device)
+    every = _largest_weights(tree, r, rays)
+    r.stop_thresh = thresh
+    out = _largest_weights(tree, r, rays)
+    _at_odd_addresses(tree)
+    want = _largest_weights(tree, r, rays)
+    assert (want > 0).sum() < (every > 0).sum()
+    assert torch.equal(out, want)           # the same products
+    csrc.check_device_status()
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("fmt", ["RGBA", "SH9", "SH25"])
+def test_sample_cap(fmt, grad, cuda_device):
+    # With a step size of 0 rays towards -x do not get off the plane x = 1/2 (see above), those towards
+    # +x do.  The former end at the cap with a status; the others are what they are alone.
+    tree = _eight_leaves(fmt, 1.44, cuda_device)
+    tree.data.requires_grad_(grad)
+    r = svox.VolumeRenderer(tree, step_size=0.0)
+    good = _along_x(75, 1, cuda_device)
+    want = r(good)
+    assert csrc.device_status(clear=True) == 0
+    bad = _along_x(5, -1, cuda_device)
+    mixed = svox.Rays(*[torch.cat((a[:40], b, a[40:])) for a, b in zip(good, bad)])
+    out = r(mixed)
+    assert csrc.device_status(clear=True) == 7
+    assert torch.equal(torch.cat((out[:40], out[45:])), want)
+    assert torch.isfinite(out).all()
 
 
 @pytest.mark.parametrize("fmt,refine,n_rays", [("RGBA", 5, 50000), ("SH9", 4, 12000),
