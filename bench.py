@@ -60,10 +60,10 @@ METRICS = {
 # traffic grows with the rays; the scatter's does not (the gradient is written once whatever the
 # number of rays), so no scaled figure is given for it.  Printed only together with
 # `traffic_source`, which names the capture.
-NCU_TRAFFIC = {"forward": 8 * (1.657777e9 + 0.381872e9), "backward": None}
+NCU_TRAFFIC = {"forward": 8 * (1.658330e9 + 0.382424e9), "backward": None}
 NCU_TRAFFIC_SOURCE = ("ncu of render_queue_kernel<9,2,768> at 2^17 rays x 8 "
                       "(profiles/training_step_rays131072_ncu_full.md); valid for the kernel as "
-                      "of library version " + "0.4.4")
+                      "of library version " + "0.4.5")
 
 
 def parse():

@@ -31,7 +31,7 @@ typedef enum {
     SVOXB_ERR_NULL = 1,        /* a required pointer is null                 */
     SVOXB_ERR_SHAPE = 2,       /* a size is negative / inconsistent          */
     SVOXB_ERR_FORMAT = 3,      /* data format not supported by this build    */
-    SVOXB_ERR_OPTION = 4,      /* invalid render option (e.g. step_size <= 0)*/
+    SVOXB_ERR_OPTION = 4,      /* invalid render option (e.g. step_size < 0) */
     SVOXB_ERR_CUDA = 5,        /* a CUDA runtime call failed                 */
     SVOXB_ERR_TREE = 6,        /* device status: descent left the node array */
     SVOXB_ERR_MARCH = 7,       /* device status: a ray hit the step cap      */
@@ -390,7 +390,8 @@ int svoxb_march_stats(const svoxb_tree* tree, const svoxb_rays* rays,
 /* Device-side anomaly report.  The kernels bound every loop (the
  * reference's descent and march are unbounded, svox/csrc/include/
  * common.cuh:67-88, rt_kernel.cu:261) and record SVOXB_ERR_TREE /
- * SVOXB_ERR_MARCH in a per-device status word instead of hanging.  This
+ * SVOXB_ERR_MARCH in a per-device status word instead of hanging.  A ray
+ * that stop_thresh has ended reports nothing from behind its stop.  This
  * call synchronises `stream`, returns the word of the current device and
  * optionally clears it. */
 int svoxb_device_status(int clear, void* stream);

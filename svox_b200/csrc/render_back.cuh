@@ -4,8 +4,9 @@
 // step lane i forms the gradient of record i in its staging row and the warp flushes the rows with
 // red.global.add.v4.f32, 16 bytes per lane.
 //
-// The march is the forward's as it was before that was shortened further: in this kernel the shorter form
-// raised an illegal instruction, whose cause reading did not show.
+// The march is the forward's as it was before that was shortened further.  A trial of the shorter form in
+// here ended in an illegal instruction, in a test that launches the plain forward and then this
+// kernel; which of the two raised it was not established, and no cause was found by reading.
 #pragma once
 
 #include "render_queue.cuh"

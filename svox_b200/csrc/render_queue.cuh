@@ -15,17 +15,18 @@
 //           its ray's transmittance and sums in march order, which keeps the reference's order of accumulation
 //           (svox/csrc/rt_kernel.cu:282-295) whatever the batches are.
 //
-// Bound: issue slots where neighbouring rays share records (images: 60 % of the slots used), DRAM
+// Bound: issue slots where neighbouring rays share records (images: 61 % of the slots used), DRAM
 // too where every sample's record misses (rays in random order: 16 GB for 2^20 rays of the 512^3
 // shell scene).  So the march is kept short: an 800x800 view of the shell scene with SH16 records takes
-// 0.512 G warp instructions for 2.28 M iterations and 0.49 M batches of items.  The leaf's corner
+// 0.504 G warp instructions: 2.28 M iterations of 94, 0.49 M batches of items at 390 (325 with 9 logged
+// functions), the rest pushes and refills.  The leaf's corner
 // comes from truncating additions, its exit distance from five operations per axis, two axes to
 // an instruction; lanes between samples compute along instead of branching; the index entry of a
 // sample is requested one iteration ahead so that the queue's work covers its latency; and a block holds
 // four warps so that shared memory and the L1 can be balanced (kMarchBlocks).
 //
-// What the march's instructions were, and what became of them (0.583 G before; a tenth of them were
-// branches and their reconvergence, another tenth constants and addresses worked out again):
+// What the march's instructions were, and what became of them (0.583 G before; 15 % of them were
+// branches and their reconvergence, 9 % constants and addresses worked out again):
 //  - the early stop summed as optical depth, where it was an exponential and a branch per sample;
 //  - one word for a lane's state and the samples it has left; seldom cases behind one vote;
 //  - items in one or two stores; the product of length and density formed by the march's lanes;
@@ -33,10 +34,10 @@
 //  - nothing of a ray's set-up or of the log's layout kept in registers through the march (the
 //    compiler moved it out of the loop, then spilled: the logged SH9 march 16 % slower), and the
 //    lane, the queue's place and the policy not worked out again.
-// us before and after, whole call: 800x800 view, SH16 1135 and 1040, SH4 858 and 758, SH9 with
-// thresholds 760 and 671; 65536 RGBA rays with gradient 233 and 216; 2^20 SH9 rays with gradient
-// 5712 and 5560 (bound by memory); four 1080p views of the 1024^3 scene 20.2 and 18.8 ms.  (Dot
-// products with two coefficients per instruction: level for SH9 to SH25, 9 % slower for RGBA.)
+// us before and after, whole call: 800x800 view, SH16 1133 and 1044, SH4 859 and 762, SH9 with
+// thresholds 757 and 660; 65536 RGBA rays with gradient 233 and 218; 2^20 SH9 rays with gradient
+// 5640 and 5566 (bound by memory); four 1080p views of the 1024^3 scene 20.2 and 18.6 ms.  (Dot
+// products with two coefficients per instruction: level for SH9 to SH25.)
 //
 // Lanes whose ray has ended wait until `refill` of them do; then the queue is drained, their
 // results are written and they take new rays from a block-wide ticket counter together (the
@@ -373,10 +374,10 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
     }
     // Kept in registers: left to itself the compiler works these three out again at every use.
     int lane = threadIdx.x & 31;
-    uint32_t place = (uint32_t)__cvta_generic_to_shared(s_raw) + (threadIdx.x >> 5) * (uint32_t)sizeof(WQ);
+    uint32_t queue = (uint32_t)__cvta_generic_to_shared(s_raw) + (threadIdx.x >> 5) * (uint32_t)sizeof(WQ);
     unsigned below = (1u << lane) - 1u;
-    asm volatile("" : "+r"(lane), "+r"(place), "+r"(below));
-    WQ& q = *reinterpret_cast<WQ*>(__cvta_shared_to_generic(place));
+    asm volatile("" : "+r"(lane), "+r"(queue), "+r"(below));
+    WQ& q = *reinterpret_cast<WQ*>(__cvta_shared_to_generic(queue));
     const uint64_t pol_stream = l2_policy_stream(), pol_keep = l2_policy_keep();
     __syncthreads();
     const float d_rgb_pad = 1 + 2 * opt.rgb_padding;
@@ -709,10 +710,10 @@ render_queue_kernel(TreeArgs tr, Source src, svoxb_render_options opt, TreeIndex
                 const int gs = shape.granule_shift;
                 const int64_t first =
                     ((int64_t)blockIdx.x + (int64_t)gridDim.x * (ticket >> gs)) << gs;
-                const int64_t place = first + (ticket & ((1u << gs) - 1u));
+                const int64_t turn = first + (ticket & ((1u << gs) - 1u));
                 if (first >= tickets) {
                     state = kExhausted;
-                } else if (place < tickets && (ray = rays.pick(place)) >= 0) {
+                } else if (turn < tickets && (ray = rays.pick(turn)) >= 0) {
                     rays.load(ray, tree, how, r);
                     ray_setup(r, tree.scaling);
                     if (!r.hit || !(r.tmin < r.tmax)) {

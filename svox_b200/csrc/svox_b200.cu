@@ -1198,7 +1198,7 @@ int svoxb_allreduce_multimem(float* multicast, int64_t n_floats, int rank, int w
     return SVOXB_OK;
 }
 
-const char* svoxb_version(void) { return "0.4.4"; }
+const char* svoxb_version(void) { return "0.4.5"; }
 
 // Test hook (include/svox_b200_testing.h): key 5 = MB of gradient one replay bin spans,
 // key 7 = bricks below the render leaf table on / off.
